@@ -20,8 +20,8 @@
 // the x coupling of level l is cx/4^l, rows unchanged), one damped z-line
 // Jacobi sweep (omega = 2/3) before and after the coarse correction, each
 // column's tridiagonal z operator solved exactly by a partitioned solver,
-// full-weighting restriction, linear interpolation, and an exact solve of the
-// one-column coarsest level. With the same damped sweep before and after and
+// full-weighting restriction, linear interpolation, and an exact Fourier-mode
+// solve of the coarsest level (spectral_kernels.cuh). With the same damped sweep before and after and
 // P = 2 R^T the V-cycle is a symmetric positive definite preconditioner.
 #pragma once
 
@@ -247,27 +247,6 @@ __global__ void __launch_bounds__(32 * kMaxSeg) k_line_sweep(SweepArgs<P> a) {
     line_sweep<P, LS>(a.L, a.z, blockIdx.x * 32, a.f, a.xin, a.xc, a.pitch_c, a.nc, a.out, a.omega, shY);
 }
 
-template <typename P>
-struct RestrictArgs {
-    int nxl, pitch, NK;   // fine level
-    ZOps z;
-    const double* cx;
-    const P *f, *x;
-    P* fc;                // coarse rhs, [NK][pitch_c]
-    int pitch_c;
-};
-
-// fc[j] = 1/4 r[2j-1] + 1/2 r[2j] + 1/4 r[2j+1], r = f - S x (periodic).
-template <typename P>
-__device__ __forceinline__ void restrict_point(const RestrictArgs<P>& a, int j, int kk) {
-    const int i0 = 2 * j, im = (i0 == 0) ? a.nxl - 1 : i0 - 1, ip = i0 + 1;
-    const size_t row = (size_t)kk * a.pitch;
-    P r0 = a.f[row + i0] - s_apply(a.x, a.pitch, a.nxl, a.NK, a.z, a.cx, kk, i0);
-    P rm = a.f[row + im] - s_apply(a.x, a.pitch, a.nxl, a.NK, a.z, a.cx, kk, im);
-    P rp = a.f[row + ip] - s_apply(a.x, a.pitch, a.nxl, a.NK, a.z, a.cx, kk, ip);
-    a.fc[(size_t)kk * a.pitch_c + j] = P(0.25) * rm + P(0.5) * r0 + P(0.25) * rp;
-}
-
 // Pre-smoothing from a zero iterate fused with the restriction of the new
 // residual: x = omega * Dline^{-1} f (no neighbour values needed), then
 // r = f - S x and fc = full weighting of r. A block's 32 lanes cover fine
@@ -346,178 +325,6 @@ __global__ void __launch_bounds__(32 * kMaxSeg) k_presmooth_restrict(LineLevel L
             if (j < len && owned && (lane & 1) == 0)
                 fc[(size_t)(a + j) * pitch_c + (col >> 1)] = P(0.25) * rm + P(0.5) * r + P(0.25) * rp;
         }
-    }
-}
-
-// Exact solve on a level of nc <= 32 columns. The operator is separable (x
-// coefficients depend on the row only, periodic in x), so a real orthonormal
-// Fourier basis Q (nc x nc) diagonalises its x part: mode m needs the
-// tridiagonal z solve of (cx mu_m + ru + rd, -ru, -rd), mu_m the eigenvalue
-// of the periodic [-1 2 -1]. One block: f and Q are staged in shared memory,
-// each (mode lane, segment warp) transforms its rows and runs the partitioned
-// solve with that mode's precomputed factors (warp 0 solving every mode's
-// reduced system), and the inverse transform writes x.
-struct ModeSolve {
-    int nc, pitch, NK, S;
-    const double* Q;                  // [nc][nc], Q[col*nc + m]
-    const double *lo, *inv, *cp, *gL, *gR;   // [NK][nc]: mode fastest (coalesced)
-    const double* band;               // [5][2S][nc]
-};
-
-// Segment Thomas pass of one mode (factors interleaved by mode, stride nc).
-template <typename P, int LS>
-__device__ __forceinline__ void seg_thomas_modes(const ModeSolve& M, int m, int a, int len, P (&r)[LS]) {
-    const int nc = M.nc;
-    P prev = P(0);
-#pragma unroll
-    for (int j = 0; j < LS; j++) {
-        if (j < len) {
-            const size_t e = (size_t)(a + j) * nc + m;
-            prev = (r[j] - P(M.lo[e]) * prev) * P(M.inv[e]);
-            r[j] = prev;
-        }
-    }
-    P next = P(0);
-#pragma unroll
-    for (int j = LS - 1; j >= 0; j--) {
-        if (j < len) {
-            next = r[j] - P(M.cp[(size_t)(a + j) * nc + m]) * next;
-            r[j] = next;
-        }
-    }
-}
-
-template <typename P, int LS>
-__global__ void __launch_bounds__(32 * kMaxSeg) k_coarse_modes(ModeSolve M, const P* f, P* x) {
-    extern __shared__ unsigned char smem_raw[];
-    P* fs = reinterpret_cast<P*>(smem_raw);             // [NK][nc]: f, later the mode solution
-    P* xh = fs;                                         // (f is dead after the first barrier)
-    P* bs = fs + (size_t)M.NK * M.nc;                   // [5][2S][nc] band
-    __shared__ P shY[2 * kMaxSeg * 32];
-    __shared__ P Qs[32 * 32];    // Q[col][m]: forward transform, lanes = m
-    __shared__ P QT[32 * 32];    // Q[col][m] at [m][col]: inverse, lanes = col
-    const int nc = M.nc, NK = M.NK, S = M.S;
-    for (int t = threadIdx.x; t < NK * nc; t += blockDim.x) {
-        int kk = t / nc, c = t % nc;
-        fs[t] = f[(size_t)kk * M.pitch + c];
-    }
-    stage_band(M.band, 10 * S * nc, bs);
-    for (int t = threadIdx.x; t < nc * nc; t += blockDim.x) {
-        Qs[t] = P(M.Q[t]);
-        QT[(t % nc) * nc + t / nc] = P(M.Q[t]);
-    }
-    __syncthreads();
-    const int lane = threadIdx.x & 31, s = threadIdx.x >> 5;
-    const bool act = (s < S) && (lane < nc);
-    const int a = (s < S) ? (s * NK) / S : 0, b = (s < S) ? ((s + 1) * NK) / S : 0, len = b - a;
-    const int m = lane;
-    P y[LS];
-    if (act) {
-#pragma unroll
-        for (int j = 0; j < LS; j++) {
-            P v = P(0);
-            if (j < len) {
-                const P* row = fs + (size_t)(a + j) * nc;
-#pragma unroll 8
-                for (int c = 0; c < nc; c++) v += Qs[c * nc + m] * row[c];
-            }
-            y[j] = v;
-        }
-        seg_thomas_modes<P, LS>(M, m, a, len, y);
-        P ylast = y[0];
-#pragma unroll
-        for (int j = 0; j < LS; j++)
-            if (j == len - 1) ylast = y[j];
-        shY[(2 * s) * 32 + lane] = y[0];
-        shY[(2 * s + 1) * 32 + lane] = ylast;
-    }
-    P XL, XR;
-    segment_couplings(bs + m, nc, S, shY, lane, s, lane < nc, XL, XR);
-    if (act) {
-#pragma unroll
-        for (int j = 0; j < LS; j++) {
-            if (j < len) {
-                const int kk = a + j;
-                xh[(size_t)kk * nc + m] = y[j] - P(M.gL[(size_t)kk * nc + m]) * XL - P(M.gR[(size_t)kk * nc + m]) * XR;
-            }
-        }
-    }
-    __syncthreads();
-    if (act) {   // lane = output column
-        const int cc = lane;
-        for (int j = 0; j < len; j++) {
-            const int kk = a + j;
-            const P* row = xh + (size_t)kk * nc;
-            P v = P(0);
-#pragma unroll 8
-            for (int q = 0; q < nc; q++) v += QT[q * nc + cc] * row[q];
-            x[(size_t)kk * M.pitch + cc] = v;
-        }
-    }
-}
-
-// The coarse end of the V-cycle in one block, with block barriers between
-// phases. Levels wider than 32 columns are swept strip by strip. When NX is a
-// power of two the last level has one column, its operator has no x part,
-// and one exact line solve (omega = 1) finishes it; otherwise the last level
-// has an odd column count and gets coarse_sweeps damped sweeps from zero.
-constexpr int kMaxCoarseLevels = 8;
-
-template <typename P>
-struct CoarseCycleArgs {
-    int nlev;                          // levels handled by the block (>= 1)
-    LineLevel L[kMaxCoarseLevels];
-    ZOps z;
-    const P* f0;                       // rhs of its first level
-    P* f[kMaxCoarseLevels];            // rhs of the following levels
-    P* x[kMaxCoarseLevels];            // pre-smoothed iterates; coarsest solution
-    P* y[kMaxCoarseLevels];            // post-smoothed results (y[0] = output)
-    P omega;
-    int coarse_sweeps;                 // 1 = exact solve of a single column
-};
-
-template <typename P, int LS>
-__device__ __forceinline__ void sweep_all(const LineLevel& L, const ZOps& z, const P* f, const P* xin,
-                                          const P* xc, int pitch_c, int nc, P* out, P omega, P* shY) {
-    for (int c0 = 0; c0 < L.nxl; c0 += 32) line_sweep<P, LS>(L, z, c0, f, xin, xc, pitch_c, nc, out, omega, shY);
-}
-
-template <typename P, int LS>
-__global__ void __launch_bounds__(32 * kMaxSeg) k_mg_coarse_cycle(CoarseCycleArgs<P> a) {
-    __shared__ P shY[kShY + kShBand];
-    const int n = a.nlev;
-    for (int l = 0; l < n - 1; l++) {
-        const P* fl = (l == 0) ? a.f0 : a.f[l];
-        sweep_all<P, LS>(a.L[l], a.z, fl, nullptr, nullptr, 0, 0, a.x[l], a.omega, shY);
-        RestrictArgs<P> ra{a.L[l].nxl, a.L[l].pitch, a.L[l].NK, a.z, a.L[l].cx, fl, a.x[l], a.f[l + 1],
-                           a.L[l + 1].pitch};
-        const int nc = a.L[l].nxl >> 1, tot = nc * a.L[l].NK;
-        for (int t = threadIdx.x; t < tot; t += blockDim.x) restrict_point(ra, t % nc, t / nc);
-        __syncthreads();
-    }
-    {
-        const int c = n - 1;
-        const P* fl = (n == 1) ? a.f0 : a.f[c];
-        P* target = (n == 1) ? a.y[0] : a.x[c];
-        P* other = (n == 1) ? a.x[0] : a.y[c];
-        const int K = a.coarse_sweeps;
-        if (K <= 1) {
-            sweep_all<P, LS>(a.L[c], a.z, fl, nullptr, nullptr, 0, 0, target, P(1), shY);
-        } else {
-            P* dst = (K & 1) ? target : other;
-            const P* cur = nullptr;
-            for (int it = 0; it < K; it++) {
-                sweep_all<P, LS>(a.L[c], a.z, fl, cur, nullptr, 0, 0, dst, a.omega, shY);
-                cur = dst;
-                dst = (dst == target) ? other : target;
-            }
-        }
-    }
-    for (int l = n - 2; l >= 0; l--) {
-        const P* fl = (l == 0) ? a.f0 : a.f[l];
-        const P* coarse = (l + 1 == n - 1) ? a.x[n - 1] : a.y[l + 1];
-        sweep_all<P, LS>(a.L[l], a.z, fl, a.x[l], coarse, a.L[l + 1].pitch, a.L[l + 1].nxl, a.y[l], a.omega,
-                         shY);
     }
 }
 

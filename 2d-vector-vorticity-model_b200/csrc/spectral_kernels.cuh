@@ -1,4 +1,4 @@
-// Exact preconditioner of the cal_w operator by Fourier modes in x.
+// Exact solve of the cal_w operator by Fourier modes in x.
 //
 // The operator (PoissonSolver::InitPoissonMatrix, src/PoissonSolver.cpp:760-796,
 // in the symmetric form S of poisson_kernels.cuh) has coefficients that depend
@@ -340,5 +340,162 @@ __device__ __forceinline__ void k_spec_inverse_body(const SpecArgs<P>& a, P* out
 }
 template <typename P>
 __global__ void k_spec_inverse(SpecArgs<P> a, P* out) { k_spec_inverse_body<P>(a, out); }
+
+// ---------------------------------------------------------------------------
+// Row transforms of any length nc by the transform's own sums, for the levels
+// a multigrid cycle solves exactly (their column counts keep the odd factor of
+// NX, where no power-of-two FFT applies). The whole solve of 1400 x 203 (one
+// iteration: two transforms, the modes, the checks and host reads): 288 us. Folding a row about its middle
+// (g_j = f_j + f_{nc-j} meets only the cosines, f_j - f_{nc-j} only the sines)
+// halves the work:
+//   Re X_m = sum_j g_j cos(2 pi m j / nc),  Im X_m = -sum_j h_j sin(2 pi m j / nc),
+//   j = 0..nc/2, m = 0..nc/2,
+// two dense products of [rows][nc/2+1] by the symmetric tables qc, qs.
+// Backwards, E_j = sum_m w_m Re X_m cos, O_j = sum_m w_m Im X_m sin give
+// x_j = (E_j - O_j) / nc and x_{nc-j} = (E_j + O_j) / nc (w_m = 2, 1 for the
+// unpaired modes). The arithmetic is nc^2 / 2 multiply-adds a row and
+// direction, bound by the FP64 pipe (64 a cycle and SM). A block takes 16 rows
+// by 32 modes (or columns): 8 warps, a quarter of them on the cosine and sine
+// products each and each over half of the staged terms, so that a coarse
+// grid's few rows still give every SM a block (100 rows of 1000: 112 blocks).
+template <typename P>
+struct DftArgs {
+    int nc, NK, pitch, mpitch;
+    const P *qc, *qs;        // cos / sin(2 pi m j / nc), [nc/2+1][mpitch], symmetric in (m, j)
+    P *sre, *sim;            // spectra, [NK][mpitch]
+};
+
+constexpr int kDftRows = 16, kDftCols = 32, kDftTerms = 32, kDftThreads = 256;
+constexpr int kDftRowPad = kDftRows + 2;   // staged rows: the transposed stores spread over the banks
+
+template <typename P>
+union DftShared {
+    struct {
+        P a[2][kDftTerms][kDftRowPad];   // folded terms of the rows: for the cosines, for the sines
+        P b[2][kDftTerms][kDftCols];     // qc, qs
+    } in;
+    P out[4][kDftRows][kDftCols];        // the groups' sums: (cosine, sine) of each half of the terms
+};
+
+// The two products of one tile. term(row, e, va, vb): the pair (cosine term,
+// sine term) number e of a row. Leaves the sums in S.out.
+template <typename P, typename Term>
+__device__ __forceinline__ void dft_tile(const DftArgs<P>& a, DftShared<P>& S, int row0, int col0, Term term) {
+    constexpr int NA = kDftRows * kDftTerms / kDftThreads, NB = kDftTerms * kDftCols / kDftThreads;
+    const int tid = threadIdx.x, n = a.nc / 2 + 1;
+    const int part = (tid >> 6) & 1, half = tid >> 7, ty = (tid >> 3) & 7, tx = tid & 7;
+    P ra[NA][2], rb[NB][2];
+    auto fetch = [&](int e0) {
+#pragma unroll
+        for (int q = 0; q < NA; q++) {
+            const int t = tid + q * kDftThreads, e = e0 + (t & (kDftTerms - 1)), row = row0 + t / kDftTerms;
+            ra[q][0] = ra[q][1] = P(0);
+            if (e < n && row < a.NK) term(row, e, ra[q][0], ra[q][1]);
+        }
+#pragma unroll
+        for (int q = 0; q < NB; q++) {
+            const int t = tid + q * kDftThreads, e = e0 + t / kDftCols;
+            const size_t at = (size_t)e * a.mpitch + col0 + (t & (kDftCols - 1));
+            rb[q][0] = e < n ? a.qc[at] : P(0);
+            rb[q][1] = e < n ? a.qs[at] : P(0);
+        }
+    };
+    P acc[2][4] = {};
+    fetch(0);
+    for (int e0 = 0; e0 < n; e0 += kDftTerms) {
+#pragma unroll
+        for (int q = 0; q < NA; q++) {
+            const int t = tid + q * kDftThreads;
+            S.in.a[0][t & (kDftTerms - 1)][t / kDftTerms] = ra[q][0];
+            S.in.a[1][t & (kDftTerms - 1)][t / kDftTerms] = ra[q][1];
+        }
+#pragma unroll
+        for (int q = 0; q < NB; q++) {
+            const int t = tid + q * kDftThreads;
+            S.in.b[0][t / kDftCols][t & (kDftCols - 1)] = rb[q][0];
+            S.in.b[1][t / kDftCols][t & (kDftCols - 1)] = rb[q][1];
+        }
+        __syncthreads();
+        if (e0 + kDftTerms < n) fetch(e0 + kDftTerms);   // in flight during the products
+#pragma unroll
+        for (int e = 0; e < kDftTerms / 2; e++) {
+            const int k = half * (kDftTerms / 2) + e;
+            P x[2], y[4];
+#pragma unroll
+            for (int i = 0; i < 2; i++) x[i] = S.in.a[part][k][2 * ty + i];
+#pragma unroll
+            for (int j = 0; j < 4; j++) y[j] = S.in.b[part][k][4 * tx + j];
+#pragma unroll
+            for (int i = 0; i < 2; i++)
+#pragma unroll
+                for (int j = 0; j < 4; j++) acc[i][j] += x[i] * y[j];
+        }
+        __syncthreads();
+    }
+#pragma unroll
+    for (int i = 0; i < 2; i++)
+#pragma unroll
+        for (int j = 0; j < 4; j++) S.out[2 * half + part][2 * ty + i][4 * tx + j] = acc[i][j];
+    __syncthreads();
+}
+
+// Spectra of the rows of f ([NK][pitch]).
+template <typename P>
+__global__ void __launch_bounds__(kDftThreads) k_dft_forward(DftArgs<P> a, const P* f) {
+    __shared__ DftShared<P> S;
+    const int row0 = blockIdx.y * kDftRows, col0 = blockIdx.x * kDftCols;
+    dft_tile(a, S, row0, col0, [&](int row, int j, P& g, P& h) {
+        const P* r = f + (size_t)row * a.pitch;
+        const P x = r[j];
+        if (j == 0 || 2 * j == a.nc) {
+            g = x;
+            h = P(0);
+        } else {
+            const P y = r[a.nc - j];
+            g = x + y;
+            h = x - y;
+        }
+    });
+    for (int t = threadIdx.x; t < kDftRows * kDftCols; t += kDftThreads) {
+        const int r = t / kDftCols, c = t % kDftCols;
+        if (row0 + r >= a.NK) continue;
+        const size_t at = (size_t)(row0 + r) * a.mpitch + col0 + c;
+        a.sre[at] = S.out[0][r][c] + S.out[2][r][c];
+        a.sim[at] = -(S.out[1][r][c] + S.out[3][r][c]);
+    }
+}
+
+// Rows of out ([NK][pitch]) from their spectra.
+template <typename P>
+__global__ void __launch_bounds__(kDftThreads) k_dft_inverse(DftArgs<P> a, P* out) {
+    __shared__ DftShared<P> S;
+    const int row0 = blockIdx.y * kDftRows, col0 = blockIdx.x * kDftCols;
+    dft_tile(a, S, row0, col0, [&](int row, int m, P& g, P& h) {
+        const P w = (m == 0 || 2 * m == a.nc) ? P(1) : P(2);
+        const size_t at = (size_t)row * a.mpitch + m;
+        g = w * a.sre[at];
+        h = w * a.sim[at];
+    });
+    const P scale = P(1) / P(a.nc);
+    for (int t = threadIdx.x; t < kDftRows * kDftCols; t += kDftThreads) {
+        const int r = t / kDftCols, j = col0 + t % kDftCols;
+        if (row0 + r >= a.NK || 2 * j > a.nc) continue;
+        const P E = S.out[0][r][j - col0] + S.out[2][r][j - col0], O = S.out[1][r][j - col0] + S.out[3][r][j - col0];
+        P* x = out + (size_t)(row0 + r) * a.pitch;
+        x[j] = (E - O) * scale;
+        if (j > 0 && 2 * j < a.nc) x[a.nc - j] = (E + O) * scale;
+    }
+}
+
+// The tables of nc columns: entry (j, m) at angle 2 pi ((j m) mod nc) / nc.
+template <typename P>
+__global__ void k_dft_tables(int nc, int mpitch, P* qc, P* qs) {
+    const int m = blockIdx.x * blockDim.x + threadIdx.x, j = blockIdx.y;
+    if (m >= mpitch) return;
+    double c = 0.0, s = 0.0;
+    if (2 * m <= nc) sincospi(2.0 * (double)(((long long)j * m) % nc) / (double)nc, &s, &c);
+    qc[(size_t)j * mpitch + m] = P(c);
+    qs[(size_t)j * mpitch + m] = P(s);
+}
 
 }  // namespace vvm

@@ -368,17 +368,8 @@ struct Arena {
     }
 };
 
-// Multigrid hierarchy for the symmetric w-equation operator, precision P.
-//
-// Levels halve the column count while it is even (x-semicoarsening); a
-// power-of-two NX ends at one column, whose operator has no x part and is
-// solved exactly by one line solve. Otherwise the coarsest level has an odd
-// column count (at most kMaxOddCoarse) and gets 2*nc + 8 damped line sweeps.
-// Levels of at most 32 columns run inside one block (k_mg_coarse_cycle).
+// The odd factor of NX at most: x-semicoarsening keeps it in every level.
 constexpr int kMaxOddCoarse = 256;
-// Dynamic shared memory of the Fourier-mode coarse solve at most (f / solution
-// and the reduced-system bands, next to 32 KB of static tiles within 227 KB).
-constexpr int kModeSmemMax = 192 * 1024;
 
 struct Recorder;
 
@@ -618,201 +609,11 @@ static HostLine factor_partitioned(const std::vector<double>& xdiag, const std::
     return h;
 }
 
+// Factors of the per-mode z solves of an operator of nc periodic columns
+// (spectral_kernels.cuh), shared by both row transforms below.
 template <typename P>
-struct Multigrid {
-    int NK = 0, nlev = 0, S = 0, LS = 8, lc = 0;   // lc: first level run in the coarse block
-    bool modes = false;        // level lc is solved exactly by Fourier modes
-    ModeSolve ms{};
-    size_t mode_smem = 0;
-    bool exact_coarsest = true;
-    int coarse_sweeps = 1;
-    std::vector<int> nx, pitch;
-    std::vector<P*> f, x, y;
-    std::vector<LineLevel> lines;
-    double *ru = nullptr, *rd = nullptr;
-    P omega = P(2.0 / 3.0);
-    Stats* stats = nullptr;
-
-    double* upload(Arena& ar, const std::vector<double>& v) {
-        double* d = ar.alloc<double>(v.size());
-        upload_now(d, v.data(), v.size() * sizeof(double));
-        return d;
-    }
-
-    void build(Arena& ar, int NX, int NKr, const std::vector<double>& cx0, const std::vector<double>& ru_h,
-               const std::vector<double>& rd_h) {
-        NK = NKr;
-        LS = NK <= 256 ? 8 : (NK <= 512 ? 16 : 32);
-        S = (NK + LS - 1) / LS;
-        int n = NX;
-        nx.push_back(n);
-        while (n % 2 == 0 && n > 1) {
-            n /= 2;
-            nx.push_back(n);
-        }
-        nlev = (int)nx.size();
-        exact_coarsest = (nx.back() == 1);
-        coarse_sweeps = exact_coarsest ? 1 : 2 * nx.back() + 8;
-        lc = nlev - 1;
-        while (lc > 0 && nx[lc - 1] <= 32) lc--;
-        if (nlev - lc > kMaxCoarseLevels) lc = nlev - kMaxCoarseLevels;
-        // exact Fourier-mode solve on the first level of at most 32 columns
-        // when its shared-memory tiles (f / solution and the reduced-system
-        // bands, next to 32 KB of static tiles) fit in 227 KB
-        for (int l = 0; l < nlev; l++) {
-            if (nx[l] <= 32 && ((size_t)NK + 10 * (size_t)S) * nx[l] * sizeof(P) <= (size_t)kModeSmemMax) {
-                modes = true;
-                lc = l;
-                nlev = l + 1;   // coarser levels are not needed
-                nx.resize(nlev);
-                break;
-            }
-        }
-        ru = upload(ar, ru_h);
-        rd = upload(ar, rd_h);
-        for (int l = 0; l < nlev; l++) {
-            int pl = round_up(nx[l], kPad);
-            pitch.push_back(pl);
-            f.push_back(l == 0 ? nullptr : ar.alloc<P>((size_t)NK * pl));
-            x.push_back(ar.alloc<P>((size_t)NK * pl));
-            y.push_back(ar.alloc<P>((size_t)NK * pl));
-            std::vector<double> c(NK), xd(NK);
-            double sc = std::pow(0.25, l);
-            bool exact = (l == nlev - 1) && exact_coarsest;
-            for (int k = 0; k < NK; k++) {
-                c[k] = cx0[k] * sc;
-                xd[k] = exact ? 0.0 : 2.0 * c[k];
-            }
-            HostLine h = factor_partitioned(xd, ru_h, rd_h, S);
-            LineLevel L{nx[l], pl, NK, S, upload(ar, c), upload(ar, h.lo), upload(ar, h.inv), upload(ar, h.cp),
-                        upload(ar, h.gL), upload(ar, h.gR), upload(ar, h.band)};
-            lines.push_back(L);
-            if (modes && l == lc) build_modes(ar, c, ru_h, rd_h, pl);
-        }
-    }
-
-    // Orthonormal real Fourier basis of nc periodic columns and the per-mode
-    // partitioned factors of (cx mu_m + ru + rd, -ru, -rd).
-    void build_modes(Arena& ar, const std::vector<double>& c, const std::vector<double>& ru_h,
-                     const std::vector<double>& rd_h, int pl) {
-        const int nc = nx[lc];
-        const double pi = 3.14159265358979323846;
-        std::vector<double> Q((size_t)nc * nc, 0.0), mu(nc, 0.0);
-        int m = 0;
-        for (int j = 0; j < nc; j++) Q[(size_t)j * nc + m] = 1.0 / std::sqrt((double)nc);
-        mu[m++] = 0.0;
-        for (int fr = 1; 2 * fr < nc; fr++) {
-            for (int j = 0; j < nc; j++) {
-                Q[(size_t)j * nc + m] = std::sqrt(2.0 / nc) * std::cos(2 * pi * fr * j / nc);
-                Q[(size_t)j * nc + m + 1] = std::sqrt(2.0 / nc) * std::sin(2 * pi * fr * j / nc);
-            }
-            mu[m] = mu[m + 1] = 2.0 - 2.0 * std::cos(2 * pi * fr / nc);
-            m += 2;
-        }
-        if (nc % 2 == 0) {
-            for (int j = 0; j < nc; j++) Q[(size_t)j * nc + m] = ((j & 1) ? -1.0 : 1.0) / std::sqrt((double)nc);
-            mu[m++] = 4.0;
-        }
-        std::vector<double> lo((size_t)NK * nc), inv((size_t)NK * nc), cp((size_t)NK * nc), gL((size_t)NK * nc),
-            gR((size_t)NK * nc), Mi((size_t)5 * 2 * S * nc);
-        const size_t S2 = 2 * (size_t)S;
-        for (int q = 0; q < nc; q++) {   // mode fastest: lanes (modes) read consecutive words
-            std::vector<double> xd(NK);
-            for (int k = 0; k < NK; k++) xd[k] = c[k] * mu[q];
-            HostLine h = factor_partitioned(xd, ru_h, rd_h, S);
-            for (int k = 0; k < NK; k++) {
-                lo[(size_t)k * nc + q] = h.lo[k];
-                inv[(size_t)k * nc + q] = h.inv[k];
-                cp[(size_t)k * nc + q] = h.cp[k];
-                gL[(size_t)k * nc + q] = h.gL[k];
-                gR[(size_t)k * nc + q] = h.gR[k];
-            }
-            for (size_t e = 0; e < 5 * S2; e++) Mi[e * nc + q] = h.band[e];
-        }
-        ms = ModeSolve{nc, pl, NK, S, upload(ar, Q), upload(ar, lo), upload(ar, inv), upload(ar, cp),
-                       upload(ar, gL), upload(ar, gR), upload(ar, Mi)};
-        mode_smem = ((size_t)NK * nc + (size_t)10 * S * nc) * sizeof(P);
-        auto setattr = [&](auto kern) {
-            // the attribute is per kernel, not per context: set the largest any
-            // context may use (the fit test above), so contexts of other sizes
-            // in the same process never lower it under each other
-            CK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, kModeSmemMax));
-        };
-        if (LS == 8) setattr(k_coarse_modes<P, 8>);
-        else if (LS == 16) setattr(k_coarse_modes<P, 16>);
-        else setattr(k_coarse_modes<P, 32>);
-    }
-
-    ZOps zops() const { return ZOps{ru, rd, NK}; }
-
-    void sweep(int l, const P* fl, const P* xin, const P* xc, int pc, int nc, P* out, P om, cudaStream_t st) {
-        SweepArgs<P> a{lines[l], zops(), fl, xin, xc, pc, nc, out, om};
-        dim3 g(cdiv(nx[l], 32)), b(32 * S);
-        if (LS == 8) LAUNCH(stats, VVM_K_MG_SWEEP, st, k_line_sweep<P, 8><<<g, b, 0, st>>>(a));
-        else if (LS == 16) LAUNCH(stats, VVM_K_MG_SWEEP, st, k_line_sweep<P, 16><<<g, b, 0, st>>>(a));
-        else LAUNCH(stats, VVM_K_MG_SWEEP, st, k_line_sweep<P, 32><<<g, b, 0, st>>>(a));
-        CKL();
-    }
-
-    // z = M r (one V(1,1) cycle); returns the buffer holding z.
-    P* apply(const P* r, cudaStream_t st) {
-        const P* fl = r;
-        for (int l = 0; l < lc; l++) {
-            // pre-smoothing from zero fused with the restriction of its residual
-            dim3 g(cdiv(nx[l], kOwned)), b(32 * S);
-            if (LS == 8) LAUNCH(stats, VVM_K_MG_SWEEP, st, k_presmooth_restrict<P, 8><<<g, b, 0, st>>>(lines[l], zops(), fl, x[l], f[l + 1], pitch[l + 1], omega));
-            else if (LS == 16) LAUNCH(stats, VVM_K_MG_SWEEP, st, k_presmooth_restrict<P, 16><<<g, b, 0, st>>>(lines[l], zops(), fl, x[l], f[l + 1], pitch[l + 1], omega));
-            else LAUNCH(stats, VVM_K_MG_SWEEP, st, k_presmooth_restrict<P, 32><<<g, b, 0, st>>>(lines[l], zops(), fl, x[l], f[l + 1], pitch[l + 1], omega));
-            CKL();
-            fl = f[l + 1];
-        }
-        P* res;
-        if (modes) {
-            P* out = (lc == 0) ? y[0] : x[lc];
-            if (LS == 8) LAUNCH(stats, VVM_K_MG_COARSE, st, k_coarse_modes<P, 8><<<1, 32 * S, mode_smem, st>>>(ms, fl, out));
-            else if (LS == 16) LAUNCH(stats, VVM_K_MG_COARSE, st, k_coarse_modes<P, 16><<<1, 32 * S, mode_smem, st>>>(ms, fl, out));
-            else LAUNCH(stats, VVM_K_MG_COARSE, st, k_coarse_modes<P, 32><<<1, 32 * S, mode_smem, st>>>(ms, fl, out));
-            CKL();
-            res = out;
-        } else {
-            // levels lc..nlev-1 in one block
-            CoarseCycleArgs<P> ca{};
-            ca.nlev = nlev - lc;
-            for (int j = 0; j < ca.nlev; j++) {
-                ca.L[j] = lines[lc + j];
-                ca.f[j] = f[lc + j];
-                ca.x[j] = x[lc + j];
-                ca.y[j] = y[lc + j];
-            }
-            ca.z = zops();
-            ca.f0 = fl;
-            ca.omega = omega;
-            ca.coarse_sweeps = coarse_sweeps;
-            if (LS == 8) LAUNCH(stats, VVM_K_MG_COARSE, st, k_mg_coarse_cycle<P, 8><<<1, 32 * S, 0, st>>>(ca));
-            else if (LS == 16) LAUNCH(stats, VVM_K_MG_COARSE, st, k_mg_coarse_cycle<P, 16><<<1, 32 * S, 0, st>>>(ca));
-            else LAUNCH(stats, VVM_K_MG_COARSE, st, k_mg_coarse_cycle<P, 32><<<1, 32 * S, 0, st>>>(ca));
-            CKL();
-            res = y[lc];
-        }
-        for (int l = lc - 1; l >= 0; l--) {
-            const P* fl2 = (l == 0) ? r : f[l];
-            sweep(l, fl2, x[l], res, pitch[l + 1], nx[l + 1], y[l], omega, st);
-            res = y[l];
-        }
-        return res;
-    }
-};
-
-// Exact Fourier-mode preconditioner (spectral_kernels.cuh); NX a power of two.
-template <typename P>
-struct Spectral {
+struct ModeFactors {
     SpecArgs<P> a{};
-    P* out = nullptr;
-    size_t smem = 0;
-    int threads = 0;
-    Stats* stats = nullptr;
-
-    static bool supports(int NX) { return NX >= 4 && NX <= 8192 && (NX & (NX - 1)) == 0; }
 
     static P* upload(Arena& ar, const std::vector<double>& v) {
         std::vector<P> h(v.begin(), v.end());
@@ -821,23 +622,16 @@ struct Spectral {
         return d;
     }
 
-    void build(Arena& ar, int NX, int NK, int pitch, const std::vector<double>& cx0, const std::vector<double>& ru,
-               const std::vector<double>& rd) {
-        int logN = 0;
-        while ((1 << logN) < NX) logN++;
-        const int M = NX / 2 + 1, mp = round_up(M, 32);
+    void build_factors(Arena& ar, int nc, int NK, int pitch, const std::vector<double>& cx0,
+                       const std::vector<double>& ru, const std::vector<double>& rd) {
+        const int M = nc / 2 + 1, mp = round_up(M, 32);
         const double pi = 3.14159265358979323846;
-        std::vector<double> twr(NX / 2), twi(NX / 2);
-        for (int j = 0; j < NX / 2; j++) {
-            twr[j] = std::cos(2.0 * pi * j / NX);
-            twi[j] = -std::sin(2.0 * pi * j / NX);
-        }
         // twisted factorisation of each mode's z operator (spectral_kernels.cuh):
         // rows 0..mid eliminated downwards, mid+1..NK-1 upwards
         const int mid = (NK - 1) / 2;
         std::vector<double> inv((size_t)NK * mp, 0.0), cp((size_t)NK * mp, 0.0), den(mp, 0.0);
         for (int m = 0; m < M; m++) {
-            const double mu = 2.0 - 2.0 * std::cos(2.0 * pi * m / NX);
+            const double mu = 2.0 - 2.0 * std::cos(2.0 * pi * m / nc);
             double up_over_piv = 0.0;   // ru_{k-1} / piv_{k-1}
             for (int k = 0; k <= mid; k++) {
                 const double piv = cx0[k] * mu + ru[k] + rd[k] - (k > 0 ? rd[k] * up_over_piv : 0.0);
@@ -854,14 +648,11 @@ struct Spectral {
             }
             den[m] = 1.0 / (1.0 - cp[(size_t)mid * mp + m] * cp[(size_t)(mid + 1) * mp + m]);
         }
-        a.NX = NX;
-        a.logN = logN;
+        a.NX = nc;
         a.NK = NK;
         a.pitch = pitch;
         a.mpitch = mp;
         a.mid = mid;
-        a.twr = upload(ar, twr);
-        a.twi = upload(ar, twi);
         a.inv = upload(ar, inv);
         a.cp = upload(ar, cp);
         a.den = upload(ar, den);
@@ -869,6 +660,39 @@ struct Spectral {
         a.ru = upload(ar, ru);
         a.sre = ar.alloc<P>((size_t)NK * mp);
         a.sim = ar.alloc<P>((size_t)NK * mp);
+    }
+
+    void solve_modes(Stats* stats, cudaStream_t st) {
+        klaunch<k_spec_modes_seg_body<P>, 64 * kModeSegs>(stats, VVM_K_MG_COARSE, st, k_spec_modes_seg<P>,
+                                                          dim3(cdiv(a.NX / 2 + 1, 32)), dim3(64 * kModeSegs), 0, a);
+    }
+};
+
+// Exact Fourier-mode preconditioner (spectral_kernels.cuh); NX a power of two.
+template <typename P>
+struct Spectral : ModeFactors<P> {
+    using ModeFactors<P>::a;
+    P* out = nullptr;
+    size_t smem = 0;
+    int threads = 0;
+    Stats* stats = nullptr;
+
+    static bool supports(int NX) { return NX >= 4 && NX <= 8192 && (NX & (NX - 1)) == 0; }
+
+    void build(Arena& ar, int NX, int NK, int pitch, const std::vector<double>& cx0, const std::vector<double>& ru,
+               const std::vector<double>& rd) {
+        int logN = 0;
+        while ((1 << logN) < NX) logN++;
+        const double pi = 3.14159265358979323846;
+        std::vector<double> twr(NX / 2), twi(NX / 2);
+        for (int j = 0; j < NX / 2; j++) {
+            twr[j] = std::cos(2.0 * pi * j / NX);
+            twi[j] = -std::sin(2.0 * pi * j / NX);
+        }
+        this->build_factors(ar, NX, NK, pitch, cx0, ru, rd);
+        a.logN = logN;
+        a.twr = this->upload(ar, twr);
+        a.twi = this->upload(ar, twi);
         out = ar.alloc<P>((size_t)NK * pitch);
         smem = 3 * (size_t)NX * sizeof(P);   // the row pair (re, im) and the twiddles
         threads = std::max(32, std::min(NX / 2, 512));
@@ -883,8 +707,7 @@ struct Spectral {
         const int rows2 = cdiv(a.NK, 2);
         klaunch<k_spec_forward_body<P>, 1024>(stats, VVM_K_MG_SWEEP, st, k_spec_forward<P>, dim3(rows2), dim3(threads),
                                               smem, a, r);
-        klaunch<k_spec_modes_seg_body<P>, 64 * kModeSegs>(stats, VVM_K_MG_COARSE, st, k_spec_modes_seg<P>,
-                                                          dim3(cdiv(a.NX / 2 + 1, 32)), dim3(64 * kModeSegs), 0, a);
+        this->solve_modes(stats, st);
         klaunch<k_spec_inverse_body<P>, 1024>(stats, VVM_K_MG_SWEEP, st, k_spec_inverse<P>, dim3(rows2), dim3(threads),
                                               smem, a, dst);
     }
@@ -892,6 +715,133 @@ struct Spectral {
     P* apply(const P* r, cudaStream_t st) {
         apply_to(r, out, st);
         return out;
+    }
+};
+
+// The same exact solve on a level of any column count (k_dft_forward).
+template <typename P>
+struct DftSolve : ModeFactors<P> {
+    using ModeFactors<P>::a;
+    DftArgs<P> d{};
+
+    void build(Arena& ar, int nc, int NK, int pitch, const std::vector<double>& cx0, const std::vector<double>& ru,
+               const std::vector<double>& rd) {
+        this->build_factors(ar, nc, NK, pitch, cx0, ru, rd);
+        const int n = nc / 2 + 1;
+        P *qc = ar.alloc<P>((size_t)n * a.mpitch), *qs = ar.alloc<P>((size_t)n * a.mpitch);
+        k_dft_tables<P><<<dim3(cdiv(a.mpitch, 64), n), 64>>>(nc, a.mpitch, qc, qs);
+        CKL();
+        CK(cudaStreamSynchronize(nullptr));
+        d = DftArgs<P>{nc, NK, pitch, a.mpitch, qc, qs, a.sre, a.sim};
+    }
+
+    // dst = (the level's operator)^{-1} r (to round-off).
+    void apply_to(Stats* stats, const P* r, P* dst, cudaStream_t st) {
+        const dim3 g(cdiv(d.nc / 2 + 1, kDftCols), cdiv(d.NK, kDftRows)), b(kDftThreads);
+        LAUNCH(stats, VVM_K_MG_COARSE, st, k_dft_forward<P><<<g, b, 0, st>>>(d, r));
+        CKL();
+        this->solve_modes(stats, st);
+        LAUNCH(stats, VVM_K_MG_COARSE, st, k_dft_inverse<P><<<g, b, 0, st>>>(d, dst));
+        CKL();
+    }
+};
+
+// Multigrid hierarchy for the symmetric w-equation operator, precision P.
+// The last level is solved exactly by its Fourier modes (DftSolve), whatever
+// its odd factor. Rows of at most kExactFinest columns are not coarsened at
+// all: the transform's nc^2 / 2 multiply-adds a row still cost less than the
+// nine or ten cycles of a multigrid PCG to 1e-12 (us a solve on a B200, exact
+// / levels down to 512 columns: 1000 x 101 190 / 1090, 1400 x 203 288 / 1640,
+// 2048 x 256 572 / 1906, 3072 x 128 614 / 1845, 4096 x 256 1776 / 2556; with
+// damped sweeps on the odd level, as before, 1400 x 203 took 226,800).
+// Longer rows halve (x-semicoarsening) until they have at most kExactCoarse
+// (4096 x 256: 2953 / 2556 / 2813 us a solve down to 1024 / 512 / 256).
+constexpr int kExactFinest = 4096, kExactCoarse = 512;
+
+template <typename P>
+struct Multigrid {
+    int NK = 0, nlev = 0, S = 0, LS = 8;
+    DftSolve<P> coarsest;      // exact solve of the last level
+    std::vector<int> nx, pitch;
+    std::vector<P*> f, x, y;
+    std::vector<LineLevel> lines;
+    double *ru = nullptr, *rd = nullptr;
+    P omega = P(2.0 / 3.0);
+    Stats* stats = nullptr;
+
+    double* upload(Arena& ar, const std::vector<double>& v) {
+        double* d = ar.alloc<double>(v.size());
+        upload_now(d, v.data(), v.size() * sizeof(double));
+        return d;
+    }
+
+    // cycle = false: the finest level's operator and line factors only.
+    void build(Arena& ar, int NX, int NKr, const std::vector<double>& cx0, const std::vector<double>& ru_h,
+               const std::vector<double>& rd_h, bool cycle) {
+        NK = NKr;
+        LS = NK <= 256 ? 8 : (NK <= 512 ? 16 : 32);
+        S = (NK + LS - 1) / LS;
+        int n = NX;
+        nx.push_back(n);
+        while (cycle && NX > kExactFinest && n > kExactCoarse) {
+            n /= 2;
+            nx.push_back(n);
+        }
+        nlev = (int)nx.size();
+        ru = upload(ar, ru_h);
+        rd = upload(ar, rd_h);
+        for (int l = 0; l < nlev; l++) {
+            int pl = round_up(nx[l], kPad);
+            pitch.push_back(pl);
+            f.push_back(cycle && l > 0 ? ar.alloc<P>((size_t)NK * pl) : nullptr);
+            x.push_back(cycle ? ar.alloc<P>((size_t)NK * pl) : nullptr);
+            y.push_back(cycle && l < nlev - 1 ? ar.alloc<P>((size_t)NK * pl) : nullptr);
+            std::vector<double> c(NK), xd(NK);
+            double sc = std::pow(0.25, l);
+            for (int k = 0; k < NK; k++) {
+                c[k] = cx0[k] * sc;
+                xd[k] = 2.0 * c[k];
+            }
+            HostLine h = factor_partitioned(xd, ru_h, rd_h, S);
+            LineLevel L{nx[l], pl, NK, S, upload(ar, c), upload(ar, h.lo), upload(ar, h.inv), upload(ar, h.cp),
+                        upload(ar, h.gL), upload(ar, h.gR), upload(ar, h.band)};
+            lines.push_back(L);
+            if (cycle && l == nlev - 1) coarsest.build(ar, nx[l], NK, pl, c, ru_h, rd_h);
+        }
+    }
+
+    ZOps zops() const { return ZOps{ru, rd, NK}; }
+
+    void sweep(int l, const P* fl, const P* xin, const P* xc, int pc, int nc, P* out, P om, cudaStream_t st) {
+        SweepArgs<P> a{lines[l], zops(), fl, xin, xc, pc, nc, out, om};
+        dim3 g(cdiv(nx[l], 32)), b(32 * S);
+        if (LS == 8) LAUNCH(stats, VVM_K_MG_SWEEP, st, k_line_sweep<P, 8><<<g, b, 0, st>>>(a));
+        else if (LS == 16) LAUNCH(stats, VVM_K_MG_SWEEP, st, k_line_sweep<P, 16><<<g, b, 0, st>>>(a));
+        else LAUNCH(stats, VVM_K_MG_SWEEP, st, k_line_sweep<P, 32><<<g, b, 0, st>>>(a));
+        CKL();
+    }
+
+    // z = M r (one V(1,1) cycle; the exact solve alone when the finest level
+    // is the last); returns the buffer holding z.
+    P* apply(const P* r, cudaStream_t st) {
+        const P* fl = r;
+        for (int l = 0; l < nlev - 1; l++) {
+            // pre-smoothing from zero fused with the restriction of its residual
+            dim3 g(cdiv(nx[l], kOwned)), b(32 * S);
+            if (LS == 8) LAUNCH(stats, VVM_K_MG_SWEEP, st, k_presmooth_restrict<P, 8><<<g, b, 0, st>>>(lines[l], zops(), fl, x[l], f[l + 1], pitch[l + 1], omega));
+            else if (LS == 16) LAUNCH(stats, VVM_K_MG_SWEEP, st, k_presmooth_restrict<P, 16><<<g, b, 0, st>>>(lines[l], zops(), fl, x[l], f[l + 1], pitch[l + 1], omega));
+            else LAUNCH(stats, VVM_K_MG_SWEEP, st, k_presmooth_restrict<P, 32><<<g, b, 0, st>>>(lines[l], zops(), fl, x[l], f[l + 1], pitch[l + 1], omega));
+            CKL();
+            fl = f[l + 1];
+        }
+        P* res = x[nlev - 1];
+        coarsest.apply_to(stats, fl, res, st);
+        for (int l = nlev - 2; l >= 0; l--) {
+            const P* fl2 = (l == 0) ? r : f[l];
+            sweep(l, fl2, x[l], res, pitch[l + 1], nx[l + 1], y[l], omega, st);
+            res = y[l];
+        }
+        return res;
     }
 };
 
@@ -1479,7 +1429,7 @@ struct PCG {
             rw[kk] = unweighted ? 1.0 : rhow[k] / a[k];
         }
         mg.stats = stats;
-        mg.build(ar, NX, NK, cx0, ru, rd);
+        mg.build(ar, NX, NK, cx0, ru, rd, !spectral);
         pitch = mg.pitch[0];
         if (spectral) {
             sp.stats = stats;

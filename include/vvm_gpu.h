@@ -48,7 +48,10 @@ extern "C" {
                              FP64 Poisson residual, refinement and reductions */
 
 /* Preconditioner of the Poisson CG (cal_w). */
-#define VVM_SOLVER_MGPCG 0    /* geometric multigrid: x-semicoarsening, z-line relaxation */
+#define VVM_SOLVER_MGPCG 0    /* geometric multigrid: x-semicoarsening, z-line relaxation, the
+                                 last level solved exactly by its Fourier modes (up to 4096
+                                 columns the finest level is the last); any NX whose odd
+                                 factor is at most 256 */
 #define VVM_SOLVER_LEARNED 1  /* learned BF16 conv preconditioner in flexible CG,
                                  multigrid-PCG as fallback (vvm_gpu_learned_*) */
 #define VVM_SOLVER_SPECTRAL 2 /* exact Fourier-mode solve (row FFTs in x, one
