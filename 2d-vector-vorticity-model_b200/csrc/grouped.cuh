@@ -94,11 +94,4 @@ __global__ void k_group_cond(const int* const* __restrict__ flags, int n, cudaGr
     if (threadIdx.x == 0) cudaGraphSetConditional(h, any ? 1u : 0u);
 }
 
-// Clears `bytes` bytes at ptrs[blockIdx.z] (a device memset a case).
-__global__ void k_group_zero(unsigned char* const* __restrict__ ptrs, size_t bytes) {
-    unsigned char* p = ptrs[blockIdx.z];
-    for (size_t j = blockIdx.x * (size_t)blockDim.x + threadIdx.x; j < bytes; j += (size_t)gridDim.x * blockDim.x)
-        p[j] = 0;
-}
-
 }  // namespace vvm

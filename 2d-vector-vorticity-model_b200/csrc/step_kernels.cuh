@@ -749,6 +749,8 @@ struct KesslerArgs {
     Consts c;
     Profiles p;
     T *thp, *qvp, *qcp, *qrp;
+    T* out[4];        // where th, qv, qc, qr go (in place, or the diffusion's inputs)
+    int halo;         // write their ghost images too
     T *d_auto, *d_accr, *d_evap, *d_cond;  // diagnostics (may be null)
     double* partial;
     int nvp;  // accumulate NVP sums
@@ -839,10 +841,12 @@ __device__ __forceinline__ void k_kessler_body(const KesslerArgs<T>& a) {
             a.d_evap[id] = T(rates[2]);
             a.d_cond[id] = T(rates[3]);
         }
-        a.thp[id] = T(th - th0);
-        a.qvp[id] = T(qv - qv0);
-        a.qcp[id] = T(qc);
-        a.qrp[id] = T(qr);
+        const T res[4] = {T(th - th0), T(qv - qv0), T(qc), T(qr)};
+#pragma unroll
+        for (int f = 0; f < 4; f++) {
+            if (a.halo) store_center(a.out[f], d, i, k, res[f]);
+            else a.out[f][id] = res[f];
+        }
         if (a.nvp) {
             C q[3] = {qv, qc, qr};
 #pragma unroll
@@ -875,47 +879,68 @@ struct RKArgs {
     Profiles p;
     const T *u, *w, *thp;
     T *RKM, *RKH;
+    unsigned* kmax;   // [2], 0 before: the largest RKM, RKH (float bits, rounded up)
 };
+
+// Raises *m to the largest of the block's values v (positive floats compared
+// as their bits; a NaN's bits are above all of them). Blocks that would not
+// raise it issue no atomic.
+__device__ __forceinline__ void block_max_bits(unsigned v, unsigned* sh, unsigned* m) {
+    const int tid = threadIdx.x + blockDim.x * threadIdx.y;
+    v = __reduce_max_sync(0xffffffffu, v);
+    if ((tid & 31) == 0) sh[tid >> 5] = v;
+    __syncthreads();
+    if (tid == 0) {
+        for (int w = 1; w < (int)(blockDim.x * blockDim.y) >> 5; w++) v = max(v, sh[w]);
+        if (v > *(volatile unsigned*)m) atomicMax(m, v);
+    }
+}
+__device__ __forceinline__ unsigned bits_up(double x) { return __float_as_uint(__double2float_ru(x)); }
+__device__ __forceinline__ unsigned bits_up(float x) { return __float_as_uint(x); }
 
 template <typename T>
 __device__ __forceinline__ void k_rkm_rkh_body(const RKArgs<T>& a) {
     const Dims& d = a.d;
     const int i = 1 + blockIdx.x * blockDim.x + threadIdx.x;
     const int k = 1 + blockIdx.y * blockDim.y + threadIdx.y;
-    if (i > d.nx - 2 || k > d.nz - 2) return;
-    const T* u = a.u;
-    const T* w = a.w;
-    T Rzeta = T(0.5) * ((w[d.at(i + 1, k + 1)] + w[d.at(i + 1, k)]) - (w[d.at(i - 1, k + 1)] + w[d.at(i - 1, k)])) * T(a.c.r2dx) +
-              T(0.5) * ((u[d.at(i + 1, k + 1)] + u[d.at(i, k + 1)]) - (u[d.at(i + 1, k - 1)] + u[d.at(i, k - 1)])) * T(a.p.r2dzcc[k]);
-    T rot = (u[d.at(i + 1, k)] - u[d.at(i, k)]) * T(a.c.rdx) + (w[d.at(i, k + 1)] - w[d.at(i, k)]) * T(a.p.rdzc[k]);
-    T Rotat = rot * rot;
-    T th0 = a.thp[d.at(i, k)];
-    T dth = a.thp[d.at(i, k + 1)] - a.thp[d.at(i, k - 1)];
-    if constexpr (kPert<T>) {       // perturbation storage: add the profile parts
-        th0 += T(a.p.ref[0][k]);
-        dth += T(a.p.g0[0][k]);
+    __shared__ unsigned sh[2][32];
+    T km = T(0), kh = T(0);
+    if (i <= d.nx - 2 && k <= d.nz - 2) {
+        const T* u = a.u;
+        const T* w = a.w;
+        T Rzeta = T(0.5) * ((w[d.at(i + 1, k + 1)] + w[d.at(i + 1, k)]) - (w[d.at(i - 1, k + 1)] + w[d.at(i - 1, k)])) * T(a.c.r2dx) +
+                  T(0.5) * ((u[d.at(i + 1, k + 1)] + u[d.at(i, k + 1)]) - (u[d.at(i + 1, k - 1)] + u[d.at(i, k - 1)])) * T(a.p.r2dzcc[k]);
+        T rot = (u[d.at(i + 1, k)] - u[d.at(i, k)]) * T(a.c.rdx) + (w[d.at(i, k + 1)] - w[d.at(i, k)]) * T(a.p.rdzc[k]);
+        T Rotat = rot * rot;
+        T th0 = a.thp[d.at(i, k)];
+        T dth = a.thp[d.at(i, k + 1)] - a.thp[d.at(i, k - 1)];
+        if constexpr (kPert<T>) {       // perturbation storage: add the profile parts
+            th0 += T(a.p.ref[0][k]);
+            dth += T(a.p.g0[0][k]);
+        }
+        T def2 = Rzeta * Rzeta + T(2.) * Rotat;
+        T Ri = (T(a.c.gravity) / th0 * dth * T(a.p.r2dzcc[k])) / def2;
+        T lam = T(a.p.lambda2[k]);
+        if (Ri < T(0)) {
+            km = lam * sqrt(def2) * sqrt(T(1.) - T(16.) * Ri);
+            kh = lam * sqrt(def2) * T(1.4) * sqrt(T(1.) - T(40.) * Ri);
+        } else if (T(0) < Ri && Ri < T(0.25)) {
+            km = lam * sqrt(def2) * pow(T(1.) - T(4.) * Ri, T(4));
+            kh = lam * sqrt(def2) * T(1.4) * (T(1.) - T(1.2) * Ri) * pow(T(1.) - T(4.) * Ri, T(4));
+        } else {
+            km = T(0.);
+            kh = T(0.);
+        }
+        const T kmax = T(a.p.kmax[k]);
+        km = smax(km, T(10.));
+        kh = smax(kh, T(10.));
+        km = smin(km, kmax);
+        kh = smin(kh, kmax);
+        store_center(a.RKM, d, i, k, km);
+        store_center(a.RKH, d, i, k, kh);
     }
-    T def2 = Rzeta * Rzeta + T(2.) * Rotat;
-    T Ri = (T(a.c.gravity) / th0 * dth * T(a.p.r2dzcc[k])) / def2;
-    T lam = T(a.p.lambda2[k]);
-    T km, kh;
-    if (Ri < T(0)) {
-        km = lam * sqrt(def2) * sqrt(T(1.) - T(16.) * Ri);
-        kh = lam * sqrt(def2) * T(1.4) * sqrt(T(1.) - T(40.) * Ri);
-    } else if (T(0) < Ri && Ri < T(0.25)) {
-        km = lam * sqrt(def2) * pow(T(1.) - T(4.) * Ri, T(4));
-        kh = lam * sqrt(def2) * T(1.4) * (T(1.) - T(1.2) * Ri) * pow(T(1.) - T(4.) * Ri, T(4));
-    } else {
-        km = T(0.);
-        kh = T(0.);
-    }
-    const T kmax = T(a.p.kmax[k]);
-    km = smax(km, T(10.));
-    kh = smax(kh, T(10.));
-    km = smin(km, kmax);
-    kh = smin(kh, kmax);
-    store_center(a.RKM, d, i, k, km);
-    store_center(a.RKH, d, i, k, kh);
+    block_max_bits(bits_up(km), sh[0], a.kmax);
+    block_max_bits(bits_up(kh), sh[1], a.kmax + 1);
 }
 template <typename T>
 __global__ void k_rkm_rkh(RKArgs<T> a) { k_rkm_rkh_body<T>(a); }
@@ -1060,8 +1085,9 @@ __device__ __forceinline__ void k_gs_tiles_body(const GSArgs<T>& a, const GSTile
     if (threadIdx.x == 0) any_changed = 0;
     __syncthreads();
     constexpr bool first = FIRST;
-    // a pass launched after the sweep converged has nothing to do
-    if (!FIRST && !*(volatile int*)&t.ctl->more) return;
+    // a pass launched after the sweep converged has nothing to do, nor has
+    // pass 1 once the passes have begun (a loop body launches both kernels)
+    if (FIRST ? t.ctl->pass != 0 : !*(volatile int*)&t.ctl->more) return;
     const int pass = FIRST ? 1 : t.ctl->pass + 1;
     const int q = pass & 1, qp = q ^ 1;
     const int tile = blockIdx.x * 4 + wid;
@@ -1351,6 +1377,390 @@ __device__ __forceinline__ void k_gs_tiles_body(const GSArgs<T>& a, const GSTile
 }
 template <typename T, bool FIRST>
 __global__ void __launch_bounds__(128, kGSTileMinBlocks<T>) k_gs_tiles(GSArgs<T> a, GSTileArgs<T> t, cudaGraphConditionalHandle h) { k_gs_tiles_body<T, FIRST>(a, t, h); }
+
+// ---------------------------------------------------------------------------
+// The same recurrence in one pass, for the coefficients a step normally has.
+//
+// With beta the largest B + C of the grid, an error of a cell's inflow is
+// beta^n of itself n cells later, so a tile needs no exact inflow: started
+// hz rows below and 16 cells left of the cells it owns, from the old values
+// (which differ from the new ones by beta times the field's local change), its
+// owned cells are off by beta^(hz+1) of that change. hz is the least number of
+// rows that puts this below 2^-56 (FP32: 2^-28), from the largest eddy
+// coefficient of the grid (k_rkm_rkh), usually 4 to 8; where more than
+// kGWHaloMax would be needed (B + C above about 0.1, FP32 0.3) the kernel
+// writes nothing and asks for the repeated passes above instead. Along a row
+// the same bound cuts the scan short: y left of a lane's four cells is the
+// lanes' offsets of the 8 (B <= 2^-7, FP32 2^-3.5) or 16 cells before it.
+//
+// The fields are read from one set of arrays and written to another, so every
+// tile sees the old values whatever the others have done; qv, qc and qr may
+// still lack the rescaling of NegativeValueProcess, which is then applied as
+// they are read (no pass of its own). Ghost cells are copied.
+//
+// One warp a tile of tr rows by 108 owned columns (27 lanes of 4 cells; four
+// halo lanes on the left, one on the right for the explicit terms), for zeta
+// and pairs of scalars (which share the coefficients: least work), or for one
+// field (shorter rows: least time where the grid has few tiles). Rows arrive
+// by cp.async kGWDepth ahead, each lane reading back only what it copied, so
+// no barrier is needed. Bound by the instruction issue of the few warps a
+// scheduler holds (about 350 instructions a row of a pair, 220 of a field, ~4
+// cycles each at one warp a scheduler). Measured at 2048 x 256 against the
+// three passes it replaces: 32 / 91 us FP64, 19 / 63 us FP32; 8192 x 256 FP64
+// 81 / 260, 128 x 64 12.6 / 81. A form that makes the rows' coefficients by
+// other warps first (shared memory, a barrier every 8 or 16 rows) took 34 us
+// and 90 us at the two large FP64 grids and 13.7 us at the small one.
+constexpr int kGWOwnLanes = 27, kGWLeft = 4, kGWOwn = 4 * kGWOwnLanes;
+constexpr int kGWRowsMax = 32, kGWHaloMax = 16, kGWDepth = 4, kGWWarps = 2;
+template <typename T>
+constexpr float kGWBits = sizeof(T) == 8 ? 56.f : 28.f;
+
+template <typename T>
+struct GSSweepArgs {
+    Dims d;
+    Consts c;
+    Profiles p;
+    const T* src[5];     // zeta, th, qv, qc, qr before the diffusion, ghosts included
+    T* dst[5];
+    const T *RKM, *RKH;
+    const double* nvp;   // rescaling of qv, qc, qr still to do (k_nvp_final's), or null
+    int nudge;           // fuse Nudge_theta (field 1) and Nudge_zeta (field 0)
+    int nb, nc, tr;      // bands of tr rows from k = 1, chunks of kGWOwn columns from i = 0
+    int jobs;            // 3: zeta; th, qv; qc, qr. 5: every field on its own
+    const unsigned* kmax;
+    float fz[2];         // largest C / K over the rows: Mparam, Hparam
+    GSTileCtl* ctl;      // more: the repeated passes are needed
+};
+
+template <typename T>
+struct GSSweepShared {
+    T ring[kGWDepth][4][128];            // K, then the job's fields (a power of two a slot)
+    T row[kGWRowsMax + kGWHaloMax][8];   // per row: lower and upper factors, nudging (dn, tn), profile differences
+};
+
+// The rescaling of field f (2, 3, 4): nvp_apply's with its factor taken as 1
+// where it does not rescale.
+__device__ __forceinline__ double gs_factor(const double* nvp, int f) {
+    return nvp[2 * (f - 2)] != 0.0 ? nvp[2 * (f - 2) + 1] : 1.0;
+}
+template <typename T>
+__device__ __forceinline__ T gs_finish(T fac, T v) { return v >= T(0) ? v * fac : T(0); }
+
+// The tile's constants and rolling windows; one lane's part of a row is its
+// four cells.
+template <typename T, bool MOM, int NF>
+struct GSSweepTile {
+    static constexpr int D = kGWDepth;
+    int i0, NX, f0, lane;
+    bool act, edge, own, wide;
+    size_t pitch;
+    const T* from[1 + NF];   // the next row to copy: K, then the fields
+    T* to[NF];               // the next row to store
+    T fac[NF];               // rescaling of each field (gs_factor)
+    bool fin[NF];            // it is still to do
+    T cx;
+    T Kp[4], Kc[4], lo[4], v0[NF][4], below[NF][4], klp;
+
+    __device__ __forceinline__ T* slot(GSSweepShared<T>& S, int q, int arr) const {
+        return &S.ring[q][arr][sizeof(T) == 8 ? 2 * lane : 4 * lane];
+    }
+    // copies the next row of K and the fields into slot q
+    __device__ __forceinline__ void issue(GSSweepShared<T>& S, int q, bool on) {
+        if (act && on) {
+#pragma unroll
+            for (int arr = 0; arr <= NF; arr++) {
+                T* dst = slot(S, q, arr);
+                cp_async16(dst, from[arr]);
+                if constexpr (sizeof(T) == 8) cp_async16(dst + 64, from[arr] + 2);
+                from[arr] += pitch;
+            }
+        }
+        cp_async_commit();
+    }
+    __device__ __forceinline__ static void read4(const T* s, T (&x)[4]) {
+        if constexpr (sizeof(T) == 8) {
+            const double2 u = *reinterpret_cast<const double2*>(s), w = *reinterpret_cast<const double2*>(s + 64);
+            x[0] = u.x, x[1] = u.y, x[2] = w.x, x[3] = w.y;
+        } else {
+            const float4 u = *reinterpret_cast<const float4*>(s);
+            x[0] = u.x, x[1] = u.y, x[2] = u.z, x[3] = u.w;
+        }
+    }
+    // the row in slot q (level k), finished; then the slot's next row
+    __device__ __forceinline__ void take(GSSweepShared<T>& S, const GSSweepArgs<T>& a, int q, int k, bool more, T (&Kx)[4],
+                                         T (&vx)[NF][4]) {
+        cp_async_wait<D - 1>();
+        read4(slot(S, q, 0), Kx);
+#pragma unroll
+        for (int f = 0; f < NF; f++) {
+            read4(slot(S, q, 1 + f), vx[f]);
+            if (!MOM && fin[f]) {
+                const bool full = kPert<T> && f0 + f == 2;
+                const double ref = full ? a.p.ref[1][k] : 0.0, fd = full ? gs_factor(a.nvp, 2) : 0.0;
+#pragma unroll
+                for (int e = 0; e < 4; e++)
+                    vx[f][e] = full ? T(gs_finish(fd, ref + (double)vx[f][e]) - ref) : gs_finish(fac[f], vx[f][e]);
+            }
+        }
+        issue(S, q, more);
+    }
+    __device__ __forceinline__ void store4(int f, const T (&x)[4]) const {
+        if constexpr (sizeof(T) == 8) {
+            *reinterpret_cast<double2*>(to[f]) = make_double2(x[0], x[1]);
+            *reinterpret_cast<double2*>(to[f] + 2) = make_double2(x[2], x[3]);
+        } else {
+            *reinterpret_cast<float4*>(to[f]) = make_float4(x[0], x[1], x[2], x[3]);
+        }
+    }
+
+    // Row k: its K above (Ku) and fields above (vu) arrive, its results go to
+    // `below` and, when asked for, to memory; the windows move up a row.
+    __device__ __forceinline__ void row(const T* rv, const T (&Ku)[4], const T (&vu)[NF][4], bool store) {
+        const T fd = rv[0], fu = rv[1];
+        // left, right, lower and upper coefficients (Turbulent.cpp:83-88, :107-112)
+        T B[4], R[4], C[4], U[4];
+        const T kl = __shfl_up_sync(0xffffffffu, Kc[3], 1);
+        if constexpr (MOM) {
+            T g = kl + klp;
+#pragma unroll
+            for (int e = 0; e < 4; e++) {
+                const T up = Kc[e] + (e ? Kc[e - 1] : kl);
+                B[e] = cx * g;
+                g = Kc[e] + Kp[e];
+                R[e] = cx * g;
+                C[e] = fd * lo[e];
+                U[e] = fu * up;
+                lo[e] = up;
+            }
+            klp = kl;
+        } else {
+            const T kr = __shfl_down_sync(0xffffffffu, Kc[0], 1);
+            T g = Kc[0] + kl;
+#pragma unroll
+            for (int e = 0; e < 4; e++) {
+                const T up = Ku[e] + Kc[e];
+                B[e] = cx * g;
+                g = (e < 3 ? Kc[e + 1] : kr) + Kc[e];
+                R[e] = cx * g;
+                C[e] = fd * lo[e];
+                U[e] = fu * up;
+                lo[e] = up;
+            }
+        }
+        if (edge) {   // ghosts and padding keep their values
+#pragma unroll
+            for (int e = 0; e < 4; e++)
+                if (i0 + e < 1 || i0 + e > NX) B[e] = R[e] = C[e] = U[e] = T(0);
+        }
+        const T M = (B[0] * B[1]) * (B[2] * B[3]);
+        T M2 = T(0);
+        if (wide) M2 = M * __shfl_up_sync(0xffffffffu, M, 1);
+#pragma unroll
+        for (int f = 0; f < NF; f++) {
+            const T vr = __shfl_down_sync(0xffffffffu, v0[f][0], 1);
+            // y itself, A0 + C y_below + B y_left, added up in the passes'
+            // order; in FP32 zeta's increment y - v, whose terms are all
+            // small beside v: one rounding at v's size a step, not four.
+            constexpr bool kInc = kPert<T> && MOM;
+            T vl = T(0);
+            if constexpr (kInc) vl = __shfl_up_sync(0xffffffffu, v0[f][3], 1);
+            T x[4];
+#pragma unroll
+            for (int e = 0; e < 4; e++) {
+                const T v = v0[f][e], right = e < 3 ? v0[f][e + 1] : vr;
+                T du = vu[f][e] - v, dd = v;
+                if (kPert<T> && !MOM && f0 + f <= 2) {   // th', qv' about a profile
+                    du += rv[5 + 2 * f];
+                    dd += rv[4 + 2 * f];
+                }
+                if constexpr (kInc)
+                    x[e] = (R[e] * (right - v) + B[e] * ((e ? v0[f][e - 1] : vl) - v)) + (U[e] * du + C[e] * (below[f][e] - dd));
+                else
+                    x[e] = v + (R[e] * (right - v) - B[e] * v) + (U[e] * du - C[e] * dd) + C[e] * below[f][e];
+            }
+            // the lane's offset with no inflow, then the lanes' before it
+            T P = ((x[0] * B[1] + x[1]) * B[2] + x[2]) * B[3] + x[3];
+            T q = __shfl_up_sync(0xffffffffu, P, 1);
+            if (lane >= 1) P += M * q;
+            if (wide) {
+                q = __shfl_up_sync(0xffffffffu, P, 2);
+                if (lane >= 2) P += M2 * q;
+            }
+            T y = __shfl_up_sync(0xffffffffu, P, 1);
+            if (lane == 0) y = kInc ? T(0) : v0[f][0];
+            T out[4];
+#pragma unroll
+            for (int e = 0; e < 4; e++) {
+                y = x[e] + B[e] * y;
+                out[e] = kInc ? v0[f][e] + y : y;
+                below[f][e] = out[e];
+            }
+            if ((MOM || (f == 0 && f0 == 1)) && rv[2] != T(0)) {   // Nudge_zeta, Nudge_theta
+#pragma unroll
+                for (int e = 0; e < 4; e++)
+                    if (i0 + e >= 1 && i0 + e <= NX) out[e] = out[e] - rv[2] * (out[e] - rv[3]);
+            }
+            if (store) {
+                if (own) store4(f, out);
+                to[f] += pitch;
+            }
+#pragma unroll
+            for (int e = 0; e < 4; e++) v0[f][e] = vu[f][e];
+        }
+#pragma unroll
+        for (int e = 0; e < 4; e++) {
+            Kp[e] = Kc[e];
+            Kc[e] = Ku[e];
+        }
+    }
+};
+
+template <typename T, bool MOM, int NF>
+__device__ __forceinline__ void gs_sweep_tile(const GSSweepArgs<T>& a, GSSweepShared<T>& S, int f0, int b, int c, int hz,
+                                              bool wide) {
+    constexpr int D = kGWDepth;
+    const Dims& d = a.d;
+    const int kend = d.nz - 2;
+    const int k0 = 1 + b * a.tr, kl = min(k0 + a.tr - 1, kend), ks = max(1, k0 - hz);
+    GSSweepTile<T, MOM, NF> t;
+    t.lane = threadIdx.x & 31;
+    t.f0 = f0;
+    t.NX = d.nx - 2;
+    t.pitch = d.pitch;
+    t.i0 = c * kGWOwn + 4 * (t.lane - kGWLeft);
+    t.act = t.i0 >= 0 && t.i0 < d.pitch;
+    t.edge = t.i0 < 1 || t.i0 + 3 > t.NX;
+    t.own = t.act && t.lane >= kGWLeft && t.lane < kGWLeft + kGWOwnLanes;
+    t.wide = wide;
+    t.cx = T(0.5) * T(a.c.rdx2 * a.c.dt);
+    t.from[0] = (MOM ? a.RKM : a.RKH) + d.at(t.i0, ks - 1);
+#pragma unroll
+    for (int f = 0; f < NF; f++) {
+        t.from[1 + f] = a.src[f0 + f] + d.at(t.i0, ks - 1);
+        t.to[f] = a.dst[f0 + f] + d.at(t.i0, k0);
+        t.fin[f] = !MOM && a.nvp && f0 + f >= 2;
+        t.fac[f] = t.fin[f] ? T(gs_factor(a.nvp, f0 + f)) : T(1);
+    }
+    if (!t.act) {   // lanes outside the array: zeros
+        for (int q = 0; q < D; q++)
+            for (int arr = 0; arr <= NF; arr++)
+                for (int e = 0; e < (sizeof(T) == 8 ? 2 : 4); e++) {
+                    t.slot(S, q, arr)[e] = T(0);
+                    if (sizeof(T) == 8) t.slot(S, q, arr)[64 + e] = T(0);
+                }
+    }
+    const int n = kl - ks + 3;   // rows to copy: ks-1 .. kl+1
+#pragma unroll
+    for (int q = 0; q < D; q++) t.issue(S, q, q < n);
+    for (int r = t.lane; r <= kl - ks; r += 32) {   // the rows' scalars
+        const int k = ks + r;
+        T* rv = S.row[r];
+        const T cz = MOM ? T(a.p.gsM_cz[k]) : T(a.p.gsS_cz[k]);
+        rv[0] = cz * (T(0.5) * (MOM ? T(a.p.gsM_rhod[k]) : T(a.p.gsS_rhod[k])));
+        rv[1] = cz * (T(0.5) * (MOM ? T(a.p.rhou[k]) : T(a.p.rhow[k + 1])));
+        T dn = T(0), tn = T(0);   // out = y - dn (y - tn)
+        if (a.nudge && f0 == 0) dn = T(a.p.dtcgr_zeta[k]);
+        if (a.nudge && f0 == 1) {
+            dn = T(a.p.dtcgr_th[k]);
+            tn = kPert<T> ? T(-a.p.dn[0][k]) : T(a.p.thb_init[k]);
+        }
+        rv[2] = dn;
+        rv[3] = tn;
+        if (kPert<T> && !MOM) {   // th', qv': their profiles' differences
+#pragma unroll
+            for (int f = 0; f < NF; f++)
+                if (f0 + f <= 2) {
+                    rv[4 + 2 * f] = T(a.p.d0[f0 + f - 1][k]);
+                    rv[5 + 2 * f] = T(a.p.d0[f0 + f - 1][k + 1]);
+                }
+        }
+    }
+    __syncwarp();
+    t.take(S, a, 0, ks - 1, D < n, t.Kp, t.below);
+    if (ks == 1 && t.own) {   // the ghost row under the grid
+#pragma unroll
+        for (int f = 0; f < NF; f++) {
+            t.to[f] -= t.pitch;
+            t.store4(f, t.below[f]);
+            t.to[f] += t.pitch;
+        }
+    }
+    t.take(S, a, 1, ks, D + 1 < n, t.Kc, t.v0);
+    t.klp = T(0);
+    if constexpr (MOM) {
+        t.klp = __shfl_up_sync(0xffffffffu, t.Kp[3], 1);
+        t.lo[0] = t.Kp[0] + t.klp;
+#pragma unroll
+        for (int e = 1; e < 4; e++) t.lo[e] = t.Kp[e] + t.Kp[e - 1];
+    } else {
+#pragma unroll
+        for (int e = 0; e < 4; e++) t.lo[e] = t.Kc[e] + t.Kp[e];
+    }
+    // not unrolled: a tile runs few rows, and fetching four times the code
+    // costs more than the moves it would save (13 rows: 14.8 against 12.6 us)
+    int q = 2;
+#pragma unroll 1
+    for (int k = ks; k <= kl; k++) {
+        T Ku[4], vu[NF][4];
+        t.take(S, a, q, k + 1, k + D < kl + 1, Ku, vu);
+        q = (q + 1) & (D - 1);
+        t.row(S.row[k - ks], Ku, vu, k >= k0);
+    }
+    if (kl == kend && t.own) {   // the ghost row over the grid
+#pragma unroll
+        for (int f = 0; f < NF; f++) t.store4(f, t.v0[f]);
+    }
+    cp_async_wait<0>();
+}
+
+template <typename T>
+__device__ __forceinline__ void k_gs_sweep_body(const GSSweepArgs<T>& a, cudaGraphConditionalHandle h) {
+    __shared__ __align__(16) GSSweepShared<T> S[kGWWarps];
+    const float cx = (float)(a.c.rdx2 * a.c.dt);
+    const float km = __uint_as_float(a.kmax[0]), kh = __uint_as_float(a.kmax[1]);
+    // bits an inflow error loses a cell, with a little to spare for the roundings here
+    const float l = -log2f(1.001f * fmaxf(km * (cx + a.fz[0]), kh * (cx + a.fz[1])));
+    const float lx = -log2f(1.001f * cx * fmaxf(km, kh));
+    const int hz = max(1, (int)ceilf(kGWBits<T> / l) - 1);
+    const bool ok = km == km && kh == kh && l > 0.f && hz <= kGWHaloMax && 16.f * lx >= kGWBits<T>;
+    if (threadIdx.x == 0 && blockIdx.x == 0 && blockIdx.y == 0) {
+        a.ctl->more = ok ? 0 : 1;
+        if (h) cudaGraphSetConditional(h, ok ? 0u : 1u);
+    }
+    if (!ok) return;
+    const int wid = threadIdx.x >> 5;
+    const int tile = blockIdx.x * kGWWarps + wid;
+    if (tile >= a.jobs * a.nb * a.nc) return;
+    const int c = tile % a.nc, b = (tile / a.nc) % a.nb, job = tile / (a.nc * a.nb);
+    const bool wide = 8.f * lx < kGWBits<T>;
+    if (job == 0) gs_sweep_tile<T, true, 1>(a, S[wid], 0, b, c, hz, wide);
+    else if (a.jobs == 3) gs_sweep_tile<T, false, 2>(a, S[wid], 2 * job - 1, b, c, hz, wide);
+    else gs_sweep_tile<T, false, 1>(a, S[wid], job, b, c, hz, wide);
+}
+template <typename T>
+__global__ void __launch_bounds__(32 * kGWWarps) k_gs_sweep(GSSweepArgs<T> a, cudaGraphConditionalHandle h) { k_gs_sweep_body<T>(a, h); }
+
+// The inputs of the repeated passes, which run in place: src, finished, copied
+// to dst (ghosts too). Nothing to do once a sweep's passes have begun.
+template <typename T>
+__device__ __forceinline__ void k_gs_inputs_body(const GSSweepArgs<T>& a) {
+    if (a.ctl->pass != 0) return;
+    const Dims& d = a.d;
+    const int i = blockIdx.x * blockDim.x + threadIdx.x, k = blockIdx.y * blockDim.y + threadIdx.y;
+    if (i >= d.nx || k >= d.nz) return;
+    const size_t id = d.at(i, k);
+#pragma unroll
+    for (int f = 0; f < 5; f++) {
+        T v = a.src[f][id];
+        if (a.nvp && f >= 2) {
+            if (kPert<T> && f == 2) v = T(gs_finish(gs_factor(a.nvp, 2), a.p.ref[1][k] + (double)v) - a.p.ref[1][k]);
+            else v = gs_finish(T(gs_factor(a.nvp, f)), v);
+        }
+        a.dst[f][id] = v;
+    }
+}
+template <typename T>
+__global__ void k_gs_inputs(GSSweepArgs<T> a) { k_gs_inputs_body<T>(a); }
 
 // ---------------------------------------------------------------------------
 // The second schedule of the same recurrence: one thread-block cluster a field.
@@ -1800,6 +2210,7 @@ struct MeanArgs {
     double *thb, *qvb, *thvb;
     double* ubar;   // [0] ubarTop, [1] ubarTopp
     int rotate_ubar;
+    unsigned* kmax;   // [2]: cleared for the next step's k_rkm_rkh (may be null)
 };
 
 template <typename T>
@@ -1824,6 +2235,7 @@ __device__ __forceinline__ void k_update_mean_body(const MeanArgs<T>& a) {
         if (k == 1) { a.thb[0] = tb; a.qvb[0] = qb; a.thvb[0] = tv; }
         if (k == d.nz - 2) { a.thb[d.nz - 1] = tb; a.qvb[d.nz - 1] = qb; a.thvb[d.nz - 1] = tv; }
         if (k == 1 && a.rotate_ubar) a.ubar[0] = a.ubar[1];
+        if (k == 1 && a.kmax) a.kmax[0] = a.kmax[1] = 0u;
     }
 }
 template <typename T>

@@ -454,20 +454,19 @@ struct Timed {
 //
 // A batch steps the cases of one shape as grouped launches (grouped.cuh).
 // To build them, each case's step is first recorded instead of issued: the
-// kernels with their launch shapes and argument packs, the clears of small
-// control blocks, and the graph loops with the points where a case decides
-// whether its loop goes on (its flag, an int in device memory). The batch
+// kernels with their launch shapes and argument packs, and the graph loops with
+// the points where a case decides whether its loop goes on (its flag, an int
+// in device memory). The batch
 // then checks that the recordings of a group agree op for op and replays
 // them side by side.
 struct RecOp {
-    enum Kind { KERNEL, ZERO, COND_NEXT, COND_LOOP, LOOP_BEGIN, LOOP_END } kind = KERNEL;
+    enum Kind { KERNEL, COND_NEXT, COND_LOOP, LOOP_BEGIN, LOOP_END } kind = KERNEL;
     const void* fn = nullptr;           // KERNEL: the grouped kernel
     dim3 grid, block;
     size_t smem = 0;
     std::vector<unsigned char> pack;    // KERNEL: this case's arguments
     size_t align = 16;
-    void* ptr = nullptr;                // ZERO: what to clear; COND_*: the case's loop flag (int)
-    size_t bytes = 0;                   // ZERO
+    void* ptr = nullptr;                // COND_*: the case's loop flag (int)
 };
 struct Recorder {
     std::vector<RecOp> ops;
@@ -507,19 +506,6 @@ void klaunch(Stats* s, int id, cudaStream_t st, void (*k)(A...), dim3 g, dim3 b,
     }
     LAUNCH(s, id, st, k<<<g, b, smem, st>>>(args...));
     CKL();
-}
-
-// cudaMemsetAsync(p, 0, bytes, st), or its record.
-inline void zero_async(Stats* s, void* p, size_t bytes, cudaStream_t st) {
-    if (s && s->rec) {
-        RecOp op;
-        op.kind = RecOp::ZERO;
-        op.ptr = p;
-        op.bytes = bytes;
-        s->rec->ops.push_back(std::move(op));
-        return;
-    }
-    CK(cudaMemsetAsync(p, 0, bytes, st));
 }
 
 // Marks where a case has decided whether a graph loop runs (another) pass:
@@ -1546,6 +1532,7 @@ template <typename T>
 struct Fields {
     T *zeta[2] = {}, *th[2] = {}, *qv[2] = {}, *qc[2] = {}, *qr[2] = {};
     T *u = nullptr, *w = nullptr, *RKM = nullptr, *RKH = nullptr;
+    T* pre[5] = {};   // zeta, th, qv, qc, qr as the diffusion reads them (it writes the future level)
     T* hist[NHIST][2] = {};
     T *d_auto = nullptr, *d_accr = nullptr, *d_evap = nullptr, *d_cond = nullptr;
     T *precip = nullptr, *th_forcing = nullptr;
@@ -1569,6 +1556,12 @@ struct vvm_gpu_ctx {
     bool spectral = false;   // VVM_SOLVER_SPECTRAL
     int tune_gs_tr = 0;      // rows of a Gauss-Seidel tile (0: automatic)
     GSTileCtl* gsctl = nullptr;   // pass state of the Gauss-Seidel tiles
+    unsigned* kmax = nullptr;     // [2]: largest RKM, RKH of the step (k_rkm_rkh)
+    float gs_fz[2] = {};          // largest lower coefficient per K: Mparam, Hparam
+    // a whole step runs: zeta, th, qv, qc, qr go to Fields::pre on their way
+    // to the diffusion, which writes the future level (routine calls keep
+    // them in the future level throughout)
+    bool in_step = false;
     int* sc_host_i = nullptr;     // pinned: the tiles' "another pass" flag read by the host loop
     // learned preconditioner (VVM_SOLVER_LEARNED)
     std::unique_ptr<LearnedNet> net;
@@ -1743,6 +1736,8 @@ void alloc_fields(vvm_gpu_ctx* c) {
     F.w = c->ar.alloc<T>(n);
     F.RKM = c->ar.alloc<T>(n);
     F.RKH = c->ar.alloc<T>(n);
+    F.pre[0] = c->ar.alloc<T>(5 * n);
+    for (int f = 1; f < 5; f++) F.pre[f] = F.pre[0] + f * n;
     for (int h = 0; h < NHIST; h++)
         for (int s = 0; s < 2; s++) F.hist[h][s] = c->ar.alloc<T>(n);
     F.d_auto = c->ar.alloc<T>(n);
@@ -1757,18 +1752,26 @@ void alloc_fields(vvm_gpu_ctx* c) {
     F.gsRight = c->ar.alloc<T>(2 * 5 * nc * (rows + kGSTileRowsMax));
     F.gsTop = c->ar.alloc<T>(2 * 5 * nc * (size_t)cdiv((int)rows, kGSTileRowsMin) * kGTCols);
     if (!c->gsctl) c->gsctl = c->ar.alloc<GSTileCtl>(1);
+    if (!c->kmax) c->kmax = c->ar.alloc<unsigned>(2);
     if (!c->sc_host_i) CK(cudaMallocHost(&c->sc_host_i, sizeof(int)));
 }
 
 // ---------------------------------------------------------------- routines
 
+// The vorticity between its advection and its diffusion.
+template <typename T>
+T* zeta_pre(vvm_gpu_ctx* c) {
+    Fields<T>& F = fields<T>(c);
+    return c->in_step ? F.pre[0] : F.zeta[1 - c->cur];
+}
+
 template <typename T>
 void launch_pzeta(vvm_gpu_ctx* c) {
     Fields<T>& F = fields<T>(c);
-    int now = c->cur, fut = 1 - c->cur;
+    int now = c->cur;
     AB2 ab = AB2::of(c->step);
     PZetaArgs<T> a{c->d, c->c, c->profiles(), F.zeta[now], F.u, F.w, F.th[now], F.qv[now], F.qc[now], F.qr[now],
-                   F.zeta[fut], F.hist[H_ZETA][ab.sn], F.hist[H_ZETA][ab.so], F.hist[H_BUOY][ab.sn],
+                   zeta_pre<T>(c), F.hist[H_ZETA][ab.sn], F.hist[H_ZETA][ab.so], F.hist[H_BUOY][ab.sn],
                    F.hist[H_BUOY][ab.so], ab};
     dim3 g(cdiv(c->d.nx - 2, kPZBX), cdiv(c->d.nz - 3, kPZBZ));
     klaunch<k_pzeta_body<T>, kPZBX * kPZBZ>(&c->stats, VVM_K_PZETA, c->stream, k_pzeta<T>, g, dim3(kPZBX, kPZBZ), 0, a);
@@ -1863,16 +1866,21 @@ void launch_pubartop(vvm_gpu_ctx* c) {
     klaunch<k_pubartop_body<T>, 1024>(&c->stats, VVM_K_PUBAR, c->stream, k_pubartop<T>, dim3(1), dim3(1024), 0, a);
 }
 
-// finish_advection: the step's own sequence, where the finish of the
-// advection (k_apply's NVP rescaling and AddForcing of th, qv, qc, qr, whose
-// NVP sums k_padv left) is applied as Kessler reads each value.
+// In a whole step the finish of the advection (k_apply's NVP rescaling and
+// AddForcing of th, qv, qc, qr, whose NVP sums k_padv left) is applied as
+// Kessler reads each value, and the finish of Kessler (the rescaling of qv, qc,
+// qr) as the diffusion reads them: two passes over four fields less, and the
+// ghost images are written by Kessler itself.
 template <typename T>
-void launch_kessler(vvm_gpu_ctx* c, bool halo, bool finish_advection = false) {
+void launch_kessler(vvm_gpu_ctx* c) {
     Fields<T>& F = fields<T>(c);
     int fut = 1 - c->cur;
     KesslerArgs<T> a{c->d, c->c, c->profiles(), F.th[fut], F.qv[fut], F.qc[fut], F.qr[fut],
+                     {F.th[fut], F.qv[fut], F.qc[fut], F.qr[fut]}, 0,
                      F.d_auto, F.d_accr, F.d_evap, F.d_cond, c->partial, 1};
-    if (finish_advection) {
+    if (c->in_step) {
+        for (int f = 0; f < 4; f++) a.out[f] = F.pre[1 + f];
+        a.halo = 1;
         a.do_pre = 1;
         a.pre.nvp = c->nvp;
         a.pre.th_forcing = F.th_forcing;
@@ -1885,7 +1893,7 @@ void launch_kessler(vvm_gpu_ctx* c, bool halo, bool finish_advection = false) {
     klaunch<k_kessler_body<T>, 256>(&c->stats, VVM_K_KESSLER, c->stream, k_kessler<T>, g, c->blk(), 0, a);
     klaunch<k_nvp_final_body, 1024>(&c->stats, VVM_K_APPLY, c->stream, k_nvp_final, dim3(1), dim3(1024), 0,
                                     (const double*)c->partial, (int)(g.x * g.y), c->nvp);
-    launch_apply<T>(c, halo ? (F_TH | F_QV | F_QC | F_QR) : (F_QV | F_QC | F_QR), F_QV | F_QC | F_QR, false, halo);
+    if (!c->in_step) launch_apply<T>(c, F_QV | F_QC | F_QR, F_QV | F_QC | F_QR, false, false);
 }
 
 cudaGraphConditionalHandle new_handle(cudaStream_t st) {
@@ -2057,69 +2065,119 @@ void launch_gs_cluster(vvm_gpu_ctx* c, GSArgs<T> g) {
     CKL();
 }
 
-// Later Gauss-Seidel passes a step graph runs before its WHILE node (the
-// typical sweep is pass 1 and two more).
-constexpr int kGSGraphPasses = 2;
-// The Gauss-Seidel schedule: kGSSchedCluster (one cluster a field) or a tile
-// height. Automatic: tiles of 16 rows in FP64, 8 in FP32 (the fastest at
-// 2048 x 256 on a B200: FP64 0.365 / 0.376 ms a step with 16 / 8 rows, FP32
-// 0.305 / 0.301 ms); a batch's autotuner also tries the cluster schedule.
+// The Gauss-Seidel schedule: the single pass (k_gs_sweep), with the repeated
+// passes over tiles where its coefficients are too large; the tuning knob sets
+// those tiles' rows (automatic: 16 in FP64, 8 in FP32, the fastest at 2048 x
+// 256), or kGSSchedCluster for one cluster a field.
 constexpr int kGSSchedCluster = 1;
 inline int gs_tile_rows(const vvm_gpu_ctx* c) {
     return c->tune_gs_tr ? c->tune_gs_tr : (c->mixed ? kGSTileRowsDefault : 2 * kGSTileRowsDefault);
 }
 inline bool gs_schedule_ok(int v) { return v == 0 || v == kGSSchedCluster || gs_tile_rows_ok(v); }
+// Rows and jobs of a single-pass tile: the grid and the precision alone decide,
+// so a case alone and in a batch computes the same bits. Tall tiles repeat
+// fewer halo rows, short ones of single fields finish sooner: the tallest that
+// still gives every SM about four warps (FP32, whose rows are cheaper, eight),
+// us a sweep with 8 rows of a field / 8, 16, 32 rows of pairs: 128 x 64 FP64
+// 12.7 / 16.7, 22.9, 34.2; 1024 x 128 16.7 / 18.8, 22.9, 35.1; 2048 x 256
+// 39.8 / 37.2, 32.6, 39.3 (FP32 18.7 / 18.8, 22.8, 34.6); 8192 x 256 116 /
+// 105, 88, 82 (FP32 45.9 / 42.3, 37.2, 42.9).
+struct GSSweepShape {
+    int tr, jobs;
+};
+inline GSSweepShape gs_sweep_shape(const Dims& d, bool mixed) {
+    const int nc = cdiv(d.nx, kGWOwn), want = (mixed ? 8 : 4) * 148;
+    for (int tr : {32, 16, 8})
+        if (3 * nc * cdiv(d.nz - 2, tr) >= want) return {tr, 3};
+    return {8, 5};
+}
 
 template <typename T>
 void launch_turbulence(vvm_gpu_ctx* c, bool nudge, long long* recorded_in_loops = nullptr) {
     Fields<T>& F = fields<T>(c);
     int fut = 1 - c->cur;
-    RKArgs<T> r{c->d, c->c, c->profiles(), F.u, F.w, F.th[fut], F.RKM, F.RKH};
-    klaunch<k_rkm_rkh_body<T>, 256>(&c->stats, VVM_K_RKM, c->stream, k_rkm_rkh<T>, c->grid_interior(1), c->blk(), 0, r);
-    GSArgs<T> g{c->d, c->c, c->profiles(), {F.zeta[fut], F.th[fut], F.qv[fut], F.qc[fut], F.qr[fut]},
-                F.RKM, F.RKH, 0x1f, nudge ? 1 : 0, F.gsA, nullptr, nullptr, nullptr};
-    if (c->tune_gs_tr == kGSSchedCluster) {
-        launch_gs_cluster<T>(c, g);
-        return;
+    cudaStream_t st = c->stream;
+    T* v[5] = {F.zeta[fut], F.th[fut], F.qv[fut], F.qc[fut], F.qr[fut]};
+    RKArgs<T> r{c->d, c->c, c->profiles(), F.u, F.w, c->in_step ? F.pre[1] : v[1], F.RKM, F.RKH, c->kmax};
+    if (!recorded_in_loops) {   // a graph's steps leave both as they found them
+        CK(cudaMemsetAsync(c->kmax, 0, 2 * sizeof(unsigned), st));
+        CK(cudaMemsetAsync(c->gsctl, 0, sizeof(GSTileCtl), st));
     }
-    // the recurrence: tiles and passes (see k_gs_tiles)
+    if (!c->in_step) {   // a routine call: the fields lie in the future level
+        for (int f = 0; f < 5; f++)
+            CK(cudaMemcpyAsync(F.pre[f], v[f], c->d.cells() * sizeof(T), cudaMemcpyDeviceToDevice, st));
+    }
+    klaunch<k_rkm_rkh_body<T>, 256>(&c->stats, VVM_K_RKM, st, k_rkm_rkh<T>, c->grid_interior(1), c->blk(), 0, r);
+    GSSweepArgs<T> w{};
+    w.d = c->d;
+    w.c = c->c;
+    w.p = c->profiles();
+    for (int f = 0; f < 5; f++) {
+        w.src[f] = F.pre[f];
+        w.dst[f] = v[f];
+    }
+    w.RKM = F.RKM;
+    w.RKH = F.RKH;
+    w.nvp = c->in_step ? c->nvp : nullptr;
+    w.nudge = nudge ? 1 : 0;
+    const GSSweepShape shape = gs_sweep_shape(c->d, c->mixed);
+    w.tr = shape.tr;
+    w.jobs = shape.jobs;
+    w.nb = cdiv(c->d.nz - 2, w.tr);
+    w.nc = cdiv(c->d.nx, kGWOwn);
+    w.kmax = c->kmax;
+    w.fz[0] = c->gs_fz[0];
+    w.fz[1] = c->gs_fz[1];
+    w.ctl = c->gsctl;
+    GSArgs<T> g{c->d, c->c, c->profiles(), {v[0], v[1], v[2], v[3], v[4]},
+                F.RKM, F.RKH, 0x1f, nudge ? 1 : 0, F.gsA, nullptr, nullptr, nullptr};
+    // the repeated passes: tiles of tr rows (see k_gs_tiles)
     const int tr = gs_tile_rows(c);
     const int nb = cdiv(c->d.nz - 2, tr), nc = cdiv(c->d.pitch, kGTCols);
     GSTileArgs<T> t{nb, nc, tr, F.gsRight, F.gsTop, c->gsctl, recorded_in_loops ? c->d_exec : nullptr};
     const int tblocks = cdiv(5 * nb * nc, 4);
-    const int maxp = std::max(2, nb + nc - 1);
-    cudaStream_t st = c->stream;
-    zero_async(&c->stats, c->gsctl, sizeof(GSTileCtl), st);   // a fresh sweep
-    klaunch<k_gs_tiles_body<T, true>, 128, kGSTileMinBlocks<T>>(&c->stats, VVM_K_GS, st, k_gs_tiles<T, true>, dim3(tblocks), dim3(128), 0,
-                                              g, t, (cudaGraphConditionalHandle)0);   // pass 1
+    auto inputs = [&](cudaStream_t s) {
+        klaunch<k_gs_inputs_body<T>, 256>(&c->stats, VVM_K_GS, s, k_gs_inputs<T>, c->grid_all(), c->blk(), 0, w);
+    };
+    auto pass = [&](cudaStream_t s, auto first, cudaGraphConditionalHandle h) {
+        constexpr bool F1 = decltype(first)::value;
+        klaunch<k_gs_tiles_body<T, F1>, 128, kGSTileMinBlocks<T>>(&c->stats, VVM_K_GS, s, k_gs_tiles<T, F1>, dim3(tblocks),
+                                                                  dim3(128), 0, g, t, h);
+    };
+    if (c->tune_gs_tr == kGSSchedCluster) {
+        inputs(st);
+        launch_gs_cluster<T>(c, g);
+        return;
+    }
+    const cudaGraphConditionalHandle h = recorded_in_loops ? new_handle_reset(&c->stats, st) : 0;
+    klaunch<k_gs_sweep_body<T>, 32 * kGWWarps>(&c->stats, VVM_K_GS, st, k_gs_sweep<T>,
+                                               dim3(cdiv(w.jobs * w.nb * w.nc, kGWWarps)), dim3(32 * kGWWarps), 0, w, h);
     if (recorded_in_loops) {
-        // graph capture: the typical passes 2..kGSGraphPasses+1 unconditionally
-        // (each returns at once if the sweep already converged, and the last
-        // block of each sets the condition below), then a WHILE node that runs
-        // further passes only when they are needed
-        const cudaGraphConditionalHandle h = new_handle_reset(&c->stats, st);
-        GSTileArgs<T> tu = t;
-        tu.exec = nullptr;   // counted with the graph's static kernels
-        for (int p = 0; p < kGSGraphPasses; p++)
-            klaunch<k_gs_tiles_body<T, false>, 128, kGSTileMinBlocks<T>>(&c->stats, VVM_K_GS, st, k_gs_tiles<T, false>, dim3(tblocks),
-                                                       dim3(128), 0, g, tu, h);
+        // graph capture: a WHILE node that the sweep's kernel opens only when
+        // the passes are needed; its body runs the first (inputs, pass 1)
+        // once and then a later pass each time round
         record_cond(&c->stats, &c->gsctl->more, true);
         cudaGraph_t body = add_while(&c->stats, st, h);
         BodyCapture bc(c->cap[0], body, &c->stats);
         const long long n0 = c->stats.launches;
-        klaunch<k_gs_tiles_body<T, false>, 128, kGSTileMinBlocks<T>>(&c->stats, VVM_K_GS, bc.s, k_gs_tiles<T, false>, dim3(tblocks),
-                                                   dim3(128), 0, g, t, h);
+        inputs(bc.s);
+        pass(bc.s, std::true_type{}, 0);
+        pass(bc.s, std::false_type{}, h);
         record_cond(&c->stats, &c->gsctl->more, false);
         bc.end();
         *recorded_in_loops += c->stats.launches - n0;
         return;
     }
-    for (int p = 2; p <= maxp; p++) {
-        LAUNCH(&c->stats, VVM_K_GS, st, k_gs_tiles<T, false><<<tblocks, 128, 0, st>>>(g, t, 0));
-        CKL();
+    const int maxp = std::max(2, nb + nc - 1);
+    for (int p = 1; p <= maxp; p++) {
         CK(cudaMemcpyAsync(c->sc_host_i, &c->gsctl->more, sizeof(int), cudaMemcpyDeviceToHost, st));
         CK(cudaStreamSynchronize(st));
         if (!*c->sc_host_i) break;
+        if (p == 1) {
+            inputs(st);
+            pass(st, std::true_type{}, 0);
+        }
+        pass(st, std::false_type{}, 0);
     }
 }
 
@@ -2139,7 +2197,7 @@ void launch_update_mean(vvm_gpu_ctx* c, bool rotate) {
     Fields<T>& F = fields<T>(c);
     int fut = 1 - c->cur;
     MeanArgs<T> a{c->d, c->offset_th(), c->offset_qv(), F.th[fut], F.qv[fut], c->thb, c->qvb, c->thvb,
-                  c->ubar, rotate ? 1 : 0};
+                  c->ubar, rotate ? 1 : 0, c->in_step ? c->kmax : nullptr};
     klaunch<k_update_mean_body<T>, 256>(&c->stats, VVM_K_MEAN, c->stream, k_update_mean<T>, dim3(c->d.nz - 2),
                                         dim3(256), 0, a);
 }
@@ -2552,13 +2610,12 @@ template <typename T>
 int launch_cal_w(vvm_gpu_ctx* c, long long* recorded_in_loops = nullptr, cudaEvent_t before_w = nullptr) {
     ensure_poisson(c);
     Fields<T>& F = fields<T>(c);
-    int fut = 1 - c->cur;
     int NX = c->d.nx - 2, NK = c->d.nz - 3;
     int pitch = c->pcg64->pitch;
     dim3 B(64, 4), G(cdiv(NX, 64), cdiv(NK, 4));
     klaunch<k_poisson_rhs_body<T>, 256>(&c->stats, VVM_K_POISSON_RHS, c->stream, k_poisson_rhs<T>, G, B, 0, c->d,
                                         c->c.dx, (const double*)c->rhow, (const double*)c->rwres,
-                                        (const T*)F.zeta[fut], c->Wf, pitch, c->wpartial, c->pcg64->arrive,
+                                        (const T*)zeta_pre<T>(c), c->Wf, pitch, c->wpartial, c->pcg64->arrive,
                                         c->pcg64->sc);   // sets sc->bb
     const bool warm = c->desc.warm_start != 0;
     const int maxit = c->desc.poisson_maxit > 0 ? c->desc.poisson_maxit : 200;
@@ -2599,8 +2656,7 @@ int launch_cal_w(vvm_gpu_ctx* c, long long* recorded_in_loops = nullptr, cudaEve
 template <typename T>
 void launch_cal_u(vvm_gpu_ctx* c) {
     Fields<T>& F = fields<T>(c);
-    int fut = 1 - c->cur;
-    CalUArgs<T> a{c->d, c->c, c->profiles(), F.u, F.w, F.zeta[fut], c->ubar};
+    CalUArgs<T> a{c->d, c->c, c->profiles(), F.u, F.w, zeta_pre<T>(c), c->ubar};
     klaunch<k_cal_u_columns_body<T>, 32 * kColSeg>(&c->stats, VVM_K_CAL_U, c->stream, k_cal_u_columns<T>,
                                                    dim3(cdiv(c->d.nx - 2, 32)), dim3(32 * kColSeg), 0, a);
 }
@@ -2636,10 +2692,9 @@ int launch_calpsiuw(vvm_gpu_ctx* c) {
     ensure_psi(c);
     PCG<double>& P = *c->pcg_psi;
     Fields<T>& F = fields<T>(c);
-    const int fut = 1 - c->cur;
     const int NX = c->d.nx - 2, NK = c->d.nz - 3, pitch = P.pitch;
     dim3 B(64, 4), G(cdiv(NX, 64), cdiv(NK, 4));
-    LAUNCH(&c->stats, VVM_K_POISSON_RHS, c->stream, k_psi_rhs<T><<<G, B, 0, c->stream>>>(c->d, c->c.dx, F.zeta[fut], c->psi_f, pitch, c->wpartial));
+    LAUNCH(&c->stats, VVM_K_POISSON_RHS, c->stream, k_psi_rhs<T><<<G, B, 0, c->stream>>>(c->d, c->c.dx, zeta_pre<T>(c), c->psi_f, pitch, c->wpartial));
     CKL();
     LAUNCH(&c->stats, VVM_K_CG, c->stream, k_cg_scalar<<<1, 1024, 0, c->stream>>>(c->wpartial, c->wnpart, P.sc, CG_SET_BB));
     CKL();
@@ -2688,6 +2743,10 @@ struct OnStream {   // issues a scope's launches on another stream
 template <typename T>
 int run_step(vvm_gpu_ctx* c, long long* recorded_in_loops = nullptr) {
     c->step++;                                                 // Iteration.cpp:246
+    struct InStep {
+        bool& f;
+        ~InStep() { f = false; }
+    } in_step{c->in_step = true};
     const bool sf = (c->desc.flags & VVM_FLAG_STREAMFUNCTION) != 0;
     // The step's kernels form two chains (in a captured step, two branches of
     // the graph; the results are those of the reference's order, since
@@ -2712,7 +2771,7 @@ int run_step(vvm_gpu_ctx* c, long long* recorded_in_loops = nullptr) {
             if (!sf) launch_pubartop<T>(c);                    // pubarTop_pt
             launch_padv<T>(c, F_TH | F_QV | F_QC | F_QR, F_QV | F_QC | F_QR, true, true);  // pth, pqv, pqc, pqr
             CK(cudaEventRecord(c->fork_ev[1], c->side));   // u and w read, ubarTopp written
-            launch_kessler<T>(c, true, true);                  // NVP + AddForcing, Kessler + NVP x3 + halos
+            launch_kessler<T>(c);                              // NVP + AddForcing, Kessler + NVP sums + halos
         }
         try {
             launch_pzeta<T>(c);                                // pzeta_pt
@@ -2741,7 +2800,7 @@ int run_step(vvm_gpu_ctx* c, long long* recorded_in_loops = nullptr) {
         // NVP and AddForcing of the advected fields run inside Kessler's
         // kernel (nothing before it reads th, qv, qc, qr; their halos come
         // after it)
-        launch_kessler<T>(c, true, true);
+        launch_kessler<T>(c);
     }
     // The first updateMean of the step (Iteration.cpp:408) only writes thb,
     // qvb, thvb, which nextTimeStep's updateMean overwrites before any read.
@@ -3021,13 +3080,12 @@ bool same_ops(const Recorder& a, const Recorder& b) {
              x.block.x != y.block.x || x.block.y != y.block.y || x.block.z != y.block.z || x.smem != y.smem ||
              x.pack.size() != y.pack.size()))
             return false;
-        if (x.kind == RecOp::ZERO && x.bytes != y.bytes) return false;
     }
     return true;
 }
 
 // The device arrays of one group's replay: per kernel op the n argument
-// packs, per clear the n targets, per condition point the n flags.
+// packs, per condition point the n flags.
 struct GroupArrays {
     std::vector<size_t> off;   // per op: offset of its array in the blob
     std::vector<unsigned char> host;
@@ -3051,7 +3109,7 @@ GroupArrays group_arrays(const std::vector<Recorder>& recs) {
         if (op.kind == RecOp::KERNEL) {
             stride[j] = op.pack.size();   // sizeof the pack: the kernel indexes packs[blockIdx.z]
             A.off[j] = place(stride[j] * n);
-        } else if (op.kind == RecOp::ZERO || op.kind == RecOp::COND_NEXT || op.kind == RecOp::COND_LOOP) {
+        } else if (op.kind == RecOp::COND_NEXT || op.kind == RecOp::COND_LOOP) {
             A.off[j] = place(sizeof(void*) * n);
         }
     }
@@ -3061,7 +3119,7 @@ GroupArrays group_arrays(const std::vector<Recorder>& recs) {
         for (size_t i = 0; i < n; i++) {
             const RecOp& op = recs[i].ops[j];
             if (k == RecOp::KERNEL) memcpy(&A.host[A.off[j] + i * stride[j]], op.pack.data(), op.pack.size());
-            else if (k == RecOp::ZERO || k == RecOp::COND_NEXT || k == RecOp::COND_LOOP)
+            else if (k == RecOp::COND_NEXT || k == RecOp::COND_LOOP)
                 memcpy(&A.host[A.off[j] + i * sizeof(void*)], &op.ptr, sizeof(void*));
         }
     }
@@ -3105,11 +3163,6 @@ long long group_replay(const std::vector<Recorder>& recs, const GroupArrays& A, 
             if (open.empty()) outside++;
             break;
         }
-        case RecOp::ZERO:
-            k_group_zero<<<dim3(1, 1, n), 128, 0, cur()>>>(reinterpret_cast<unsigned char* const*>(arr), op.bytes);
-            CKL();
-            if (open.empty()) outside++;
-            break;
         case RecOp::COND_NEXT:
             next_h = new_handle(cur());
             next_flags = arr;
@@ -3721,6 +3774,14 @@ int upload_profiles(vvm_gpu_ctx* c, const vvm_gpu_host_state* s) {
         upload_profile(c, scz.data(), c->gsS_cz);
         upload_profile(c, srd.data(), c->gsS_rhod);
         upload_profile(c, dzw.data(), c->lv_dzw);
+        // the largest lower coefficient of the diffusion per K (k_gs_sweep)
+        double fm = 0.0, fs = 0.0;
+        for (int k = 1; k <= nz - 2; k++) {
+            fm = std::max(fm, mcz[k] * mrd[k]);
+            fs = std::max(fs, scz[k] * srd[k]);
+        }
+        c->gs_fz[0] = (float)fm;
+        c->gs_fz[1] = (float)fs;
     }
     // the first nudged level (NumericalProcess.cpp:62: 12000 / dz + 1); on
     // stretched levels the last face at or below 12 km
@@ -4205,7 +4266,7 @@ ROUTINE(vvm_gpu_halo_all, { DISPATCH(ctx, launch_halo_all)(ctx); return VVM_GPU_
 ROUTINE(vvm_gpu_pubartop, { DISPATCH(ctx, launch_pubartop)(ctx); return VVM_GPU_OK; })
 ROUTINE(vvm_gpu_cal_w, { ctx->last_graph = false; return DISPATCH(ctx, launch_cal_w)(ctx, nullptr, nullptr); })
 ROUTINE(vvm_gpu_cal_u, { DISPATCH(ctx, launch_cal_u)(ctx); return VVM_GPU_OK; })
-ROUTINE(vvm_gpu_kessler, { DISPATCH(ctx, launch_kessler)(ctx, false, false); return VVM_GPU_OK; })
+ROUTINE(vvm_gpu_kessler, { DISPATCH(ctx, launch_kessler)(ctx); return VVM_GPU_OK; })
 ROUTINE(vvm_gpu_update_mean, { DISPATCH(ctx, launch_update_mean)(ctx, false); return VVM_GPU_OK; })
 ROUTINE(vvm_gpu_turbulence, { DISPATCH(ctx, launch_turbulence)(ctx, false, nullptr); return VVM_GPU_OK; })
 ROUTINE(vvm_gpu_nudge, {

@@ -1,0 +1,86 @@
+"""The in-place diffusion sweep in one pass (and the repeated passes it asks for
+when its coefficients are too large) against the sequential sweep of the C
+restatement, at grids around its tiles: 108 owned columns (104 to 110 and 215
+to 217 columns with ghosts), bands of 8 rows and one row more, the smallest
+grid.
+
+dt sets the size of the coefficients B + C ~ 2 K dt / dx^2 of the random state
+(K up to ~100 m^2/s at dx = 200 m): a short tail (dt = 1), the long one (dt =
+8), the repeated passes (dt = 60). Tolerance: a cell takes about 20 operations
+on values of its neighbourhood, 20 * 2^-53 ~ 2e-15 relative in FP64 (bound
+1e-13); the mixed step's K is itself formed in FP32 from differences of
+neighbours (bound 1e-5).
+"""
+import numpy as np
+import pytest
+
+from conftest import rel_l2
+
+pytestmark = pytest.mark.gpu
+
+PAIRS = (("zetap", 0), ("thp", 1), ("qvp", 2), ("qcp", 3), ("qrp", 4))
+
+
+@pytest.fixture(scope="module")
+def G():
+    from vvm_b200 import build, gpu
+    build.build()
+    return gpu
+
+
+@pytest.mark.parametrize("precision", [0, 1])
+@pytest.mark.parametrize("dt", [1.0, 8.0, 60.0])
+@pytest.mark.parametrize("NX,NZ", [(4, 4), (104, 8), (106, 9), (108, 17), (213, 16), (215, 25), (256, 40)])
+def test_diffusion_matches_sequential_sweep(G, NX, NZ, dt, precision):
+    from oracle.models import PortModel
+    from vvm_b200.initial_state import random_state
+    st = random_state(NX, NZ, dt=dt, seed=NX + NZ)
+    rng = np.random.default_rng(NX)
+    for n in ("zeta", "th", "qv", "qc", "qr"):
+        st.fields[n + "p"] = st.fields[n] * (1.0 + 1e-3 * rng.standard_normal(st.fields[n].shape))
+    m = PortModel(st.grid)
+    m.load(st)
+    m.call("RKM_RKH")
+    ref = m.dump()
+    g = G.VVMGpu(st.grid, precision=precision)
+    g.upload(st)
+    g.call("turbulence")
+    out = g.download()
+    g.close()
+    for n, _ in PAIRS:
+        assert rel_l2(out.fields[n], ref.fields[n]) <= (1e-13 if precision == 0 else 1e-5), n
+    assert rel_l2(out.fields["qcp"], st.fields["qcp"]) > 1e-5   # it diffused
+
+
+@pytest.mark.parametrize("precision,dt", [(0, 10.0), (1, 30.0)])
+def test_repeated_passes_from_graphs(G, precision, dt):
+    """Coefficients the single pass does not take (dx = 40 m, K = 10 m^2/s at
+    least): the passes of a step graph and of a grouped launch give what the
+    host's loop gives, bit for bit."""
+    from vvm_b200.initial_state import warm_bubble
+    sts = [warm_bubble(128, 24, 40.0, 40.0, dt, amp=a, radius=400.0, zc=400.0) for a in (0.1, 0.2)]
+    host = []
+    for st in sts:
+        g = G.VVMGpu(st.grid, precision=precision, solver=G.VVM_SOLVER_SPECTRAL)
+        g.upload(st)
+        g.profile(True)      # timed steps run kernel by kernel from the host
+        g.step(6)
+        host.append(g.download())
+        g.close()
+        g = G.VVMGpu(st.grid, precision=precision, solver=G.VVM_SOLVER_SPECTRAL)
+        g.upload(st)
+        g.step(6)
+        alone = g.download()
+        g.close()
+        for n in ("zeta", "th", "qv", "qc", "qr", "u", "w"):
+            assert np.isfinite(alone.fields[n]).all() and np.array_equal(alone.fields[n], host[-1].fields[n]), n
+    b = G.VVMBatch([st.grid for st in sts], precision=precision)
+    b.upload(sts)
+    b.step(6)
+    b.synchronize()
+    assert b.grouping() == 1
+    for c, ref in zip(b.cases, host):
+        out = c.download()
+        for n in ("zeta", "th", "qv", "qc", "qr", "u", "w"):
+            assert np.array_equal(out.fields[n], ref.fields[n]), n
+    b.close()
