@@ -61,11 +61,11 @@ __global__ void __launch_bounds__(MAXT, MINB)
     kcall<Body>(packs[blockIdx.z], std::index_sequence_for<A...>{});
 }
 
-// The scalar advection's pack: its four tensor maps stay in global memory,
-// where TMA reads them.
+// The scalar advection's pack: its tensor maps stay in global memory, where
+// TMA reads them.
 template <typename T>
 struct PAdvPack {
-    CUtensorMap m[4];
+    PAdvMaps m;
     PAdvArgs<T> a;
 };
 
@@ -76,14 +76,14 @@ __device__ __forceinline__ void tensormap_acquire(const CUtensorMap* m) {
                  : "memory");
 }
 
-template <typename T>
-__global__ void __launch_bounds__(kPAdvBX * kPAdvBZ, 4)
+template <typename T, int R>
+__global__ void __launch_bounds__(kPAdvLanes* kPAdvWarps, kPAdvMinBlocks<T>)
     k_padv_grouped(const PAdvPack<T>* __restrict__ packs, const int* const* __restrict__ gate) {
     if (gate && !*(const volatile int*)gate[blockIdx.z]) return;
     const PAdvPack<T>& p = packs[blockIdx.z];
     if (threadIdx.x == 0 && threadIdx.y == 0)
-        for (int f = 0; f < 4; f++) tensormap_acquire(&p.m[f]);
-    k_padv_body<T>(&p.m[0], &p.m[1], &p.m[2], &p.m[3], p.a);
+        for (int f = 0; f < 6; f++) tensormap_acquire(&p.m.m[f]);
+    k_padv_body<T, F_TH | F_QV | F_QC | F_QR, R>(p.m, p.a);
 }
 
 // The group's loop condition: another iteration while any case's flag is set.

@@ -290,92 +290,15 @@ struct PAdvArgs {
     T* precip;         // [nx]
     double* partial;   // [gridDim.x*gridDim.y][6]: (pos, neg) of qv, qc, qr
     int* err;          // device error word (kStageErrWait), may be null
-    int mask;          // F_* fields to advect
     int nvp_mask;      // F_* fields whose NVP sums are wanted
-    int do_vt;         // sedimentation of qr (with F_QR)
-    int do_precip;     // surface rain diagnostic
+    int do_precip;     // surface rain diagnostic (with F_QR)
     AB2 ab;
 };
 
-// The velocity part of one face's flux, shared by every advected field:
-// flux = base (v0 + vm) - 1/3 (c1 (v0 - vm) - c2 (vm - vmm) - c3 (v0 - vm)
-// - c4 (vp - v0)), the bracket only away from the boundaries (hi = 0 there).
-// Each coefficient is formed exactly as the per-field expressions of
-// Advection.cpp:40-50 form it.
-template <typename T>
-struct Face {
-    T base, c1, c2, c3, c4;
-    bool hi;
+// The tensor maps of th, qv, qc, qr, u, w (box kPAdvVX by the tile's staged rows).
+struct PAdvMaps {
+    CUtensorMap m[6];
 };
-
-// x face (i-1/2, k), i = 1..nx-2 (Advection.cpp:36,40-44).
-template <typename T>
-__device__ __forceinline__ Face<T> face_u(const PAdvArgs<T>& a, int i, int k) {
-    const Dims& d = a.d;
-    Face<T> F;
-    const T ru = T(a.p.rhou[k]);
-    const T ui = a.u[d.at(i, k)];
-    F.base = ru * ui;
-    F.hi = (i >= 2 && i <= d.nx - 3 && k >= 2 && k <= d.nz - 3);
-    F.c1 = F.c2 = F.c3 = F.c4 = T(0);
-    if (F.hi) {
-        const T um = a.u[d.at(i - 1, k)], up = a.u[d.at(i + 1, k)];
-        F.c1 = ru * plus_part(ui);
-        F.c2 = sqrt(ru * plus_part(ui) * ru * plus_part(um));
-        F.c3 = ru * minus_part(ui);
-        F.c4 = sqrt(fabs(ru * minus_part(ui) * ru * minus_part(up)));
-    }
-    return F;
-}
-
-// z face (i, k-1/2), k = 1..nz-2 (Advection.cpp:37,46-50).
-template <typename T>
-__device__ __forceinline__ Face<T> face_w(const PAdvArgs<T>& a, int i, int k) {
-    const Dims& d = a.d;
-    Face<T> F;
-    const T rk = T(a.p.rhow[k]);
-    const T wk = a.w[d.at(i, k)];
-    F.base = rk * wk;
-    F.hi = (i >= 2 && i <= d.nx - 3 && k >= 2 && k <= d.nz - 3);
-    F.c1 = F.c2 = F.c3 = F.c4 = T(0);
-    if (F.hi) {
-        const T rkm = T(a.p.rhow[k - 1]), rkp = T(a.p.rhow[k + 1]);
-        const T wm = a.w[d.at(i, k - 1)], wp = a.w[d.at(i, k + 1)];
-        F.c1 = rk * plus_part(wk);
-        F.c2 = sqrt(rk * plus_part(wk) * rkm * plus_part(wm));
-        F.c3 = rk * minus_part(wk);
-        F.c4 = sqrt(fabs(rk * minus_part(wk) * rkp * minus_part(wp)));
-    }
-    return F;
-}
-
-// Flux through a face from the field values vmm, vm | v0, vp across it.
-template <typename T>
-__device__ __forceinline__ T face_flux(const Face<T>& F, T vmm, T vm, T v0, T vp) {
-    T f = F.base * (v0 + vm);
-    if (F.hi) f += T(-1. / 3.) * (F.c1 * (v0 - vm) - F.c2 * (vm - vmm) - F.c3 * (v0 - vm) - F.c4 * (vp - v0));
-    return f;
-}
-
-// The same with the third-order differences of a perturbation v' about a
-// profile: dk = (v0 - vm) + d0[k] etc. (mixed step, z faces of th and qv).
-template <typename T>
-__device__ __forceinline__ T face_flux_pert(const Face<T>& F, T vmm, T vm, T v0, T vp, T dkm0, T dk0, T dkp0) {
-    T f = F.base * (v0 + vm);
-    if (F.hi) {
-        const T dk = (v0 - vm) + dk0, dkm = (vm - vmm) + dkm0, dkp = (vp - v0) + dkp0;
-        f += T(-1. / 3.) * (F.c1 * dk - F.c2 * dkm - F.c3 * dk - F.c4 * dkp);
-    }
-    return f;
-}
-
-// Sedimentation flux at (i, k-1/2), k = 1..nz-2 (Advection.cpp:165-166).
-template <typename T>
-__device__ __forceinline__ T vt_flux(const PAdvArgs<T>& a, const T* qr, int i, int k) {
-    T s = qr[a.d.at(i, k)] + qr[a.d.at(i, k - 1)];
-    T VT = T(1E-2) * (T(3634) * pow(T(a.p.vt_c1[k]) * s, T(0.1346)) * T(a.p.vt_fac[k]));
-    return T(a.p.rhow[k]) * VT * s;
-}
 
 // Final sums of NegativeValueProcess and its rescaling factor
 // (MicroPhysics.cpp:125-127): nvp[2f] = 1 if positives are rescaled,
@@ -415,93 +338,115 @@ __device__ __forceinline__ void nvp_finish(const double* partial, int nblocks, d
 
 __global__ void k_nvp_final(const double* partial, int nblocks, double* nvp);
 
-// Tile of k_padv: 32 x 8 cells a block of 32 x 8 threads. The four fields
-// are staged into shared memory with two halo cells a side (one TMA box a
-// field, issued first); every face of the tile (33 x 8 x-faces, 32 x 9 z-faces) is then
-// evaluated once, by one thread: its velocity part (in registers) once for
-// all fields, its flux once per field and, for qr, its sedimentation flux,
-// into shared memory; a cell differences the four fluxes around it. The expressions are the per-cell ones of
-// Advection.cpp:36-58, so each cell's tendency is what a thread computing
-// its own four faces would get, at about half the arithmetic (two square
-// roots a face, one pow a sedimentation face) and with every stencil read
-// from shared memory.
-constexpr int kPAdvBX = 32, kPAdvBZ = 8;
+// Tile of k_padv: 31 x 8R cells a block of 32 x 8 threads, R rows a thread.
+// th, qv, qc, qr, u and w are staged into shared memory with two halo cells a
+// side (one TMA box a field, issued first) and the rows' coefficients beside
+// them. A lane evaluates the x face west of its cell once, the velocity part
+// for all fields, and takes the east flux from the next lane (the last lane
+// owns no cell); going up its rows it carries each field's z flux, so a face
+// between two of its rows is evaluated once too. Of the two square roots of a
+// face's bracket (Advection.cpp:40-50) the wind's sign leaves one that is not
+// zero, so one is taken; flux divergences multiply by r2d / rhou of the row
+// instead of dividing (two roundings either way); a sedimentation flux of no
+// rain needs no pow. The sums of NegativeValueProcess are reduced once for a
+// thread's R cells.
+// Bound by instruction issue: 35 us at 2048 x 256 FP64 and 89 at 8192 x 256,
+// from 51 and 179 with two roots, a division a term, every flux through shared
+// memory and a reduction a cell (FP32 44 -> 23).
+constexpr int kPAdvLanes = 32, kPAdvWarps = 8, kPAdvBX = 31;
 constexpr int kStageErrWait = 4;   // device error word: a stencil's TMA staging wait gave up
+// The staged box of one field: rows k0-2 .. k0+BZ+1 and 40 columns from the
+// halo's first one, i0-2, rounded down to a 16-byte boundary (TMA requires x *
+// element size to be a multiple of 16).
+constexpr int kPAdvVX = 40;
+constexpr int padv_rows(int R) { return kPAdvWarps * R; }
 
-// The staged box of one field: rows k0-2 .. k0+BZ+1 and 40 columns from x0,
-// the halo's first column i0-2 rounded down to a 16-byte boundary (TMA
-// requires x * element size to be a multiple of 16): x0 = i0-2 - kPAdvOff.
-constexpr int kPAdvVX = 40, kPAdvVZ = kPAdvBZ + 4;
-template <typename T>
-constexpr int kPAdvOff = sizeof(T) == 8 ? 1 : 3;
-
-template <typename T>
+template <typename T, int R>
 struct PAdvShared {
-    static constexpr int BX = kPAdvBX, BZ = kPAdvBZ, VX = kPAdvVX, VZ = kPAdvVZ;
-    T v[4][VZ][VX];           // th, qv, qc, qr: rows k0-2.., columns x0.. (each box a multiple of 128 bytes)
-    T fx[4][BZ][BX + 1];      // x fluxes of each field
-    T fz[4][BZ + 1][BX];      // z fluxes of each field
-    T gz[BZ + 1][BX];         // sedimentation fluxes of qr
-    double red[32 * 6];       // block_sum scratch
+    static constexpr int BZ = padv_rows(R), VZ = BZ + 4;
+    T v[6][VZ][kPAdvVX];     // th, qv, qc, qr, u, w: each box a multiple of 128 bytes
+    // rows k0-1 .. k0+BZ+1: rhou, rhow, r2dx / rhou, r2dzc / rhou, vt_c1,
+    // vt_fac; mixed, of th0 and qv0: 2 ref, s0, g0, d0
+    T row[BZ + 3][kPert<T> ? 14 : 6];
+    double red[kPAdvWarps][6];
 };
 
-// Sedimentation flux from s = qr(k) + qr(k-1) at (i, k-1/2) (vt_flux's expression).
+// The velocity part of one face's flux, shared by every advected field:
+// flux = base (v0 + vm) - 1/3 (c (v0 - vm) - s dv), dv the difference across
+// the upwind neighbour face (Advection.cpp:36-50 with the terms that the
+// wind's sign makes zero left out); c = s = 0 next to the boundaries.
 template <typename T>
-__device__ __forceinline__ T vt_flux_s(const PAdvArgs<T>& a, T s, int k) {
-    T VT = T(1E-2) * (T(3634) * pow(T(a.p.vt_c1[k]) * s, T(0.1346)) * T(a.p.vt_fac[k]));
-    return T(a.p.rhow[k]) * VT * s;
+struct Face {
+    T base, c, s;
+    bool pos;   // wind towards +
+};
+// m the face's density, mm and mp the neighbour faces'; v its wind, vm and vp theirs.
+template <typename T>
+__device__ __forceinline__ Face<T> face_of(bool hi, T m, T mm, T mp, T v, T vm, T vp) {
+    Face<T> F;
+    F.base = m * v;
+    F.pos = v > T(0);
+    F.c = F.s = T(0);
+    if (hi) {
+        F.c = fabs(F.base);
+        F.s = sqrt(fabs(F.base * (F.pos ? mm : mp) * (F.pos ? plus_part(vm) : minus_part(vp))));
+    }
+    return F;
+}
+template <typename T>
+__device__ __forceinline__ T face_flux(const Face<T>& F, T d, T dm, T dp, T sum) {
+    return F.base * sum + T(-1. / 3.) * (F.c * d - F.s * (F.pos ? dm : dp));
 }
 
-// Dynamic shared memory: sizeof(PAdvShared<T>) (about 36 KB FP64, 19 KB
-// mixed). At most 64 registers a thread, four blocks a SM (neither step
-// spills). map[f]: the tensor map of a.now[f], box {kPAdvVX, kPAdvVZ}.
-// The maps are read where they lie (a kernel parameter, or global memory
-// for a grouped launch): TMA takes their addresses.
-template <typename T>
-__device__ __forceinline__ void k_padv_body(const CUtensorMap* m0, const CUtensorMap* m1, const CUtensorMap* m2,
-                                            const CUtensorMap* m3, const PAdvArgs<T>& a) {
-    constexpr int BX = kPAdvBX, BZ = kPAdvBZ, VX = kPAdvVX, VZ = kPAdvVZ, OFF = kPAdvOff<T>;
+// MASK: the F_* fields advected; NVP sums and the precipitation go with it
+// (a.nvp_mask, a.do_precip). maps: the tensor maps of th, qv, qc, qr, u, w,
+// read where they lie (a kernel parameter, or global memory for a grouped
+// launch): TMA takes their addresses.
+template <typename T, int MASK, int R>
+__device__ __forceinline__ void k_padv_body(const PAdvMaps& maps, const PAdvArgs<T>& a) {
+    using Sh = PAdvShared<T, R>;
+    constexpr int BZ = Sh::BZ, VZ = Sh::VZ, VX = kPAdvVX, AL = 16 / sizeof(T);
     extern __shared__ __align__(128) unsigned char padv_smem[];
     __shared__ uint64_t stage_bar;
-    PAdvShared<T>& S = *reinterpret_cast<PAdvShared<T>*>(padv_smem);
+    Sh& S = *reinterpret_cast<Sh*>(padv_smem);
     const Dims& d = a.d;
-    const int tx = threadIdx.x, ty = threadIdx.y, tid = tx + BX * ty;
-    const int i0 = 1 + blockIdx.x * BX, k0 = 1 + blockIdx.y * BZ;
-    const int i = i0 + tx, k = k0 + ty;
-    const bool act = (i <= d.nx - 2 && k <= d.nz - 2);
+    const int lane = threadIdx.x, wid = threadIdx.y, tid = lane + kPAdvLanes * wid;
+    const int i0 = 1 + blockIdx.x * kPAdvBX, k0 = 1 + blockIdx.y * BZ;
+    const int x0 = (i0 - 2) & ~(AL - 1);
+    const int i = i0 + lane;
 
-    // Stage the fields, one TMA box each: points outside the array read as
-    // zero and are never used, since a face reads its outer neighbours only
-    // where the third-order bracket applies (2 <= index <= n-3).
+    // Points outside the array read as zero; a face reads its outer neighbours
+    // only where the bracket applies (2 <= index <= n-3).
     const uint32_t bar = smem_u32(&stage_bar);
     if (tid == 0) mbar_init1(bar);
     __syncthreads();
     if (tid == 0) {
-        const CUtensorMap* maps[4] = {m0, m1, m2, m3};
-        uint32_t bytes = 0;
-        for (int f = 0; f < 4; f++)
-            if (a.mask & (1 << f)) bytes += VZ * VX * sizeof(T);
-        mbar_expect_tx(bar, bytes);
-        for (int f = 0; f < 4; f++)
-            if (a.mask & (1 << f)) tma_load_2d(smem_u32(&S.v[f][0][0]), maps[f], i0 - 2 - OFF, k0 - 2, bar);
+        constexpr int nf = ((MASK >> 0) & 1) + ((MASK >> 1) & 1) + ((MASK >> 2) & 1) + ((MASK >> 3) & 1) + 2;
+        mbar_expect_tx(bar, nf * VZ * VX * sizeof(T));
+#pragma unroll
+        for (int f = 0; f < 6; f++)
+            if (f >= 4 || (MASK & (1 << f))) tma_load_2d(smem_u32(&S.v[f][0][0]), &maps.m[f], x0, k0 - 2, bar);
     }
-
-    // Faces: x face (r, c) is fi = i0 + c, between cells fi-1 and fi, on row
-    // k0 + r; the east face of cell nx-2 is the halo copy of face 1
-    // (BoundaryProcess2D_center on flux_u, Advection.cpp:55). z face (r, c) is
-    // fk = k0 + r, between cells fk-1 and fk, in column i0 + c; face nz-1
-    // carries no flux (Advection.cpp:57-58).
-    auto xface_ok = [&](int r, int c) { return k0 + r <= d.nz - 2 && i0 + c <= d.nx - 1; };
-    auto zface_ok = [&](int r, int c) { return k0 + r <= d.nz - 2 && i0 + c <= d.nx - 2; };
-    auto zflux_ok = [&](int r, int c) { return k0 + r <= d.nz - 1 && i0 + c <= d.nx - 2; };
-    auto xface_i = [&](int c) { int fi = i0 + c; return fi == d.nx - 1 ? 1 : fi; };
-
-    // velocity parts of the thread's own faces, its cell's west and bottom
-    // ones, while the copies are in flight
-    const bool xo = xface_ok(ty, tx), zo = zface_ok(ty, tx), zfo = zflux_ok(ty, tx);
-    Face<T> Fx{}, Fz{};
-    if (xo) Fx = face_u(a, xface_i(tx), k0 + ty);
-    if (zo) Fz = face_w(a, i0 + tx, k0 + ty);
+    for (int t = tid; t < BZ + 3; t += kPAdvLanes * kPAdvWarps) {
+        const int k = k0 - 1 + t;
+        if (k > d.nz - 1) break;
+        T* r = S.row[t];
+        r[0] = T(a.p.rhou[k]);
+        r[1] = T(a.p.rhow[k]);
+        r[2] = T(a.c.r2dx) / r[0];
+        r[3] = T(a.p.r2dzc[k]) / r[0];
+        r[4] = T(a.p.vt_c1[k]);
+        r[5] = T(a.p.vt_fac[k]);
+        if constexpr (kPert<T>) {
+#pragma unroll
+            for (int f = 0; f < 2; f++) {
+                r[6 + f] = T(2.0 * a.p.ref[f][k]);
+                r[8 + f] = T(a.p.s0[f][k]);
+                r[10 + f] = T(a.p.g0[f][k]);
+                r[12 + f] = T(a.p.d0[f][k]);
+            }
+        }
+    }
     const bool ok = mbar_wait_bounded(bar, 0);
     if (__syncthreads_or(!ok)) {   // the copies never landed: report and leave
         if (tid == 0 && a.err) atomicOr(a.err, kStageErrWait);
@@ -509,130 +454,158 @@ __device__ __forceinline__ void k_padv_body(const CUtensorMap* m0, const CUtenso
         return;
     }
 
-    // staged column of index ii: ii - (i0 - 2) + OFF
-    auto xflux = [&](const Face<T>& F, int f, int r, int c) {
-        if (i0 + c == d.nx - 1) {   // face 1 (no bracket), read where it lies
-            const T* v = a.now[f];
-            return face_flux(F, T(0), v[d.at(0, k0 + r)], v[d.at(1, k0 + r)], T(0));
-        }
-        const T* row = &S.v[f][r + 2][c + OFF];   // columns fi-2 .. fi+1
-        return face_flux(F, F.hi ? row[0] : T(0), row[1], row[2], F.hi ? row[3] : T(0));
-    };
-    // th and qv of the mixed step take the perturbation form (third-order
-    // differences with the profile's d0)
-    auto zflux = [&](const Face<T>& F, int f, int r, int c) {
-        const int fk = k0 + r;
-        if (fk == d.nz - 1) return T(0);
-        const T vmm = S.v[f][r][c + 2 + OFF], vm = S.v[f][r + 1][c + 2 + OFF], v0 = S.v[f][r + 2][c + 2 + OFF],
-                vp = S.v[f][r + 3][c + 2 + OFF];   // rows fk-2 .. fk+1
-        if (kPert<T> && f < 2 && F.hi) {
-            const double* d0 = a.p.d0[f];
-            return face_flux_pert(F, vmm, vm, v0, vp, T(d0[fk - 1]), T(d0[fk]), T(d0[fk + 1]));
-        }
-        return face_flux(F, F.hi ? vmm : T(0), vm, v0, F.hi ? vp : T(0));
-    };
-    auto gflux = [&](int r, int c) {
-        const int fk = k0 + r;
-        return fk == d.nz - 1 ? T(0) : vt_flux_s(a, S.v[3][r + 2][c + 2 + OFF] + S.v[3][r + 1][c + 2 + OFF], fk);
-    };
-
-    const bool vt = (a.mask & F_QR) && a.do_vt;
-    for (int f = 0; f < 4; f++) {
-        if (!(a.mask & (1 << f))) continue;
-        if (xo) S.fx[f][ty][tx] = xflux(Fx, f, ty, tx);
-        if (zfo) S.fz[f][ty][tx] = zflux(Fz, f, ty, tx);
-    }
-    if (vt && zfo) S.gz[ty][tx] = gflux(ty, tx);
-    // the tile's east column of x faces (warp 0, lanes 0..7, one a row) and
-    // its top row of z faces (warp 1)
-    if (ty == 0 && tx < BZ && xface_ok(tx, BX)) {
-        const Face<T> F = face_u(a, xface_i(BX), k0 + tx);
-        for (int f = 0; f < 4; f++)
-            if (a.mask & (1 << f)) S.fx[f][tx][BX] = xflux(F, f, tx, BX);
-    }
-    if (ty == 1 && zflux_ok(BZ, tx)) {
+    const int c = i0 - x0 + lane;                 // the lane's column in the tile
+    const bool cell = lane < kPAdvBX && i <= d.nx - 2;
+    const bool wrap = (i == d.nx - 1);            // the east face of cell nx-2: the halo copy of face 1
+    const bool xhi = i >= 2 && i <= d.nx - 3;
+    constexpr bool vt = (MASK & F_QR) != 0;       // sedimentation goes with qr
+    const T dt15 = T(1.5 * a.c.dt), dt05 = T(0.5 * a.c.dt);
+    const T* const u = &S.v[4][0][0];
+    const T* const w = &S.v[5][0][0];
+    // z fluxes of the fields and of the rain's fall at face k (between rows
+    // k-1 and k); none at the top face (Advection.cpp:57-58, :170-171)
+    T fz[4] = {T(0), T(0), T(0), T(0)}, gz = T(0);
+    auto zfaces = [&](int k, T (&f4)[4], T& g) {
+        const int r = k - k0 + 2, at = r * VX + c;
+        const T* q = S.row[k - k0 + 1];
+        const bool hi = xhi && k >= 2 && k <= d.nz - 3;
         Face<T> F{};
-        if (zface_ok(BZ, tx)) F = face_w(a, i0 + tx, k0 + BZ);
-        for (int f = 0; f < 4; f++)
-            if (a.mask & (1 << f)) S.fz[f][BZ][tx] = zflux(F, f, BZ, tx);
-        if (vt) S.gz[BZ][tx] = gflux(BZ, tx);
-    }
-    __syncthreads();
+        const bool top = k > d.nz - 2;
+        if (!top) {
+            const T wk = w[at];
+            F = face_of(hi, q[1], S.row[k - k0][1], S.row[k - k0 + 2][1], wk, w[at - VX], w[at + VX]);
+        }
+#pragma unroll
+        for (int f = 0; f < 4; f++) {
+            if (!(MASK & (1 << f))) continue;
+            const T* v = &S.v[f][0][0] + at;
+            const T vmm = v[-2 * VX], vm = v[-VX], v0 = v[0], vp = v[VX];
+            T dd = v0 - vm, dm = vm - vmm, dp = vp - v0;
+            if (kPert<T> && f < 2 && hi) {   // third-order differences with the profile's (mixed step)
+                dd += q[12 + f];
+                dm += S.row[k - k0][12 + f];
+                dp += S.row[k - k0 + 2][12 + f];
+            }
+            f4[f] = top ? T(0) : face_flux(F, dd, dm, dp, v0 + vm);
+            if (f == 3) {
+                const T sm = v0 + vm;
+                g = T(0);
+                if (!top && sm != T(0)) {   // Advection.cpp:165-166
+                    const T VT = T(1E-2) * (T(3634) * pow(q[4] * sm, T(0.1346)) * q[5]);
+                    g = q[1] * VT * sm;
+                }
+            }
+        }
+    };
 
     double sums[6] = {0, 0, 0, 0, 0, 0};
-    if (act) {
+    const int ka = k0 + wid * R;
+    if (ka <= d.nz - 2) zfaces(ka, fz, gz);
+#pragma unroll 1
+    for (int j = 0; j < R; j++) {
+        const int k = ka + j;
+        if (k > d.nz - 2) break;   // uniform over the warp
+        const int at = (k - k0 + 2) * VX + c;
         const size_t id = d.at(i, k);
-        const T dt15 = T(1.5 * a.c.dt), dt05 = T(0.5 * a.c.dt);
-        const T ru = T(a.p.rhou[k]);
-        // mixed step: one division for the cell's flux divergences (the FP64
-        // step keeps the reference's (difference * r2d) / rhou per term)
-        const T sx = kPert<T> ? T(a.c.r2dx) / ru : T(0), sz = kPert<T> ? T(a.p.r2dzc[k]) / ru : T(0);
-        const int ip = (i == d.nx - 2) ? 1 : i + 1;
-        const bool top = (k == d.nz - 2);
-        for (int f = 0; f < 4; f++) {
-            if (!(a.mask & (1 << f))) continue;
-            const T fu_0 = S.fx[f][ty][tx], fu_p = S.fx[f][ty][tx + 1];
-            const T fw_0 = S.fz[f][ty][tx], fw_p = S.fz[f][ty + 1][tx];
-            T px, pz;
-            if (!kPert<T> || f >= 2) {
-                if constexpr (kPert<T>) {
-                    px = (fu_p - fu_0) * sx;
-                    pz = (fw_p - fw_0) * sz;
-                } else {
-                    px = (fu_p - fu_0) * T(a.c.r2dx) / ru;
-                    pz = (fw_p - fw_0) * T(a.p.r2dzc[k]) / ru;
-                }
-            } else {
-                // v = v0(k) + v': the v0 parts of both fluxes are added in
-                // difference form, 2 v0 (u[i+1] - u[i]) in x and
-                // s0[k+1] (m[k+1] - m[k]) + m[k] g0[k] in z, m = rhow w.
-                T m0 = T(a.p.rhow[k]) * a.w[d.at(i, k)];
-                T refz = top ? -m0 * T(a.p.s0[f][k])
-                             : T(a.p.s0[f][k + 1]) * (T(a.p.rhow[k + 1]) * a.w[d.at(i, k + 1)] - m0) +
-                                   m0 * T(a.p.g0[f][k]);
-                T refx = T(2.0 * a.p.ref[f][k]) * (a.u[d.at(ip, k)] - a.u[d.at(i, k)]);
-                px = (fu_p - fu_0) * sx + refx * T(a.c.r2dx);
-                pz = (fw_p - fw_0 + refz) * sz;
-            }
-            T t = -px - pz;
-            T o = ab2_push(a.hn[f], a.ho[f], id, t, a.ab);
-            T out = S.v[f][ty + 2][tx + 2 + OFF] + dt15 * t - dt05 * o;
-            if (f == 3 && vt) {
-                const T gp = S.gz[ty + 1][tx], g0 = S.gz[ty][tx];
-                T tv = kPert<T> ? (gp - g0) * sz : (gp - g0) * T(a.p.r2dzc[k]) / ru;
-                T ov = ab2_push(a.hvt_n, a.hvt_o, id, tv, a.ab);
-                out += dt15 * tv - dt05 * ov;
-            }
-            a.fut[f][id] = out;
-            if (f >= 1 && (a.nvp_mask & (1 << f))) {
-                double full = (double)out;
-                if (kPert<T> && f == 1) full += a.p.ref[1][k];
-                if (full >= 0.0) sums[2 * (f - 1)] += full;
-                else sums[2 * (f - 1) + 1] += full;
-            }
+        const T* q = S.row[k - k0 + 1];
+        T o[4], ovt = T(0);
+        if (cell && !a.ab.first) {   // the previous tendencies, in flight during the fluxes
+#pragma unroll
+            for (int f = 0; f < 4; f++)
+                if (MASK & (1 << f)) o[f] = a.ho[f][id];
+            if (vt) ovt = a.hvt_o[id];
         }
-        if (a.do_precip && k == 1) {
-            const T* qr = a.now[3];
-            T q1 = qr[d.at(i, 1)];
+        // x face west of the cell (or, at nx-1, face 1, from where it lies)
+        Face<T> F = face_of(xhi && k >= 2 && k <= d.nz - 3, q[0], q[0], q[0], wrap ? a.u[d.at(1, k)] : u[at], u[at - 1], u[at + 1]);
+        T fu[4], zu[4], gu;
+#pragma unroll
+        for (int f = 0; f < 4; f++) {
+            if (!(MASK & (1 << f))) continue;
+            const T* v = &S.v[f][0][0] + at;
+            T vm = v[-1], v0 = v[0];
+            if (wrap) {
+                vm = a.now[f][d.at(0, k)];
+                v0 = a.now[f][d.at(1, k)];
+            }
+            fu[f] = face_flux(F, v0 - vm, vm - v[-2], v[1] - v0, v0 + vm);
+        }
+        zfaces(k + 1, zu, gu);
+#pragma unroll
+        for (int f = 0; f < 4; f++) {
+            if (!(MASK & (1 << f))) continue;
+            const T fe = __shfl_down_sync(0xffffffffu, fu[f], 1);
+            T px = (fe - fu[f]) * q[2], pz = (zu[f] - fz[f]) * q[3];
+            if constexpr (kPert<T>) {
+                if (f < 2) {
+                    // v = v0(k) + v': the v0 parts of both fluxes are added in
+                    // difference form, 2 v0 (u[i+1] - u[i]) in x and
+                    // s0[k+1] (m[k+1] - m[k]) + m[k] g0[k] in z, m = rhow w.
+                    const T m0 = q[1] * w[at];
+                    const T refz = (k == d.nz - 2) ? -m0 * q[8 + f]
+                                                   : S.row[k - k0 + 2][8 + f] * (S.row[k - k0 + 2][1] * w[at + VX] - m0) + m0 * q[10 + f];
+                    const T ue = (i == d.nx - 2) ? a.u[d.at(1, k)] : u[at + 1];
+                    px = (fe - fu[f]) * q[2] + q[6 + f] * (ue - u[at]) * T(a.c.r2dx);
+                    pz = (zu[f] - fz[f] + refz) * q[3];
+                }
+            }
+            const T t = -px - pz;
+            T tv = T(0);
+            if (f == 3) tv = (gu - gz) * q[3];
+            if (cell) {
+                if (a.ab.first) {
+                    o[f] = t;
+                    a.ho[f][id] = t;
+                    if (f == 3) {
+                        ovt = tv;
+                        a.hvt_o[id] = tv;
+                    }
+                }
+                a.hn[f][id] = t;
+                T out = S.v[f][k - k0 + 2][c] + dt15 * t - dt05 * o[f];
+                if (f == 3) {
+                    a.hvt_n[id] = tv;
+                    out += dt15 * tv - dt05 * ovt;
+                }
+                a.fut[f][id] = out;
+                if (f >= 1 && (a.nvp_mask & (1 << f))) {
+                    double full = (double)out;
+                    if (kPert<T> && f == 1) full += a.p.ref[1][k];
+                    if (full >= 0.0) sums[2 * (f - 1)] += full;
+                    else sums[2 * (f - 1) + 1] += full;
+                }
+            }
+            fz[f] = zu[f];
+        }
+        gz = gu;
+        if (a.do_precip && k == 1 && cell) {
+            const T q1 = S.v[3][2][c];
             T VT = T(1E-2) * (T(3634) * pow(T(a.p.pf1) * q1, T(0.1346)) * T(a.p.pf2));
-            T rain = -T(a.p.rhou[1]) * (T(0.5) * (a.w[d.at(i, 2)] + T(0)) - VT) * q1;
+            T rain = -q[0] * (T(0.5) * (w[at + VX] + T(0)) - VT) * q1;
             a.precip[i] = (rain < T(0)) ? T(0) : rain;
         }
     }
-    if (a.nvp_mask) {
-        block_sum(sums, S.red);
-        if (tid == 0) {
-            double* out = a.partial + (size_t)(blockIdx.x + gridDim.x * blockIdx.y) * 6;
+    if (a.nvp_mask) {   // the block's sums, in a fixed order
 #pragma unroll
-            for (int j = 0; j < 6; j++) out[j] = sums[j];
+        for (int m = 0; m < 6; m++) sums[m] = warp_sum(sums[m]);
+        if (lane == 0) {
+#pragma unroll
+            for (int m = 0; m < 6; m++) S.red[wid][m] = sums[m];
+        }
+        __syncthreads();
+        if (tid < 6) {
+            double t = 0.0;
+            for (int q = 0; q < kPAdvWarps; q++) t += S.red[q][tid];
+            a.partial[(size_t)(blockIdx.x + gridDim.x * blockIdx.y) * 6 + tid] = t;
         }
     }
 }
+// Blocks a SM by shared memory at four rows a thread: three in FP64, six in FP32.
 template <typename T>
-__global__ void __launch_bounds__(kPAdvBX * kPAdvBZ, 4)
-    k_padv(const __grid_constant__ CUtensorMap m0, const __grid_constant__ CUtensorMap m1,
-           const __grid_constant__ CUtensorMap m2, const __grid_constant__ CUtensorMap m3, PAdvArgs<T> a) {
-    k_padv_body<T>(&m0, &m1, &m2, &m3, a);
+constexpr int kPAdvMinBlocks = sizeof(T) == 8 ? 3 : 4;
+template <typename T, int MASK, int R>
+__global__ void __launch_bounds__(kPAdvLanes* kPAdvWarps, kPAdvMinBlocks<T>)
+    k_padv(const __grid_constant__ PAdvMaps maps, PAdvArgs<T> a) {
+    k_padv_body<T, MASK, R>(maps, a);
 }
 
 // ---------------------------------------------------------------------------

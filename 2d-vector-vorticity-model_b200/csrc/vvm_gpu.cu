@@ -1698,9 +1698,6 @@ struct vvm_gpu_ctx {
     const double* offset_qv() const { return mixed ? pref[1] : nullptr; }
     dim3 blk() const { return dim3(64, 4); }
     dim3 grid_interior(int k0) const { return dim3(cdiv(d.nx - 2, 64), cdiv(d.nz - 1 - k0, 4)); }
-    // k_padv's tiles of kPAdvBX x kPAdvBZ interior cells
-    dim3 padv_blk() const { return dim3(kPAdvBX, kPAdvBZ); }
-    dim3 padv_grid() const { return dim3(cdiv(d.nx - 2, kPAdvBX), cdiv(d.nz - 2, kPAdvBZ)); }
     dim3 grid_all() const { return dim3(cdiv(d.nx, 64), cdiv(d.nz, 4)); }
 };
 
@@ -1777,8 +1774,17 @@ void launch_pzeta(vvm_gpu_ctx* c) {
     klaunch<k_pzeta_body<T>, kPZBX * kPZBZ>(&c->stats, VVM_K_PZETA, c->stream, k_pzeta<T>, g, dim3(kPZBX, kPZBZ), 0, a);
 }
 
-template <typename T>
-void launch_padv(vvm_gpu_ctx* c, int mask, int nvp_mask, bool vt, bool precip) {
+// Rows a thread of k_padv takes: four share their z fluxes and amortise the
+// reduction, one finishes sooner where the grid is small (us a launch with 1 /
+// 4 rows, FP64: 128 x 64 10.6 / 16.8; 8192 x 256 98.8 / 89.0, FP32 82.3 /
+// 66.0; the step of 512 x 128 84.1 / 82.0, of 2048 x 256 199.5 / 195.5).
+inline int padv_rows_a_thread(const Dims& d) {
+    return cdiv(d.nx - 2, kPAdvBX) * cdiv(d.nz - 2, padv_rows(4)) >= 64 ? 4 : 1;
+}
+
+// MASK: the fields advected. Surface rain and sedimentation go with qr.
+template <typename T, int MASK>
+void launch_padv(vvm_gpu_ctx* c) {
     Fields<T>& F = fields<T>(c);
     int now = c->cur, fut = 1 - c->cur;
     AB2 ab = AB2::of(c->step);
@@ -1801,28 +1807,32 @@ void launch_padv(vvm_gpu_ctx* c, int mask, int nvp_mask, bool vt, bool precip) {
     a.hvt_o = F.hist[H_VT][ab.so];
     a.precip = F.precip;
     a.partial = c->partial;
-    a.mask = mask;
-    a.nvp_mask = nvp_mask;
-    a.do_vt = vt;
-    a.do_precip = precip;
+    a.nvp_mask = MASK & ~F_TH;
+    a.do_precip = (MASK & F_QR) != 0;
     a.ab = ab;
     a.err = c->d_err;
-    dim3 g = c->padv_grid();
-    CUtensorMap m[4];
-    for (int f = 0; f < 4; f++)
-        m[f] = field_map(a.now[f], c->d.nx, c->d.nz, c->d.pitch, (int)sizeof(T), kPAdvVX, kPAdvVZ);
+    constexpr int ALL = F_TH | F_QV | F_QC | F_QR;
+    const int R = MASK == ALL ? padv_rows_a_thread(c->d) : 1;
+    const dim3 g(cdiv(c->d.nx - 2, kPAdvBX), cdiv(c->d.nz - 2, padv_rows(R))), blk(kPAdvLanes, kPAdvWarps);
+    PAdvMaps m;
+    for (int f = 0; f < 6; f++)
+        m.m[f] = field_map(f < 4 ? a.now[f] : f == 4 ? a.u : a.w, c->d.nx, c->d.nz, c->d.pitch, (int)sizeof(T), kPAdvVX,
+                           padv_rows(R) + 4);
+    const size_t smem = R == 4 ? sizeof(PAdvShared<T, 4>) : sizeof(PAdvShared<T, 1>);
     if (c->stats.rec) {
-        PAdvPack<T> p;
-        for (int f = 0; f < 4; f++) p.m[f] = m[f];
-        p.a = a;
-        record_kernel(&c->stats, reinterpret_cast<const void*>(&k_padv_grouped<T>), g, c->padv_blk(),
-                      sizeof(PAdvShared<T>), &p, sizeof(p), alignof(PAdvPack<T>));
+        if (MASK != ALL) throw CudaError{"grouped launch: the advection of single fields has no grouped form"};
+        PAdvPack<T> p{m, a};
+        const void* fn = R == 4 ? reinterpret_cast<const void*>(&k_padv_grouped<T, 4>)
+                                : reinterpret_cast<const void*>(&k_padv_grouped<T, 1>);
+        record_kernel(&c->stats, fn, g, blk, smem, &p, sizeof(p), alignof(PAdvPack<T>));
+    } else if (MASK == ALL && R == 4) {
+        LAUNCH(&c->stats, VVM_K_PADV, c->stream, k_padv<T, ALL, 4><<<g, blk, smem, c->stream>>>(m, a));
+        CKL();
     } else {
-        LAUNCH(&c->stats, VVM_K_PADV, c->stream,
-               k_padv<T><<<g, c->padv_blk(), sizeof(PAdvShared<T>), c->stream>>>(m[0], m[1], m[2], m[3], a));
+        LAUNCH(&c->stats, VVM_K_PADV, c->stream, k_padv<T, MASK, 1><<<g, blk, smem, c->stream>>>(m, a));
         CKL();
     }
-    if (nvp_mask)
+    if (a.nvp_mask)
         klaunch<k_nvp_final_body, 1024>(&c->stats, VVM_K_APPLY, c->stream, k_nvp_final, dim3(1), dim3(1024), 0,
                                         (const double*)c->partial, (int)(g.x * g.y), c->nvp);
 }
@@ -2769,7 +2779,7 @@ int run_step(vvm_gpu_ctx* c, long long* recorded_in_loops = nullptr) {
         {
             OnStream os(c, c->side);
             if (!sf) launch_pubartop<T>(c);                    // pubarTop_pt
-            launch_padv<T>(c, F_TH | F_QV | F_QC | F_QR, F_QV | F_QC | F_QR, true, true);  // pth, pqv, pqc, pqr
+            launch_padv<T, F_TH | F_QV | F_QC | F_QR>(c);  // pth, pqv, pqc, pqr
             CK(cudaEventRecord(c->fork_ev[1], c->side));   // u and w read, ubarTopp written
             launch_kessler<T>(c);                              // NVP + AddForcing, Kessler + NVP sums + halos
         }
@@ -2789,7 +2799,7 @@ int run_step(vvm_gpu_ctx* c, long long* recorded_in_loops = nullptr) {
         join_side(c, 2);
     } else {
         launch_pzeta<T>(c);                                    // pzeta_pt
-        launch_padv<T>(c, F_TH | F_QV | F_QC | F_QR, F_QV | F_QC | F_QR, true, true);  // pth, pqv, pqc, pqr
+        launch_padv<T, F_TH | F_QV | F_QC | F_QR>(c);  // pth, pqv, pqc, pqr
         if (sf) {
             rc = launch_calpsiuw<T>(c);
         } else {
@@ -4105,13 +4115,11 @@ int vvm_gpu_create(const vvm_gpu_desc* desc, int device, vvm_gpu_ctx** out) {
         c->ubar = c->ar.alloc<double>(2);
         c->dubar = c->ar.alloc<double>(2);
         // block partials of k_padv and k_kessler (NegativeValueProcess sums)
-        dim3 g = c->grid_interior(1), ga = c->padv_grid();
-        c->npart = std::max(g.x * g.y, ga.x * ga.y);
+        dim3 g = c->grid_interior(1);
+        c->npart = std::max((int)(g.x * g.y), cdiv(D.NX, kPAdvBX) * cdiv(D.NZ, padv_rows(1)));
         c->partial = c->ar.alloc<double>((size_t)c->npart * 6);
-        CK(cudaFuncSetAttribute(k_padv<double>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                (int)sizeof(PAdvShared<double>)));
-        CK(cudaFuncSetAttribute(k_padv<float>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                (int)sizeof(PAdvShared<float>)));
+        CK(cudaFuncSetAttribute(k_padv<double, F_TH | F_QV | F_QC | F_QR, 4>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                (int)sizeof(PAdvShared<double, 4>)));
         c->nvp = c->ar.alloc<double>(6);
         c->staging = c->ar.alloc<double>((size_t)c->d.nx * c->d.nz * 2);
         c->wctl = c->ar.alloc<CGCtl>(1);
@@ -4229,22 +4237,22 @@ int vvm_gpu_get_step(vvm_gpu_ctx* ctx, int* step) {
 
 ROUTINE(vvm_gpu_pzeta, { DISPATCH(ctx, launch_pzeta)(ctx); return VVM_GPU_OK; })
 ROUTINE(vvm_gpu_pth, {
-    DISPATCH(ctx, launch_padv)(ctx, F_TH, 0, false, false);
+    ctx->mixed ? launch_padv<float, F_TH>(ctx) : launch_padv<double, F_TH>(ctx);
     DISPATCH(ctx, launch_apply)(ctx, F_TH, 0, false, true);
     return VVM_GPU_OK;
 })
 ROUTINE(vvm_gpu_pqv, {
-    DISPATCH(ctx, launch_padv)(ctx, F_QV, F_QV, false, false);
+    ctx->mixed ? launch_padv<float, F_QV>(ctx) : launch_padv<double, F_QV>(ctx);
     DISPATCH(ctx, launch_apply)(ctx, F_QV, F_QV, false, true);
     return VVM_GPU_OK;
 })
 ROUTINE(vvm_gpu_pqc, {
-    DISPATCH(ctx, launch_padv)(ctx, F_QC, F_QC, false, false);
+    ctx->mixed ? launch_padv<float, F_QC>(ctx) : launch_padv<double, F_QC>(ctx);
     DISPATCH(ctx, launch_apply)(ctx, F_QC, F_QC, false, true);
     return VVM_GPU_OK;
 })
 ROUTINE(vvm_gpu_pqr, {
-    DISPATCH(ctx, launch_padv)(ctx, F_QR, F_QR, true, true);
+    ctx->mixed ? launch_padv<float, F_QR>(ctx) : launch_padv<double, F_QR>(ctx);
     DISPATCH(ctx, launch_apply)(ctx, F_QR, F_QR, false, true);
     return VVM_GPU_OK;
 })
