@@ -61,12 +61,12 @@ __global__ void __launch_bounds__(MAXT, MINB)
     kcall<Body>(packs[blockIdx.z], std::index_sequence_for<A...>{});
 }
 
-// The scalar advection's pack: its tensor maps stay in global memory, where
-// TMA reads them.
-template <typename T>
-struct PAdvPack {
-    PAdvMaps m;
-    PAdvArgs<T> a;
+// The pack of a kernel that stages its fields by TMA: its tensor maps stay in
+// global memory, where TMA reads them.
+template <int N, typename A>
+struct TilePack {
+    FieldMaps<N> m;
+    A a;
 };
 
 // A tensor map that a host copy wrote to global memory, made visible to the
@@ -76,14 +76,28 @@ __device__ __forceinline__ void tensormap_acquire(const CUtensorMap* m) {
                  : "memory");
 }
 
-template <typename T, int R>
-__global__ void __launch_bounds__(kPAdvLanes* kPAdvWarps, kPAdvMinBlocks<T>)
-    k_padv_grouped(const PAdvPack<T>* __restrict__ packs, const int* const* __restrict__ gate) {
-    if (gate && !*(const volatile int*)gate[blockIdx.z]) return;
-    const PAdvPack<T>& p = packs[blockIdx.z];
+template <int N, typename A>
+__device__ __forceinline__ void tensormaps_acquire(const TilePack<N, A>& p) {
     if (threadIdx.x == 0 && threadIdx.y == 0)
-        for (int f = 0; f < 6; f++) tensormap_acquire(&p.m.m[f]);
+        for (int f = 0; f < N; f++) tensormap_acquire(&p.m.m[f]);
+}
+
+template <typename T, int R>
+__global__ void __launch_bounds__(kTileLanes* kTileWarps, kPAdvMinBlocks<T>)
+    k_padv_grouped(const TilePack<6, PAdvArgs<T>>* __restrict__ packs, const int* const* __restrict__ gate) {
+    if (gate && !*(const volatile int*)gate[blockIdx.z]) return;
+    const TilePack<6, PAdvArgs<T>>& p = packs[blockIdx.z];
+    tensormaps_acquire(p);
     k_padv_body<T, F_TH | F_QV | F_QC | F_QR, R>(p.m, p.a);
+}
+
+template <typename T, int R>
+__global__ void __launch_bounds__(kTileLanes* kTileWarps, 4)
+    k_pzeta_grouped(const TilePack<7, PZetaArgs<T>>* __restrict__ packs, const int* const* __restrict__ gate) {
+    if (gate && !*(const volatile int*)gate[blockIdx.z]) return;
+    const TilePack<7, PZetaArgs<T>>& p = packs[blockIdx.z];
+    tensormaps_acquire(p);
+    k_pzeta_body<T, R>(p.m, p.a);
 }
 
 // The group's loop condition: another iteration while any case's flag is set.

@@ -25,6 +25,7 @@ struct Profiles {
     const double *vt_c1;      // (1E-3*rhow[k])*0.5            Advection.cpp:165
     const double *vt_fac;     // pow(rhow[k]/rhow[1], -0.5)    Advection.cpp:165
     const double *pc;         // 380/(pow(pib,Cp/Rd)*P0)       MicroPhysics.cpp:10,82
+    const double *lvcp;       // Lv/(Cp*pib)                    MicroPhysics.cpp:24,108
     const double *dtcgr_th;   // dt*CGR of Nudge_theta (0 below k_start)
     const double *dtcgr_zeta; // dt*CGR of Nudge_zeta (0 below k_start or case 2)
     const double *q1ls, *q2ls;  // large-scale forcing profiles (may be all zero)
@@ -100,171 +101,214 @@ struct PZetaArgs {
     const T *zeta, *u, *w, *th, *qv, *qc, *qr;
     T* zetap;
     T *hz_n, *hz_o, *hb_n, *hb_o;  // dzeta_advect, dth_buoyancy slots
+    int* err;                      // device error word (kStageErrWait), may be null
     AB2 ab;
 };
 
-// x-face mass flux Uw of Advection_zeta (Advection.cpp:90) from global
-// memory: the halo face of k_pzeta's first tile.
-template <typename T>
-__device__ __forceinline__ T zeta_Uw(const PZetaArgs<T>& a, int i, int k) {
-    const Dims& d = a.d;
-    return T(0.25) * (T(a.p.rhou[k]) * (a.u[d.at(i + 1, k)] + a.u[d.at(i, k)]) +
-                      T(a.p.rhou[k - 1]) * (a.u[d.at(i + 1, k - 1)] + a.u[d.at(i, k - 1)]));
-}
+// Tile of k_pzeta: 31 x 8R zeta points a block of 32 x 8 threads, R rows a
+// thread. zeta, u, w, th, qv, qc and qr are staged by TMA (one box a field).
+// A lane is the x face fi = i0 - 1 + lane and the point west of it: it
+// evaluates the face once and takes its point's west flux from the lane before
+// (lane 0 owns no point). Going up its rows it carries the z flux, the staggered
+// mass fluxes Uw, Wu (Advection.cpp:90-91) and the buoyancy difference of the
+// row below, so each is formed once. As in k_padv one square root a face, no
+// division but the buoyancy's by thvb. Bound by instruction issue: 28 -> 22 us
+// at 2048 x 256 FP64, 25 -> 16 FP32; 96 -> 57 and 84 -> 42 at 8192 x 256 (from
+// staging loops that divide for their indexes, two roots a face and every flux
+// through shared memory).
+constexpr int kStageErrWait = 4;   // device error word: a stencil's TMA staging wait gave up
+constexpr int kTileLanes = 32, kTileWarps = 8, kTileBX = 31;   // blocks of k_pzeta and k_padv
+// The staged box of one field: the tile's rows with two halo rows a side and 40
+// columns from the halo's first one, i0-2, rounded down to a 16-byte boundary
+// (TMA requires x * element size to be a multiple of 16).
+constexpr int kTileVX = 40;
+constexpr int tile_rows(int R) { return kTileWarps * R; }
 
-// Tile of k_pzeta: 32 x 8 zeta points a block of 32 x 8 threads. zeta, u, w,
-// th, qv, qc and qr are staged into shared memory (cp.async); the staggered
-// mass fluxes Uw, Wu (Advection.cpp:90-91) are formed once a face point, the
-// x and z fluxes once a face, and each point then differences its four
-// fluxes and forms its buoyancy from the staged values.
-constexpr int kPZBX = 32, kPZBZ = 8;
-
-template <typename T>
-struct PZetaShared {
-    static constexpr int BX = kPZBX, BZ = kPZBZ;
-    T z[BZ + 4][BX + 4];      // zeta: rows k0-2.., columns i0-2..
-    T u[BZ + 1][BX + 4];      // u: rows k0-1.., columns i0-2..
-    T w[BZ + 4][BX + 1];      // w: rows k0-2.., columns i0-1..
-    T q[4][BZ + 1][BX + 1];   // th, qv, qc, qr: rows k0-1.., columns i0-1..
-    T U[BZ][BX + 3];          // Uw at x faces fi = i0-2.., rows k0..
-    T W[BZ + 3][BX];          // Wu at z faces fk = k0-2.., columns i0..
-    T fu[BZ][BX + 1];         // flux_u at fi = i0-1..
-    T fw[BZ + 1][BX];         // flux_w at fk = k0-1..
+// Tensor maps of a tile kernel's fields (box kTileVX by its staged rows).
+template <int N>
+struct FieldMaps {
+    CUtensorMap m[N];
 };
 
+// The velocity part of one face's flux, shared by every advected field:
+// flux = base (v0 + vm) - 1/3 (c (v0 - vm) - s dv), dv the difference across
+// the upwind neighbour face (Advection.cpp:36-50, :107-118 with the terms that
+// the wind's sign makes zero left out); c = s = 0 next to the boundaries.
 template <typename T>
-__device__ __forceinline__ void k_pzeta_body(const PZetaArgs<T>& a) {
-    constexpr int BX = kPZBX, BZ = kPZBZ, NT = BX * BZ;
-    __shared__ PZetaShared<T> S;
-    const Dims& d = a.d;
-    const int tx = threadIdx.x, ty = threadIdx.y, tid = tx + BX * ty;
-    const int i0 = 1 + blockIdx.x * BX, k0 = 2 + blockIdx.y * BZ;
-    const int i = i0 + tx, k = k0 + ty;
-    const bool act = (i <= d.nx - 2 && k <= d.nz - 2);
-
-    // Stage: points outside the array are skipped; none of them is read (a
-    // flux reads its outer neighbours only where the third-order bracket
-    // applies, 2 <= index <= n-3).
-    auto stage = [&](T* dst, const T* src, int rows, int cols, int kb, int ib) {
-        for (int t = tid; t < rows * cols; t += NT) {
-            const int r = t / cols, c = t - r * cols;
-            const int kk = kb + r, ii = ib + c;
-            if (kk >= 0 && kk <= d.nz - 1 && ii >= 0 && ii <= d.nx - 1) cp_async_elem(dst + t, src + d.at(ii, kk));
-        }
-    };
-    stage(&S.z[0][0], a.zeta, BZ + 4, BX + 4, k0 - 2, i0 - 2);
-    stage(&S.u[0][0], a.u, BZ + 1, BX + 4, k0 - 1, i0 - 2);
-    stage(&S.w[0][0], a.w, BZ + 4, BX + 1, k0 - 2, i0 - 1);
-    const T* qs[4] = {a.th, a.qv, a.qc, a.qr};
-#pragma unroll
-    for (int f = 0; f < 4; f++) stage(&S.q[f][0][0], qs[f], BZ + 1, BX + 1, k0 - 1, i0 - 1);
-    cp_async_commit();
-    cp_async_wait<0>();
-    __syncthreads();
-
-    // Uw(fi, k), fi = 0..nx-2, and Wu(i, fk), fk = 1..nz-2 (Advection.cpp:90-91)
-    for (int t = tid; t < BZ * (BX + 3); t += NT) {
-        const int r = t / (BX + 3), c = t - r * (BX + 3);
-        const int fi = i0 - 2 + c, kk = k0 + r;
-        if (fi >= 0 && fi <= d.nx - 2 && kk <= d.nz - 2) {
-            const int uc = c, ur = r + 1;   // u at (fi, kk) in the staged tile
-            S.U[r][c] = T(0.25) * (T(a.p.rhou[kk]) * (S.u[ur][uc + 1] + S.u[ur][uc]) +
-                                   T(a.p.rhou[kk - 1]) * (S.u[ur - 1][uc + 1] + S.u[ur - 1][uc]));
-        }
+struct Face {
+    T base, c, s;
+    bool pos;   // wind towards +
+};
+// base: the face's mass flux; mm, mp: the densities times winds vm, vp of the
+// neighbour faces on either side enter as mm * vm, mp * vp.
+template <typename T>
+__device__ __forceinline__ Face<T> face_of(bool hi, T base, T mm, T vm, T mp, T vp) {
+    Face<T> F;
+    F.base = base;
+    F.pos = base > T(0);
+    F.c = F.s = T(0);
+    if (hi) {
+        F.c = fabs(base);
+        F.s = sqrt(fabs(base * (F.pos ? mm : mp) * (F.pos ? plus_part(vm) : minus_part(vp))));
     }
-    for (int t = tid; t < (BZ + 3) * BX; t += NT) {
-        const int r = t / BX, c = t - r * BX;
-        const int fk = k0 - 2 + r, ii = i0 + c;
-        if (fk >= 1 && fk <= d.nz - 2 && ii <= d.nx - 2) {
-            const int wc = c + 1, wr = r;   // w at (ii, fk)
-            S.W[r][c] = T(0.25) * (T(a.p.rhow[fk + 1]) * (S.w[wr + 1][wc] + S.w[wr + 1][wc - 1]) +
-                                   T(a.p.rhow[fk]) * (S.w[wr][wc] + S.w[wr][wc - 1]));
-        }
-    }
-    __syncthreads();
-
-    // x flux at face (fi+1/2, k), fi = 1..nx-2 (Advection.cpp:107,111-114);
-    // the west face of point 1 is the halo copy of face nx-2 (Advection.cpp:123)
-    for (int t = tid; t < BZ * (BX + 1); t += NT) {
-        const int r = t / (BX + 1), c = t - r * (BX + 1);
-        const int fi = i0 - 1 + c, kk = k0 + r;
-        if (kk > d.nz - 2 || fi > d.nx - 2) continue;
-        T f;
-        if (fi == 0) {
-            const int e = d.nx - 2;   // no bracket at nx-2
-            f = zeta_Uw(a, e, kk) * (a.zeta[d.at(e + 1, kk)] + a.zeta[d.at(e, kk)]);
-        } else {
-            const T U = S.U[r][c + 1];
-            const T* zr = &S.z[r + 2][c];   // zeta at fi-1 .. fi+2
-            f = U * (zr[2] + zr[1]);
-            if (fi >= 2 && fi <= d.nx - 3 && kk >= 2 && kk <= d.nz - 3) {
-                const T Um = S.U[r][c], Up = S.U[r][c + 2];
-                const T z0 = zr[0], z1 = zr[1], z2 = zr[2], z3 = zr[3];
-                f += T(-1. / 3.) * (plus_part(U) * (z2 - z1) - sqrt(plus_part(U) * plus_part(Um)) * (z1 - z0) -
-                                    minus_part(U) * (z2 - z1) - sqrt(fabs(minus_part(U) * minus_part(Up))) * (z3 - z2));
-            }
-        }
-        S.fu[r][c] = f;
-    }
-    // z flux at face (i, fk+1/2), fk = 1..nz-2 (Advection.cpp:108,115-118)
-    for (int t = tid; t < (BZ + 1) * BX; t += NT) {
-        const int r = t / BX, c = t - r * BX;
-        const int fk = k0 - 1 + r, ii = i0 + c;
-        if (fk > d.nz - 2 || ii > d.nx - 2) continue;
-        const T W = S.W[r + 1][c];
-        const int zc = c + 2, zr = r + 1;   // zeta (ii, fk) in the staged tile
-        T f = W * (S.z[zr + 1][zc] + S.z[zr][zc]);
-        if (ii >= 2 && ii <= d.nx - 3 && fk >= 2 && fk <= d.nz - 3) {
-            const T Wm = S.W[r][c], Wp = S.W[r + 2][c];
-            const T z0 = S.z[zr - 1][zc], z1 = S.z[zr][zc], z2 = S.z[zr + 1][zc], z3 = S.z[zr + 2][zc];
-            f += T(-1. / 3.) * (plus_part(W) * (z2 - z1) - sqrt(plus_part(W) * plus_part(Wm)) * (z1 - z0) -
-                                minus_part(W) * (z2 - z1) - sqrt(fabs(minus_part(W) * minus_part(Wp))) * (z3 - z2));
-        }
-        S.fw[r][c] = f;
-    }
-    __syncthreads();
-    if (!act) return;
-
-    const size_t id = d.at(i, k);
-    const T dt15 = T(1.5 * a.c.dt), dt05 = T(0.5 * a.c.dt);
-    const T fu_i = S.fu[ty][tx + 1], fu_m = S.fu[ty][tx];
-    const T fw_k = S.fw[ty + 1][tx], fw_m = S.fw[ty][tx];
-    T rw = T(a.p.rhow[k]);
-    T px = (fu_i - fu_m) * T(a.c.r2dx) / rw;
-    T pz = (fw_k - fw_m) * T(a.p.r2dzw[k]) / rw;
-    T tz = -px - pz;
-    T oz = ab2_push(a.hz_n, a.hz_o, id, tz, a.ab);
-    T zp = S.z[ty + 2][tx + 2] + dt15 * tz - dt05 * oz;
-    // Bouyancy (Buoyancy.cpp:25-48); staged q[f][r][c] is (i0-1+c, k0-1+r)
-    const int r1 = ty + 1, r0 = ty, c1 = tx + 1, c0 = tx;
-    auto Q = [&](int f, int r, int c) { return S.q[f][r][c]; };
-    T g_rw = T(a.c.gravity) / rw;
-    T b;
-    if constexpr (!kPert<T>) {
-        auto thv = [&](int r, int c) { return Q(0, r, c) * (T(1) + T(0.608) * Q(1, r, c)); };   // Buoyancy.cpp:3-9
-        b = g_rw * T(0.5) *
-            ((thv(r1, c1) - thv(r1, c0)) / T(a.p.thvb[k]) + (thv(r0, c1) - thv(r0, c0)) / T(a.p.thvb[k - 1])) *
-            T(a.c.rdx);
-    } else {
-        // thv(i) - thv(i-1) from perturbations th', qv' about th0(k), qv0(k):
-        // dth' + 0.608 (th0 dqv' + qv0 dth' + (th'q')_i - (th'q')_{i-1}); the
-        // large reference values never enter a difference
-        auto thv_dx = [&](int r, int kk) {
-            T t1 = Q(0, r, c1), t0 = Q(0, r, c0), q1 = Q(1, r, c1), q0 = Q(1, r, c0);
-            T dt = t1 - t0, dq = q1 - q0;
-            return dt + T(0.608) * (T(a.p.ref[0][kk]) * dq + T(a.p.ref[1][kk]) * dt + (t1 * q1 - t0 * q0));
-        };
-        b = g_rw * T(0.5) * (thv_dx(r1, k) / T(a.p.thvb[k]) + thv_dx(r0, k - 1) / T(a.p.thvb[k - 1])) * T(a.c.rdx);
-    }
-    T bc = g_rw * (T(0.5) * (Q(2, r1, c1) + Q(2, r0, c1)) - T(0.5) * (Q(2, r1, c0) + Q(2, r0, c0))) * T(a.c.rdx);
-    T br = g_rw * (T(0.5) * (Q(3, r1, c1) + Q(3, r0, c1)) - T(0.5) * (Q(3, r1, c0) + Q(3, r0, c0))) * T(a.c.rdx);
-    T tb = b + (-bc - br);
-    T ob = ab2_push(a.hb_n, a.hb_o, id, tb, a.ab);
-    zp += (dt15 * tb) - (dt05 * ob);
-    store_westdown(a.zetap, d, i, k, zp);
+    return F;
 }
 template <typename T>
-__global__ void __launch_bounds__(kPZBX * kPZBZ) k_pzeta(PZetaArgs<T> a) { k_pzeta_body<T>(a); }
+__device__ __forceinline__ T face_flux(const Face<T>& F, T d, T dm, T dp, T sum) {
+    return F.base * sum + T(-1. / 3.) * (F.c * d - F.s * (F.pos ? dm : dp));
+}
+
+template <typename T, int R>
+struct PZetaShared {
+    static constexpr int BZ = tile_rows(R), VZ = BZ + 4;
+    T v[7][VZ][kTileVX];     // zeta, u, w, th, qv, qc, qr: rows k0-2..
+    // rows k0-2 .. k0+BZ+2: rhou, rhow, r2dx / rhow, r2dzw / rhow, g / rhow,
+    // thvb; mixed: the reference th0, qv0
+    T row[BZ + 5][kPert<T> ? 8 : 6];
+};
+
+template <typename T, int R>
+__device__ __forceinline__ void k_pzeta_body(const FieldMaps<7>& maps, const PZetaArgs<T>& a) {
+    using Sh = PZetaShared<T, R>;
+    constexpr int BZ = Sh::BZ, VZ = Sh::VZ, VX = kTileVX, AL = 16 / sizeof(T);
+    extern __shared__ __align__(128) unsigned char pzeta_smem[];
+    __shared__ uint64_t stage_bar;
+    Sh& S = *reinterpret_cast<Sh*>(pzeta_smem);
+    const Dims& d = a.d;
+    const int lane = threadIdx.x, wid = threadIdx.y, tid = lane + kTileLanes * wid;
+    const int i0 = 1 + blockIdx.x * kTileBX, k0 = 2 + blockIdx.y * BZ;
+    const int x0 = (i0 - 2) & ~(AL - 1);
+    const int i = i0 - 1 + lane;   // the lane's face, and the point west of it
+
+    const uint32_t bar = smem_u32(&stage_bar);
+    if (tid == 0) mbar_init1(bar);
+    __syncthreads();
+    if (tid == 0) {
+        mbar_expect_tx(bar, 7 * VZ * VX * sizeof(T));
+#pragma unroll
+        for (int f = 0; f < 7; f++) tma_load_2d(smem_u32(&S.v[f][0][0]), &maps.m[f], x0, k0 - 2, bar);
+    }
+    for (int t = tid; t < BZ + 5; t += kTileLanes * kTileWarps) {
+        const int k = k0 - 2 + t;
+        if (k > d.nz - 1) break;
+        T* r = S.row[t];
+        r[0] = T(a.p.rhou[k]);
+        r[1] = T(a.p.rhow[k]);
+        r[2] = T(a.c.r2dx) / r[1];
+        r[3] = T(a.p.r2dzw[k]) / r[1];
+        r[4] = T(a.c.gravity) / r[1];
+        r[5] = T(a.p.thvb[k]);
+        if constexpr (kPert<T>) {
+            r[6] = T(a.p.ref[0][k]);
+            r[7] = T(a.p.ref[1][k]);
+        }
+    }
+    const bool ok = mbar_wait_bounded(bar, 0);
+    if (__syncthreads_or(!ok)) {   // the copies never landed: report and leave
+        if (tid == 0 && a.err) atomicOr(a.err, kStageErrWait);
+        mbar_wait_bounded(bar, 0);
+        return;
+    }
+
+    const int c = i - x0;
+    const bool point = lane >= 1 && i <= d.nx - 2;
+    const bool wrap = (i == 0);    // the west face of point 1: the halo copy of face nx-2 (Advection.cpp:123)
+    const bool xhi = i >= 2 && i <= d.nx - 3;
+    const T dt15 = T(1.5 * a.c.dt), dt05 = T(0.5 * a.c.dt);
+    const T* const zeta = &S.v[0][0][c];
+    const T* const u = &S.v[1][0][c];
+    const T* const w = &S.v[2][0][c];
+    auto row = [&](int k) { return S.row[k - k0 + 2]; };
+    auto at = [&](int k) { return (k - k0 + 2) * VX; };
+    auto su = [&](int k, int e) { return row(k)[0] * (u[at(k) + e + 1] + u[at(k) + e]); };    // rhou (u_{i+1} + u_i) at i + e
+    auto sw = [&](int k) { return row(k)[1] * (w[at(k)] + w[at(k) - 1]); };                  // rhow (w_i + w_{i-1})
+    // flux_w at face k (between rows k and k+1) from Wu there and beside it
+    auto zflux = [&](int k, T Wm, T W, T Wp) {
+        const T* z = zeta + at(k);
+        const Face<T> F = face_of(xhi && k >= 2 && k <= d.nz - 3, W, T(1), Wm, T(1), Wp);
+        return face_flux(F, z[VX] - z[0], z[0] - z[-VX], z[2 * VX] - z[VX], z[VX] + z[0]);
+    };
+    // (thv_i - thv_{i-1}) / thvb of row k (Buoyancy.cpp:3-9, :25-28)
+    auto thv_dx = [&](int k) {
+        const T *th = &S.v[3][0][c] + at(k), *qv = &S.v[4][0][c] + at(k), *r = row(k);
+        if constexpr (!kPert<T>) {
+            return (th[0] * (T(1) + T(0.608) * qv[0]) - th[-1] * (T(1) + T(0.608) * qv[-1])) / r[5];
+        } else {
+            // from perturbations th', qv' about th0(k), qv0(k): dth' + 0.608
+            // (th0 dqv' + qv0 dth' + (th'q')_i - (th'q')_{i-1}); the large
+            // reference values never enter a difference
+            const T dth = th[0] - th[-1], dq = qv[0] - qv[-1];
+            return (dth + T(0.608) * (r[6] * dq + r[7] * dth + (th[0] * qv[0] - th[-1] * qv[-1]))) / r[5];
+        }
+    };
+    const int ka = k0 + wid * R;
+    if (ka > d.nz - 2) return;
+    T um = su(ka - 1, -1), u0 = su(ka - 1, 0), up = su(ka - 1, 1);   // the row below
+    T w1 = sw(ka), w2 = sw(ka + 1);
+    T Wm = T(0.25) * (w1 + sw(ka - 1)), W = T(0.25) * (w2 + w1);     // Wu at faces ka-1, ka
+    T fz = zflux(ka - 1, T(0.25) * (sw(ka - 1) + sw(ka - 2)), Wm, W);
+    T D = thv_dx(ka - 1);
+#pragma unroll 1
+    for (int j = 0; j < R; j++) {
+        const int k = ka + j;
+        if (k > d.nz - 2) break;   // uniform over the warp
+        const T* r = row(k);
+        const size_t id = d.at(i, k);
+        T oz = T(0), ob = T(0);
+        if (point && !a.ab.first) {   // the previous tendencies, in flight during the fluxes
+            oz = a.hz_o[id];
+            ob = a.hb_o[id];
+        }
+        // x face (i+1/2, k)
+        const T vm = su(k, -1), v0 = su(k, 0), vp = su(k, 1);
+        const T* z = zeta + at(k);
+        T U = T(0.25) * (v0 + u0), z1 = z[0], z2 = z[1];
+        if (wrap) {
+            const int e = d.nx - 2;
+            U = T(0.25) * (r[0] * (a.u[d.at(e + 1, k)] + a.u[d.at(e, k)]) + row(k - 1)[0] * (a.u[d.at(e + 1, k - 1)] + a.u[d.at(e, k - 1)]));
+            z1 = a.zeta[d.at(e, k)];
+            z2 = a.zeta[d.at(e + 1, k)];
+        }
+        const Face<T> F = face_of(xhi && k <= d.nz - 3, U, T(1), T(0.25) * (vm + um), T(1), T(0.25) * (vp + up));
+        const T fu = face_flux(F, z2 - z1, z1 - z[-1], z[2] - z2, z2 + z1);
+        um = vm;
+        u0 = v0;
+        up = vp;
+        // z face (i, k+1/2)
+        const T w3 = k + 2 <= d.nz - 1 ? sw(k + 2) : T(0);
+        const T Wp = T(0.25) * (w3 + w2);
+        const T fk = zflux(k, Wm, W, Wp);
+        Wm = W;
+        W = Wp;
+        w2 = w3;
+        const T px = (fu - __shfl_up_sync(0xffffffffu, fu, 1)) * r[2], pz = (fk - fz) * r[3];
+        fz = fk;
+        // Bouyancy (Buoyancy.cpp:25-48)
+        const T Dk = thv_dx(k);
+        const T *qc = &S.v[5][0][c] + at(k), *qr = &S.v[6][0][c] + at(k);
+        const T b = r[4] * T(0.5) * (Dk + D) * T(a.c.rdx);
+        const T bc = r[4] * (T(0.5) * (qc[0] + qc[-VX]) - T(0.5) * (qc[-1] + qc[-VX - 1])) * T(a.c.rdx);
+        const T br = r[4] * (T(0.5) * (qr[0] + qr[-VX]) - T(0.5) * (qr[-1] + qr[-VX - 1])) * T(a.c.rdx);
+        D = Dk;
+        if (!point) continue;
+        const T tz = -px - pz, tb = b + (-bc - br);
+        if (a.ab.first) {
+            a.hz_o[id] = oz = tz;
+            a.hb_o[id] = ob = tb;
+        }
+        a.hz_n[id] = tz;
+        a.hb_n[id] = tb;
+        T zp = z[0] + dt15 * tz - dt05 * oz;
+        zp += (dt15 * tb) - (dt05 * ob);
+        store_westdown(a.zetap, d, i, k, zp);
+    }
+}
+// Blocks a SM: what shared memory holds at the rows a thread of pzeta_rows.
+template <typename T, int R>
+__global__ void __launch_bounds__(kTileLanes* kTileWarps, 4)
+    k_pzeta(const __grid_constant__ FieldMaps<7> maps, PZetaArgs<T> a) {
+    k_pzeta_body<T, R>(maps, a);
+}
 
 // ---------------------------------------------------------------------------
 // Scalar advection (Advection_thermo, Advection.cpp:25-81) of th, qv, qc, qr,
@@ -293,11 +337,6 @@ struct PAdvArgs {
     int nvp_mask;      // F_* fields whose NVP sums are wanted
     int do_precip;     // surface rain diagnostic (with F_QR)
     AB2 ab;
-};
-
-// The tensor maps of th, qv, qc, qr, u, w (box kPAdvVX by the tile's staged rows).
-struct PAdvMaps {
-    CUtensorMap m[6];
 };
 
 // Final sums of NegativeValueProcess and its rescaling factor
@@ -353,65 +392,30 @@ __global__ void k_nvp_final(const double* partial, int nblocks, double* nvp);
 // Bound by instruction issue: 35 us at 2048 x 256 FP64 and 89 at 8192 x 256,
 // from 51 and 179 with two roots, a division a term, every flux through shared
 // memory and a reduction a cell (FP32 44 -> 23).
-constexpr int kPAdvLanes = 32, kPAdvWarps = 8, kPAdvBX = 31;
-constexpr int kStageErrWait = 4;   // device error word: a stencil's TMA staging wait gave up
-// The staged box of one field: rows k0-2 .. k0+BZ+1 and 40 columns from the
-// halo's first one, i0-2, rounded down to a 16-byte boundary (TMA requires x *
-// element size to be a multiple of 16).
-constexpr int kPAdvVX = 40;
-constexpr int padv_rows(int R) { return kPAdvWarps * R; }
-
 template <typename T, int R>
 struct PAdvShared {
-    static constexpr int BZ = padv_rows(R), VZ = BZ + 4;
-    T v[6][VZ][kPAdvVX];     // th, qv, qc, qr, u, w: each box a multiple of 128 bytes
+    static constexpr int BZ = tile_rows(R), VZ = BZ + 4;
+    T v[6][VZ][kTileVX];     // th, qv, qc, qr, u, w: each box a multiple of 128 bytes
     // rows k0-1 .. k0+BZ+1: rhou, rhow, r2dx / rhou, r2dzc / rhou, vt_c1,
     // vt_fac; mixed, of th0 and qv0: 2 ref, s0, g0, d0
     T row[BZ + 3][kPert<T> ? 14 : 6];
-    double red[kPAdvWarps][6];
+    double red[kTileWarps][6];
 };
-
-// The velocity part of one face's flux, shared by every advected field:
-// flux = base (v0 + vm) - 1/3 (c (v0 - vm) - s dv), dv the difference across
-// the upwind neighbour face (Advection.cpp:36-50 with the terms that the
-// wind's sign makes zero left out); c = s = 0 next to the boundaries.
-template <typename T>
-struct Face {
-    T base, c, s;
-    bool pos;   // wind towards +
-};
-// m the face's density, mm and mp the neighbour faces'; v its wind, vm and vp theirs.
-template <typename T>
-__device__ __forceinline__ Face<T> face_of(bool hi, T m, T mm, T mp, T v, T vm, T vp) {
-    Face<T> F;
-    F.base = m * v;
-    F.pos = v > T(0);
-    F.c = F.s = T(0);
-    if (hi) {
-        F.c = fabs(F.base);
-        F.s = sqrt(fabs(F.base * (F.pos ? mm : mp) * (F.pos ? plus_part(vm) : minus_part(vp))));
-    }
-    return F;
-}
-template <typename T>
-__device__ __forceinline__ T face_flux(const Face<T>& F, T d, T dm, T dp, T sum) {
-    return F.base * sum + T(-1. / 3.) * (F.c * d - F.s * (F.pos ? dm : dp));
-}
 
 // MASK: the F_* fields advected; NVP sums and the precipitation go with it
 // (a.nvp_mask, a.do_precip). maps: the tensor maps of th, qv, qc, qr, u, w,
 // read where they lie (a kernel parameter, or global memory for a grouped
 // launch): TMA takes their addresses.
 template <typename T, int MASK, int R>
-__device__ __forceinline__ void k_padv_body(const PAdvMaps& maps, const PAdvArgs<T>& a) {
+__device__ __forceinline__ void k_padv_body(const FieldMaps<6>& maps, const PAdvArgs<T>& a) {
     using Sh = PAdvShared<T, R>;
-    constexpr int BZ = Sh::BZ, VZ = Sh::VZ, VX = kPAdvVX, AL = 16 / sizeof(T);
+    constexpr int BZ = Sh::BZ, VZ = Sh::VZ, VX = kTileVX, AL = 16 / sizeof(T);
     extern __shared__ __align__(128) unsigned char padv_smem[];
     __shared__ uint64_t stage_bar;
     Sh& S = *reinterpret_cast<Sh*>(padv_smem);
     const Dims& d = a.d;
-    const int lane = threadIdx.x, wid = threadIdx.y, tid = lane + kPAdvLanes * wid;
-    const int i0 = 1 + blockIdx.x * kPAdvBX, k0 = 1 + blockIdx.y * BZ;
+    const int lane = threadIdx.x, wid = threadIdx.y, tid = lane + kTileLanes * wid;
+    const int i0 = 1 + blockIdx.x * kTileBX, k0 = 1 + blockIdx.y * BZ;
     const int x0 = (i0 - 2) & ~(AL - 1);
     const int i = i0 + lane;
 
@@ -427,7 +431,7 @@ __device__ __forceinline__ void k_padv_body(const PAdvMaps& maps, const PAdvArgs
         for (int f = 0; f < 6; f++)
             if (f >= 4 || (MASK & (1 << f))) tma_load_2d(smem_u32(&S.v[f][0][0]), &maps.m[f], x0, k0 - 2, bar);
     }
-    for (int t = tid; t < BZ + 3; t += kPAdvLanes * kPAdvWarps) {
+    for (int t = tid; t < BZ + 3; t += kTileLanes * kTileWarps) {
         const int k = k0 - 1 + t;
         if (k > d.nz - 1) break;
         T* r = S.row[t];
@@ -455,7 +459,7 @@ __device__ __forceinline__ void k_padv_body(const PAdvMaps& maps, const PAdvArgs
     }
 
     const int c = i0 - x0 + lane;                 // the lane's column in the tile
-    const bool cell = lane < kPAdvBX && i <= d.nx - 2;
+    const bool cell = lane < kTileBX && i <= d.nx - 2;
     const bool wrap = (i == d.nx - 1);            // the east face of cell nx-2: the halo copy of face 1
     const bool xhi = i >= 2 && i <= d.nx - 3;
     constexpr bool vt = (MASK & F_QR) != 0;       // sedimentation goes with qr
@@ -473,7 +477,7 @@ __device__ __forceinline__ void k_padv_body(const PAdvMaps& maps, const PAdvArgs
         const bool top = k > d.nz - 2;
         if (!top) {
             const T wk = w[at];
-            F = face_of(hi, q[1], S.row[k - k0][1], S.row[k - k0 + 2][1], wk, w[at - VX], w[at + VX]);
+            F = face_of(hi, q[1] * wk, S.row[k - k0][1], w[at - VX], S.row[k - k0 + 2][1], w[at + VX]);
         }
 #pragma unroll
         for (int f = 0; f < 4; f++) {
@@ -516,7 +520,7 @@ __device__ __forceinline__ void k_padv_body(const PAdvMaps& maps, const PAdvArgs
             if (vt) ovt = a.hvt_o[id];
         }
         // x face west of the cell (or, at nx-1, face 1, from where it lies)
-        Face<T> F = face_of(xhi && k >= 2 && k <= d.nz - 3, q[0], q[0], q[0], wrap ? a.u[d.at(1, k)] : u[at], u[at - 1], u[at + 1]);
+        const Face<T> F = face_of(xhi && k >= 2 && k <= d.nz - 3, q[0] * (wrap ? a.u[d.at(1, k)] : u[at]), q[0], u[at - 1], q[0], u[at + 1]);
         T fu[4], zu[4], gu;
 #pragma unroll
         for (int f = 0; f < 4; f++) {
@@ -594,7 +598,7 @@ __device__ __forceinline__ void k_padv_body(const PAdvMaps& maps, const PAdvArgs
         __syncthreads();
         if (tid < 6) {
             double t = 0.0;
-            for (int q = 0; q < kPAdvWarps; q++) t += S.red[q][tid];
+            for (int q = 0; q < kTileWarps; q++) t += S.red[q][tid];
             a.partial[(size_t)(blockIdx.x + gridDim.x * blockIdx.y) * 6 + tid] = t;
         }
     }
@@ -603,8 +607,8 @@ __device__ __forceinline__ void k_padv_body(const PAdvMaps& maps, const PAdvArgs
 template <typename T>
 constexpr int kPAdvMinBlocks = sizeof(T) == 8 ? 3 : 4;
 template <typename T, int MASK, int R>
-__global__ void __launch_bounds__(kPAdvLanes* kPAdvWarps, kPAdvMinBlocks<T>)
-    k_padv(const __grid_constant__ PAdvMaps maps, PAdvArgs<T> a) {
+__global__ void __launch_bounds__(kTileLanes* kTileWarps, kPAdvMinBlocks<T>)
+    k_padv(const __grid_constant__ FieldMaps<6> maps, PAdvArgs<T> a) {
     k_padv_body<T, MASK, R>(maps, a);
 }
 
@@ -724,9 +728,8 @@ struct KesslerArgs {
     T *thp, *qvp, *qcp, *qrp;
     T* out[4];        // where th, qv, qc, qr go (in place, or the diffusion's inputs)
     int halo;         // write their ghost images too
-    T *d_auto, *d_accr, *d_evap, *d_cond;  // diagnostics (may be null)
-    double* partial;
-    int nvp;  // accumulate NVP sums
+    double* partial;  // NVP sums of each block
+    int rows;         // rows a thread
     // The finish of the advection step (k_apply's rescaling and forcing of
     // th, qv, qc, qr) applied to each value as it is read, in place of a
     // k_apply launch whose halo images the apply after Kessler rewrites.
@@ -734,10 +737,12 @@ struct KesslerArgs {
     int do_pre;
 };
 
-// One cell of Kessler warm rain in compute type C; writes the four rates.
+// One cell of Kessler warm rain in compute type C.
+// Cells without rain (or, for the accretion, without cloud) have rates that
+// are exactly zero there, so their pow and exp are left out; lvcp = lv / (cp pib).
 template <typename C>
 __device__ __forceinline__ void kessler_cell(C& th, C& qv, C& qc, C& qr, C dt, C lv, C cp, C pib, C rhou,
-                                             C pc, C pb, C rates[4]) {
+                                             C pc, C pb, C lvcp) {
     {   // autoconversion
         C qcplus = smax(C(0), qc);
         C ar = C(0.001) * (qcplus - C(0.001));
@@ -745,18 +750,20 @@ __device__ __forceinline__ void kessler_cell(C& th, C& qv, C& qc, C& qr, C dt, C
         C arcrdt = smin(ar * dt, qcplus);
         qc = qc - arcrdt;
         qr = qr + arcrdt;
-        rates[0] = arcrdt;
     }
     {   // accretion
         C qcplus = smax(C(0), qc), qrplus = smax(C(0), qr);
-        C cr = C(2.2) * qcplus * (pow(qrplus, C(0.875)));
-        C arcrdt = smin(cr * dt, qcplus);
+        C arcrdt = C(0);
+        if (qcplus != C(0) && qrplus != C(0)) {
+            C cr = C(2.2) * qcplus * (pow(qrplus, C(0.875)));
+            arcrdt = smin(cr * dt, qcplus);
+        }
         qc = qc - arcrdt;
         qr = qr + arcrdt;
-        rates[1] = arcrdt;
     }
-    {   // evaporation of rain
-        C qrplus = smax(C(0), qr), qvplus = smax(C(0), qv);
+    C qrplus = smax(C(0), qr);
+    if (qrplus != C(0)) {   // evaporation of rain
+        C qvplus = smax(C(0), qv);
         C qvs = pc * exp(C(17.27) * (pib * th - C(273.)) / (pib * th - C(36.)));
         C deficit = smax((C(1.) - qvplus / qvs), C(0.));
         C coef = C(1.6) + C(124.9) * pow((C(1E-3) * rhou * qrplus), C(0.2046));
@@ -765,8 +772,7 @@ __device__ __forceinline__ void kessler_cell(C& th, C& qv, C& qc, C& qr, C dt, C
         C erdt = smin(qrplus, smax(C(0.), er * dt));
         qr = qr - erdt;
         qv = qv + erdt;
-        th = th - lv * erdt / (cp * pib);
-        rates[2] = erdt;
+        th = th - lvcp * erdt;
     }
     {   // saturation adjustment
         C qvs = pc * exp(C(17.27) * (pib * th - C(273.)) / (pib * th - C(36.)));
@@ -776,24 +782,34 @@ __device__ __forceinline__ void kessler_cell(C& th, C& qv, C& qc, C& qr, C dt, C
         if (fabs(cnd) > qc && cnd < C(0)) cnd = -qc;
         qv = qv - cnd;
         qc = qc + cnd;
-        th = th + lv / (cp * pib) * cnd;
-        rates[3] = cnd;
+        th = th + lvcp * cnd;
     }
 }
 
 // The mixed step runs this kernel's arithmetic in FP64 on its FP32 storage:
 // the saturation adjustment subtracts qvs from qv, which cancel to a few
 // units of the FP32 epsilon near saturation.
+// A block of 32 x 8 threads takes 32 columns by 8 a.rows rows, a thread a.rows
+// of a column, and reduces the sums once for them. Bound by instruction issue
+// and its latencies (FP64 exp, divisions; pow in rain), so registers are held
+// to four blocks a SM (a few spills; 24.6, 21.9, 18.9 us at two, three, four):
+// 26 -> 19 us at 2048 x 256, 81 -> 50 at 8192 x 256, with rain in a small part
+// of the grid.
+constexpr int kKesslerWarps = 8;
 template <typename T>
 __device__ __forceinline__ void k_kessler_body(const KesslerArgs<T>& a) {
     using C = double;
-    __shared__ double sh[32 * 6];
+    __shared__ double red[kKesslerWarps][6];
     const Dims& d = a.d;
-    const int i = 1 + blockIdx.x * blockDim.x + threadIdx.x;
-    const int k = 1 + blockIdx.y * blockDim.y + threadIdx.y;
-    const bool act = (i <= d.nx - 2 && k <= d.nz - 2);
+    const int lane = threadIdx.x, wid = threadIdx.y;
+    const int i = 1 + blockIdx.x * 32 + lane;
+    const int ka = 1 + (blockIdx.y * kKesslerWarps + wid) * a.rows;
     double sums[6] = {0, 0, 0, 0, 0, 0};
-    if (act) {
+#pragma unroll 1
+    for (int j = 0; j < a.rows; j++) {
+        const int k = ka + j;
+        if (k > d.nz - 2) break;   // uniform over the warp
+        if (i > d.nx - 2) continue;
         const size_t id = d.at(i, k);
         const C th0 = kPert<T> ? a.p.ref[0][k] : 0.0, qv0 = kPert<T> ? a.p.ref[1][k] : 0.0;
         T tv = a.thp[id], qvv = a.qvp[id], qcv = a.qcp[id], qrv = a.qrp[id];
@@ -805,41 +821,38 @@ __device__ __forceinline__ void k_kessler_body(const KesslerArgs<T>& a) {
             qrv = finish_value(a.pre, a.p, dt, 3, qrv, k, id);
         }
         C th = th0 + (C)tv, qv = qv0 + (C)qvv, qc = qcv, qr = qrv;
-        C rates[4];
         kessler_cell<C>(th, qv, qc, qr, a.c.dt, a.c.lv, a.c.cp, a.p.pib[k], a.p.rhou[k], a.p.pc[k], a.p.pb[k],
-                        rates);
-        if (a.d_auto) {
-            a.d_auto[id] = T(rates[0]);
-            a.d_accr[id] = T(rates[1]);
-            a.d_evap[id] = T(rates[2]);
-            a.d_cond[id] = T(rates[3]);
-        }
+                        a.p.lvcp[k]);
         const T res[4] = {T(th - th0), T(qv - qv0), T(qc), T(qr)};
 #pragma unroll
         for (int f = 0; f < 4; f++) {
             if (a.halo) store_center(a.out[f], d, i, k, res[f]);
             else a.out[f][id] = res[f];
         }
-        if (a.nvp) {
-            C q[3] = {qv, qc, qr};
+        const C q[3] = {qv, qc, qr};
 #pragma unroll
-            for (int f = 0; f < 3; f++) {
-                if (q[f] >= C(0)) sums[2 * f] += (double)q[f];
-                else sums[2 * f + 1] += (double)q[f];
-            }
+        for (int f = 0; f < 3; f++) {
+            if (q[f] >= C(0)) sums[2 * f] += q[f];
+            else sums[2 * f + 1] += q[f];
         }
     }
-    if (a.nvp) {
-        block_sum(sums, sh);
-        if (threadIdx.x == 0 && threadIdx.y == 0) {
-            double* out = a.partial + (size_t)(blockIdx.x + gridDim.x * blockIdx.y) * 6;
+    // the block's sums, in a fixed order
 #pragma unroll
-            for (int j = 0; j < 6; j++) out[j] = sums[j];
-        }
+    for (int m = 0; m < 6; m++) sums[m] = warp_sum(sums[m]);
+    if (lane == 0) {
+#pragma unroll
+        for (int m = 0; m < 6; m++) red[wid][m] = sums[m];
+    }
+    __syncthreads();
+    const int tid = lane + 32 * wid;
+    if (tid < 6) {
+        double t = 0.0;
+        for (int q = 0; q < kKesslerWarps; q++) t += red[q][tid];
+        a.partial[(size_t)(blockIdx.x + gridDim.x * blockIdx.y) * 6 + tid] = t;
     }
 }
 template <typename T>
-__global__ void k_kessler(KesslerArgs<T> a) { k_kessler_body<T>(a); }
+__global__ void __launch_bounds__(32 * kKesslerWarps, 4) k_kessler(KesslerArgs<T> a) { k_kessler_body<T>(a); }
 
 // ---------------------------------------------------------------------------
 // Eddy coefficients (Turbulence::RKM_RKH, Turbulent.cpp:5-45) with their

@@ -1534,7 +1534,6 @@ struct Fields {
     T *u = nullptr, *w = nullptr, *RKM = nullptr, *RKH = nullptr;
     T* pre[5] = {};   // zeta, th, qv, qc, qr as the diffusion reads them (it writes the future level)
     T* hist[NHIST][2] = {};
-    T *d_auto = nullptr, *d_accr = nullptr, *d_evap = nullptr, *d_cond = nullptr;
     T *precip = nullptr, *th_forcing = nullptr;
     T* gsA = nullptr;                                   // Gauss-Seidel constant terms, [5][cells]
     T *gsC = nullptr, *gsB = nullptr;                   // and coefficients (cluster schedule; on first use)
@@ -1597,7 +1596,7 @@ struct vvm_gpu_ctx {
     bool has_state = false, has_forcing_th = false, has_q = false;
     // profiles
     double *rhou = nullptr, *rhow = nullptr, *thvb = nullptr, *thb = nullptr, *qvb = nullptr,
-           *thb_init = nullptr, *qvb0 = nullptr, *pib = nullptr, *pb = nullptr, *lambda2 = nullptr,
+           *thb_init = nullptr, *qvb0 = nullptr, *pib = nullptr, *pb = nullptr, *lambda2 = nullptr, *lvcp = nullptr,
            *z = nullptr, *z_zeta = nullptr, *vt_c1 = nullptr, *vt_fac = nullptr, *pc = nullptr,
            *dtcgr_th = nullptr, *dtcgr_zeta = nullptr, *q1ls = nullptr, *q2ls = nullptr;
     double pf1 = 0, pf2 = 0;
@@ -1686,7 +1685,7 @@ struct vvm_gpu_ctx {
     }
 
     Profiles profiles() const {
-        return Profiles{rhou, rhow, thvb, thb_init, qvb0, pib, pb, lambda2, vt_c1, vt_fac, pc,
+        return Profiles{rhou, rhow, thvb, thb_init, qvb0, pib, pb, lambda2, vt_c1, vt_fac, pc, lvcp,
                         dtcgr_th, dtcgr_zeta, q1ls, q2ls, pf1, pf2,
                         {pref[0], pref[1]}, {pd0[0], pd0[1]}, {ps0[0], ps0[1]}, {pg0[0], pg0[1]},
                         {pdn[0], pdn[1]},
@@ -1737,10 +1736,6 @@ void alloc_fields(vvm_gpu_ctx* c) {
     for (int f = 1; f < 5; f++) F.pre[f] = F.pre[0] + f * n;
     for (int h = 0; h < NHIST; h++)
         for (int s = 0; s < 2; s++) F.hist[h][s] = c->ar.alloc<T>(n);
-    F.d_auto = c->ar.alloc<T>(n);
-    F.d_accr = c->ar.alloc<T>(n);
-    F.d_evap = c->ar.alloc<T>(n);
-    F.d_cond = c->ar.alloc<T>(n);
     F.precip = c->ar.alloc<T>(c->d.nx);
     F.th_forcing = c->ar.alloc<T>(n);
     F.gsA = c->ar.alloc<T>(5 * n);
@@ -1762,16 +1757,38 @@ T* zeta_pre(vvm_gpu_ctx* c) {
     return c->in_step ? F.pre[0] : F.zeta[1 - c->cur];
 }
 
-template <typename T>
-void launch_pzeta(vvm_gpu_ctx* c) {
+// Rows a thread of k_pzeta takes: two in FP64, four in FP32 (what leaves shared
+// memory for four or five blocks a SM), one where that gives fewer blocks than
+// there are SMs. us a launch with 1 / 2 / 4 rows: 8192 x 256 FP64 67 / 57 / 72,
+// FP32 46 / 46 / 42; 2048 x 256 FP64 23 / 22 / 24, FP32 18 / 17 / 16; 128 x 64
+// 10.6 / 12.1 / 14.0.
+template <typename T, int R>
+void launch_pzeta_r(vvm_gpu_ctx* c) {
     Fields<T>& F = fields<T>(c);
     int now = c->cur;
     AB2 ab = AB2::of(c->step);
     PZetaArgs<T> a{c->d, c->c, c->profiles(), F.zeta[now], F.u, F.w, F.th[now], F.qv[now], F.qc[now], F.qr[now],
                    zeta_pre<T>(c), F.hist[H_ZETA][ab.sn], F.hist[H_ZETA][ab.so], F.hist[H_BUOY][ab.sn],
-                   F.hist[H_BUOY][ab.so], ab};
-    dim3 g(cdiv(c->d.nx - 2, kPZBX), cdiv(c->d.nz - 3, kPZBZ));
-    klaunch<k_pzeta_body<T>, kPZBX * kPZBZ>(&c->stats, VVM_K_PZETA, c->stream, k_pzeta<T>, g, dim3(kPZBX, kPZBZ), 0, a);
+                   F.hist[H_BUOY][ab.so], c->d_err, ab};
+    const T* staged[7] = {a.zeta, a.u, a.w, a.th, a.qv, a.qc, a.qr};
+    FieldMaps<7> m;
+    for (int f = 0; f < 7; f++)
+        m.m[f] = field_map(staged[f], c->d.nx, c->d.nz, c->d.pitch, (int)sizeof(T), kTileVX, tile_rows(R) + 4);
+    const dim3 g(cdiv(c->d.nx - 2, kTileBX), cdiv(c->d.nz - 3, tile_rows(R))), blk(kTileLanes, kTileWarps);
+    if (c->stats.rec) {
+        TilePack<7, PZetaArgs<T>> p{m, a};
+        record_kernel(&c->stats, reinterpret_cast<const void*>(&k_pzeta_grouped<T, R>), g, blk, sizeof(PZetaShared<T, R>),
+                      &p, sizeof(p), alignof(decltype(p)));
+    } else {
+        LAUNCH(&c->stats, VVM_K_PZETA, c->stream, k_pzeta<T, R><<<g, blk, sizeof(PZetaShared<T, R>), c->stream>>>(m, a));
+        CKL();
+    }
+}
+template <typename T>
+void launch_pzeta(vvm_gpu_ctx* c) {
+    constexpr int R = sizeof(T) == 8 ? 2 : 4;
+    if (cdiv(c->d.nx - 2, kTileBX) * cdiv(c->d.nz - 3, tile_rows(R)) >= 148) launch_pzeta_r<T, R>(c);
+    else launch_pzeta_r<T, 1>(c);
 }
 
 // Rows a thread of k_padv takes: four share their z fluxes and amortise the
@@ -1779,7 +1796,7 @@ void launch_pzeta(vvm_gpu_ctx* c) {
 // 4 rows, FP64: 128 x 64 10.6 / 16.8; 8192 x 256 98.8 / 89.0, FP32 82.3 /
 // 66.0; the step of 512 x 128 84.1 / 82.0, of 2048 x 256 199.5 / 195.5).
 inline int padv_rows_a_thread(const Dims& d) {
-    return cdiv(d.nx - 2, kPAdvBX) * cdiv(d.nz - 2, padv_rows(4)) >= 64 ? 4 : 1;
+    return cdiv(d.nx - 2, kTileBX) * cdiv(d.nz - 2, tile_rows(4)) >= 64 ? 4 : 1;
 }
 
 // MASK: the fields advected. Surface rain and sedimentation go with qr.
@@ -1813,18 +1830,18 @@ void launch_padv(vvm_gpu_ctx* c) {
     a.err = c->d_err;
     constexpr int ALL = F_TH | F_QV | F_QC | F_QR;
     const int R = MASK == ALL ? padv_rows_a_thread(c->d) : 1;
-    const dim3 g(cdiv(c->d.nx - 2, kPAdvBX), cdiv(c->d.nz - 2, padv_rows(R))), blk(kPAdvLanes, kPAdvWarps);
-    PAdvMaps m;
+    const dim3 g(cdiv(c->d.nx - 2, kTileBX), cdiv(c->d.nz - 2, tile_rows(R))), blk(kTileLanes, kTileWarps);
+    FieldMaps<6> m;
     for (int f = 0; f < 6; f++)
-        m.m[f] = field_map(f < 4 ? a.now[f] : f == 4 ? a.u : a.w, c->d.nx, c->d.nz, c->d.pitch, (int)sizeof(T), kPAdvVX,
-                           padv_rows(R) + 4);
+        m.m[f] = field_map(f < 4 ? a.now[f] : f == 4 ? a.u : a.w, c->d.nx, c->d.nz, c->d.pitch, (int)sizeof(T), kTileVX,
+                           tile_rows(R) + 4);
     const size_t smem = R == 4 ? sizeof(PAdvShared<T, 4>) : sizeof(PAdvShared<T, 1>);
     if (c->stats.rec) {
         if (MASK != ALL) throw CudaError{"grouped launch: the advection of single fields has no grouped form"};
-        PAdvPack<T> p{m, a};
+        TilePack<6, PAdvArgs<T>> p{m, a};
         const void* fn = R == 4 ? reinterpret_cast<const void*>(&k_padv_grouped<T, 4>)
                                 : reinterpret_cast<const void*>(&k_padv_grouped<T, 1>);
-        record_kernel(&c->stats, fn, g, blk, smem, &p, sizeof(p), alignof(PAdvPack<T>));
+        record_kernel(&c->stats, fn, g, blk, smem, &p, sizeof(p), alignof(decltype(p)));
     } else if (MASK == ALL && R == 4) {
         LAUNCH(&c->stats, VVM_K_PADV, c->stream, k_padv<T, ALL, 4><<<g, blk, smem, c->stream>>>(m, a));
         CKL();
@@ -1887,7 +1904,11 @@ void launch_kessler(vvm_gpu_ctx* c) {
     int fut = 1 - c->cur;
     KesslerArgs<T> a{c->d, c->c, c->profiles(), F.th[fut], F.qv[fut], F.qc[fut], F.qr[fut],
                      {F.th[fut], F.qv[fut], F.qc[fut], F.qr[fut]}, 0,
-                     F.d_auto, F.d_accr, F.d_evap, F.d_cond, c->partial, 1};
+                     c->partial};
+    // two rows a thread where that still gives every SM a block (us a launch with
+    // 1 / 2 / 4 rows, FP64: 8192 x 256 56 / 50 / 50, 2048 x 256 20 / 19 / 23,
+    // 128 x 64 10.2 / 13.1 / 18.8)
+    a.rows = cdiv(c->d.nx - 2, 32) * cdiv(c->d.nz - 2, 2 * kKesslerWarps) >= 148 ? 2 : 1;
     if (c->in_step) {
         for (int f = 0; f < 4; f++) a.out[f] = F.pre[1 + f];
         a.halo = 1;
@@ -1899,8 +1920,9 @@ void launch_kessler(vvm_gpu_ctx* c) {
         // status_for_adding_forcing (Iteration.cpp:276-277), as launch_apply forms it
         a.pre.forcing_th = c->has_forcing_th && (c->step * c->desc.dt <= c->desc.addforcingtime);
     }
-    dim3 g = c->grid_interior(1);
-    klaunch<k_kessler_body<T>, 256>(&c->stats, VVM_K_KESSLER, c->stream, k_kessler<T>, g, c->blk(), 0, a);
+    const dim3 g(cdiv(c->d.nx - 2, 32), cdiv(c->d.nz - 2, kKesslerWarps * a.rows));
+    klaunch<k_kessler_body<T>, 32 * kKesslerWarps, 4>(&c->stats, VVM_K_KESSLER, c->stream, k_kessler<T>, g,
+                                                   dim3(32, kKesslerWarps), 0, a);
     klaunch<k_nvp_final_body, 1024>(&c->stats, VVM_K_APPLY, c->stream, k_nvp_final, dim3(1), dim3(1024), 0,
                                     (const double*)c->partial, (int)(g.x * g.y), c->nvp);
     if (!c->in_step) launch_apply<T>(c, F_QV | F_QC | F_QR, F_QV | F_QC | F_QR, false, false);
@@ -3707,11 +3729,12 @@ int upload_profiles(vvm_gpu_ctx* c, const vvm_gpu_host_state* s) {
     upload_profile(c, s->z_zeta, c->z_zeta);
     upload_profile(c, s->lambda2, c->lambda2);
     const vvm_gpu_desc& D = c->desc;
-    std::vector<double> vt1(nz), vtf(nz), pc(nz), cth(nz, 0.0), cze(nz, 0.0), q1(nz, 0.0), q2(nz, 0.0);
+    std::vector<double> vt1(nz), vtf(nz), pc(nz), lvcp(nz), cth(nz, 0.0), cze(nz, 0.0), q1(nz, 0.0), q2(nz, 0.0);
     for (int k = 0; k < nz; k++) {
         vt1[k] = 1E-3 * s->rhow[k] * 0.5;                            // Advection.cpp:165
         vtf[k] = std::pow(s->rhow[k] / s->rhow[1], -0.5);
         pc[k] = 380. / (std::pow(s->pib[k], D.cp / D.rd) * D.p0);    // MicroPhysics.cpp:10
+        lvcp[k] = D.lv / (D.cp * s->pib[k]);                         // MicroPhysics.cpp:24
     }
     // Vertical level metric of the stencils (the C restatement's levels(),
     // oracle/vvm_oracle.c, formula for formula): with dc[k] = 2 (z[k] -
@@ -3820,6 +3843,7 @@ int upload_profiles(vvm_gpu_ctx* c, const vvm_gpu_host_state* s) {
     upload_profile(c, vt1.data(), c->vt_c1);
     upload_profile(c, vtf.data(), c->vt_fac);
     upload_profile(c, pc.data(), c->pc);
+    upload_profile(c, lvcp.data(), c->lvcp);
     upload_profile(c, cth.data(), c->dtcgr_th);
     upload_profile(c, cze.data(), c->dtcgr_zeta);
     upload_profile(c, q1.data(), c->q1ls);
@@ -4101,7 +4125,7 @@ int vvm_gpu_create(const vvm_gpu_desc* desc, int device, vvm_gpu_ctx** out) {
         int nz = c->d.nz;
         double** profs[] = {&c->rhou, &c->rhow, &c->thvb, &c->thb, &c->qvb, &c->thb_init, &c->qvb0,
                             &c->pib, &c->pb, &c->lambda2, &c->z, &c->z_zeta, &c->vt_c1, &c->vt_fac,
-                            &c->pc, &c->dtcgr_th, &c->dtcgr_zeta, &c->q1ls, &c->q2ls, &c->rwres,
+                            &c->pc, &c->lvcp, &c->dtcgr_th, &c->dtcgr_zeta, &c->q1ls, &c->q2ls, &c->rwres,
                             &c->lv_r2dzc, &c->lv_r2dzw, &c->lv_rdzc, &c->lv_r2dzcc, &c->lv_kmax, &c->gsM_cz,
                             &c->gsM_rhod, &c->gsS_cz, &c->gsS_rhod, &c->lv_dzw};
         for (double** p : profs) *p = c->ar.alloc<double>(nz);
@@ -4115,9 +4139,10 @@ int vvm_gpu_create(const vvm_gpu_desc* desc, int device, vvm_gpu_ctx** out) {
         c->ubar = c->ar.alloc<double>(2);
         c->dubar = c->ar.alloc<double>(2);
         // block partials of k_padv and k_kessler (NegativeValueProcess sums)
-        dim3 g = c->grid_interior(1);
-        c->npart = std::max((int)(g.x * g.y), cdiv(D.NX, kPAdvBX) * cdiv(D.NZ, padv_rows(1)));
+        c->npart = std::max(cdiv(D.NX, 32) * cdiv(D.NZ, kKesslerWarps), cdiv(D.NX, kTileBX) * cdiv(D.NZ, tile_rows(1)));
         c->partial = c->ar.alloc<double>((size_t)c->npart * 6);
+        CK(cudaFuncSetAttribute(k_pzeta<double, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(PZetaShared<double, 2>)));
+        CK(cudaFuncSetAttribute(k_pzeta<float, 4>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(PZetaShared<float, 4>)));
         CK(cudaFuncSetAttribute(k_padv<double, F_TH | F_QV | F_QC | F_QR, 4>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                 (int)sizeof(PAdvShared<double, 4>)));
         c->nvp = c->ar.alloc<double>(6);
