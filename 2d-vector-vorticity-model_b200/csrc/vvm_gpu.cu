@@ -311,6 +311,51 @@ __global__ void k_to_host_layout(Dims d, const T* src, int sk, int off, const do
     }
 }
 
+// The seven prognostic fields at once, blockIdx.z the field; host image f at
+// staging + f * nx * nz. Tiles through shared memory, so both sides are read and
+// written in runs of 32.
+template <typename T>
+struct LayoutArgs {
+    Dims d;
+    double* staging;
+    T* f[7];
+    const double* ref[7];
+};
+template <typename T>
+__global__ void k_from_host_layouts(LayoutArgs<T> a) {
+    __shared__ double tile[32][33];
+    const Dims& d = a.d;
+    const int i0 = blockIdx.x * 32, k0 = blockIdx.y * 32, f = blockIdx.z;
+    const double* src = a.staging + (size_t)f * d.nx * d.nz;
+    const int kk = k0 + threadIdx.x;
+    const double ref = (a.ref[f] && kk < d.nz) ? a.ref[f][kk] : 0.0;
+    for (int r = threadIdx.y; r < 32; r += blockDim.y)
+        if (i0 + r < d.nx && kk < d.nz) {
+            const double v = src[(size_t)(i0 + r) * d.nz + kk];
+            tile[r][threadIdx.x] = a.ref[f] ? v - ref : v;
+        }
+    __syncthreads();
+    for (int r = threadIdx.y; r < 32; r += blockDim.y)
+        if (i0 + (int)threadIdx.x < d.nx && k0 + r < d.nz) a.f[f][d.at(i0 + threadIdx.x, k0 + r)] = T(tile[threadIdx.x][r]);
+}
+template <typename T>
+__global__ void k_to_host_layouts(LayoutArgs<T> a) {
+    __shared__ double tile[32][33];
+    const Dims& d = a.d;
+    const int i0 = blockIdx.x * 32, k0 = blockIdx.y * 32, f = blockIdx.z;
+    double* dst = a.staging + (size_t)f * d.nx * d.nz;
+    for (int r = threadIdx.y; r < 32; r += blockDim.y)
+        if (i0 + (int)threadIdx.x < d.nx && k0 + r < d.nz) {
+            double v = (double)a.f[f][d.at(i0 + threadIdx.x, k0 + r)];
+            if (a.ref[f]) v += a.ref[f][k0 + r];
+            tile[r][threadIdx.x] = v;
+        }
+    __syncthreads();
+    const int kk = k0 + threadIdx.x;
+    for (int r = threadIdx.y; r < 32; r += blockDim.y)
+        if (i0 + r < d.nx && kk < d.nz) dst[(size_t)(i0 + r) * d.nz + kk] = tile[threadIdx.x][r];
+}
+
 }  // namespace vvm
 
 // ===========================================================================
@@ -347,21 +392,38 @@ inline void upload_now(void* dst, const void* src, size_t nb) {
     CK(cudaStreamSynchronize(nullptr));
 }
 
+// Small allocations are carved from slabs: a context makes about a hundred,
+// and a cudaMalloc, a clear and a wait for each took most of its creation (128 x
+// 64: 2 ms). ptrs and bytes list the slabs.
 struct Arena {
+    static constexpr size_t kSlab = size_t(2) << 20, kAlign = 256;
     std::vector<void*> ptrs;
     std::vector<size_t> bytes;
-    template <typename X>
-    X* alloc(size_t n) {
+    char* slab = nullptr;
+    size_t left = 0;
+    void* raw(size_t nb) {
         void* p = nullptr;
-        const size_t nb = std::max<size_t>(n, 1) * sizeof(X);
         CK(cudaMalloc(&p, nb));
+        ptrs.push_back(p);
+        bytes.push_back(nb);
         CK(cudaMemset(p, 0, nb));
         // complete before returning: a context's stream may be non-blocking,
         // and work on it is not ordered after the legacy stream
         CK(cudaStreamSynchronize(nullptr));
-        ptrs.push_back(p);
-        bytes.push_back(nb);
-        return static_cast<X*>(p);
+        return p;
+    }
+    template <typename X>
+    X* alloc(size_t n) {
+        const size_t nb = (std::max<size_t>(n, 1) * sizeof(X) + kAlign - 1) / kAlign * kAlign;
+        if (nb > kSlab / 2) return static_cast<X*>(raw(nb));
+        if (nb > left) {
+            slab = static_cast<char*>(raw(kSlab));
+            left = kSlab;
+        }
+        X* p = reinterpret_cast<X*>(slab);
+        slab += nb;
+        left -= nb;
+        return p;
     }
     ~Arena() {
         for (void* p : ptrs) cudaFree(p);
@@ -1162,7 +1224,7 @@ struct LearnedNet {
     int NX = 0, NK = 0, H[4] = {}, W[4] = {};
     float *w = nullptr, *g = nullptr, *m = nullptr, *v = nullptr;
     uint4 *pk = nullptr, *pkT = nullptr;       // packed forward / adjoint operands, 6 x 1152
-    float *x0 = nullptr, *z0 = nullptr, *dz = nullptr;
+    float *x0 = nullptr, *z0 = nullptr, *dz = nullptr, *t0 = nullptr;   // t0: the target of an evaluation
     __nv_bfloat16 *h[4] = {}, *pl[4] = {}, *u[3] = {}, *gg[3] = {};
     __nv_bfloat16 *dgb[4] = {}, *dub[3] = {}, *dpb[4] = {}, *dh3 = nullptr;
     double *part = nullptr, *lt = nullptr;
@@ -1225,6 +1287,7 @@ struct LearnedNet {
         x0 = ar.alloc<float>(n0);
         z0 = ar.alloc<float>(n0);
         dz = ar.alloc<float>(n0);
+        t0 = ar.alloc<float>(n0);
         for (int l = 0; l < 4; l++) {
             const size_t nl = (size_t)H[l] * W[l] * kNetC;
             h[l] = ar.alloc<__nv_bfloat16>(nl);
@@ -1602,6 +1665,8 @@ struct vvm_gpu_ctx {
     double pf1 = 0, pf2 = 0;
     // perturbation profiles of th (0) and qv (1); used by the mixed step
     double *pref[2] = {}, *pd0[2] = {}, *ps0[2] = {}, *pg0[2] = {}, *pdn[2] = {};
+    double* prof = nullptr;          // the profiles above, one block
+    std::vector<double> h_prof;      // its host image while a state is uploaded
     std::vector<double> h_rhou, h_rhow;
     // vertical metric of the cal_w operator: a_k = (z_k - z_{k-1}) / dx, h_k =
     // dx / (2 (z_k - z_zeta_k)); exactly 1 on uniform levels. `stretched`:
@@ -1618,7 +1683,8 @@ struct vvm_gpu_ctx {
     double* dubar = nullptr;  // [2]
     double *partial = nullptr, *nvp = nullptr;
     int npart = 0;
-    double* staging = nullptr;   // nx*nz*2 doubles
+    double* staging = nullptr;   // staging_slots() host images of a field
+    int* err_host = nullptr;     // pinned copy of d_err (downloads)
     // Poisson
     bool poisson_ready = false;
     std::unique_ptr<PCG<double>> pcg64;
@@ -1681,6 +1747,7 @@ struct vvm_gpu_ctx {
         if (pcg_psi) pcg_psi->release();
         if (sc_host) cudaFreeHost(sc_host);
         if (sc_host_i) cudaFreeHost(sc_host_i);
+        if (err_host) cudaFreeHost(err_host);
         if (own) cudaStreamDestroy(own);
     }
 
@@ -3560,6 +3627,24 @@ int batch_guarded(vvm_gpu_batch* b, Fn fn) {
 
 // ---------------------------------------------------------------- transfer
 
+// The prognostic transfers of a small field: the copies of all seven and one
+// layout kernel, on the context's stream. Of a large one: each field's copy on
+// the copy stream beside the previous field's layout kernel, two staging slots
+// alternating. The line lies where a field's copy (51 GB/s) takes as long as the
+// calls that pipelining adds (six a field, about 2 us each): 512 KB.
+constexpr size_t kSmallField = 512 * 1024;
+inline bool small_field(const Dims& d) { return (size_t)d.nx * d.nz * sizeof(double) <= kSmallField; }
+inline int staging_slots(const Dims& d) { return small_field(d) ? 7 : 2; }
+
+template <typename T>
+LayoutArgs<T> layout_args(vvm_gpu_ctx* c) {
+    Fields<T>& F = fields<T>(c);
+    const int now = c->cur;
+    return LayoutArgs<T>{c->d, c->staging, {F.zeta[now], F.th[now], F.qv[now], F.qc[now], F.qr[now], F.u, F.w},
+                         {nullptr, c->offset_th(), c->offset_qv(), nullptr, nullptr, nullptr, nullptr}};
+}
+inline dim3 layout_grid(const Dims& d) { return dim3(cdiv(d.nx, 32), cdiv(d.nz, 32), 7); }
+
 template <typename T>
 void upload_field(vvm_gpu_ctx* c, const double* host, int sk, int off, T* dst, const double* ref = nullptr) {
     size_t n = (size_t)c->d.nx * c->d.nz * sk;
@@ -3635,18 +3720,28 @@ void download_field(vvm_gpu_ctx* c, const T* src, int sk, int off, double* host,
     }
 }
 
+// Sets a profile in the host image of the profile block; upload_profiles copies
+// the block at its end.
 void upload_profile(vvm_gpu_ctx* c, const double* h, double* dptr) {
-    CK(cudaMemcpyAsync(dptr, h, c->d.nz * sizeof(double), cudaMemcpyHostToDevice, c->stream));
-    CK(cudaStreamSynchronize(c->stream));
+    std::copy(h, h + c->d.nz, c->h_prof.begin() + (dptr - c->prof));
 }
 
 template <typename T>
 int upload_prognostic_t(vvm_gpu_ctx* c, const vvm_gpu_host_state* s) {
     Fields<T>& F = fields<T>(c);
-    int now = c->cur, fut = 1 - c->cur;
+    int now = c->cur;
     const double* req[] = {s->zeta, s->th, s->qv, s->qc, s->qr, s->u, s->w};
     for (const double* p : req)
         if (!p) return fail(c, VVM_GPU_EINVAL, "upload: prognostic field pointer is NULL");
+    if (small_field(c->d)) {
+        const size_t nf = (size_t)c->d.nx * c->d.nz;
+        for (int f = 0; f < 7; f++)
+            CK(cudaMemcpyAsync(c->staging + f * nf, req[f], nf * sizeof(double), cudaMemcpyHostToDevice, c->stream));
+        const LayoutArgs<T> a = layout_args<T>(c);
+        LAUNCH(&c->stats, VVM_K_MEAN, c->stream, k_from_host_layouts<T><<<layout_grid(c->d), dim3(32, 8), 0, c->stream>>>(a));
+        CKL();
+        return VVM_GPU_OK;
+    }
     // the fields' copies back to back on the copy stream, two staging slots
     // alternating, each slot's layout kernel on the context's stream: the
     // link stays busy while the previous field is rearranged
@@ -3671,7 +3766,6 @@ int upload_prognostic_t(vvm_gpu_ctx* c, const vvm_gpu_host_state* s) {
         CKL();
         CK(cudaEventRecord(c->xev[slot][1], c->stream));
     }
-    (void)fut;
     return VVM_GPU_OK;
 }
 
@@ -3695,8 +3789,20 @@ int upload_state_t(vvm_gpu_ctx* c, const vvm_gpu_host_state* s) {
     up_or_zero(s->RKH, 1, 0, F.RKH);
     double* hs[NHIST] = {s->dzeta_advect, s->dth_buoyancy, s->dth_advect, s->dqv_advect,
                          s->dqc_advect, s->dqr_advect, s->dqr_VT};
-    for (int h = 0; h < NHIST; h++)
-        for (int sl = 0; sl < 2; sl++) up_or_zero(hs[h], 2, sl, F.hist[h][sl]);
+    const dim3 lb(32, 8), lg(cdiv(c->d.nx, 32), cdiv(c->d.nz, 8));
+    for (int h = 0; h < NHIST; h++) {   // one copy holds both slots
+        if (hs[h])
+            CK(cudaMemcpyAsync(c->staging, hs[h], 2 * (size_t)c->d.nx * c->d.nz * sizeof(double), cudaMemcpyHostToDevice, c->stream));
+        for (int sl = 0; sl < 2; sl++) {
+            if (!hs[h]) {
+                CK(cudaMemsetAsync(F.hist[h][sl], 0, n * sizeof(T), c->stream));
+                continue;
+            }
+            LAUNCH(&c->stats, VVM_K_MEAN, c->stream,
+                   k_from_host_layout<T><<<lg, lb, 0, c->stream>>>(c->d, c->staging, 2, sl, nullptr, F.hist[h][sl]));
+            CKL();
+        }
+    }
     // regenerated each forced step unless the uploaded field is to be kept
     c->has_forcing_th = (s->init_th_forcing != nullptr) || !(c->desc.flags & VVM_FLAG_FIXED_FORCING);
     up_or_zero(s->init_th_forcing, 1, 0, F.th_forcing);
@@ -3906,6 +4012,7 @@ int upload_profiles(vvm_gpu_ctx* c, const vvm_gpu_host_state* s) {
         c->pcg64.reset();
         c->pcg32.reset();
     }
+    CK(cudaMemcpyAsync(c->prof, c->h_prof.data(), c->h_prof.size() * sizeof(double), cudaMemcpyHostToDevice, c->stream));
     double ub[2] = {s->ubarTop, s->ubarTopp};
     CK(cudaMemcpyAsync(c->ubar, ub, sizeof(ub), cudaMemcpyHostToDevice, c->stream));
     CK(cudaMemcpyAsync(c->dubar, s->dubarTop_advect, 2 * sizeof(double), cudaMemcpyHostToDevice, c->stream));
@@ -3921,6 +4028,19 @@ int download_prognostic_t(vvm_gpu_ctx* c, vvm_gpu_host_state* s) {
     struct { double* h; T* dptr; const double* ref; } m[] = {
         {s->zeta, F.zeta[now], nullptr}, {s->th, F.th[now], c->offset_th()}, {s->qv, F.qv[now], c->offset_qv()},
         {s->qc, F.qc[now], nullptr}, {s->qr, F.qr[now], nullptr}, {s->u, F.u, nullptr}, {s->w, F.w, nullptr}};
+    // the error word comes with the fields: no call of its own after them
+    *c->err_host = 0;
+    CK(cudaMemcpyAsync(c->err_host, c->d_err, sizeof(int), cudaMemcpyDeviceToHost, c->stream));
+    if (small_field(c->d)) {
+        const size_t nf = (size_t)c->d.nx * c->d.nz;
+        const LayoutArgs<T> a = layout_args<T>(c);
+        LAUNCH(&c->stats, VVM_K_MEAN, c->stream, k_to_host_layouts<T><<<layout_grid(c->d), dim3(32, 8), 0, c->stream>>>(a));
+        CKL();
+        for (int f = 0; f < 7; f++)
+            if (m[f].h) CK(cudaMemcpyAsync(m[f].h, c->staging + f * nf, nf * sizeof(double), cudaMemcpyDeviceToHost, c->stream));
+        CK(cudaStreamSynchronize(c->stream));
+        return VVM_GPU_OK;
+    }
     // each field's layout kernel into one of two staging slots on the
     // context's stream, its copy to the host on the copy stream: the link
     // stays busy while the next field is rearranged; one wait at the end
@@ -3943,7 +4063,7 @@ int download_prognostic_t(vvm_gpu_ctx* c, vvm_gpu_host_state* s) {
     // later work on the context's stream may reuse the staging slots
     CK(cudaEventRecord(c->xev[0][0], c->xfer));
     CK(cudaStreamWaitEvent(c->stream, c->xev[0][0], 0));
-    CK(cudaStreamSynchronize(c->xfer));
+    CK(cudaStreamSynchronize(f ? c->xfer : c->stream));   // (the error word's copy precedes every layout kernel)
     return VVM_GPU_OK;
 }
 
@@ -4021,10 +4141,11 @@ int need_uniform(vvm_gpu_ctx* c) {
 
 
 // Reads and clears the device error word (after the stream's work is done).
-int device_errors(vvm_gpu_ctx* c) {
+int device_errors(vvm_gpu_ctx* c, bool downloaded = false) {
     if (!c->d_err) return VVM_GPU_OK;
     int h = 0;
-    CK(cudaMemcpy(&h, c->d_err, sizeof(int), cudaMemcpyDeviceToHost));
+    if (downloaded) h = *c->err_host;
+    else CK(cudaMemcpy(&h, c->d_err, sizeof(int), cudaMemcpyDeviceToHost));
     if (!h) return VVM_GPU_OK;
     CK(cudaMemsetAsync(c->d_err, 0, sizeof(int), c->stream));
     CK(cudaStreamSynchronize(c->stream));
@@ -4128,13 +4249,21 @@ int vvm_gpu_create(const vvm_gpu_desc* desc, int device, vvm_gpu_ctx** out) {
                             &c->pc, &c->lvcp, &c->dtcgr_th, &c->dtcgr_zeta, &c->q1ls, &c->q2ls, &c->rwres,
                             &c->lv_r2dzc, &c->lv_r2dzw, &c->lv_rdzc, &c->lv_r2dzcc, &c->lv_kmax, &c->gsM_cz,
                             &c->gsM_rhod, &c->gsS_cz, &c->gsS_rhod, &c->lv_dzw};
-        for (double** p : profs) *p = c->ar.alloc<double>(nz);
+        const size_t np = sizeof(profs) / sizeof(profs[0]) + 10;
+        c->h_prof.assign(np * nz, 0.0);
+        c->prof = c->ar.alloc<double>(np * nz);
+        double* at = c->prof;
+        auto take = [&](double*& p) {
+            p = at;
+            at += nz;
+        };
+        for (double** p : profs) take(*p);
         for (int j = 0; j < 2; j++) {
-            c->pref[j] = c->ar.alloc<double>(nz);
-            c->pd0[j] = c->ar.alloc<double>(nz);
-            c->ps0[j] = c->ar.alloc<double>(nz);
-            c->pg0[j] = c->ar.alloc<double>(nz);
-            c->pdn[j] = c->ar.alloc<double>(nz);
+            take(c->pref[j]);
+            take(c->pd0[j]);
+            take(c->ps0[j]);
+            take(c->pg0[j]);
+            take(c->pdn[j]);
         }
         c->ubar = c->ar.alloc<double>(2);
         c->dubar = c->ar.alloc<double>(2);
@@ -4146,7 +4275,8 @@ int vvm_gpu_create(const vvm_gpu_desc* desc, int device, vvm_gpu_ctx** out) {
         CK(cudaFuncSetAttribute(k_padv<double, F_TH | F_QV | F_QC | F_QR, 4>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                 (int)sizeof(PAdvShared<double, 4>)));
         c->nvp = c->ar.alloc<double>(6);
-        c->staging = c->ar.alloc<double>((size_t)c->d.nx * c->d.nz * 2);
+        c->staging = c->ar.alloc<double>((size_t)c->d.nx * c->d.nz * staging_slots(c->d));
+        CK(cudaMallocHost(&c->err_host, sizeof(int)));
         c->wctl = c->ar.alloc<CGCtl>(1);
         c->d_exec = c->ar.alloc<long long>(1);
         c->d_err = c->ar.alloc<int>(1);
@@ -4235,7 +4365,7 @@ int vvm_gpu_download_prognostic(vvm_gpu_ctx* ctx, vvm_gpu_host_state* st) {
     return guarded(ctx, [&] {
         if (int rc = need_state(ctx)) return rc;
         if (int rc = DISPATCH(ctx, download_prognostic_t)(ctx, st)) return rc;
-        return device_errors(ctx);
+        return device_errors(ctx, true);
     });
 }
 
@@ -4494,8 +4624,7 @@ int vvm_gpu_learned_eval(vvm_gpu_ctx* ctx, const float* x, const float* t, float
         N.forward(st);
         if (z) CK(cudaMemcpyAsync(z, N.z0, n0 * sizeof(float), cudaMemcpyDeviceToHost, st));
         if (t) {
-            Arena tmp;
-            float* td = tmp.alloc<float>(n0);
+            float* td = N.t0;
             CK(cudaMemcpyAsync(td, t, n0 * sizeof(float), cudaMemcpyHostToDevice, st));
             CK(cudaMemsetAsync(N.g, 0, LearnedNet::kParams * sizeof(float), st));
             N.loss(td, 1.f, st);

@@ -159,6 +159,21 @@ def _ptr(a):
     return a.ctypes.data_as(_dp) if a is not None else None
 
 
+_PROGNOSTIC = ("zeta", "th", "qv", "qc", "qr", "u", "w")
+_SLOT = [(n, getattr(HostState, n).offset // 8) for n in _PROGNOSTIC]
+
+
+def _prognostic_state(arrays):
+    """HostState of the prognostic fields alone: their addresses set as words
+    of the structure (a ctypes pointer object a field costs more than the
+    small transfers themselves)."""
+    hs = HostState()
+    words = np.frombuffer(hs, dtype=np.uint64)
+    for (n, at), a in zip(_SLOT, arrays):
+        words[at] = a.__array_interface__["data"][0]
+    return hs
+
+
 def poisson_solve_noalloc(NX: int, NZ: int, rhou: np.ndarray, rhow: np.ndarray, d_b: int, d_W: int,
                           tol: float = 1e-10, maxit: int = 10000, stream: int = 0):
     """vvm_gpu_poisson_solve_noalloc: the cal_w solve on caller-owned device
@@ -336,18 +351,11 @@ class VVMGpu:
         return st
 
     def upload_prognostic(self, fields: dict):
-        hs = HostState()
-        keep = []
-        for n in ("zeta", "th", "qv", "qc", "qr", "u", "w"):
-            a = np.ascontiguousarray(fields[n], dtype=np.float64)
-            keep.append(a)
-            setattr(hs, n, _ptr(a))
-        self._check(self.L.vvm_gpu_upload_prognostic(self.h, ctypes.byref(hs)))
+        keep = [np.ascontiguousarray(fields[n], dtype=np.float64) for n in _PROGNOSTIC]
+        self._check(self.L.vvm_gpu_upload_prognostic(self.h, ctypes.byref(_prognostic_state(keep))))
 
     def download_prognostic(self, out: dict):
-        hs = HostState()
-        for n in ("zeta", "th", "qv", "qc", "qr", "u", "w"):
-            setattr(hs, n, _ptr(out[n]))
+        hs = _prognostic_state([out[n] for n in _PROGNOSTIC])
         self._check(self.L.vvm_gpu_download_prognostic(self.h, ctypes.byref(hs)))
 
     # -- stepping ----------------------------------------------------------
