@@ -608,57 +608,149 @@ __global__ void k_net_up_add(const __nv_bfloat16* lo, const __nv_bfloat16* skip,
     bf16x8_store(out + act_at(y, q, x, W), a);
 }
 
-// dW[t][ci][co] += sum_p X[p + off(t)][ci] dY[p][co] over one tile of 128
-// pixels of a row (grid = H * ceil(W / 128), 256 threads; 36 weights a thread).
-__global__ void __launch_bounds__(256) k_net_wgrad32(const __nv_bfloat16* X, const __nv_bfloat16* dY, float* dW,
-                                                     int H, int W) {
-    __shared__ __nv_bfloat16 sx[3][kConvSpan][kNetC];
-    __shared__ __nv_bfloat16 sy[kConvTile][kNetC];
-    const int tiles = (W + kConvTile - 1) / kConvTile;
-    const int y = blockIdx.x / tiles, x0 = (blockIdx.x % tiles) * kConvTile;
-    const int n = min(kConvTile, W - x0);
-    for (int j = threadIdx.x; j < 3 * kConvSpan * 4; j += blockDim.x) {
-        const int q = j & 3, p = (j >> 2) % kConvSpan, dy = (j >> 2) / kConvSpan;
-        const int yy = y + dy - 1, xx = ((x0 + p - 1) % W + W) % W;
-        uint4 v = make_uint4(0, 0, 0, 0);
-        if (yy >= 0 && yy < H) v = *reinterpret_cast<const uint4*>(X + act_at(yy, q, xx, W));
-        *reinterpret_cast<uint4*>(&sx[dy][p][8 * q]) = v;
+// dW[t][ci][co] += sum_p X[p + off(t)][ci] dY[p][co]: nine 32 x 32 products over
+// all pixels, on the tensor cores (bf16 operands, FP32 accumulators). A block
+// takes a strip of 128 pixels and walks `rows` rows of it; warp t holds tap t's
+// 32 x 32 sums (eight 16 x 8 tiles) in registers throughout and adds them to dW
+// at the end. Pixels are the contraction: both operands lie with the channels
+// of a pixel together, so both are loaded transposed (ldmatrix), a tap's shift
+// being a shift of the rows it starts from. (A tap's product has 32 rows, below
+// the 64 that a tcgen05 operand needs at least, and taps cannot share one: each
+// meets dY at its own shift. At 16 MB of operands for 2.4 GFLOP the kernel is
+// bound by its loads and issue anyway.) Rows of X come by cp.async one row
+// ahead, each read once; a pixel's four 16-byte chunks are rotated by
+// (pixel / 2) mod 4 so that eight consecutive pixels meet all banks.
+// 128 x 1024 pixels: 21 us, from 295 with a multiply-add of two conversions
+// and two shared loads a term.
+constexpr int kWgPix = kConvTile, kWgThreads = 9 * 32;
+
+struct WgradShared {
+    uint4 x[4][kWgPix + 2][4];   // rows y-1 .. y+2 of X, pixels x0-1 ..
+    uint4 y[2][kWgPix][4];       // rows y, y+1 of dY
+};
+__device__ __forceinline__ int wg_slot(int p, int q) { return q ^ ((p >> 1) & 3); }
+__device__ __forceinline__ void ldmatrix4_trans(uint32_t (&r)[4], const uint4* p) {
+    asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0, %1, %2, %3}, [%4];"
+                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3])
+                 : "r"(smem_u32(p))
+                 : "memory");
+}
+__device__ __forceinline__ void mma_bf16(float (&c)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {
+    asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, {%0, %1, %2, %3};"
+                 : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
+                 : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
+}
+__device__ __forceinline__ void wg_copy16(uint4* dst, const __nv_bfloat16* src) {
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(smem_u32(dst)), "l"(src) : "memory");
+}
+
+__global__ void __launch_bounds__(kWgThreads) k_net_wgrad32(const __nv_bfloat16* X, const __nv_bfloat16* dY, float* dW,
+                                                            int H, int W, int rows) {
+    extern __shared__ __align__(16) unsigned char wgrad_smem[];
+    WgradShared& S = *reinterpret_cast<WgradShared*>(wgrad_smem);
+    const int tid = threadIdx.x, lane = tid & 31, tap = tid >> 5, dy = tap / 3, dx = tap % 3;
+    const int x0 = blockIdx.x * kWgPix, n = min(kWgPix, W - x0);
+    const int y0 = blockIdx.y * rows, y1 = min(y0 + rows, H);
+    // rows outside the grid and pixels beyond its end are zero
+    auto load_x = [&](int y) {
+        for (int j = tid; j < 4 * (kWgPix + 2); j += kWgThreads) {
+            const int q = j / (kWgPix + 2), p = j - q * (kWgPix + 2);   // pixels fastest: consecutive chunks
+            uint4* dst = &S.x[(y + 4) & 3][p][wg_slot(p, q)];
+            if (y >= 0 && y < H && p < n + 2) wg_copy16(dst, X + act_at(y, q, wrapx(x0 + p - 1, W), W));
+            else *dst = make_uint4(0, 0, 0, 0);
+        }
+    };
+    auto load_y = [&](int y) {
+        for (int j = tid; j < 4 * kWgPix; j += kWgThreads) {
+            const int q = j / kWgPix, p = j - q * kWgPix;
+            uint4* dst = &S.y[y & 1][p][wg_slot(p, q)];
+            if (y < H && p < n) wg_copy16(dst, dY + act_at(y, q, x0 + p, W));
+            else *dst = make_uint4(0, 0, 0, 0);
+        }
+    };
+    float acc[2][4][4] = {};
+    load_x(y0 - 1);
+    load_x(y0);
+    load_x(y0 + 1);
+    load_y(y0);
+    asm volatile("cp.async.commit_group;\n" ::: "memory");
+    const int m = lane >> 3, r8 = lane & 7;
+    for (int y = y0; y < y1; y++) {
+        if (y + 1 < y1) {   // the next row, in flight during the products
+            load_x(y + 2);
+            load_y(y + 1);
+        }
+        asm volatile("cp.async.commit_group;\n" ::: "memory");
+        asm volatile("cp.async.wait_group 1;\n" ::: "memory");
+        __syncthreads();
+        const uint4(*xs)[4] = S.x[(y + dy - 1 + 4) & 3];
+        const uint4(*ys)[4] = S.y[y & 1];
+        for (int k = 0; k < n; k += 16) {
+            uint32_t a[2][4], b[2][4];
+            const int pa = k + dx + (m >> 1) * 8 + r8, pb = k + (m & 1) * 8 + r8;
+#pragma unroll
+            for (int h = 0; h < 2; h++) {
+                ldmatrix4_trans(a[h], &xs[pa][wg_slot(pa, 2 * h + (m & 1))]);
+                ldmatrix4_trans(b[h], &ys[pb][wg_slot(pb, 2 * h + (m >> 1))]);
+            }
+#pragma unroll
+            for (int i = 0; i < 2; i++)
+#pragma unroll
+                for (int j = 0; j < 4; j++) mma_bf16(acc[i][j], a[i], b[j >> 1][2 * (j & 1)], b[j >> 1][2 * (j & 1) + 1]);
+        }
+        __syncthreads();
     }
-    for (int j = threadIdx.x; j < kConvTile * 4; j += blockDim.x) {
-        const int q = j & 3, m = j >> 2;
-        uint4 v = make_uint4(0, 0, 0, 0);
-        if (m < n) v = *reinterpret_cast<const uint4*>(dY + act_at(y, q, x0 + m, W));
-        *reinterpret_cast<uint4*>(&sy[m][8 * q]) = v;
-    }
-    __syncthreads();
-    for (int j = threadIdx.x; j < 9 * kNetC * kNetC; j += blockDim.x) {
-        const int co = j % kNetC, ci = (j / kNetC) % kNetC, t = j / (kNetC * kNetC);
-        const int dy = t / 3, dx = t % 3;
-        float acc = 0.f;
-        for (int m = 0; m < n; m++) acc += __bfloat162float(sx[dy][m + dx][ci]) * __bfloat162float(sy[m][co]);
-        atomicAdd(dW + j, acc);
-    }
+    asm volatile("cp.async.wait_group 0;\n" ::: "memory");
+    const int g = lane >> 2, c = 2 * (lane & 3);
+#pragma unroll
+    for (int i = 0; i < 2; i++)
+#pragma unroll
+        for (int j = 0; j < 4; j++) {
+            float* w = dW + ((size_t)tap * kNetC + 16 * i + g) * kNetC + 8 * j + c;
+            atomicAdd(reinterpret_cast<float2*>(w), make_float2(acc[i][j][0], acc[i][j][1]));
+            atomicAdd(reinterpret_cast<float2*>(w + 8 * kNetC), make_float2(acc[i][j][2], acc[i][j][3]));
+        }
 }
 
 // dw[t][c] += sum_p s[p + off(t)] d[p][c]: the weight gradient of the lift
 // (s = its FP32 input, d = the gradient of its output) and, with the roles
 // read the other way, of the projection (s = dz at p, d = g at p + off(t)).
-// mode 0: lift, s shifted; mode 1: projection, d shifted. One block of 288
-// threads (one weight each) per row.
-__global__ void k_net_wgrad_edge(const float* s, const __nv_bfloat16* d, float* dw, int H, int W, int mode) {
-    const int y = blockIdx.x;
-    const int j = threadIdx.x;   // (t, c)
-    if (j >= 9 * kNetC) return;
-    const int t = j / kNetC, c = j % kNetC, dy = t / 3 - 1, dx = t % 3 - 1;
-    const int yy = y + dy;
-    if (yy < 0 || yy >= H) return;
+// mode 0: lift, s shifted; mode 1: projection, d shifted. A block stages 128
+// pixels of a row (three rows of the shifted operand) and its 288 threads, one
+// weight each, run over them; `rows` rows a block. 128 x 1024 pixels: 23 and 19 us,
+// from 96 and 127 with one block a row reading global memory term by term.
+__global__ void __launch_bounds__(9 * kNetC) k_net_wgrad_edge(const float* s, const __nv_bfloat16* d, float* dw, int H, int W,
+                                                              int mode, int rows) {
+    __shared__ float ss[3][kWgPix + 2];
+    __shared__ __align__(16) __nv_bfloat16 sd[3][kWgPix + 2][kNetC];
+    const int tid = threadIdx.x, t = tid / kNetC, c = tid % kNetC, dy = t / 3, dx = t % 3;
+    const int x0 = blockIdx.x * kWgPix, n = min(kWgPix, W - x0);
+    const int y0 = blockIdx.y * rows, y1 = min(y0 + rows, H);
+    const int hs = mode == 0 ? 1 : 0, hd = 1 - hs;   // halo of each operand
     float acc = 0.f;
-    for (int x = 0; x < W; x++) {
-        const int xs = wrapx(x + dx, W);
-        if (mode == 0) acc += s[(size_t)yy * W + xs] * __bfloat162float(d[act_at(y, c >> 3, x, W) + (c & 7)]);
-        else acc += s[(size_t)y * W + x] * __bfloat162float(d[act_at(yy, c >> 3, xs, W) + (c & 7)]);
+    for (int y = y0; y < y1; y++) {
+        __syncthreads();
+        for (int j = tid; j < (2 * hs + 1) * (kWgPix + 2); j += blockDim.x) {
+            const int r = j / (kWgPix + 2), p = j - r * (kWgPix + 2), yy = y + r - hs;
+            float v = 0.f;
+            if (yy >= 0 && yy < H && p < n + 2) v = s[(size_t)yy * W + wrapx(x0 + p - 1, W)];
+            ss[r][p] = v;
+        }
+        for (int j = tid; j < (2 * hd + 1) * 4 * (kWgPix + 2); j += blockDim.x) {
+            const int r = j / (4 * (kWgPix + 2)), e = j - r * 4 * (kWgPix + 2), q = e / (kWgPix + 2), p = e - q * (kWgPix + 2);
+            const int yy = y + r - hd;
+            uint4 v = make_uint4(0, 0, 0, 0);
+            if (yy >= 0 && yy < H && p < n + 2) v = *reinterpret_cast<const uint4*>(d + act_at(yy, q, wrapx(x0 + p - 1, W), W));
+            *reinterpret_cast<uint4*>(&sd[r][p][8 * q]) = v;
+        }
+        __syncthreads();
+        // pixel m of the strip is column m + 1 of both tiles
+        const float* sp = &ss[hs ? dy : 0][hs ? dx : 1];
+        const __nv_bfloat16* dp = &sd[hd ? dy : 0][hd ? dx : 1][c];
+#pragma unroll 4
+        for (int m = 0; m < n; m++) acc += sp[m] * __bfloat162float(dp[m * kNetC]);
     }
-    atomicAdd(dw + j, acc);
+    atomicAdd(dw + tid, acc);
 }
 
 // Loss of one pair: the S-norm error that the preconditioner's Galerkin step

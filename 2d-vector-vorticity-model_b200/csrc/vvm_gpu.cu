@@ -1309,6 +1309,7 @@ struct LearnedNet {
         sz = ar.alloc<float>(n0);
         st = ar.alloc<float>(n0);
         err = ar.alloc<int>(1);
+        CK(cudaFuncSetAttribute(k_net_wgrad32, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(WgradShared)));
         init_weights(seed);
     }
 
@@ -1367,7 +1368,19 @@ struct LearnedNet {
         CKL();
     }
     void wgrad(const __nv_bfloat16* X, const __nv_bfloat16* dY, int c, int l, cudaStream_t st) {
-        LAUNCH(stats, VVM_K_LEARNED, st, k_net_wgrad32<<<H[l] * cdiv(W[l], kConvTile), 256, 0, st>>>(X, dY, g + kConvs + (size_t)c * kConvSize, H[l], W[l]));
+        const dim3 grid = wgrad_grid(l, 1);
+        LAUNCH(stats, VVM_K_LEARNED, st, k_net_wgrad32<<<grid, kWgThreads, sizeof(WgradShared), st>>>(X, dY, g + kConvs + (size_t)c * kConvSize, H[l], W[l], cdiv(H[l], grid.y)));
+        CKL();
+    }
+    // Strips of 128 pixels by groups of rows: about `a_sm` blocks a SM, so that few blocks add
+    // their sums to the same weights.
+    dim3 wgrad_grid(int l, int a_sm) const {
+        const int strips = cdiv(W[l], kWgPix), groups = std::max(1, std::min(H[l], a_sm * 148 / strips));
+        return dim3(strips, cdiv(H[l], cdiv(H[l], groups)));
+    }
+    void wgrad_edge(const float* s, const __nv_bfloat16* d, float* dw, int mode, cudaStream_t st) {
+        const dim3 grid = wgrad_grid(0, 4);
+        LAUNCH(stats, VVM_K_LEARNED, st, k_net_wgrad_edge<<<grid, 9 * kNetC, 0, st>>>(s, d, dw, H[0], W[0], mode, cdiv(H[0], grid.y)));
         CKL();
     }
 
@@ -1398,8 +1411,7 @@ struct LearnedNet {
 
     // g += d loss / d w for the gradient dz of the output (after forward()).
     void backward(cudaStream_t st) {
-        LAUNCH(stats, VVM_K_LEARNED, st, k_net_wgrad_edge<<<H[0], 9 * kNetC, 0, st>>>(dz, gg[0], g + kProj, H[0], W[0], 1));
-        CKL();
+        wgrad_edge(dz, gg[0], g + kProj, 1, st);
         LAUNCH(stats, VVM_K_LEARNED, st, k_net_proj_adj<<<cdiv(H[0] * W[0], 128), 128, 0, st>>>(dz, w + kProj, dgb[0], H[0], W[0]));
         CKL();
         // up path, level 0 first: du_l = U_l^T dg_l; dg_{l+1} = up^T du_l; dh_l = du_l
@@ -1417,8 +1429,7 @@ struct LearnedNet {
             up_add(dpb[l], dub[l - 1], dub[l - 1], l - 1, 0.25f, st);   // dh_{l-1} lives in du_{l-1}
             dh = dub[l - 1];
         }
-        LAUNCH(stats, VVM_K_LEARNED, st, k_net_wgrad_edge<<<H[0], 9 * kNetC, 0, st>>>(x0, dub[0], g + kLift, H[0], W[0], 0));
-        CKL();
+        wgrad_edge(x0, dub[0], g + kLift, 0, st);
     }
 
     // loss of z0 against target t (FP32 [H0][W0]): the S-norm error left by
