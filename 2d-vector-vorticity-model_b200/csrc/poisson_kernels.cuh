@@ -535,4 +535,58 @@ template <typename P>
 __global__ void k_cg_check(VecArgs<P> v, const P* f, P* x, P* r, double* partial, CGScalars* sc, CGCtl* ctl,
                            unsigned* arrive, cudaGraphConditionalHandle h, double tol2, int maxit) { k_cg_check_body<P>(v, f, x, r, partial, sc, ctl, arrive, h, tol2, maxit); }
 
+// Rows a thread of k_spec_check takes: a quarter of the blocks to count in
+// (2048 x 256: 10 us with one row).
+constexpr int kCheckRows = 4;
+
+// The check of a direct solve x = S^{-1} f: as k_cg_check, with ||b||^2 (b = -rw f)
+// summed in the same pass (nothing before it needs it; x = 0 where b = 0
+// already). partial: two values a block.
+__device__ __forceinline__ void k_spec_check_body(const VecArgs<double>& v, const double* f, const double* x, double* r, double* partial,
+                                                  CGScalars* sc, CGCtl* ctl, unsigned* arrive, cudaGraphConditionalHandle h,
+                                                  double tol2, int maxit) {
+    __shared__ double sh[64];
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    double s[2] = {0, 0};
+#pragma unroll 4
+    for (int q = 0; q < kCheckRows; q++) {
+        const int kk = (blockIdx.y * kCheckRows + q) * blockDim.y + threadIdx.y;
+        if (i >= v.nx || kk >= v.NK) break;
+        const size_t id = (size_t)kk * v.pitch + i;
+        const double fv = f[id], rv = fv - s_apply(x, v.pitch, v.nx, v.NK, v.z, v.cx, kk, i);
+        r[id] = rv;
+        const double w = v.rhow_k[kk], wr = w * rv, wb = w * fv;
+        s[0] += wr * wr;
+        s[1] += wb * wb;
+    }
+    block_sum(s, sh);
+    const unsigned nb = gridDim.x * gridDim.y;
+    if (threadIdx.x == 0 && threadIdx.y == 0) {
+        double* p = partial + 2 * (size_t)(blockIdx.x + gridDim.x * blockIdx.y);
+        p[0] = s[0];
+        p[1] = s[1];
+    }
+    if (!arrive_last(arrive, nb)) return;
+    const int nt = blockDim.x * blockDim.y, tid = threadIdx.x + blockDim.x * threadIdx.y;
+    double t[2] = {0, 0};
+    for (int b = tid; b < (int)nb; b += nt) {
+        t[0] += __ldcg(partial + 2 * b);
+        t[1] += __ldcg(partial + 2 * b + 1);
+    }
+    block_sum(t, sh);
+    if (tid == 0) {
+        const double rr = t[0], bb = t[1];
+        sc->rr = rr;
+        sc->bb = bb;
+        ctl->it = 0;
+        ctl->total = 0;
+        ctl->relres = (bb > 0.0) ? sqrt(rr / bb) : 0.0;
+        const bool more = (bb > 0.0) && (rr > tol2 * bb) && (maxit > 0) && isfinite(rr);
+        ctl->more = more ? 1 : 0;
+        if (h) cudaGraphSetConditional(h, more ? 1u : 0u);
+    }
+}
+__global__ void k_spec_check(VecArgs<double> v, const double* f, const double* x, double* r, double* partial, CGScalars* sc,
+                             CGCtl* ctl, unsigned* arrive, cudaGraphConditionalHandle h, double tol2, int maxit);
+
 }  // namespace vvm

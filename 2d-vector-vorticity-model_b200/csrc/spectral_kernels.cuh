@@ -139,9 +139,9 @@ __device__ __forceinline__ void fft_shared(P* re, P* im, const P* tw, const Spec
 
 __device__ __forceinline__ int bitrev(int j, int logN) { return (int)(__brev((unsigned)j) >> (32 - logN)); }
 
-// Spectra of rows 2b and 2b+1 of r ([NK][pitch]).
-template <typename P>
-__device__ __forceinline__ void k_spec_forward_body(const SpecArgs<P>& a, const P* r) {
+// Spectra of rows 2b and 2b+1 of the field load(row, column).
+template <typename P, typename Load>
+__device__ __forceinline__ void spec_forward(const SpecArgs<P>& a, Load load) {
     extern __shared__ unsigned char smem_raw[];
     P* re = reinterpret_cast<P*>(smem_raw);
     P* im = re + a.NX;
@@ -151,8 +151,8 @@ __device__ __forceinline__ void k_spec_forward_body(const SpecArgs<P>& a, const 
     load_twiddles(tw, a);
     for (int j = threadIdx.x; j < a.NX; j += blockDim.x) {
         const int jr = sw(bitrev(j, a.logN));
-        re[jr] = r[(size_t)k0 * a.pitch + j];
-        im[jr] = two ? r[(size_t)k1 * a.pitch + j] : P(0);
+        re[jr] = load(k0, j);
+        im[jr] = two ? load(k1, j) : P(0);
     }
     __syncthreads();
     fft_shared(re, im, tw, a, false);
@@ -168,6 +168,11 @@ __device__ __forceinline__ void k_spec_forward_body(const SpecArgs<P>& a, const 
             a.sim[(size_t)k1 * a.mpitch + m] = P(0.5) * (nr - zr);
         }
     }
+}
+// ... of r ([NK][pitch]).
+template <typename P>
+__device__ __forceinline__ void k_spec_forward_body(const SpecArgs<P>& a, const P* r) {
+    spec_forward(a, [&](int k, int j) { return r[(size_t)k * a.pitch + j]; });
 }
 template <typename P>
 __global__ void k_spec_forward(SpecArgs<P> a, const P* r) { k_spec_forward_body<P>(a, r); }
@@ -304,9 +309,10 @@ __device__ __forceinline__ void k_spec_modes_seg_body(const SpecArgs<P>& a) {
 template <typename P>
 __global__ void __launch_bounds__(64 * kModeSegs) k_spec_modes_seg(SpecArgs<P> a) { k_spec_modes_seg_body<P>(a); }
 
-// Rows 2b and 2b+1 of out ([NK][pitch]) from their spectra, scaled by 1/NX.
-template <typename P>
-__device__ __forceinline__ void k_spec_inverse_body(const SpecArgs<P>& a, P* out) {
+// Rows 2b and 2b+1 from their spectra, scaled by 1/NX, given to store(row,
+// column, value).
+template <typename P, typename Store>
+__device__ __forceinline__ void spec_inverse(const SpecArgs<P>& a, Store store) {
     extern __shared__ unsigned char smem_raw[];
     P* re = reinterpret_cast<P*>(smem_raw);
     P* im = re + a.NX;
@@ -334,9 +340,14 @@ __device__ __forceinline__ void k_spec_inverse_body(const SpecArgs<P>& a, P* out
     fft_shared(re, im, tw, a, true);
     const P scale = P(1) / P(N);
     for (int j = threadIdx.x; j < N; j += blockDim.x) {
-        out[(size_t)k0 * a.pitch + j] = re[sw(j)] * scale;
-        if (two) out[(size_t)k1 * a.pitch + j] = im[sw(j)] * scale;
+        store(k0, j, re[sw(j)] * scale);
+        if (two) store(k1, j, im[sw(j)] * scale);
     }
+}
+// ... to out ([NK][pitch]).
+template <typename P>
+__device__ __forceinline__ void k_spec_inverse_body(const SpecArgs<P>& a, P* out) {
+    spec_inverse(a, [&](int k, int j, P v) { out[(size_t)k * a.pitch + j] = v; });
 }
 template <typename P>
 __global__ void k_spec_inverse(SpecArgs<P> a, P* out) { k_spec_inverse_body<P>(a, out); }

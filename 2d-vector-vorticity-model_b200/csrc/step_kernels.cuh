@@ -88,6 +88,59 @@ __device__ __forceinline__ void cp_async_elem(T* smem, const T* gmem) {
 }
 
 // ---------------------------------------------------------------------------
+// Domain-mean top wind tendency (PoissonSolver::pubarTop_pt,
+// PoissonSolver.cpp:655-676). One block of 256 threads; in a whole step an
+// extra block of k_pzeta, which reads the same time level (a launch of its own
+// stood 9 us at the head of the scalars' chain).
+
+template <typename T>
+struct PubarArgs {
+    Dims d;
+    Consts c;
+    Profiles p;
+    const T *u, *w, *RKM;
+    double* ubar;     // [0] ubarTop, [1] ubarTopp
+    double* dubar;    // dubarTop_advect[2]
+    AB2 ab;
+};
+
+template <typename T>
+__device__ __forceinline__ void k_pubartop_body(const PubarArgs<T>& a) {
+    __shared__ double sh[32 * 3];
+    const Dims& d = a.d;
+    const int tid = threadIdx.x + blockDim.x * threadIdx.y, nt = blockDim.x * blockDim.y;
+    const int t = d.nz - 2, b = d.nz - 3, top = d.nz - 1;
+    const double* rhou = a.p.rhou;
+    const double* rhow = a.p.rhow;
+    double s[3] = {0, 0, 0};
+#pragma unroll 4
+    for (int i = 1 + tid; i < d.nx - 1; i += nt) {
+        double ut = a.u[d.at(i, t)], ub = a.u[d.at(i, b)], utop = a.u[d.at(i, top)];
+        double wt = a.w[d.at(i, t)], wtm = a.w[d.at(i - 1, t)];
+        const T* K = a.RKM;
+        s[0] += 0.25 * (rhou[t] * ut + rhou[b] * ub) * (wt + wtm);
+        s[1] += rhow[top] * 0.25 * ((double)K[d.at(i, top)] + K[d.at(i, t)] + K[d.at(i - 1, top)] + K[d.at(i - 1, t)]) *
+                (a.p.rdz_up * (utop - ut));
+        s[2] += rhow[t] * 0.25 * ((double)K[d.at(i, t)] + K[d.at(i, b)] + K[d.at(i - 1, t)] + K[d.at(i - 1, b)]) *
+                (a.c.rdx * (wt - wtm) + a.p.rdz_dn * (ut - ub));
+    }
+    block_sum(s, sh);
+    if (tid == 0) {
+        double n = (double)(d.nx - 2.);
+        double down = s[0] / n, kup = s[1] / n, kdown = s[2] / n;
+        double pa = (-down) * a.p.rdz_c / rhou[t];
+        double pb = (kup - kdown) * a.p.rdz_c / rhou[t];
+        double tend = -pa + pb;
+        double old = a.ab.first ? tend : a.dubar[a.ab.so];
+        a.dubar[a.ab.sn] = tend;
+        if (a.ab.first) a.dubar[a.ab.so] = tend;
+        a.ubar[1] = a.ubar[0] + 1.5 * a.c.dt * tend - 0.5 * a.c.dt * old;
+    }
+}
+template <typename T>
+__global__ void k_pubartop(PubarArgs<T> a) { k_pubartop_body<T>(a); }
+
+// ---------------------------------------------------------------------------
 // Vorticity advection + buoyancy + westdown halo of zetap
 // (Iteration::pzeta_pt: Advection.cpp:84-149, Buoyancy.cpp:11-58,
 // Boundary.cpp:21-30). One thread per interior zeta point (i, k),
@@ -103,6 +156,8 @@ struct PZetaArgs {
     T *hz_n, *hz_o, *hb_n, *hb_o;  // dzeta_advect, dth_buoyancy slots
     int* err;                      // device error word (kStageErrWait), may be null
     AB2 ab;
+    PubarArgs<T> pubar;            // pubarTop_pt, by one block past the tiles
+    int do_pubar;
 };
 
 // Tile of k_pzeta: 31 x 8R zeta points a block of 32 x 8 threads, R rows a
@@ -171,12 +226,17 @@ template <typename T, int R>
 __device__ __forceinline__ void k_pzeta_body(const FieldMaps<7>& maps, const PZetaArgs<T>& a) {
     using Sh = PZetaShared<T, R>;
     constexpr int BZ = Sh::BZ, VZ = Sh::VZ, VX = kTileVX, AL = 16 / sizeof(T);
+    if (a.do_pubar && blockIdx.y == 0) {   // the first row of blocks: it starts with the first wave
+        if (blockIdx.x == 0) k_pubartop_body<T>(a.pubar);
+        return;
+    }
+    const int by = blockIdx.y - (a.do_pubar ? 1 : 0);
     extern __shared__ __align__(128) unsigned char pzeta_smem[];
     __shared__ uint64_t stage_bar;
     Sh& S = *reinterpret_cast<Sh*>(pzeta_smem);
     const Dims& d = a.d;
     const int lane = threadIdx.x, wid = threadIdx.y, tid = lane + kTileLanes * wid;
-    const int i0 = 1 + blockIdx.x * kTileBX, k0 = 2 + blockIdx.y * BZ;
+    const int i0 = 1 + blockIdx.x * kTileBX, k0 = 2 + by * BZ;
     const int x0 = (i0 - 2) & ~(AL - 1);
     const int i = i0 - 1 + lane;   // the lane's face, and the point west of it
 
@@ -2205,9 +2265,27 @@ __device__ __forceinline__ void k_update_mean_body(const MeanArgs<T>& a) {
     const Dims& d = a.d;
     const int k = 1 + blockIdx.x;
     double s[2] = {0, 0};
-    for (int i = 1 + threadIdx.x; i <= d.nx - 2; i += blockDim.x) {
-        s[0] += (double)a.thp[d.at(i, k)];
-        s[1] += (double)a.qvp[d.at(i, k)];
+    // eight loads in flight a thread: the rows come from L2 or memory, and a
+    // loop of single loads waited for each
+    const T *th = a.thp + d.at(0, k), *qv = a.qvp + d.at(0, k);
+    const int step = blockDim.x;
+    int i = 1 + threadIdx.x;
+    for (; i + 3 * step <= d.nx - 2; i += 4 * step) {
+        T x[4], y[4];
+#pragma unroll
+        for (int e = 0; e < 4; e++) {
+            x[e] = th[i + e * step];
+            y[e] = qv[i + e * step];
+        }
+#pragma unroll
+        for (int e = 0; e < 4; e++) {
+            s[0] += (double)x[e];
+            s[1] += (double)y[e];
+        }
+    }
+    for (; i <= d.nx - 2; i += step) {
+        s[0] += (double)th[i];
+        s[1] += (double)qv[i];
     }
     block_sum(s, sh);
     if (threadIdx.x == 0) {
@@ -2226,55 +2304,6 @@ __device__ __forceinline__ void k_update_mean_body(const MeanArgs<T>& a) {
 }
 template <typename T>
 __global__ void k_update_mean(MeanArgs<T> a) { k_update_mean_body<T>(a); }
-
-// ---------------------------------------------------------------------------
-// Domain-mean top wind tendency (PoissonSolver::pubarTop_pt,
-// PoissonSolver.cpp:655-676). One block.
-
-template <typename T>
-struct PubarArgs {
-    Dims d;
-    Consts c;
-    Profiles p;
-    const T *u, *w, *RKM;
-    double* ubar;     // [0] ubarTop, [1] ubarTopp
-    double* dubar;    // dubarTop_advect[2]
-    AB2 ab;
-};
-
-template <typename T>
-__device__ __forceinline__ void k_pubartop_body(const PubarArgs<T>& a) {
-    __shared__ double sh[32 * 3];
-    const Dims& d = a.d;
-    const int t = d.nz - 2, b = d.nz - 3, top = d.nz - 1;
-    const double* rhou = a.p.rhou;
-    const double* rhow = a.p.rhow;
-    double s[3] = {0, 0, 0};
-    for (int i = 1 + threadIdx.x; i < d.nx - 1; i += blockDim.x) {
-        double ut = a.u[d.at(i, t)], ub = a.u[d.at(i, b)], utop = a.u[d.at(i, top)];
-        double wt = a.w[d.at(i, t)], wtm = a.w[d.at(i - 1, t)];
-        const T* K = a.RKM;
-        s[0] += 0.25 * (rhou[t] * ut + rhou[b] * ub) * (wt + wtm);
-        s[1] += rhow[top] * 0.25 * ((double)K[d.at(i, top)] + K[d.at(i, t)] + K[d.at(i - 1, top)] + K[d.at(i - 1, t)]) *
-                (a.p.rdz_up * (utop - ut));
-        s[2] += rhow[t] * 0.25 * ((double)K[d.at(i, t)] + K[d.at(i, b)] + K[d.at(i - 1, t)] + K[d.at(i - 1, b)]) *
-                (a.c.rdx * (wt - wtm) + a.p.rdz_dn * (ut - ub));
-    }
-    block_sum(s, sh);
-    if (threadIdx.x == 0) {
-        double n = (double)(d.nx - 2.);
-        double down = s[0] / n, kup = s[1] / n, kdown = s[2] / n;
-        double pa = (-down) * a.p.rdz_c / rhou[t];
-        double pb = (kup - kdown) * a.p.rdz_c / rhou[t];
-        double tend = -pa + pb;
-        double old = a.ab.first ? tend : a.dubar[a.ab.so];
-        a.dubar[a.ab.sn] = tend;
-        if (a.ab.first) a.dubar[a.ab.so] = tend;
-        a.ubar[1] = a.ubar[0] + 1.5 * a.c.dt * tend - 0.5 * a.c.dt * old;
-    }
-}
-template <typename T>
-__global__ void k_pubartop(PubarArgs<T> a) { k_pubartop_body<T>(a); }
 
 // ---------------------------------------------------------------------------
 // cal_u (PoissonSolver.cpp:580-653): the top-row wind from the periodic chi

@@ -204,6 +204,47 @@ __device__ __forceinline__ void k_w_from_W_body(const Dims& d, const double* rho
 template <typename T>
 __global__ void k_w_from_W(Dims d, const double* rhow, const double* W, int pitch_f, T* w) { k_w_from_W_body<T>(d, rhow, W, pitch_f, w); }
 
+// k_poisson_rhs's right-hand side formed as the row transform loads it (f is
+// stored too, for the residual check), and w = W / rhow_k stored beside W by
+// the inverse transform: launches of their own read and wrote the same rows
+// again (2048 x 256: 10 and 3 us).
+template <typename T>
+struct SpecFieldArgs {
+    SpecArgs<double> sp;
+    Dims d;
+    double dx;
+    const double *rhow, *rw;
+    const T* zetap;
+    double *f, *W;   // [NK][sp.pitch]
+    T* w;
+};
+template <typename T>
+__device__ __forceinline__ void k_spec_forward_rhs_body(const SpecFieldArgs<T>& a) {
+    spec_forward(a.sp, [&](int kk, int ii) {
+        const int i = ii + 1, k = kk + 2;
+        const double b = a.rhow[k] * a.rhow[k] * ((double)a.zetap[a.d.at(i + 1, k)] - (double)a.zetap[a.d.at(i, k)]) * a.dx;
+        const double f = -b / a.rw[k];
+        a.f[(size_t)kk * a.sp.pitch + ii] = f;
+        return f;
+    });
+}
+template <typename T>
+__global__ void k_spec_forward_rhs(SpecFieldArgs<T> a) { k_spec_forward_rhs_body<T>(a); }
+template <typename T>
+__device__ __forceinline__ void k_spec_inverse_w_body(const SpecFieldArgs<T>& a) {
+    spec_inverse(a.sp, [&](int kk, int ii, double v) {
+        a.W[(size_t)kk * a.sp.pitch + ii] = v;
+        store_westdown(a.w, a.d, ii + 1, kk + 2, T(v / a.rhow[kk + 2]));
+    });
+}
+template <typename T>
+__global__ void k_spec_inverse_w(SpecFieldArgs<T> a) { k_spec_inverse_w_body<T>(a); }
+
+__global__ void k_spec_check(VecArgs<double> v, const double* f, const double* x, double* r, double* partial, CGScalars* sc,
+                             CGCtl* ctl, unsigned* arrive, cudaGraphConditionalHandle h, double tol2, int maxit) {
+    k_spec_check_body(v, f, x, r, partial, sc, ctl, arrive, h, tol2, maxit);
+}
+
 // The streamfunction formulation (PoissonSolver::calpsiuw, STREAMFUNCTION,
 // src/PoissonSolver.cpp:124-177). Its matrix (src/PoissonSolver.cpp:726-756,
 // POISSONPARAM = 0) is -S with S the symmetric w-equation operator of
@@ -748,6 +789,12 @@ struct Spectral : ModeFactors<P> {
         const int smax = 3 * 8192 * (int)sizeof(P);
         CK(cudaFuncSetAttribute(k_spec_forward<P>, cudaFuncAttributeMaxDynamicSharedMemorySize, smax));
         CK(cudaFuncSetAttribute(k_spec_inverse<P>, cudaFuncAttributeMaxDynamicSharedMemorySize, smax));
+        if constexpr (sizeof(P) == 8) {
+            CK(cudaFuncSetAttribute(k_spec_forward_rhs<double>, cudaFuncAttributeMaxDynamicSharedMemorySize, smax));
+            CK(cudaFuncSetAttribute(k_spec_forward_rhs<float>, cudaFuncAttributeMaxDynamicSharedMemorySize, smax));
+            CK(cudaFuncSetAttribute(k_spec_inverse_w<double>, cudaFuncAttributeMaxDynamicSharedMemorySize, smax));
+            CK(cudaFuncSetAttribute(k_spec_inverse_w<float>, cudaFuncAttributeMaxDynamicSharedMemorySize, smax));
+        }
     }
 
     // dst = S^{-1} r (to round-off).
@@ -758,6 +805,19 @@ struct Spectral : ModeFactors<P> {
         this->solve_modes(stats, st);
         klaunch<k_spec_inverse_body<P>, 1024>(stats, VVM_K_MG_SWEEP, st, k_spec_inverse<P>, dim3(rows2), dim3(threads),
                                               smem, a, dst);
+    }
+    // W = S^{-1} f with f from zetap and w from W (FP64 operators); before_w: w's
+    // readers so far.
+    template <typename T>
+    void apply_fields(SpecFieldArgs<T> q, cudaStream_t st, cudaEvent_t before_w) {
+        q.sp = a;
+        const int rows2 = cdiv(a.NK, 2);
+        klaunch<k_spec_forward_rhs_body<T>, 1024>(stats, VVM_K_MG_SWEEP, st, k_spec_forward_rhs<T>, dim3(rows2),
+                                                  dim3(threads), smem, q);
+        this->solve_modes(stats, st);
+        if (before_w) CK(cudaStreamWaitEvent(st, before_w, 0));
+        klaunch<k_spec_inverse_w_body<T>, 1024>(stats, VVM_K_MG_SWEEP, st, k_spec_inverse_w<T>, dim3(rows2), dim3(threads),
+                                                smem, q);
     }
     // z = S^{-1} r; returns the buffer holding z.
     P* apply(const P* r, cudaStream_t st) {
@@ -1500,7 +1560,7 @@ struct PCG {
         q = ar.alloc<P>((size_t)NK * pitch);
         dim3 g = grid();
         npart = g.x * g.y;
-        partial = ar.alloc<double>(npart);
+        partial = ar.alloc<double>(npart + 2 * g.x);   // k_spec_check: two values a block of kCheckRows x 4 rows
         rhow_k = ar.alloc<double>(NK);
         upload_now(rhow_k, rw.data(), NK * sizeof(double));
         sc = ar.alloc<CGScalars>(1);
@@ -1835,6 +1895,12 @@ T* zeta_pre(vvm_gpu_ctx* c) {
     return c->in_step ? F.pre[0] : F.zeta[1 - c->cur];
 }
 
+template <typename T>
+PubarArgs<T> pubar_args(vvm_gpu_ctx* c) {
+    Fields<T>& F = fields<T>(c);
+    return PubarArgs<T>{c->d, c->c, c->profiles(), F.u, F.w, F.RKM, c->ubar, c->dubar, AB2::of(c->step)};
+}
+
 // Rows a thread of k_pzeta takes: two in FP64, four in FP32 (what leaves shared
 // memory for four or five blocks a SM), one where that gives fewer blocks than
 // there are SMs. us a launch with 1 / 2 / 4 rows: 8192 x 256 FP64 67 / 57 / 72,
@@ -1847,12 +1913,13 @@ void launch_pzeta_r(vvm_gpu_ctx* c) {
     AB2 ab = AB2::of(c->step);
     PZetaArgs<T> a{c->d, c->c, c->profiles(), F.zeta[now], F.u, F.w, F.th[now], F.qv[now], F.qc[now], F.qr[now],
                    zeta_pre<T>(c), F.hist[H_ZETA][ab.sn], F.hist[H_ZETA][ab.so], F.hist[H_BUOY][ab.sn],
-                   F.hist[H_BUOY][ab.so], c->d_err, ab};
+                   F.hist[H_BUOY][ab.so], c->d_err, ab, pubar_args<T>(c),
+                   c->in_step && !(c->desc.flags & VVM_FLAG_STREAMFUNCTION)};
     const T* staged[7] = {a.zeta, a.u, a.w, a.th, a.qv, a.qc, a.qr};
     FieldMaps<7> m;
     for (int f = 0; f < 7; f++)
         m.m[f] = field_map(staged[f], c->d.nx, c->d.nz, c->d.pitch, (int)sizeof(T), kTileVX, tile_rows(R) + 4);
-    const dim3 g(cdiv(c->d.nx - 2, kTileBX), cdiv(c->d.nz - 3, tile_rows(R))), blk(kTileLanes, kTileWarps);
+    const dim3 g(cdiv(c->d.nx - 2, kTileBX), cdiv(c->d.nz - 3, tile_rows(R)) + a.do_pubar), blk(kTileLanes, kTileWarps);
     if (c->stats.rec) {
         TilePack<7, PZetaArgs<T>> p{m, a};
         record_kernel(&c->stats, reinterpret_cast<const void*>(&k_pzeta_grouped<T, R>), g, blk, sizeof(PZetaShared<T, R>),
@@ -1966,9 +2033,8 @@ void launch_halo_all(vvm_gpu_ctx* c) {
 
 template <typename T>
 void launch_pubartop(vvm_gpu_ctx* c) {
-    Fields<T>& F = fields<T>(c);
-    PubarArgs<T> a{c->d, c->c, c->profiles(), F.u, F.w, F.RKM, c->ubar, c->dubar, AB2::of(c->step)};
-    klaunch<k_pubartop_body<T>, 1024>(&c->stats, VVM_K_PUBAR, c->stream, k_pubartop<T>, dim3(1), dim3(1024), 0, a);
+    LAUNCH(&c->stats, VVM_K_PUBAR, c->stream, k_pubartop<T><<<1, 256, 0, c->stream>>>(pubar_args<T>(c)));
+    CKL();
 }
 
 // In a whole step the finish of the advection (k_apply's NVP rescaling and
@@ -2627,6 +2693,67 @@ int solve_w(vvm_gpu_ctx* c, double bb, double tol, bool warm) {
 
 // ---------------------------------------------------------------- graphs
 
+template <typename T>
+SpecFieldArgs<T> spec_fields(vvm_gpu_ctx* c) {
+    return SpecFieldArgs<T>{{}, c->d, c->c.dx, c->rhow, c->rwres, zeta_pre<T>(c), c->Wf, c->W, fields<T>(c).w};
+}
+template <typename T>
+void launch_w_from_W(vvm_gpu_ctx* c, cudaStream_t st) {
+    klaunch<k_w_from_W_body<T>, 256>(&c->stats, VVM_K_POISSON_RHS, st, k_w_from_W<T>, c->grid_interior(2), c->blk(), 0,
+                                     c->d, (const double*)c->rhow, (const double*)c->W, c->pcg64->pitch, fields<T>(c).w);
+}
+
+// The direct solve of cal_w, W and w in three launches, and the check of its
+// residual, which sets the condition h (0: none).
+template <typename T>
+void launch_spectral_w(vvm_gpu_ctx* c, cudaEvent_t before_w, cudaGraphConditionalHandle h, int maxit) {
+    PCG<double>& P = *c->pcg64;
+    P.sp.apply_fields(spec_fields<T>(c), c->stream, before_w);
+    const dim3 B = P.block(), G(P.grid().x, cdiv(P.NK, (int)B.y * kCheckRows));
+    klaunch<k_spec_check_body, 256>(&c->stats, VVM_K_CG, c->stream, k_spec_check, G, B, 0, P.vargs(), (const double*)c->Wf,
+                                    (const double*)c->W, P.r, P.partial, P.sc, P.ctl, P.arrive, h,
+                                    c->desc.poisson_tol * c->desc.poisson_tol, maxit);
+}
+
+// Records cal_w by the direct solve (graph capture): only if its check fails,
+// CG iterations from W, with w formed anew. Returns the kernels recorded
+// inside that loop.
+template <typename T>
+long long record_spectral(vvm_gpu_ctx* c, cudaEvent_t before_w, int maxit) {
+    PCG<double>& P = *c->pcg64;
+    cudaGraphConditionalHandle h = new_handle(&c->stats, c->stream);
+    launch_spectral_w<T>(c, before_w, h, maxit);
+    record_cond(&c->stats, &P.ctl->more, true);
+    cudaGraph_t body = add_while(&c->stats, c->stream, h);
+    BodyCapture bc(c->cap[0], body, &c->stats);
+    const long long n0 = c->stats.launches;
+    const int nb = P.record_iteration(c->W, bc.s);
+    launch_w_from_W<T>(c, bc.s);   // before the loop's test, which closes a grouped case's gate
+    klaunch<k_loop_plain_body, 32>(&c->stats, VVM_K_CG, bc.s, k_loop_plain, dim3(1), dim3(1), 0, (const CGScalars*)P.sc,
+                                   P.ctl, h, c->desc.poisson_tol * c->desc.poisson_tol, maxit, 0, c->d_exec, nb + 2);
+    record_cond(&c->stats, &P.ctl->more, false);
+    bc.end();
+    return c->stats.launches - n0;
+}
+
+// ... without capture: the host reads the check's result.
+template <typename T>
+int run_spectral(vvm_gpu_ctx* c, cudaEvent_t before_w, int maxit) {
+    PCG<double>& P = *c->pcg64;
+    launch_spectral_w<T>(c, before_w, 0, maxit);
+    CGCtl ctl;
+    CK(cudaMemcpyAsync(c->sc_host, &P.sc->bb, sizeof(double), cudaMemcpyDeviceToHost, c->stream));
+    CK(cudaMemcpyAsync(&ctl, P.ctl, sizeof(ctl), cudaMemcpyDeviceToHost, c->stream));
+    CK(cudaStreamSynchronize(c->stream));
+    c->last_iters = 0;
+    c->last_relres = ctl.relres;
+    if (ctl.more) {
+        c->last_iters = P.solve(c->Wf, c->W, true, *c->sc_host, c->desc.poisson_tol, maxit, c->stream, &c->last_relres);
+        launch_w_from_W<T>(c, c->stream);
+    }
+    return (c->last_relres <= c->desc.poisson_tol) ? VVM_GPU_OK : VVM_GPU_ENOCONV;
+}
+
 // Records the cal_w solve with device-side loop control (graph capture on
 // c->stream). The FP64 step: one PCG loop to tol. The mixed step: FP64
 // residual refinement around an FP32 PCG loop. Returns the number of
@@ -2642,9 +2769,8 @@ long long record_solve(vvm_gpu_ctx* c, double tol, int maxit, bool warm) {
     // learned: the flexible-CG loop, then the check below, whose plain PCG
     // loop runs only if the flexible CG stopped at its cap (the fallback)
     if (learned) in_bodies += record_fcg(c, tol, c->learned_cap);
-    if (c->spectral) P64.sp.apply_to(c->Wf, c->W, st);   // direct solve; the loop below checks it
-    else if (!warm && !learned) CK(cudaMemsetAsync(c->W, 0, (size_t)P64.NK * P64.pitch * sizeof(double), st));
-    if (!c->mixed || c->spectral || learned) {
+    if (!warm && !learned) CK(cudaMemsetAsync(c->W, 0, (size_t)P64.NK * P64.pitch * sizeof(double), st));
+    if (!c->mixed || learned) {
         cudaGraphConditionalHandle h = new_handle(&c->stats, st);
         klaunch<k_cg_check_body<double>, 256>(&c->stats, VVM_K_CG, st, k_cg_check<double>, G, B, 0, v,
                                               (const double*)c->Wf, c->W, P64.r, P64.partial, P64.sc, P64.ctl,
@@ -2723,28 +2849,34 @@ int launch_cal_w(vvm_gpu_ctx* c, long long* recorded_in_loops = nullptr, cudaEve
     int NX = c->d.nx - 2, NK = c->d.nz - 3;
     int pitch = c->pcg64->pitch;
     dim3 B(64, 4), G(cdiv(NX, 64), cdiv(NK, 4));
+    const int maxit = c->desc.poisson_maxit > 0 ? c->desc.poisson_maxit : 200;
+    if (c->spectral) {
+        int rc = VVM_GPU_OK;
+        if (recorded_in_loops) *recorded_in_loops = record_spectral<T>(c, before_w, maxit);
+        else rc = run_spectral<T>(c, before_w, maxit);
+        c->nsolves++;
+        return rc;
+    }
     klaunch<k_poisson_rhs_body<T>, 256>(&c->stats, VVM_K_POISSON_RHS, c->stream, k_poisson_rhs<T>, G, B, 0, c->d,
                                         c->c.dx, (const double*)c->rhow, (const double*)c->rwres,
                                         (const T*)zeta_pre<T>(c), c->Wf, pitch, c->wpartial, c->pcg64->arrive,
                                         c->pcg64->sc);   // sets sc->bb
     const bool warm = c->desc.warm_start != 0;
-    const int maxit = c->desc.poisson_maxit > 0 ? c->desc.poisson_maxit : 200;
     if (recorded_in_loops) {   // graph capture: the loops run on the device
-        if (warm && !c->spectral) {
+        if (warm) {
             LAUNCH(&c->stats, VVM_K_POISSON_RHS, c->stream, k_extrapolate<<<G, B, 0, c->stream>>>(NX, NK, pitch, c->W, c->Wprev));
             CKL();
         }
         *recorded_in_loops = record_solve(c, c->desc.poisson_tol, maxit, warm);
         c->nsolves++;
         if (before_w) CK(cudaStreamWaitEvent(c->stream, before_w, 0));
-        klaunch<k_w_from_W_body<T>, 256>(&c->stats, VVM_K_POISSON_RHS, c->stream, k_w_from_W<T>, c->grid_interior(2),
-                                         c->blk(), 0, c->d, (const double*)c->rhow, (const double*)c->W, pitch, F.w);
+        launch_w_from_W<T>(c, c->stream);
         return VVM_GPU_OK;
     }
     CK(cudaMemcpyAsync(c->sc_host, &c->pcg64->sc->bb, sizeof(double), cudaMemcpyDeviceToHost, c->stream));
     CK(cudaStreamSynchronize(c->stream));
     double bb = *c->sc_host;
-    if (warm && !c->spectral) {
+    if (warm) {
         // the previous solution(s) as the initial guess: linear extrapolation
         // once two exist (the reference starts every solve from zero)
         if (c->nsolves >= 2) {
@@ -2758,8 +2890,7 @@ int launch_cal_w(vvm_gpu_ctx* c, long long* recorded_in_loops = nullptr, cudaEve
     int rc = solve_w(c, bb, c->desc.poisson_tol, warm);
     c->nsolves++;
     if (before_w) CK(cudaStreamWaitEvent(c->stream, before_w, 0));
-    LAUNCH(&c->stats, VVM_K_POISSON_RHS, c->stream, k_w_from_W<T><<<c->grid_interior(2), c->blk(), 0, c->stream>>>(c->d, c->rhow, c->W, pitch, F.w));
-    CKL();
+    launch_w_from_W<T>(c, c->stream);
     return rc;
 }
 
@@ -2861,13 +2992,12 @@ int run_step(vvm_gpu_ctx* c, long long* recorded_in_loops = nullptr) {
     // The step's kernels form two chains (in a captured step, two branches of
     // the graph; the results are those of the reference's order, since
     // neither chain reads what the other writes before they meet):
-    //  main: pzeta_pt (writes zetap and its tendencies), cal_w up to its
-    //        solution W, then, once the side chain has read w and u and
-    //        written ubarTopp, w from W and cal_u (which reads ubarTopp);
-    //  side: pubarTop_pt (reads u, w, RKM; writes ubar, dubar), the scalar
-    //        advection (writes the future th, qv, qc, qr and their
-    //        tendencies), their NVP rescaling and AddForcing, Kessler, its
-    //        NVP and the halos of th, qv, qc, qr.
+    //  main: pzeta_pt (writes zetap and its tendencies) with pubarTop_pt (reads
+    //        u, w, RKM; writes ubar, dubar), cal_w up to its solution W, then,
+    //        once the side chain has read w and u, w from W and cal_u;
+    //  side: the scalar advection (writes the future th, qv, qc, qr and their
+    //        tendencies) and their NVP sums, then Kessler on its rescaled and
+    //        forced values, with its own NVP sums and the halos.
     // They meet before the turbulence. A batch's cases are already parallel
     // branches of its graph: there every case runs as one chain, in the
     // reference's order; so does a profiled step, whose event timers should
@@ -2878,13 +3008,12 @@ int run_step(vvm_gpu_ctx* c, long long* recorded_in_loops = nullptr) {
         fork_side(c, 0);
         {
             OnStream os(c, c->side);
-            if (!sf) launch_pubartop<T>(c);                    // pubarTop_pt
             launch_padv<T, F_TH | F_QV | F_QC | F_QR>(c);  // pth, pqv, pqc, pqr
-            CK(cudaEventRecord(c->fork_ev[1], c->side));   // u and w read, ubarTopp written
+            CK(cudaEventRecord(c->fork_ev[1], c->side));   // u and w read
             launch_kessler<T>(c);                              // NVP + AddForcing, Kessler + NVP sums + halos
         }
         try {
-            launch_pzeta<T>(c);                                // pzeta_pt
+            launch_pzeta<T>(c);                                // pzeta_pt, pubarTop_pt
             if (sf) {
                 CK(cudaStreamWaitEvent(c->stream, c->fork_ev[1], 0));
                 rc = launch_calpsiuw<T>(c);                    // calpsiuw (Iteration.cpp:289-290)
@@ -2903,7 +3032,6 @@ int run_step(vvm_gpu_ctx* c, long long* recorded_in_loops = nullptr) {
         if (sf) {
             rc = launch_calpsiuw<T>(c);
         } else {
-            launch_pubartop<T>(c);
             rc = launch_cal_w<T>(c, recorded_in_loops);
             launch_cal_u<T>(c);
         }
