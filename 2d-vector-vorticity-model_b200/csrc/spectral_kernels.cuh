@@ -309,6 +309,129 @@ __device__ __forceinline__ void k_spec_modes_seg_body(const SpecArgs<P>& a) {
 template <typename P>
 __global__ void __launch_bounds__(64 * kModeSegs) k_spec_modes_seg(SpecArgs<P> a) { k_spec_modes_seg_body<P>(a); }
 
+// The same solve with a segment's rows (at most kModeRows) held in registers:
+// every load of a thread is issued at once, where k_spec_modes_seg waits for
+// each row's in each of its four sweeps (one block a SM or less: latency is all
+// it spends). A thread a mode and segment, 16 modes a block; us with k_spec_modes_seg
+// / 16 segments of 8 rows / 32 of 4: 2048 x 256 17.4 / 8 / 8, 8192 x 256 19 / 14 /
+// 22, 128 x 64 6.3 / 4 / 4. Taller grids would spill, and keep k_spec_modes_seg.
+constexpr int kModeRows = 8, kModeRegSegs = 16, kModeRegThreads = 512;
+
+template <typename P>
+__device__ __forceinline__ void k_spec_modes_reg_body(const SpecArgs<P>& a) {
+    constexpr int S = kModeRegSegs, ML = kModeRegThreads / (2 * S), R = kModeRows;
+    __shared__ P shA[2][S][ML][3];   // (A re, A im, B) per half, segment, mode
+    __shared__ P shY[2][ML][2];      // the halves' last rows after elimination
+    const int ml = threadIdx.x % ML, idx = threadIdx.x / ML;
+    const int h = idx / S, sg = idx % S;
+    const int m = blockIdx.x * ML + ml;
+    const bool on = m <= a.NX / 2;
+    const int NK = a.NK, mid = a.mid;
+    const size_t mp = a.mpitch;
+    const P* __restrict__ lc = h ? a.ru : a.rd;
+    // this half's rows in elimination order: k(j) = k0 + dir j, j < n
+    const int n = h ? NK - 1 - mid : mid + 1;
+    const int dir = h ? -1 : 1, k0 = h ? NK - 1 : 0;
+    const int L = (n + S - 1) / S;
+    const int j0 = min(n, sg * L), cnt = on ? min(n, j0 + L) - j0 : 0;
+    auto at = [&](int q) { return (size_t)(k0 + dir * (j0 + q)) * mp + m; };
+
+    P fr[R], fi[R], iv[R], cp[R], c[R];
+#pragma unroll
+    for (int q = 0; q < R; q++) {
+        const bool in = q < cnt;
+        fr[q] = in ? a.sre[at(q)] : P(0);
+        fi[q] = in ? a.sim[at(q)] : P(0);
+        iv[q] = in ? a.inv[at(q)] : P(0);
+        cp[q] = in ? a.cp[at(q)] : P(0);
+        c[q] = in ? lc[k0 + dir * (j0 + q)] : P(0);
+    }
+    P cpm = P(0), cqm = P(0), dn = P(0);
+    if (on) {
+        cpm = a.cp[(size_t)mid * mp + m];
+        dn = a.den[m];
+        if (mid + 1 < NK) cqm = a.cp[(size_t)(mid + 1) * mp + m];
+    }
+    // elimination: the segment's map
+    P Ar = P(0), Ai = P(0), Bm = P(1);
+#pragma unroll
+    for (int q = 0; q < R; q++)
+        if (q < cnt) {
+            const P e = c[q] * iv[q];
+            Ar = fr[q] * iv[q] + e * Ar;
+            Ai = fi[q] * iv[q] + e * Ai;
+            Bm = e * Bm;
+        }
+    shA[h][sg][ml][0] = Ar;
+    shA[h][sg][ml][1] = Ai;
+    shA[h][sg][ml][2] = Bm;
+    if (threadIdx.x < 4 * ML) (&shY[0][0][0])[threadIdx.x] = P(0);   // an empty half: 0
+    __syncthreads();
+    P yr = P(0), yi = P(0);
+    for (int t = 0; t < sg; t++) {
+        const P b = shA[h][t][ml][2];
+        yr = shA[h][t][ml][0] + b * yr;
+        yi = shA[h][t][ml][1] + b * yi;
+    }
+#pragma unroll
+    for (int q = 0; q < R; q++)
+        if (q < cnt) {
+            yr = (fr[q] + c[q] * yr) * iv[q];
+            yi = (fi[q] + c[q] * yi) * iv[q];
+            fr[q] = yr;
+            fi[q] = yi;
+        }
+    const bool last = cnt > 0 && j0 + cnt == n;   // holds the meeting row
+    if (last) {
+        shY[h][ml][0] = yr;
+        shY[h][ml][1] = yi;
+    }
+    __syncthreads();
+    // the meeting rows mid (half 0) and mid + 1 (half 1)
+    const P ymr = shY[0][ml][0], ymi = shY[0][ml][1], zr = shY[1][ml][0], zi = shY[1][ml][1];
+    P wr = (ymr - cpm * zr) * dn, wi = (ymi - cpm * zi) * dn;
+    if (h) {
+        wr = zr - cqm * wr;
+        wi = zi - cqm * wi;
+    }
+    // back-substitution outwards: the segment's map over its rows but the meeting one
+    const int back = last ? cnt - 1 : cnt;
+    Ar = P(0);
+    Ai = P(0);
+    Bm = P(1);
+#pragma unroll
+    for (int q = R - 1; q >= 0; q--)
+        if (q < back) {
+            Ar = fr[q] - cp[q] * Ar;
+            Ai = fi[q] - cp[q] * Ai;
+            Bm = -cp[q] * Bm;
+        }
+    // (shA's first maps were read before the barrier above)
+    shA[h][sg][ml][0] = Ar;
+    shA[h][sg][ml][1] = Ai;
+    shA[h][sg][ml][2] = Bm;
+    __syncthreads();
+    if (last) {
+        a.sre[at(cnt - 1)] = wr;
+        a.sim[at(cnt - 1)] = wi;
+    }
+    for (int t = S - 1; t > sg; t--) {
+        const P b = shA[h][t][ml][2];
+        wr = shA[h][t][ml][0] + b * wr;
+        wi = shA[h][t][ml][1] + b * wi;
+    }
+#pragma unroll
+    for (int q = R - 1; q >= 0; q--)
+        if (q < back) {
+            wr = fr[q] - cp[q] * wr;
+            wi = fi[q] - cp[q] * wi;
+            a.sre[at(q)] = wr;
+            a.sim[at(q)] = wi;
+        }
+}
+template <typename P>
+__global__ void __launch_bounds__(kModeRegThreads) k_spec_modes_reg(SpecArgs<P> a) { k_spec_modes_reg_body<P>(a); }
+
 // Rows 2b and 2b+1 from their spectra, scaled by 1/NX, given to store(row,
 // column, value).
 template <typename P, typename Store>

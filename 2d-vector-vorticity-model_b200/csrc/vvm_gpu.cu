@@ -751,7 +751,14 @@ struct ModeFactors {
         a.sim = ar.alloc<P>((size_t)NK * mp);
     }
 
+    // in registers up to 2 x kModeRegSegs x kModeRows rows
     void solve_modes(Stats* stats, cudaStream_t st) {
+        if (a.NK <= 2 * kModeRegSegs * kModeRows) {
+            klaunch<k_spec_modes_reg_body<P>, kModeRegThreads>(stats, VVM_K_MG_COARSE, st, k_spec_modes_reg<P>,
+                                                               dim3(cdiv(a.NX / 2 + 1, kModeRegThreads / (2 * kModeRegSegs))),
+                                                               dim3(kModeRegThreads), 0, a);
+            return;
+        }
         klaunch<k_spec_modes_seg_body<P>, 64 * kModeSegs>(stats, VVM_K_MG_COARSE, st, k_spec_modes_seg<P>,
                                                           dim3(cdiv(a.NX / 2 + 1, 32)), dim3(64 * kModeSegs), 0, a);
     }

@@ -168,3 +168,25 @@ def test_spectral_cal_w_at_edge_sizes(gpu, nx, nz, d):
     for f in ("w", "u"):
         assert np.abs(m[f]).max() > 0
         assert rel_l2(a[f], m[f]) <= 1e-8, (f, rel_l2(a[f], m[f]))
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("nk", [3, 4, 16, 31, 33, 255, 256, 257])
+def test_spectral_modes_at_every_height(gpu, nk):
+    """The z solve in registers (to 256 rows) and beyond: the direct solve of a
+    random right-hand side leaves a residual at round-off (1e-12: the
+    operator's condition number at 257 rows of 32 columns, about 1e4, times
+    2^-53 times the transforms' growth), without CG iterations."""
+    from vvm_b200.initial_state import warm_bubble
+    from oracle.models import PortModel
+    nx, nz = 32, nk + 1
+    st = warm_bubble(nx, nz, 200.0, 15000.0 / nz)
+    g = gpu.VVMGpu(st.grid, warm_start=False, solver=gpu.VVM_SOLVER_SPECTRAL)
+    g.upload(st)
+    m = PortModel(st.grid)
+    m.load(st)
+    b = np.random.default_rng(nk).standard_normal(nx * nk)
+    W, it, rel = g.poisson_solve(b, tol=1e-10)
+    g.close()
+    assert it == 0 and rel <= 1e-12
+    assert rel_l2(m.apply_A(W), b) <= 1e-12
