@@ -1476,6 +1476,10 @@ struct GSSweepArgs {
     const unsigned* kmax;
     float fz[2];         // largest C / K over the rows: Mparam, Hparam
     GSTileCtl* ctl;      // more: the repeated passes are needed
+    // a captured step that puts its rare loops at its end (run_step_direct):
+    // the solve's check has failed; set when the end has to run
+    const int* solve_more;
+    int* redo;
 };
 
 template <typename T>
@@ -1771,7 +1775,9 @@ __device__ __forceinline__ void k_gs_sweep_body(const GSSweepArgs<T>& a, cudaGra
     const bool ok = km == km && kh == kh && l > 0.f && hz <= kGWHaloMax && 16.f * lx >= kGWBits<T>;
     if (threadIdx.x == 0 && blockIdx.x == 0 && blockIdx.y == 0) {
         a.ctl->more = ok ? 0 : 1;
-        if (h) cudaGraphSetConditional(h, ok ? 0u : 1u);
+        const bool more = !ok || (a.solve_more && *a.solve_more);
+        if (a.redo) *a.redo = more;
+        if (h) cudaGraphSetConditional(h, more ? 1u : 0u);
     }
     if (!ok) return;
     const int wid = threadIdx.x >> 5;
@@ -2218,10 +2224,12 @@ struct NudgeArgs {
     const T* qv;
     int do_th, do_zeta;
     double tau;       // moisture_nudge_time, 0 = off
+    const int* skip;  // nothing to do where *skip (may be null)
 };
 
 template <typename T>
 __device__ __forceinline__ void k_nudge_body(const NudgeArgs<T>& a) {
+    if (a.skip && *a.skip) return;
     const Dims& d = a.d;
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     const int k = blockIdx.y * blockDim.y + threadIdx.y;
@@ -2257,11 +2265,13 @@ struct MeanArgs {
     double* ubar;   // [0] ubarTop, [1] ubarTopp
     int rotate_ubar;
     unsigned* kmax;   // [2]: cleared for the next step's k_rkm_rkh (may be null)
+    const int* skip;  // nothing to do where *skip (may be null)
 };
 
 template <typename T>
 __device__ __forceinline__ void k_update_mean_body(const MeanArgs<T>& a) {
     __shared__ double sh[32 * 2];
+    if (a.skip && *a.skip) return;
     const Dims& d = a.d;
     const int k = 1 + blockIdx.x;
     double s[2] = {0, 0};

@@ -245,6 +245,13 @@ __global__ void k_spec_check(VecArgs<double> v, const double* f, const double* x
     k_spec_check_body(v, f, x, r, partial, sc, ctl, arrive, h, tol2, maxit);
 }
 
+// The rare end of a captured step (run_step_direct): opens its CG loop if the
+// solve's check failed; counts the kernels it ran outside its loops.
+__global__ void k_redo_begin(const CGCtl* ctl, cudaGraphConditionalHandle solve) {
+    cudaGraphSetConditional(solve, ctl->more ? 1u : 0u);
+}
+__global__ void k_redo_end(long long* exec, int kernels) { *exec += kernels; }
+
 // The streamfunction formulation (PoissonSolver::calpsiuw, STREAMFUNCTION,
 // src/PoissonSolver.cpp:124-177). Its matrix (src/PoissonSolver.cpp:726-756,
 // POISSONPARAM = 0) is -S with S the symmetric w-equation operator of
@@ -1760,6 +1767,7 @@ struct vvm_gpu_ctx {
     double* ubar = nullptr;   // [0] ubarTop, [1] ubarTopp
     double* dubar = nullptr;  // [2]
     double *partial = nullptr, *nvp = nullptr;
+    int* redo = nullptr;         // a captured step's end has to run (run_step_direct)
     int npart = 0;
     double* staging = nullptr;   // staging_slots() host images of a field
     int* err_host = nullptr;     // pinned copy of d_err (downloads)
@@ -1775,11 +1783,11 @@ struct vvm_gpu_ctx {
     double* Wprev = nullptr;   // previous cal_w solution (initial-guess extrapolation)
     int nsolves = 0;
     // CUDA graphs of one whole step, by (time-level buffer, step parity)
-    cudaGraphExec_t gexec[2][2] = {};
-    long long gstatic[2][2] = {};      // kernels outside the solver loops
+    cudaGraphExec_t gexec[2][2][2] = {};   // of one step, of kGraphSteps
+    long long gstatic[2][2][2] = {};       // kernels outside the solver loops
     cudaStream_t cap[2] = {};          // streams for capturing loop bodies
     cudaStream_t side = nullptr;       // the step's second chain (run_step)
-    cudaEvent_t fork_ev[3] = {};       // its fork, meeting and join points
+    cudaEvent_t fork_ev[6] = {};       // its fork, meeting and join points
     cudaStream_t xfer = nullptr;       // host copies of the prognostic transfers
     cudaEvent_t xev[2][2] = {};        // per staging slot: [0] its copy done, [1] its layout kernel done
     bool branches = true;              // use them (off inside a batch: the cases are the branches)
@@ -1798,12 +1806,13 @@ struct vvm_gpu_ctx {
     std::string err;
 
     void drop_graphs() {
-        for (auto& row : gexec)
-            for (auto& g : row)
-                if (g) {
-                    cudaGraphExecDestroy(g);
-                    g = nullptr;
-                }
+        for (auto& many : gexec)
+            for (auto& row : many)
+                for (auto& g : row)
+                    if (g) {
+                        cudaGraphExecDestroy(g);
+                        g = nullptr;
+                    }
         if (fcg_exec) cudaGraphExecDestroy(fcg_exec);
         fcg_exec = nullptr;
     }
@@ -2105,9 +2114,10 @@ cudaGraphConditionalHandle new_handle(Stats* s, cudaStream_t st) {
     return new_handle(st);
 }
 
-// Appends a WHILE node (condition h) to the graph being captured on st and
-// returns its body graph; capture on st continues after the node.
-cudaGraph_t add_while(cudaStream_t st, cudaGraphConditionalHandle h) {
+// Appends a WHILE (or IF) node (condition h) to the graph being captured on st
+// and returns its body graph; capture on st continues after the node.
+cudaGraph_t add_while(cudaStream_t st, cudaGraphConditionalHandle h,
+                      cudaGraphConditionalNodeType type = cudaGraphCondTypeWhile) {
     cudaStreamCaptureStatus status;
     cudaGraph_t g;
     const cudaGraphNode_t* deps = nullptr;
@@ -2116,7 +2126,7 @@ cudaGraph_t add_while(cudaStream_t st, cudaGraphConditionalHandle h) {
     cudaGraphNodeParams p = {};
     p.type = cudaGraphNodeTypeConditional;
     p.conditional.handle = h;
-    p.conditional.type = cudaGraphCondTypeWhile;
+    p.conditional.type = type;
     p.conditional.size = 1;
     cudaGraphNode_t node;
     CK(cudaGraphAddNode(&node, g, deps, nd, &p));
@@ -2276,21 +2286,17 @@ inline GSSweepShape gs_sweep_shape(const Dims& d, bool mixed) {
 }
 
 template <typename T>
-void launch_turbulence(vvm_gpu_ctx* c, bool nudge, long long* recorded_in_loops = nullptr) {
+void launch_rkm(vvm_gpu_ctx* c) {
     Fields<T>& F = fields<T>(c);
-    int fut = 1 - c->cur;
-    cudaStream_t st = c->stream;
+    RKArgs<T> r{c->d, c->c, c->profiles(), F.u, F.w, c->in_step ? F.pre[1] : F.th[1 - c->cur], F.RKM, F.RKH, c->kmax};
+    klaunch<k_rkm_rkh_body<T>, 256>(&c->stats, VVM_K_RKM, c->stream, k_rkm_rkh<T>, c->grid_interior(1), c->blk(), 0, r);
+}
+
+template <typename T>
+GSSweepArgs<T> gs_sweep_args(vvm_gpu_ctx* c, bool nudge) {
+    Fields<T>& F = fields<T>(c);
+    const int fut = 1 - c->cur;
     T* v[5] = {F.zeta[fut], F.th[fut], F.qv[fut], F.qc[fut], F.qr[fut]};
-    RKArgs<T> r{c->d, c->c, c->profiles(), F.u, F.w, c->in_step ? F.pre[1] : v[1], F.RKM, F.RKH, c->kmax};
-    if (!recorded_in_loops) {   // a graph's steps leave both as they found them
-        CK(cudaMemsetAsync(c->kmax, 0, 2 * sizeof(unsigned), st));
-        CK(cudaMemsetAsync(c->gsctl, 0, sizeof(GSTileCtl), st));
-    }
-    if (!c->in_step) {   // a routine call: the fields lie in the future level
-        for (int f = 0; f < 5; f++)
-            CK(cudaMemcpyAsync(F.pre[f], v[f], c->d.cells() * sizeof(T), cudaMemcpyDeviceToDevice, st));
-    }
-    klaunch<k_rkm_rkh_body<T>, 256>(&c->stats, VVM_K_RKM, st, k_rkm_rkh<T>, c->grid_interior(1), c->blk(), 0, r);
     GSSweepArgs<T> w{};
     w.d = c->d;
     w.c = c->c;
@@ -2312,75 +2318,112 @@ void launch_turbulence(vvm_gpu_ctx* c, bool nudge, long long* recorded_in_loops 
     w.fz[0] = c->gs_fz[0];
     w.fz[1] = c->gs_fz[1];
     w.ctl = c->gsctl;
-    GSArgs<T> g{c->d, c->c, c->profiles(), {v[0], v[1], v[2], v[3], v[4]},
-                F.RKM, F.RKH, 0x1f, nudge ? 1 : 0, F.gsA, nullptr, nullptr, nullptr};
-    // the repeated passes: tiles of tr rows (see k_gs_tiles)
-    const int tr = gs_tile_rows(c);
-    const int nb = cdiv(c->d.nz - 2, tr), nc = cdiv(c->d.pitch, kGTCols);
-    GSTileArgs<T> t{nb, nc, tr, F.gsRight, F.gsTop, c->gsctl, recorded_in_loops ? c->d_exec : nullptr};
-    const int tblocks = cdiv(5 * nb * nc, 4);
-    auto inputs = [&](cudaStream_t s) {
+    return w;
+}
+
+template <typename T>
+void launch_gs_sweep(vvm_gpu_ctx* c, const GSSweepArgs<T>& w, cudaGraphConditionalHandle h) {
+    klaunch<k_gs_sweep_body<T>, 32 * kGWWarps>(&c->stats, VVM_K_GS, c->stream, k_gs_sweep<T>,
+                                               dim3(cdiv(w.jobs * w.nb * w.nc, kGWWarps)), dim3(32 * kGWWarps), 0, w, h);
+}
+
+// The repeated passes a sweep may ask for: tiles of tr rows (see k_gs_tiles).
+template <typename T>
+struct GSPasses {
+    vvm_gpu_ctx* c;
+    GSSweepArgs<T> w;
+    GSArgs<T> g;
+    GSTileArgs<T> t;
+    GSPasses(vvm_gpu_ctx* c_, const GSSweepArgs<T>& w_, bool recorded) : c(c_), w(w_) {
+        Fields<T>& F = fields<T>(c);
+        g = GSArgs<T>{c->d, c->c, c->profiles(), {w.dst[0], w.dst[1], w.dst[2], w.dst[3], w.dst[4]},
+                      F.RKM, F.RKH, 0x1f, w.nudge, F.gsA, nullptr, nullptr, nullptr};
+        const int tr = gs_tile_rows(c);
+        t = GSTileArgs<T>{cdiv(c->d.nz - 2, tr), cdiv(c->d.pitch, kGTCols), tr, F.gsRight, F.gsTop, c->gsctl,
+                          recorded ? c->d_exec : nullptr};
+    }
+    int most() const { return std::max(2, t.nb + t.nc - 1); }
+    void inputs(cudaStream_t s) {
         klaunch<k_gs_inputs_body<T>, 256>(&c->stats, VVM_K_GS, s, k_gs_inputs<T>, c->grid_all(), c->blk(), 0, w);
-    };
-    auto pass = [&](cudaStream_t s, auto first, cudaGraphConditionalHandle h) {
-        constexpr bool F1 = decltype(first)::value;
-        klaunch<k_gs_tiles_body<T, F1>, 128, kGSTileMinBlocks<T>>(&c->stats, VVM_K_GS, s, k_gs_tiles<T, F1>, dim3(tblocks),
-                                                                  dim3(128), 0, g, t, h);
-    };
+    }
+    template <bool FIRST>
+    void pass(cudaStream_t s, cudaGraphConditionalHandle h) {
+        klaunch<k_gs_tiles_body<T, FIRST>, 128, kGSTileMinBlocks<T>>(&c->stats, VVM_K_GS, s, k_gs_tiles<T, FIRST>,
+                                                                     dim3(cdiv(5 * t.nb * t.nc, 4)), dim3(128), 0, g, t, h);
+    }
+    // A WHILE node (condition h) on st that the sweep's kernel opens only when
+    // the passes are needed; its body, captured on cap, runs the first
+    // (inputs, pass 1) once and then a later pass each time round. Returns the
+    // kernels of the body.
+    long long record(cudaStream_t st, cudaStream_t cap, cudaGraphConditionalHandle h) {
+        record_cond(&c->stats, &c->gsctl->more, true);
+        cudaGraph_t body = add_while(&c->stats, st, h);
+        BodyCapture bc(cap, body, &c->stats);
+        const long long n0 = c->stats.launches;
+        inputs(bc.s);
+        pass<true>(bc.s, 0);
+        pass<false>(bc.s, h);
+        record_cond(&c->stats, &c->gsctl->more, false);
+        bc.end();
+        return c->stats.launches - n0;
+    }
+};
+
+template <typename T>
+void launch_turbulence(vvm_gpu_ctx* c, bool nudge, long long* recorded_in_loops = nullptr) {
+    Fields<T>& F = fields<T>(c);
+    cudaStream_t st = c->stream;
+    const GSSweepArgs<T> w = gs_sweep_args<T>(c, nudge);
+    GSPasses<T> passes(c, w, recorded_in_loops != nullptr);
+    if (!recorded_in_loops) {   // a graph's steps leave both as they found them
+        CK(cudaMemsetAsync(c->kmax, 0, 2 * sizeof(unsigned), st));
+        CK(cudaMemsetAsync(c->gsctl, 0, sizeof(GSTileCtl), st));
+    }
+    if (!c->in_step) {   // a routine call: the fields lie in the future level
+        for (int f = 0; f < 5; f++)
+            CK(cudaMemcpyAsync(F.pre[f], w.dst[f], c->d.cells() * sizeof(T), cudaMemcpyDeviceToDevice, st));
+    }
+    launch_rkm<T>(c);
     if (c->tune_gs_tr == kGSSchedCluster) {
-        inputs(st);
-        launch_gs_cluster<T>(c, g);
+        passes.inputs(st);
+        launch_gs_cluster<T>(c, passes.g);
         return;
     }
     const cudaGraphConditionalHandle h = recorded_in_loops ? new_handle_reset(&c->stats, st) : 0;
-    klaunch<k_gs_sweep_body<T>, 32 * kGWWarps>(&c->stats, VVM_K_GS, st, k_gs_sweep<T>,
-                                               dim3(cdiv(w.jobs * w.nb * w.nc, kGWWarps)), dim3(32 * kGWWarps), 0, w, h);
+    launch_gs_sweep<T>(c, w, h);
     if (recorded_in_loops) {
-        // graph capture: a WHILE node that the sweep's kernel opens only when
-        // the passes are needed; its body runs the first (inputs, pass 1)
-        // once and then a later pass each time round
-        record_cond(&c->stats, &c->gsctl->more, true);
-        cudaGraph_t body = add_while(&c->stats, st, h);
-        BodyCapture bc(c->cap[0], body, &c->stats);
-        const long long n0 = c->stats.launches;
-        inputs(bc.s);
-        pass(bc.s, std::true_type{}, 0);
-        pass(bc.s, std::false_type{}, h);
-        record_cond(&c->stats, &c->gsctl->more, false);
-        bc.end();
-        *recorded_in_loops += c->stats.launches - n0;
+        *recorded_in_loops += passes.record(st, c->cap[0], h);
         return;
     }
-    const int maxp = std::max(2, nb + nc - 1);
-    for (int p = 1; p <= maxp; p++) {
+    for (int p = 1; p <= passes.most(); p++) {
         CK(cudaMemcpyAsync(c->sc_host_i, &c->gsctl->more, sizeof(int), cudaMemcpyDeviceToHost, st));
         CK(cudaStreamSynchronize(st));
         if (!*c->sc_host_i) break;
         if (p == 1) {
-            inputs(st);
-            pass(st, std::true_type{}, 0);
+            passes.inputs(st);
+            passes.template pass<true>(st, 0);
         }
-        pass(st, std::false_type{}, 0);
+        passes.template pass<false>(st, 0);
     }
 }
 
 template <typename T>
-void launch_nudge(vvm_gpu_ctx* c, bool th_zeta, bool qv) {
+void launch_nudge(vvm_gpu_ctx* c, bool th_zeta, bool qv, const int* skip = nullptr) {
     Fields<T>& F = fields<T>(c);
     int now = c->cur, fut = 1 - c->cur;
     NudgeArgs<T> a{c->d, c->c, c->profiles(), F.th[fut], F.zeta[fut], F.qv[fut], F.qv[now],
                    th_zeta ? 1 : 0, (th_zeta && c->desc.case_id != 2) ? 1 : 0,
-                   qv ? c->desc.moisture_nudge_time : 0.0};
+                   qv ? c->desc.moisture_nudge_time : 0.0, skip};
     klaunch<k_nudge_body<T>, 256>(&c->stats, VVM_K_MEAN, c->stream, k_nudge<T>, c->grid_all(), c->blk(), 0, a);
     CKL();
 }
 
 template <typename T>
-void launch_update_mean(vvm_gpu_ctx* c, bool rotate) {
+void launch_update_mean(vvm_gpu_ctx* c, bool rotate, const int* skip = nullptr) {
     Fields<T>& F = fields<T>(c);
     int fut = 1 - c->cur;
     MeanArgs<T> a{c->d, c->offset_th(), c->offset_qv(), F.th[fut], F.qv[fut], c->thb, c->qvb, c->thvb,
-                  c->ubar, rotate ? 1 : 0, c->in_step ? c->kmax : nullptr};
+                  c->ubar, rotate ? 1 : 0, c->in_step ? c->kmax : nullptr, skip};
     klaunch<k_update_mean_body<T>, 256>(&c->stats, VVM_K_MEAN, c->stream, k_update_mean<T>, dim3(c->d.nz - 2),
                                         dim3(256), 0, a);
 }
@@ -2710,29 +2753,23 @@ void launch_w_from_W(vvm_gpu_ctx* c, cudaStream_t st) {
                                      c->d, (const double*)c->rhow, (const double*)c->W, c->pcg64->pitch, fields<T>(c).w);
 }
 
-// The direct solve of cal_w, W and w in three launches, and the check of its
-// residual, which sets the condition h (0: none).
-template <typename T>
-void launch_spectral_w(vvm_gpu_ctx* c, cudaEvent_t before_w, cudaGraphConditionalHandle h, int maxit) {
+// The check of a direct solve's residual, which sets the condition h (0: none).
+void launch_spectral_check(vvm_gpu_ctx* c, cudaGraphConditionalHandle h, int maxit) {
     PCG<double>& P = *c->pcg64;
-    P.sp.apply_fields(spec_fields<T>(c), c->stream, before_w);
     const dim3 B = P.block(), G(P.grid().x, cdiv(P.NK, (int)B.y * kCheckRows));
     klaunch<k_spec_check_body, 256>(&c->stats, VVM_K_CG, c->stream, k_spec_check, G, B, 0, P.vargs(), (const double*)c->Wf,
                                     (const double*)c->W, P.r, P.partial, P.sc, P.ctl, P.arrive, h,
                                     c->desc.poisson_tol * c->desc.poisson_tol, maxit);
 }
 
-// Records cal_w by the direct solve (graph capture): only if its check fails,
-// CG iterations from W, with w formed anew. Returns the kernels recorded
-// inside that loop.
+// The loop that follows a check that fails (condition h, body captured on
+// cap): CG iterations from W, with w formed anew. Returns the body's kernels.
 template <typename T>
-long long record_spectral(vvm_gpu_ctx* c, cudaEvent_t before_w, int maxit) {
+long long record_spectral_loop(vvm_gpu_ctx* c, cudaStream_t cap, cudaGraphConditionalHandle h, int maxit) {
     PCG<double>& P = *c->pcg64;
-    cudaGraphConditionalHandle h = new_handle(&c->stats, c->stream);
-    launch_spectral_w<T>(c, before_w, h, maxit);
     record_cond(&c->stats, &P.ctl->more, true);
     cudaGraph_t body = add_while(&c->stats, c->stream, h);
-    BodyCapture bc(c->cap[0], body, &c->stats);
+    BodyCapture bc(cap, body, &c->stats);
     const long long n0 = c->stats.launches;
     const int nb = P.record_iteration(c->W, bc.s);
     launch_w_from_W<T>(c, bc.s);   // before the loop's test, which closes a grouped case's gate
@@ -2743,11 +2780,14 @@ long long record_spectral(vvm_gpu_ctx* c, cudaEvent_t before_w, int maxit) {
     return c->stats.launches - n0;
 }
 
+int poisson_maxit(const vvm_gpu_ctx* c) { return c->desc.poisson_maxit > 0 ? c->desc.poisson_maxit : 200; }
+
 // ... without capture: the host reads the check's result.
 template <typename T>
 int run_spectral(vvm_gpu_ctx* c, cudaEvent_t before_w, int maxit) {
     PCG<double>& P = *c->pcg64;
-    launch_spectral_w<T>(c, before_w, 0, maxit);
+    P.sp.apply_fields(spec_fields<T>(c), c->stream, before_w);
+    launch_spectral_check(c, 0, maxit);
     CGCtl ctl;
     CK(cudaMemcpyAsync(c->sc_host, &P.sc->bb, sizeof(double), cudaMemcpyDeviceToHost, c->stream));
     CK(cudaMemcpyAsync(&ctl, P.ctl, sizeof(ctl), cudaMemcpyDeviceToHost, c->stream));
@@ -2856,11 +2896,17 @@ int launch_cal_w(vvm_gpu_ctx* c, long long* recorded_in_loops = nullptr, cudaEve
     int NX = c->d.nx - 2, NK = c->d.nz - 3;
     int pitch = c->pcg64->pitch;
     dim3 B(64, 4), G(cdiv(NX, 64), cdiv(NK, 4));
-    const int maxit = c->desc.poisson_maxit > 0 ? c->desc.poisson_maxit : 200;
+    const int maxit = poisson_maxit(c);
     if (c->spectral) {
         int rc = VVM_GPU_OK;
-        if (recorded_in_loops) *recorded_in_loops = record_spectral<T>(c, before_w, maxit);
-        else rc = run_spectral<T>(c, before_w, maxit);
+        if (recorded_in_loops) {
+            const cudaGraphConditionalHandle h = new_handle(&c->stats, c->stream);
+            c->pcg64->sp.apply_fields(spec_fields<T>(c), c->stream, before_w);
+            launch_spectral_check(c, h, maxit);
+            *recorded_in_loops = record_spectral_loop<T>(c, c->cap[0], h, maxit);
+        } else {
+            rc = run_spectral<T>(c, before_w, maxit);
+        }
         c->nsolves++;
         return rc;
     }
@@ -2988,6 +3034,88 @@ struct OnStream {   // issues a scope's launches on another stream
     ~OnStream() { c->stream = saved; }
 };
 
+// One captured step of the direct solver. A WHILE node that does not open
+// still holds what follows it for 6 to 10 us, and a step with one after the
+// solve and one after the diffusion spends 18 of its 71 us (128 x 64) on them;
+// both are for what almost never happens. So the step goes on as if the
+// solve's check passed and the sweep needed no passes (main and side chains as
+// run_step's; the check beside cal_u), and one IF node at the end, beside the
+// means, does over what depended on either: the CG loop, cal_u, the
+// turbulence with its passes and the means. What they read is still there:
+// the sweep writes the future level from Fields::pre, and the means, which
+// overwrite thb, qvb and ubar, are skipped (c->redo).
+template <typename T>
+void run_step_direct(vvm_gpu_ctx* c, long long* in_loops) {
+    cudaStream_t st = c->stream, side = c->side;
+    const int maxit = poisson_maxit(c);
+    auto means = [&](const int* skip) {
+        if (c->desc.moisture_nudge_time != 0.0) launch_nudge<T>(c, false, true, skip);
+        launch_update_mean<T>(c, true, skip);                  // nextTimeStep: means, ubarTop
+    };
+    fork_side(c, 0);
+    try {
+        {
+            OnStream os(c, side);
+            launch_padv<T, F_TH | F_QV | F_QC | F_QR>(c);  // pth, pqv, pqc, pqr
+            CK(cudaEventRecord(c->fork_ev[1], side));          // u and w read
+            launch_kessler<T>(c);                              // NVP + AddForcing, Kessler + NVP sums + halos
+            CK(cudaEventRecord(c->fork_ev[3], side));
+        }
+        launch_pzeta<T>(c);                                    // pzeta_pt, pubarTop_pt
+        c->pcg64->sp.apply_fields(spec_fields<T>(c), st, c->fork_ev[1]);   // cal_w
+        c->nsolves++;
+        CK(cudaEventRecord(c->fork_ev[4], st));
+        {
+            OnStream os(c, side);
+            CK(cudaStreamWaitEvent(side, c->fork_ev[4], 0));
+            launch_spectral_check(c, 0, maxit);
+            CK(cudaEventRecord(c->fork_ev[5], side));
+        }
+        launch_cal_u<T>(c);                                    // cal_u
+        CK(cudaStreamWaitEvent(st, c->fork_ev[3], 0));
+        launch_rkm<T>(c);                                      // RKM_RKH
+        CK(cudaStreamWaitEvent(st, c->fork_ev[5], 0));
+        GSSweepArgs<T> w = gs_sweep_args<T>(c, true);          // diffusion + theta/zeta nudging
+        w.solve_more = &c->pcg64->ctl->more;
+        w.redo = c->redo;
+        const cudaGraphConditionalHandle h = new_handle_reset(&c->stats, st);
+        launch_gs_sweep<T>(c, w, h);
+        fork_side(c, 0);
+        {
+            OnStream os(c, side);
+            means(c->redo);
+        }
+        cudaGraph_t body = add_while(st, h, cudaGraphCondTypeIf);
+        {
+            BodyCapture bc(c->cap[0], body, &c->stats);
+            OnStream os(c, bc.s);
+            const long long n0 = c->stats.launches;
+            const cudaGraphConditionalHandle hs = new_handle(&c->stats, bc.s), hp = new_handle(&c->stats, bc.s);
+            LAUNCH(&c->stats, VVM_K_CG, bc.s, k_redo_begin<<<1, 1, 0, bc.s>>>(c->pcg64->ctl, hs));
+            CKL();
+            long long inner = record_spectral_loop<T>(c, c->cap[1], hs, maxit);
+            launch_cal_u<T>(c);
+            CK(cudaMemsetAsync(c->kmax, 0, 2 * sizeof(unsigned), bc.s));
+            launch_rkm<T>(c);
+            w.solve_more = nullptr;
+            w.redo = nullptr;
+            launch_gs_sweep<T>(c, w, hp);
+            inner += GSPasses<T>(c, w, true).record(bc.s, c->cap[1], hp);
+            means(nullptr);
+            const int outer = (int)(c->stats.launches - n0 - inner) + 1;
+            LAUNCH(&c->stats, VVM_K_CG, bc.s, k_redo_end<<<1, 1, 0, bc.s>>>(c->d_exec, outer));
+            CKL();
+            bc.end();
+            *in_loops += c->stats.launches - n0;
+        }
+    } catch (...) {
+        c->stream = st;
+        join_side(c, 2);
+        throw;
+    }
+    join_side(c, 2);
+}
+
 template <typename T>
 int run_step(vvm_gpu_ctx* c, long long* recorded_in_loops = nullptr) {
     c->step++;                                                 // Iteration.cpp:246
@@ -2996,6 +3124,11 @@ int run_step(vvm_gpu_ctx* c, long long* recorded_in_loops = nullptr) {
         ~InStep() { f = false; }
     } in_step{c->in_step = true};
     const bool sf = (c->desc.flags & VVM_FLAG_STREAMFUNCTION) != 0;
+    if (recorded_in_loops && c->branches && c->spectral && !sf && c->tune_gs_tr != kGSSchedCluster) {
+        run_step_direct<T>(c, recorded_in_loops);
+        c->cur = 1 - c->cur;
+        return VVM_GPU_OK;
+    }
     // The step's kernels form two chains (in a captured step, two branches of
     // the graph; the results are those of the reference's order, since
     // neither chain reads what the other writes before they meet):
@@ -3056,14 +3189,21 @@ int run_step(vvm_gpu_ctx* c, long long* recorded_in_loops = nullptr) {
     return rc;
 }
 
-// The step as one CUDA graph: every kernel of run_step, with the cal_w
-// iterations as device-controlled WHILE nodes (no host round trip). Graphs
-// are keyed by the time-level buffer and the parity of the step they run
-// (the AB2 slots alternate with it) and captured on first use.
+// Steps of one launch where a call has as many left: a graph starts a few us
+// after the one before it ends. An even number, so that the graph ends on the
+// buffers and the parity it began with; us a step with 1 / 2 / 4 / 8: 128 x 64
+// 53.8 / 52.6 / 50.6 / 50.6, 2048 x 256 141 / 139 / 139 / 138. The first call's
+// capture takes 1.1 ms with 1 (two graphs) or 2, 1.8 with 4, 3.6 with 8.
+constexpr int kGraphSteps = 2;
+
+// The step as one CUDA graph (many: kGraphSteps of them): every kernel of
+// run_step, with the loops as device-controlled WHILE nodes (no host round
+// trip). Graphs are keyed by the time-level buffer and the parity of the step
+// they run (the AB2 slots alternate with it) and captured on first use.
 template <typename T>
-cudaGraphExec_t step_graph(vvm_gpu_ctx* c) {
+cudaGraphExec_t step_graph(vvm_gpu_ctx* c, bool many) {
     const int b = c->cur, par = (c->step + 1) & 1;
-    if (c->gexec[b][par]) return c->gexec[b][par];
+    if (c->gexec[many][b][par]) return c->gexec[many][b][par];
     ensure_poisson(c);
     if (c->desc.solver == VVM_SOLVER_LEARNED) ensure_learned(c);   // allocations stay outside the capture
     const int step0 = c->step, cur0 = c->cur, ns0 = c->nsolves;
@@ -3074,7 +3214,11 @@ cudaGraphExec_t step_graph(vvm_gpu_ctx* c) {
     long long in_loops = 0;
     CK(cudaStreamBeginCapture(c->stream, cudaStreamCaptureModeRelaxed));
     try {
-        run_step<T>(c, &in_loops);
+        for (int s = 0; s < (many ? kGraphSteps : 1); s++) {
+            long long in = 0;
+            run_step<T>(c, &in);
+            in_loops += in;
+        }
     } catch (...) {
         cudaStreamEndCapture(c->stream, &g);
         if (g) cudaGraphDestroy(g);
@@ -3089,13 +3233,13 @@ cudaGraphExec_t step_graph(vvm_gpu_ctx* c) {
     c->step = step0;
     c->cur = cur0;
     c->nsolves = ns0;
-    c->gstatic[b][par] = c->stats.launches - l0 - in_loops;
+    c->gstatic[many][b][par] = c->stats.launches - l0 - in_loops;
     c->stats.launches = l0;
     cudaGraphExec_t ex = nullptr;
     cudaError_t e = cudaGraphInstantiate(&ex, g, 0);
     cudaGraphDestroy(g);
     if (e != cudaSuccess) throw CudaError{std::string("cudaGraphInstantiate: ") + cudaGetErrorString(e)};
-    c->gexec[b][par] = ex;
+    c->gexec[many][b][par] = ex;
     return ex;
 }
 
@@ -3121,14 +3265,22 @@ void sync_graph_solve(vvm_gpu_ctx* c) {
     }
 }
 
-template <typename T>
-int step_once(vvm_gpu_ctx* c) {
+// True when the case's next step may run from a captured graph (then so may
+// the ones after it).
+bool graph_ready(vvm_gpu_ctx* c) {
     const bool forcing_now = c->has_forcing_th && ((c->step + 1) * c->desc.dt <= c->desc.addforcingtime);
     const bool warm = c->desc.warm_start != 0;
-    const bool use_graph = !c->graphs_off && !c->stats.on && c->step >= 0 && !forcing_now &&
-                           c->poisson_ready && (!warm || c->nsolves >= 2) && !c->learned_collect &&
-                           !(c->desc.flags & VVM_FLAG_STREAMFUNCTION);
-    if (!use_graph) {
+    return !c->graphs_off && !c->stats.on && c->step >= 0 && !forcing_now && c->poisson_ready &&
+           (!warm || c->nsolves >= 2) && !c->learned_collect && !(c->desc.flags & VVM_FLAG_STREAMFUNCTION);
+}
+
+// Steps once, or, where `left` allows it, kGraphSteps times; returns the steps
+// taken in *taken.
+template <typename T>
+int step_some(vvm_gpu_ctx* c, int left, int* taken) {
+    *taken = 1;
+    if (!graph_ready(c)) {
+        const bool forcing_now = c->has_forcing_th && ((c->step + 1) * c->desc.dt <= c->desc.addforcingtime);
         c->last_graph = false;
         // TimeMarching makes the step's forcing field before AddForcing
         // (src/Iteration.cpp:276-283); nothing before AddForcing reads it
@@ -3138,16 +3290,24 @@ int step_once(vvm_gpu_ctx* c) {
         c->fut_is_now = true;
         return rc;
     }
-    cudaGraphExec_t ex = step_graph<T>(c);
+    const bool many = left >= kGraphSteps;
+    if (many) *taken = kGraphSteps;
+    cudaGraphExec_t ex = step_graph<T>(c, many);
     const int b = c->cur, par = (c->step + 1) & 1;
     CK(cudaGraphLaunch(ex, c->stream));
-    c->stats.launches += c->gstatic[b][par];
-    c->step++;
-    c->cur = 1 - c->cur;
-    c->nsolves++;
+    c->stats.launches += c->gstatic[many][b][par];
+    c->step += *taken;
+    if (!many) c->cur = 1 - c->cur;
+    c->nsolves += *taken;
     c->last_graph = true;
     c->fut_is_now = true;
     return VVM_GPU_OK;
+}
+
+template <typename T>
+int step_once(vvm_gpu_ctx* c) {
+    int taken;
+    return step_some<T>(c, 1, &taken);
 }
 
 // ---------------------------------------------------------------- snapshots
@@ -3194,15 +3354,6 @@ struct Snapshot {
         for (void* q : copies) cudaFree(q);
     }
 };
-
-// True when the case's next step may run from a captured graph (the test of
-// step_once).
-bool graph_ready(vvm_gpu_ctx* c) {
-    const bool forcing_now = c->has_forcing_th && ((c->step + 1) * c->desc.dt <= c->desc.addforcingtime);
-    const bool warm = c->desc.warm_start != 0;
-    return !c->graphs_off && !c->stats.on && c->step >= 0 && !forcing_now && c->poisson_ready &&
-           (!warm || c->nsolves >= 2) && !c->learned_collect && !(c->desc.flags & VVM_FLAG_STREAMFUNCTION);
-}
 
 }  // namespace
 
@@ -4421,6 +4572,7 @@ int vvm_gpu_create(const vvm_gpu_desc* desc, int device, vvm_gpu_ctx** out) {
         CK(cudaFuncSetAttribute(k_padv<double, F_TH | F_QV | F_QC | F_QR, 4>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                 (int)sizeof(PAdvShared<double, 4>)));
         c->nvp = c->ar.alloc<double>(6);
+        c->redo = c->ar.alloc<int>(1);
         c->staging = c->ar.alloc<double>((size_t)c->d.nx * c->d.nz * staging_slots(c->d));
         CK(cudaMallocHost(&c->err_host, sizeof(int)));
         c->wctl = c->ar.alloc<CGCtl>(1);
@@ -4576,10 +4728,10 @@ ROUTINE(vvm_gpu_pubartop, { DISPATCH(ctx, launch_pubartop)(ctx); return VVM_GPU_
 ROUTINE(vvm_gpu_cal_w, { ctx->last_graph = false; return DISPATCH(ctx, launch_cal_w)(ctx, nullptr, nullptr); })
 ROUTINE(vvm_gpu_cal_u, { DISPATCH(ctx, launch_cal_u)(ctx); return VVM_GPU_OK; })
 ROUTINE(vvm_gpu_kessler, { DISPATCH(ctx, launch_kessler)(ctx); return VVM_GPU_OK; })
-ROUTINE(vvm_gpu_update_mean, { DISPATCH(ctx, launch_update_mean)(ctx, false); return VVM_GPU_OK; })
+ROUTINE(vvm_gpu_update_mean, { DISPATCH(ctx, launch_update_mean)(ctx, false, nullptr); return VVM_GPU_OK; })
 ROUTINE(vvm_gpu_turbulence, { DISPATCH(ctx, launch_turbulence)(ctx, false, nullptr); return VVM_GPU_OK; })
 ROUTINE(vvm_gpu_nudge, {
-    DISPATCH(ctx, launch_nudge)(ctx, true, ctx->desc.moisture_nudge_time != 0.0);
+    DISPATCH(ctx, launch_nudge)(ctx, true, ctx->desc.moisture_nudge_time != 0.0, nullptr);
     return VVM_GPU_OK;
 })
 ROUTINE(vvm_gpu_calpsiuw, {
@@ -4597,7 +4749,7 @@ int vvm_gpu_download_psi(vvm_gpu_ctx* ctx, double* psi) {
 }
 
 ROUTINE(vvm_gpu_next_step, {
-    DISPATCH(ctx, launch_update_mean)(ctx, true);
+    DISPATCH(ctx, launch_update_mean)(ctx, true, nullptr);
     ctx->cur = 1 - ctx->cur;
     ctx->fut_is_now = true;
     return VVM_GPU_OK;
@@ -4610,8 +4762,8 @@ int vvm_gpu_step(vvm_gpu_ctx* ctx, int nsteps) {
         if (ctx->desc.flags & VVM_FLAG_STREAMFUNCTION)
             if (int rc = need_uniform(ctx)) return rc;
         int worst = VVM_GPU_OK;
-        for (int s = 0; s < nsteps; s++) {
-            int rc = DISPATCH(ctx, step_once)(ctx);
+        for (int s = 0, taken; s < nsteps; s += taken) {
+            int rc = DISPATCH(ctx, step_some)(ctx, nsteps - s, &taken);
             if (rc != VVM_GPU_OK) worst = rc;
         }
         if (worst == VVM_GPU_ENOCONV) fail(ctx, worst, "cal_w: Poisson solve did not reach its tolerance");

@@ -190,3 +190,40 @@ def test_spectral_modes_at_every_height(gpu, nk):
     g.close()
     assert it == 0 and rel <= 1e-12
     assert rel_l2(m.apply_A(W), b) <= 1e-12
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("precision", [0, 1])
+@pytest.mark.parametrize("tol,passes", [(1e-10, False), (1e-14, False), (1e-10, True), (1e-14, True)])
+def test_captured_steps_do_their_end_over(gpu, tol, passes, precision):
+    """Steps whose check fails (tol 1e-14), whose sweep needs the repeated passes
+    or both: graphs of one step and of several, whose end does over what the
+    steps went on with, equal the host's loops bit for bit, with moisture
+    nudging after the diffusion and the counts of launches alike."""
+    from vvm_b200.initial_state import warm_bubble
+    if passes:
+        st = warm_bubble(128, 24, 40.0, 40.0, 30.0 if precision else 10.0, amp=0.2, radius=400.0, zc=400.0)
+    else:
+        st = warm_bubble(128, 48)
+    st.grid.moisture_nudge_time = 600.0
+    runs, iters, launched = [], [], []
+    for profile, calls in ((True, [11]), (False, [11]), (False, [1] * 11), (False, [3, 8])):
+        g = gpu.VVMGpu(st.grid, precision=precision, solver=gpu.VVM_SOLVER_SPECTRAL, poisson_tol=tol)
+        g.upload(st)
+        if profile:
+            g.profile(True)
+        its = 0
+        for n in calls:
+            g.step(n)
+            its += g.last_solve()[0]
+        out = g.download()
+        launched.append(g.launch_count)
+        runs.append((out, g.last_solve()))
+        iters.append(its)
+        g.close()
+    assert (iters[2] > 0) == (tol == 1e-14)
+    for out, last in runs[1:]:
+        assert last == runs[0][1]
+        for f in PROG:
+            assert np.isfinite(out.fields[f]).all() and np.array_equal(out.fields[f], runs[0][0].fields[f]), f
+    assert launched[1] == launched[2] == launched[3]
