@@ -535,29 +535,48 @@ template <typename P>
 __global__ void k_cg_check(VecArgs<P> v, const P* f, P* x, P* r, double* partial, CGScalars* sc, CGCtl* ctl,
                            unsigned* arrive, cudaGraphConditionalHandle h, double tol2, int maxit) { k_cg_check_body<P>(v, f, x, r, partial, sc, ctl, arrive, h, tol2, maxit); }
 
-// Rows a thread of k_spec_check takes: a quarter of the blocks to count in
-// (2048 x 256: 10 us with one row).
-constexpr int kCheckRows = 4;
+// Rows a thread of k_spec_check takes, loaded at once, with as many blocks less
+// to count in; us a launch (events) with 1 / 2 / 4 / 8: 2048 x 256 17 / 13 / 12.6
+// / 10.6, 8192 x 256 29 / 25 / 23 / 19, 128 x 64 8.6 with each.
+constexpr int kCheckRows = 8;
 
 // The check of a direct solve x = S^{-1} f: as k_cg_check, with ||b||^2 (b = -rw f)
 // summed in the same pass (nothing before it needs it; x = 0 where b = 0
-// already). partial: two values a block.
+// already). r: the residual, where it is wanted. partial: two values a block.
 __device__ __forceinline__ void k_spec_check_body(const VecArgs<double>& v, const double* f, const double* x, double* r, double* partial,
                                                   CGScalars* sc, CGCtl* ctl, unsigned* arrive, cudaGraphConditionalHandle h,
                                                   double tol2, int maxit) {
     __shared__ double sh[64];
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    const int k0 = (blockIdx.y * blockDim.y + threadIdx.y) * kCheckRows;
     double s[2] = {0, 0};
-#pragma unroll 4
-    for (int q = 0; q < kCheckRows; q++) {
-        const int kk = (blockIdx.y * kCheckRows + q) * blockDim.y + threadIdx.y;
-        if (i >= v.nx || kk >= v.NK) break;
-        const size_t id = (size_t)kk * v.pitch + i;
-        const double fv = f[id], rv = fv - s_apply(x, v.pitch, v.nx, v.NK, v.z, v.cx, kk, i);
-        r[id] = rv;
-        const double w = v.rhow_k[kk], wr = w * rv, wb = w * fv;
-        s[0] += wr * wr;
-        s[1] += wb * wb;
+    if (i < v.nx && k0 < v.NK) {
+        const int il = (i == 0) ? v.nx - 1 : i - 1, ir = (i == v.nx - 1) ? 0 : i + 1;
+        double xc[kCheckRows + 2], xs[kCheckRows], fv[kCheckRows];   // rows k0-1 .. k0+kCheckRows
+#pragma unroll
+        for (int q = 0; q < kCheckRows + 2; q++) {
+            const int kk = k0 - 1 + q;
+            xc[q] = (kk >= 0 && kk < v.NK) ? x[(size_t)kk * v.pitch + i] : 0.0;
+            if (q < kCheckRows) {
+                const size_t row = (size_t)min(k0 + q, v.NK - 1) * v.pitch;
+                xs[q] = x[row + il] + x[row + ir];
+                fv[q] = f[row + i];
+            }
+        }
+#pragma unroll
+        for (int q = 0; q < kCheckRows; q++) {
+            const int kk = k0 + q;
+            if (kk >= v.NK) break;
+            // f - S x as s_apply forms it (x = 0 beyond the ends)
+            const double c = v.cx[kk], ru = v.z.ru[kk], rd = v.z.rd[kk], w = v.rhow_k[kk];
+            double y = (2.0 * c + ru + rd) * xc[q + 1] - c * xs[q];
+            y -= ru * xc[q + 2];
+            y -= rd * xc[q];
+            const double rv = fv[q] - y, wr = w * rv, wb = w * fv[q];
+            if (r) r[(size_t)kk * v.pitch + i] = rv;
+            s[0] += wr * wr;
+            s[1] += wb * wb;
+        }
     }
     block_sum(s, sh);
     const unsigned nb = gridDim.x * gridDim.y;

@@ -944,52 +944,70 @@ __device__ __forceinline__ void block_max_bits(unsigned v, unsigned* sh, unsigne
 __device__ __forceinline__ unsigned bits_up(double x) { return __float_as_uint(__double2float_ru(x)); }
 __device__ __forceinline__ unsigned bits_up(float x) { return __float_as_uint(x); }
 
-template <typename T>
+// R rows a thread: the rows between are loaded once, not three times, and all
+// of them at once, with a barrier and an atomic for R times as many cells.
+// Ri is compared as its numerator against its denominator (th > 0), so that
+// the cells of Ri >= 1/4, most of them, divide and take roots not at all.
+template <typename T, int R>
 __device__ __forceinline__ void k_rkm_rkh_body(const RKArgs<T>& a) {
     const Dims& d = a.d;
     const int i = 1 + blockIdx.x * blockDim.x + threadIdx.x;
-    const int k = 1 + blockIdx.y * blockDim.y + threadIdx.y;
+    const int k0 = 1 + (blockIdx.y * blockDim.y + threadIdx.y) * R;
     __shared__ unsigned sh[2][32];
-    T km = T(0), kh = T(0);
-    if (i <= d.nx - 2 && k <= d.nz - 2) {
-        const T* u = a.u;
-        const T* w = a.w;
-        T Rzeta = T(0.5) * ((w[d.at(i + 1, k + 1)] + w[d.at(i + 1, k)]) - (w[d.at(i - 1, k + 1)] + w[d.at(i - 1, k)])) * T(a.c.r2dx) +
-                  T(0.5) * ((u[d.at(i + 1, k + 1)] + u[d.at(i, k + 1)]) - (u[d.at(i + 1, k - 1)] + u[d.at(i, k - 1)])) * T(a.p.r2dzcc[k]);
-        T rot = (u[d.at(i + 1, k)] - u[d.at(i, k)]) * T(a.c.rdx) + (w[d.at(i, k + 1)] - w[d.at(i, k)]) * T(a.p.rdzc[k]);
-        T Rotat = rot * rot;
-        T th0 = a.thp[d.at(i, k)];
-        T dth = a.thp[d.at(i, k + 1)] - a.thp[d.at(i, k - 1)];
-        if constexpr (kPert<T>) {       // perturbation storage: add the profile parts
-            th0 += T(a.p.ref[0][k]);
-            dth += T(a.p.g0[0][k]);
+    unsigned kmx = 0u, khx = 0u;   // bits, above all others' where a value is NaN
+    if (i <= d.nx - 2 && k0 <= d.nz - 2) {
+        T u[R + 2][2], w[R + 1][3], th[R + 2];   // rows k0-1 .. k0+R; w from k0
+#pragma unroll
+        for (int q = 0; q < R + 2; q++) {
+            const size_t e = d.at(i, min(k0 - 1 + q, d.nz - 1));
+            u[q][0] = a.u[e];
+            u[q][1] = a.u[e + 1];
+            th[q] = a.thp[e];
+            if (q)
+#pragma unroll
+                for (int x = 0; x < 3; x++) w[q - 1][x] = a.w[e + x - 1];
         }
-        T def2 = Rzeta * Rzeta + T(2.) * Rotat;
-        T Ri = (T(a.c.gravity) / th0 * dth * T(a.p.r2dzcc[k])) / def2;
-        T lam = T(a.p.lambda2[k]);
-        if (Ri < T(0)) {
-            km = lam * sqrt(def2) * sqrt(T(1.) - T(16.) * Ri);
-            kh = lam * sqrt(def2) * T(1.4) * sqrt(T(1.) - T(40.) * Ri);
-        } else if (T(0) < Ri && Ri < T(0.25)) {
-            km = lam * sqrt(def2) * pow(T(1.) - T(4.) * Ri, T(4));
-            kh = lam * sqrt(def2) * T(1.4) * (T(1.) - T(1.2) * Ri) * pow(T(1.) - T(4.) * Ri, T(4));
-        } else {
-            km = T(0.);
-            kh = T(0.);
+#pragma unroll
+        for (int q = 0; q < R; q++) {
+            const int k = k0 + q;
+            if (k > d.nz - 2) break;
+            T Rzeta = T(0.5) * ((w[q + 1][2] + w[q][2]) - (w[q + 1][0] + w[q][0])) * T(a.c.r2dx) +
+                      T(0.5) * ((u[q + 2][1] + u[q + 2][0]) - (u[q][1] + u[q][0])) * T(a.p.r2dzcc[k]);
+            T rot = (u[q + 1][1] - u[q + 1][0]) * T(a.c.rdx) + (w[q + 1][1] - w[q][1]) * T(a.p.rdzc[k]);
+            T th0 = th[q + 1];
+            T dth = th[q + 2] - th[q];
+            if constexpr (kPert<T>) {       // perturbation storage: add the profile parts
+                th0 += T(a.p.ref[0][k]);
+                dth += T(a.p.g0[0][k]);
+            }
+            const T def2 = Rzeta * Rzeta + T(2.) * (rot * rot);
+            const T num = T(a.c.gravity) * dth * T(a.p.r2dzcc[k]), den = th0 * def2;   // Ri = num / den
+            T km = T(0.), kh = T(0.);
+            if (num < T(0.25) * den && num != T(0)) {
+                const T Ri = num / den, lam = T(a.p.lambda2[k]), ld = lam * sqrt(def2);
+                if (Ri < T(0)) {
+                    km = ld * sqrt(T(1.) - T(16.) * Ri);
+                    kh = ld * T(1.4) * sqrt(T(1.) - T(40.) * Ri);
+                } else {
+                    const T f = T(1.) - T(4.) * Ri, f4 = (f * f) * (f * f);
+                    km = ld * f4;
+                    kh = ld * T(1.4) * (T(1.) - T(1.2) * Ri) * f4;
+                }
+            }
+            const T kmax = T(a.p.kmax[k]);
+            km = smin(smax(km, T(10.)), kmax);
+            kh = smin(smax(kh, T(10.)), kmax);
+            store_center(a.RKM, d, i, k, km);
+            store_center(a.RKH, d, i, k, kh);
+            kmx = max(kmx, bits_up(km));
+            khx = max(khx, bits_up(kh));
         }
-        const T kmax = T(a.p.kmax[k]);
-        km = smax(km, T(10.));
-        kh = smax(kh, T(10.));
-        km = smin(km, kmax);
-        kh = smin(kh, kmax);
-        store_center(a.RKM, d, i, k, km);
-        store_center(a.RKH, d, i, k, kh);
     }
-    block_max_bits(bits_up(km), sh[0], a.kmax);
-    block_max_bits(bits_up(kh), sh[1], a.kmax + 1);
+    block_max_bits(kmx, sh[0], a.kmax);
+    block_max_bits(khx, sh[1], a.kmax + 1);
 }
-template <typename T>
-__global__ void k_rkm_rkh(RKArgs<T> a) { k_rkm_rkh_body<T>(a); }
+template <typename T, int R>
+__global__ void __launch_bounds__(256) k_rkm_rkh(RKArgs<T> a) { k_rkm_rkh_body<T, R>(a); }
 
 // ---------------------------------------------------------------------------
 // In-place Gauss-Seidel diffusion (Turbulence::Mparam / Hparam,

@@ -1574,7 +1574,7 @@ struct PCG {
         q = ar.alloc<P>((size_t)NK * pitch);
         dim3 g = grid();
         npart = g.x * g.y;
-        partial = ar.alloc<double>(npart + 2 * g.x);   // k_spec_check: two values a block of kCheckRows x 4 rows
+        partial = ar.alloc<double>(npart + 4 * g.x);   // k_spec_check: two values a block of 32 x 8 kCheckRows cells
         rhow_k = ar.alloc<double>(NK);
         upload_now(rhow_k, rw.data(), NK * sizeof(double));
         sc = ar.alloc<CGScalars>(1);
@@ -2289,7 +2289,15 @@ template <typename T>
 void launch_rkm(vvm_gpu_ctx* c) {
     Fields<T>& F = fields<T>(c);
     RKArgs<T> r{c->d, c->c, c->profiles(), F.u, F.w, c->in_step ? F.pre[1] : F.th[1 - c->cur], F.RKM, F.RKH, c->kmax};
-    klaunch<k_rkm_rkh_body<T>, 256>(&c->stats, VVM_K_RKM, c->stream, k_rkm_rkh<T>, c->grid_interior(1), c->blk(), 0, r);
+    // four rows a thread where that leaves every SM two blocks (us a launch with 1
+    // / 2 / 4 rows, FP64: 2048 x 256 16 / 17 / 15, 8192 x 256 40 / 46 / 35)
+    dim3 g = c->grid_interior(1);
+    if (g.x * g.y >= 4 * 2 * 148) {
+        g.y = cdiv((int)g.y, 4);
+        klaunch<k_rkm_rkh_body<T, 4>, 256>(&c->stats, VVM_K_RKM, c->stream, k_rkm_rkh<T, 4>, g, c->blk(), 0, r);
+    } else {
+        klaunch<k_rkm_rkh_body<T, 1>, 256>(&c->stats, VVM_K_RKM, c->stream, k_rkm_rkh<T, 1>, g, c->blk(), 0, r);
+    }
 }
 
 template <typename T>
@@ -2754,11 +2762,12 @@ void launch_w_from_W(vvm_gpu_ctx* c, cudaStream_t st) {
 }
 
 // The check of a direct solve's residual, which sets the condition h (0: none).
-void launch_spectral_check(vvm_gpu_ctx* c, cudaGraphConditionalHandle h, int maxit) {
+// r: where the residual goes (null: nowhere).
+void launch_spectral_check(vvm_gpu_ctx* c, double* r, cudaGraphConditionalHandle h, int maxit) {
     PCG<double>& P = *c->pcg64;
-    const dim3 B = P.block(), G(P.grid().x, cdiv(P.NK, (int)B.y * kCheckRows));
+    const dim3 B(32, 8), G(cdiv(P.NX, 32), cdiv(P.NK, 8 * kCheckRows));
     klaunch<k_spec_check_body, 256>(&c->stats, VVM_K_CG, c->stream, k_spec_check, G, B, 0, P.vargs(), (const double*)c->Wf,
-                                    (const double*)c->W, P.r, P.partial, P.sc, P.ctl, P.arrive, h,
+                                    (const double*)c->W, r, P.partial, P.sc, P.ctl, P.arrive, h,
                                     c->desc.poisson_tol * c->desc.poisson_tol, maxit);
 }
 
@@ -2787,7 +2796,7 @@ template <typename T>
 int run_spectral(vvm_gpu_ctx* c, cudaEvent_t before_w, int maxit) {
     PCG<double>& P = *c->pcg64;
     P.sp.apply_fields(spec_fields<T>(c), c->stream, before_w);
-    launch_spectral_check(c, 0, maxit);
+    launch_spectral_check(c, nullptr, 0, maxit);
     CGCtl ctl;
     CK(cudaMemcpyAsync(c->sc_host, &P.sc->bb, sizeof(double), cudaMemcpyDeviceToHost, c->stream));
     CK(cudaMemcpyAsync(&ctl, P.ctl, sizeof(ctl), cudaMemcpyDeviceToHost, c->stream));
@@ -2902,7 +2911,7 @@ int launch_cal_w(vvm_gpu_ctx* c, long long* recorded_in_loops = nullptr, cudaEve
         if (recorded_in_loops) {
             const cudaGraphConditionalHandle h = new_handle(&c->stats, c->stream);
             c->pcg64->sp.apply_fields(spec_fields<T>(c), c->stream, before_w);
-            launch_spectral_check(c, h, maxit);
+            launch_spectral_check(c, c->pcg64->r, h, maxit);
             *recorded_in_loops = record_spectral_loop<T>(c, c->cap[0], h, maxit);
         } else {
             rc = run_spectral<T>(c, before_w, maxit);
@@ -3068,7 +3077,7 @@ void run_step_direct(vvm_gpu_ctx* c, long long* in_loops) {
         {
             OnStream os(c, side);
             CK(cudaStreamWaitEvent(side, c->fork_ev[4], 0));
-            launch_spectral_check(c, 0, maxit);
+            launch_spectral_check(c, nullptr, 0, maxit);
             CK(cudaEventRecord(c->fork_ev[5], side));
         }
         launch_cal_u<T>(c);                                    // cal_u
@@ -3092,6 +3101,9 @@ void run_step_direct(vvm_gpu_ctx* c, long long* in_loops) {
             const long long n0 = c->stats.launches;
             const cudaGraphConditionalHandle hs = new_handle(&c->stats, bc.s), hp = new_handle(&c->stats, bc.s);
             LAUNCH(&c->stats, VVM_K_CG, bc.s, k_redo_begin<<<1, 1, 0, bc.s>>>(c->pcg64->ctl, hs));
+            CKL();
+            PCG<double>& P = *c->pcg64;
+            LAUNCH(&c->stats, VVM_K_CG, bc.s, k_cg_residual<double><<<P.grid(), P.block(), 0, bc.s>>>(P.vargs(), c->Wf, c->W, P.r, P.partial));
             CKL();
             long long inner = record_spectral_loop<T>(c, c->cap[1], hs, maxit);
             launch_cal_u<T>(c);
