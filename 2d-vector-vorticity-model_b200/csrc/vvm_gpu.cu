@@ -1955,9 +1955,13 @@ void launch_pzeta(vvm_gpu_ctx* c) {
 // Rows a thread of k_padv takes: four share their z fluxes and amortise the
 // reduction, one finishes sooner where the grid is small (us a launch with 1 /
 // 4 rows, FP64: 128 x 64 10.6 / 16.8; 8192 x 256 98.8 / 89.0, FP32 82.3 /
-// 66.0; the step of 512 x 128 84.1 / 82.0, of 2048 x 256 199.5 / 195.5).
+// 66.0; the step of 128 x 64 52.7 / 55.0, of 512 x 128 84.1 / 82.0, of 2048 x 256
+// 199.5 / 195.5). The line lies low, at 16 blocks with four: the scalars' chain
+// is the shorter one of a step, and a group of cases, which takes the rows a
+// case alone takes (its sums' order follows them), has the blocks of all (48 of
+// 256 x 64, 18 blocks each: 303 / 280 us a step).
 inline int padv_rows_a_thread(const Dims& d) {
-    return cdiv(d.nx - 2, kTileBX) * cdiv(d.nz - 2, tile_rows(4)) >= 64 ? 4 : 1;
+    return cdiv(d.nx - 2, kTileBX) * cdiv(d.nz - 2, tile_rows(4)) >= 16 ? 4 : 1;
 }
 
 // MASK: the fields advected. Surface rain and sedimentation go with qr.
@@ -2065,10 +2069,10 @@ void launch_kessler(vvm_gpu_ctx* c) {
     KesslerArgs<T> a{c->d, c->c, c->profiles(), F.th[fut], F.qv[fut], F.qc[fut], F.qr[fut],
                      {F.th[fut], F.qv[fut], F.qc[fut], F.qr[fut]}, 0,
                      c->partial};
-    // two rows a thread where that still gives every SM a block (us a launch with
-    // 1 / 2 / 4 rows, FP64: 8192 x 256 56 / 50 / 50, 2048 x 256 20 / 19 / 23,
-    // 128 x 64 10.2 / 13.1 / 18.8)
-    a.rows = cdiv(c->d.nx - 2, 32) * cdiv(c->d.nz - 2, 2 * kKesslerWarps) >= 148 ? 2 : 1;
+    // two rows a thread but for the smallest grids (us a launch with 1 / 2 / 4
+    // rows, FP64: 8192 x 256 56 / 50 / 50, 2048 x 256 20 / 19 / 23, 128 x 64 10.2 /
+    // 13.1 / 18.8; the step of 512 x 128, 128 blocks with two, 63.7 / 61.3)
+    a.rows = cdiv(c->d.nx - 2, 32) * cdiv(c->d.nz - 2, 2 * kKesslerWarps) >= 32 ? 2 : 1;
     if (c->in_step) {
         for (int f = 0; f < 4; f++) a.out[f] = F.pre[1 + f];
         a.halo = 1;
@@ -2289,10 +2293,11 @@ template <typename T>
 void launch_rkm(vvm_gpu_ctx* c) {
     Fields<T>& F = fields<T>(c);
     RKArgs<T> r{c->d, c->c, c->profiles(), F.u, F.w, c->in_step ? F.pre[1] : F.th[1 - c->cur], F.RKM, F.RKH, c->kmax};
-    // four rows a thread where that leaves every SM two blocks (us a launch with 1
+    // four rows a thread where that leaves every SM two blocks, as a grouped
+    // launch does (us a launch with 1
     // / 2 / 4 rows, FP64: 2048 x 256 16 / 17 / 15, 8192 x 256 40 / 46 / 35)
     dim3 g = c->grid_interior(1);
-    if (g.x * g.y >= 4 * 2 * 148) {
+    if (c->stats.rec || g.x * g.y >= 4 * 2 * 148) {
         g.y = cdiv((int)g.y, 4);
         klaunch<k_rkm_rkh_body<T, 4>, 256>(&c->stats, VVM_K_RKM, c->stream, k_rkm_rkh<T, 4>, g, c->blk(), 0, r);
     } else {
