@@ -599,7 +599,7 @@ __device__ __forceinline__ void k_spec_check_body(const VecArgs<double>& v, cons
         sc->bb = bb;
         ctl->it = 0;
         ctl->total = 0;
-        ctl->relres = (bb > 0.0) ? sqrt(rr / bb) : 0.0;
+        ctl->relres = (bb == 0.0) ? 0.0 : sqrt(rr / bb);   // NaN where b holds one
         const bool more = (bb > 0.0) && (rr > tol2 * bb) && (maxit > 0) && isfinite(rr);
         ctl->more = more ? 1 : 0;
         if (h) cudaGraphSetConditional(h, more ? 1u : 0u);

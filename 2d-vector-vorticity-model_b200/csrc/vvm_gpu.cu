@@ -798,7 +798,7 @@ struct Spectral : ModeFactors<P> {
         a.twi = this->upload(ar, twi);
         out = ar.alloc<P>((size_t)NK * pitch);
         smem = 3 * (size_t)NX * sizeof(P);   // the row pair (re, im) and the twiddles
-        threads = std::max(32, std::min(NX / 2, 512));
+        threads = std::max(32, std::min(NX / 2, 1024));
         // per-kernel attribute: the largest row any context may have (NX = 8192)
         const int smax = 3 * 8192 * (int)sizeof(P);
         CK(cudaFuncSetAttribute(k_spec_forward<P>, cudaFuncAttributeMaxDynamicSharedMemorySize, smax));
@@ -2447,7 +2447,8 @@ void launch_update_mean(vvm_gpu_ctx* c, bool rotate, const int* skip = nullptr) 
 void apply_tuning(vvm_gpu_ctx* c) {
     if (c->pcg64 && c->pcg64->spectral) {
         const int half = std::max(32, (c->d.nx - 2) / 2);
-        const int def = std::min(half, 512);
+        // (us both transforms of a step with 512 / 1024: 8192 x 256 75 / 62, 2048 x 256 30 / 28)
+        const int def = std::min(half, 1024);
         c->pcg64->sp.threads = c->tune_fft > 0 ? std::max(32, std::min(c->tune_fft, std::min(half, 1024))) : def;
     }
 }
@@ -2709,14 +2710,6 @@ int solve_w(vvm_gpu_ctx* c, double bb, double tol, bool warm) {
         c->last_relres = rel;
         return (rel <= tol) ? VVM_GPU_OK : VVM_GPU_ENOCONV;
     }
-    if (c->spectral) {   // direct solve W = S^{-1} f, checked; CG from there if the check fails
-        double rel = 0;
-        c->pcg64->sp.apply_to(c->Wf, c->W, c->stream);
-        int it = c->pcg64->solve(c->Wf, c->W, true, bb, tol, maxit, c->stream, &rel);
-        c->last_iters = it;
-        c->last_relres = rel;
-        return (rel <= tol) ? VVM_GPU_OK : VVM_GPU_ENOCONV;
-    }
     if (!c->mixed) {
         double rel = 0;
         int it = c->pcg64->solve(c->Wf, c->W, warm, bb, tol, maxit, c->stream, &rel);
@@ -2768,12 +2761,12 @@ void launch_w_from_W(vvm_gpu_ctx* c, cudaStream_t st) {
 
 // The check of a direct solve's residual, which sets the condition h (0: none).
 // r: where the residual goes (null: nowhere).
-void launch_spectral_check(vvm_gpu_ctx* c, double* r, cudaGraphConditionalHandle h, int maxit) {
+void launch_spectral_check(vvm_gpu_ctx* c, double* r, cudaGraphConditionalHandle h, double tol, int maxit) {
     PCG<double>& P = *c->pcg64;
     const dim3 B(32, 8), G(cdiv(P.NX, 32), cdiv(P.NK, 8 * kCheckRows));
     klaunch<k_spec_check_body, 256>(&c->stats, VVM_K_CG, c->stream, k_spec_check, G, B, 0, P.vargs(), (const double*)c->Wf,
                                     (const double*)c->W, r, P.partial, P.sc, P.ctl, P.arrive, h,
-                                    c->desc.poisson_tol * c->desc.poisson_tol, maxit);
+                                    tol * tol, maxit);
 }
 
 // The loop that follows a check that fails (condition h, body captured on
@@ -2796,23 +2789,28 @@ long long record_spectral_loop(vvm_gpu_ctx* c, cudaStream_t cap, cudaGraphCondit
 
 int poisson_maxit(const vvm_gpu_ctx* c) { return c->desc.poisson_maxit > 0 ? c->desc.poisson_maxit : 200; }
 
-// ... without capture: the host reads the check's result.
-template <typename T>
-int run_spectral(vvm_gpu_ctx* c, cudaEvent_t before_w, int maxit) {
+// The check without capture, after the direct solve of c->Wf into c->W: the
+// host reads its result and goes on with CG if it failed. `use` issues what
+// follows the solution, before the check is known to pass (one wait in all) and
+// again after CG.
+template <typename Use>
+int finish_spectral(vvm_gpu_ctx* c, double tol, Use use) {
     PCG<double>& P = *c->pcg64;
-    P.sp.apply_fields(spec_fields<T>(c), c->stream, before_w);
-    launch_spectral_check(c, nullptr, 0, maxit);
+    const int maxit = poisson_maxit(c);
+    launch_spectral_check(c, nullptr, 0, tol, maxit);
+    c->last_iters = 0;
+    use();
     CGCtl ctl;
     CK(cudaMemcpyAsync(c->sc_host, &P.sc->bb, sizeof(double), cudaMemcpyDeviceToHost, c->stream));
     CK(cudaMemcpyAsync(&ctl, P.ctl, sizeof(ctl), cudaMemcpyDeviceToHost, c->stream));
     CK(cudaStreamSynchronize(c->stream));
-    c->last_iters = 0;
     c->last_relres = ctl.relres;
     if (ctl.more) {
-        c->last_iters = P.solve(c->Wf, c->W, true, *c->sc_host, c->desc.poisson_tol, maxit, c->stream, &c->last_relres);
-        launch_w_from_W<T>(c, c->stream);
+        c->last_iters = P.solve(c->Wf, c->W, true, *c->sc_host, tol, maxit, c->stream, &c->last_relres);
+        use();
+        CK(cudaStreamSynchronize(c->stream));
     }
-    return (c->last_relres <= c->desc.poisson_tol) ? VVM_GPU_OK : VVM_GPU_ENOCONV;
+    return (c->last_relres <= tol) ? VVM_GPU_OK : VVM_GPU_ENOCONV;
 }
 
 // Records the cal_w solve with device-side loop control (graph capture on
@@ -2916,10 +2914,13 @@ int launch_cal_w(vvm_gpu_ctx* c, long long* recorded_in_loops = nullptr, cudaEve
         if (recorded_in_loops) {
             const cudaGraphConditionalHandle h = new_handle(&c->stats, c->stream);
             c->pcg64->sp.apply_fields(spec_fields<T>(c), c->stream, before_w);
-            launch_spectral_check(c, c->pcg64->r, h, maxit);
+            launch_spectral_check(c, c->pcg64->r, h, c->desc.poisson_tol, maxit);
             *recorded_in_loops = record_spectral_loop<T>(c, c->cap[0], h, maxit);
         } else {
-            rc = run_spectral<T>(c, before_w, maxit);
+            c->pcg64->sp.apply_fields(spec_fields<T>(c), c->stream, before_w);
+            rc = finish_spectral(c, c->desc.poisson_tol, [&]() {
+                if (c->last_iters) launch_w_from_W<T>(c, c->stream);   // CG has gone on from the solve's w
+            });
         }
         c->nsolves++;
         return rc;
@@ -3082,7 +3083,7 @@ void run_step_direct(vvm_gpu_ctx* c, long long* in_loops) {
         {
             OnStream os(c, side);
             CK(cudaStreamWaitEvent(side, c->fork_ev[4], 0));
-            launch_spectral_check(c, nullptr, 0, maxit);
+            launch_spectral_check(c, nullptr, 0, c->desc.poisson_tol, maxit);
             CK(cudaEventRecord(c->fork_ev[5], side));
         }
         launch_cal_u<T>(c);                                    // cal_u
@@ -4797,6 +4798,21 @@ int vvm_gpu_poisson_solve_device(vvm_gpu_ctx* ctx, const double* d_b, double* d_
         dim3 B(64, 4), G(cdiv(NX, 64), cdiv(NK, 4));
         LAUNCH(&ctx->stats, VVM_K_POISSON_RHS, ctx->stream, k_rhs_from_b<<<G, B, 0, ctx->stream>>>(NX, NK, ctx->rwres, d_b, ctx->Wf, pitch, ctx->wpartial));
         CKL();
+        auto pack = [&]() {
+            LAUNCH(&ctx->stats, VVM_K_POISSON_RHS, ctx->stream, k_pack_solution<<<G, B, 0, ctx->stream>>>(NX, NK, ctx->W, pitch, d_W));
+            CKL();
+        };
+        auto done = [&](int rc) {
+            if (iters) *iters = ctx->last_iters;
+            if (relres) *relres = ctx->last_relres;
+            if (rc == VVM_GPU_ENOCONV) fail(ctx, rc, "poisson_solve: tolerance not reached");
+            return rc;
+        };
+        ctx->last_graph = false;
+        if (ctx->spectral) {
+            ctx->pcg64->sp.apply_to(ctx->Wf, ctx->W, ctx->stream);
+            return done(finish_spectral(ctx, tol, pack));
+        }
         LAUNCH(&ctx->stats, VVM_K_CG, ctx->stream, k_cg_scalar<<<1, 1024, 0, ctx->stream>>>(ctx->wpartial, ctx->wnpart, ctx->pcg64->sc, CG_SET_BB));
         CKL();
         double bb = read_scalar(ctx, &ctx->pcg64->sc->bb);
@@ -4805,15 +4821,10 @@ int vvm_gpu_poisson_solve_device(vvm_gpu_ctx* ctx, const double* d_b, double* d_
             LAUNCH(&ctx->stats, VVM_K_POISSON_RHS, ctx->stream, k_unpack_solution<<<G, B, 0, ctx->stream>>>(NX, NK, d_W, ctx->W, pitch));
             CKL();
         }
-        int rc = solve_w(ctx, bb, tol, warm);
-        ctx->last_graph = false;
-        LAUNCH(&ctx->stats, VVM_K_POISSON_RHS, ctx->stream, k_pack_solution<<<G, B, 0, ctx->stream>>>(NX, NK, ctx->W, pitch, d_W));
-        CKL();
+        const int rc = solve_w(ctx, bb, tol, warm);
+        pack();
         CK(cudaStreamSynchronize(ctx->stream));
-        if (iters) *iters = ctx->last_iters;
-        if (relres) *relres = ctx->last_relres;
-        if (rc == VVM_GPU_ENOCONV) fail(ctx, rc, "poisson_solve: tolerance not reached");
-        return rc;
+        return done(rc);
     });
 }
 

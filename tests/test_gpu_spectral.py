@@ -227,3 +227,27 @@ def test_captured_steps_do_their_end_over(gpu, tol, passes, precision):
         for f in PROG:
             assert np.isfinite(out.fields[f]).all() and np.array_equal(out.fields[f], runs[0][0].fields[f]), f
     assert launched[1] == launched[2] == launched[3]
+
+
+@pytest.mark.gpu
+def test_spectral_solve_edges(gpu):
+    """What the check sees beside a passing solve: no right-hand side (W = 0,
+    nothing to iterate), a NaN in it (refused as not converged) and, after
+    those, an ordinary solve again."""
+    from vvm_b200.initial_state import warm_bubble
+    st = warm_bubble(64, 33)
+    g = gpu.VVMGpu(st.grid, solver=gpu.VVM_SOLVER_SPECTRAL)
+    g.upload(st)
+    b = np.random.default_rng(3).standard_normal(64 * 32)
+    first, it, rel = g.poisson_solve(b, tol=1e-10)
+    assert it == 0 and 0 < rel <= 1e-12
+    W, it, rel = g.poisson_solve(np.zeros_like(b), tol=1e-10)
+    assert it == 0 and rel == 0 and not W.any()
+    bad = b.copy()
+    bad[7] = np.nan
+    with pytest.raises(gpu.VVMGpuError) as e:
+        g.poisson_solve(bad, tol=1e-10)
+    assert "tolerance" in str(e.value)
+    W, it, rel = g.poisson_solve(b, tol=1e-10)
+    assert np.array_equal(W, first) and it == 0
+    g.close()
