@@ -375,8 +375,8 @@ __global__ void __launch_bounds__(kTileLanes* kTileWarps, 4)
 // rain sedimentation (Advection_qrVT, Advection.cpp:153-192), the surface
 // precipitation diagnostic (Iteration.cpp:114-119) and the per-block partial
 // sums of NegativeValueProcess (MicroPhysics.cpp:116-138). Writes the raw
-// interior future values; k_apply finishes them. One thread per interior
-// cell (i = 1..nx-2, k = 1..nz-2).
+// interior future values; Kessler's kernel (routine calls: k_apply) finishes
+// them.
 
 enum : int { F_TH = 1, F_QV = 2, F_QC = 4, F_QR = 8 };
 
@@ -792,7 +792,7 @@ struct KesslerArgs {
     int rows;         // rows a thread
     // The finish of the advection step (k_apply's rescaling and forcing of
     // th, qv, qc, qr) applied to each value as it is read, in place of a
-    // k_apply launch whose halo images the apply after Kessler rewrites.
+    // k_apply launch.
     AdvFinish<T> pre;
     int do_pre;
 };

@@ -131,12 +131,12 @@ def class_bytes(cls: str, launches: int, grid, elem: int, cg_iters: float) -> fl
     per_launch = {
         "pzeta": 12 * cells * elem,        # zeta u w th qv qc qr + 2 old hist in; zetap + 2 hist out
         "padv": 20 * cells * elem,         # u w + 4 fields + 5 old hist in; 4 fields + 5 hist out
-        "apply": 8 * cells * elem,         # 4 fields in place
-        "kessler": 12 * cells * elem,      # 4 in, 4 out, 4 rates out
+        "apply": 0,                        # the NVP sums' totals
+        "kessler": 8 * cells * elem,       # 4 in, 4 out
         "rkm": 5 * cells * elem,           # u w thp in; RKM RKH out
         "gs": 12 * cells * elem,           # per STEP, not per launch: 5 fields read
-                                           # and written in place + RKM, RKH (the
-                                           # tile passes' count varies, 3 typical)
+                                           # and written + RKM, RKH (repeated passes
+                                           # vary in number)
         "cal_u": 3 * cells * elem / 2,     # w zetap in, u out (two launches)
     }
     if cls in per_launch:

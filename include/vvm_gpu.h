@@ -296,14 +296,14 @@ int vvm_gpu_learned_time(vvm_gpu_ctx* ctx, int reps, double* ms_forward, double*
 int vvm_gpu_learned_last(vvm_gpu_ctx* ctx, int* fcg_iters, int* fell_back);
 
 /* -- launch-shape knobs --------------------------------------------------------
- * gs_tile_rows selects the Gauss-Seidel schedule: 4, 8, 16 or 32 = tiles of
- * that many rows (128 columns and one warp each; the passes run to the same
- * fixed point whatever the height, so results are identical across heights);
- * 1 = one thread-block cluster a field (a single pass, the schedule for many
- * cases stepping at once; it agrees with the tiles to round-off, its carries
+ * gs_tile_rows selects the Gauss-Seidel schedule: 4, 8, 16 or 32 = the single
+ * pass, with tiles of that many rows (128 columns and one warp each) for the
+ * repeated passes it falls back on (they run to the same fixed point whatever
+ * the height, so results are identical across heights); 1 = one thread-block
+ * cluster a field (it agrees with the others to round-off, its terms
  * associate differently). fft_threads sets the threads of a row-FFT block of
  * the spectral solve (no result changes). 0 selects the automatic value
- * (tiles of 16 rows in FP64, 8 in the mixed step; 512 threads or half the
+ * (tiles of 16 rows in FP64, 8 in the mixed step; 1024 threads or half the
  * row). Setting them drops the context's captured graphs. get
  * returns the values in use. */
 int vvm_gpu_set_tuning(vvm_gpu_ctx* ctx, int gs_tile_rows, int fft_threads);
@@ -314,8 +314,8 @@ int vvm_gpu_get_tuning(vvm_gpu_ctx* ctx, int* gs_tile_rows, int* fft_threads);
  * sizes (one context each, created from descs[i] on `device`) that advance
  * together: from the third step on, one CUDA graph per step runs every
  * case's step, launched on the batch's own stream. Cases with the same grid,
- * precision and tuning whose step uses the exact Fourier-mode solve and the
- * tiled Gauss-Seidel passes step as grouped launches: one launch a kernel
+ * precision and tuning whose step uses the exact Fourier-mode solve and not
+ * the cluster Gauss-Seidel schedule step as grouped launches: one launch a kernel
  * for all cases of the group (each case reads its own arguments and loop
  * flags), each group a parallel branch; other cases run as branches of
  * their own. Either way each case's results are those it computes alone.
