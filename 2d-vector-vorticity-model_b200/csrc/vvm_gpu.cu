@@ -1783,8 +1783,8 @@ struct vvm_gpu_ctx {
     double* Wprev = nullptr;   // previous cal_w solution (initial-guess extrapolation)
     int nsolves = 0;
     // CUDA graphs of one whole step, by (time-level buffer, step parity)
-    cudaGraphExec_t gexec[2][2][2] = {};   // of one step, of kGraphSteps
-    long long gstatic[2][2][2] = {};       // kernels outside the solver loops
+    cudaGraphExec_t gexec[2][2] = {};
+    long long gstatic[2][2] = {};      // kernels outside the solver loops
     cudaStream_t cap[2] = {};          // streams for capturing loop bodies
     cudaStream_t side = nullptr;       // the step's second chain (run_step)
     cudaEvent_t fork_ev[6] = {};       // its fork, meeting and join points
@@ -1806,13 +1806,12 @@ struct vvm_gpu_ctx {
     std::string err;
 
     void drop_graphs() {
-        for (auto& many : gexec)
-            for (auto& row : many)
-                for (auto& g : row)
-                    if (g) {
-                        cudaGraphExecDestroy(g);
-                        g = nullptr;
-                    }
+        for (auto& row : gexec)
+            for (auto& g : row)
+                if (g) {
+                    cudaGraphExecDestroy(g);
+                    g = nullptr;
+                }
         if (fcg_exec) cudaGraphExecDestroy(fcg_exec);
         fcg_exec = nullptr;
     }
@@ -3207,21 +3206,16 @@ int run_step(vvm_gpu_ctx* c, long long* recorded_in_loops = nullptr) {
     return rc;
 }
 
-// Steps of one launch where a call has as many left: a graph starts a few us
-// after the one before it ends. An even number, so that the graph ends on the
-// buffers and the parity it began with; us a step with 1 / 2 / 4 / 8: 128 x 64
-// 53.8 / 52.6 / 50.6 / 50.6, 2048 x 256 141 / 139 / 139 / 138. The first call's
-// capture takes 1.1 ms with 1 (two graphs) or 2, 1.8 with 4, 3.6 with 8.
-constexpr int kGraphSteps = 2;
-
-// The step as one CUDA graph (many: kGraphSteps of them): every kernel of
-// run_step, with the loops as device-controlled WHILE nodes (no host round
-// trip). Graphs are keyed by the time-level buffer and the parity of the step
-// they run (the AB2 slots alternate with it) and captured on first use.
+// The step as one CUDA graph: every kernel of run_step, with the loops as
+// device-controlled conditional nodes (no host round trip). Graphs are keyed
+// by the time-level buffer and the parity of the step they run (the AB2 slots
+// alternate with it) and captured on first use. (Two or four steps a graph
+// save 1 to 3 us a step, but a call of one step after calls of many would
+// then pay a capture of its own.)
 template <typename T>
-cudaGraphExec_t step_graph(vvm_gpu_ctx* c, bool many) {
+cudaGraphExec_t step_graph(vvm_gpu_ctx* c) {
     const int b = c->cur, par = (c->step + 1) & 1;
-    if (c->gexec[many][b][par]) return c->gexec[many][b][par];
+    if (c->gexec[b][par]) return c->gexec[b][par];
     ensure_poisson(c);
     if (c->desc.solver == VVM_SOLVER_LEARNED) ensure_learned(c);   // allocations stay outside the capture
     const int step0 = c->step, cur0 = c->cur, ns0 = c->nsolves;
@@ -3232,11 +3226,7 @@ cudaGraphExec_t step_graph(vvm_gpu_ctx* c, bool many) {
     long long in_loops = 0;
     CK(cudaStreamBeginCapture(c->stream, cudaStreamCaptureModeRelaxed));
     try {
-        for (int s = 0; s < (many ? kGraphSteps : 1); s++) {
-            long long in = 0;
-            run_step<T>(c, &in);
-            in_loops += in;
-        }
+        run_step<T>(c, &in_loops);
     } catch (...) {
         cudaStreamEndCapture(c->stream, &g);
         if (g) cudaGraphDestroy(g);
@@ -3251,13 +3241,13 @@ cudaGraphExec_t step_graph(vvm_gpu_ctx* c, bool many) {
     c->step = step0;
     c->cur = cur0;
     c->nsolves = ns0;
-    c->gstatic[many][b][par] = c->stats.launches - l0 - in_loops;
+    c->gstatic[b][par] = c->stats.launches - l0 - in_loops;
     c->stats.launches = l0;
     cudaGraphExec_t ex = nullptr;
     cudaError_t e = cudaGraphInstantiate(&ex, g, 0);
     cudaGraphDestroy(g);
     if (e != cudaSuccess) throw CudaError{std::string("cudaGraphInstantiate: ") + cudaGetErrorString(e)};
-    c->gexec[many][b][par] = ex;
+    c->gexec[b][par] = ex;
     return ex;
 }
 
@@ -3292,11 +3282,8 @@ bool graph_ready(vvm_gpu_ctx* c) {
            (!warm || c->nsolves >= 2) && !c->learned_collect && !(c->desc.flags & VVM_FLAG_STREAMFUNCTION);
 }
 
-// Steps once, or, where `left` allows it, kGraphSteps times; returns the steps
-// taken in *taken.
 template <typename T>
-int step_some(vvm_gpu_ctx* c, int left, int* taken) {
-    *taken = 1;
+int step_once(vvm_gpu_ctx* c) {
     if (!graph_ready(c)) {
         const bool forcing_now = c->has_forcing_th && ((c->step + 1) * c->desc.dt <= c->desc.addforcingtime);
         c->last_graph = false;
@@ -3308,24 +3295,16 @@ int step_some(vvm_gpu_ctx* c, int left, int* taken) {
         c->fut_is_now = true;
         return rc;
     }
-    const bool many = left >= kGraphSteps;
-    if (many) *taken = kGraphSteps;
-    cudaGraphExec_t ex = step_graph<T>(c, many);
+    cudaGraphExec_t ex = step_graph<T>(c);
     const int b = c->cur, par = (c->step + 1) & 1;
     CK(cudaGraphLaunch(ex, c->stream));
-    c->stats.launches += c->gstatic[many][b][par];
-    c->step += *taken;
-    if (!many) c->cur = 1 - c->cur;
-    c->nsolves += *taken;
+    c->stats.launches += c->gstatic[b][par];
+    c->step++;
+    c->cur = 1 - c->cur;
+    c->nsolves++;
     c->last_graph = true;
     c->fut_is_now = true;
     return VVM_GPU_OK;
-}
-
-template <typename T>
-int step_once(vvm_gpu_ctx* c) {
-    int taken;
-    return step_some<T>(c, 1, &taken);
 }
 
 // ---------------------------------------------------------------- snapshots
@@ -4780,8 +4759,8 @@ int vvm_gpu_step(vvm_gpu_ctx* ctx, int nsteps) {
         if (ctx->desc.flags & VVM_FLAG_STREAMFUNCTION)
             if (int rc = need_uniform(ctx)) return rc;
         int worst = VVM_GPU_OK;
-        for (int s = 0, taken; s < nsteps; s += taken) {
-            int rc = DISPATCH(ctx, step_some)(ctx, nsteps - s, &taken);
+        for (int s = 0; s < nsteps; s++) {
+            int rc = DISPATCH(ctx, step_once)(ctx);
             if (rc != VVM_GPU_OK) worst = rc;
         }
         if (worst == VVM_GPU_ENOCONV) fail(ctx, worst, "cal_w: Poisson solve did not reach its tolerance");

@@ -150,6 +150,11 @@ def class_bytes(cls: str, launches: int, grid, elem: int, cg_iters: float) -> fl
             nfine += 1
             n //= 2
         return total / max(2 * nfine, 1) * launches
+    if cls == "mg_coarse":
+        # the z solve of the modes (direct solver): spectra in and out, two factor
+        # arrays of half the size; with the row transforms of the multigrid's exact
+        # level, 2 arrays each, the mean of three launches is less
+        return 3 * unk * elem * launches
     if cls == "cg":
         # per iteration: spmv 2, update 6, dot 2, direction 3 arrays of the unknowns
         return 13 * unk * elem * cg_iters

@@ -197,8 +197,8 @@ def test_spectral_modes_at_every_height(gpu, nk):
 @pytest.mark.parametrize("tol,passes", [(1e-10, False), (1e-14, False), (1e-10, True), (1e-14, True)])
 def test_captured_steps_do_their_end_over(gpu, tol, passes, precision):
     """Steps whose check fails (tol 1e-14), whose sweep needs the repeated passes
-    or both: graphs of one step and of several, whose end does over what the
-    steps went on with, equal the host's loops bit for bit, with moisture
+    or both: step graphs, whose end does over what the step went on with, equal
+    the host's loops bit for bit, however the calls are cut, with moisture
     nudging after the diffusion and the counts of launches alike."""
     from vvm_b200.initial_state import warm_bubble
     if passes:
