@@ -14,6 +14,7 @@
 
 #include <type_traits>
 
+#include "gs_bands.cuh"
 #include "vvm_common.cuh"
 
 namespace vvm {
@@ -1688,8 +1689,8 @@ __device__ __forceinline__ void gs_sweep_tile(const GSSweepArgs<T>& a, GSSweepSh
                                               bool wide) {
     constexpr int D = kGWDepth;
     const Dims& d = a.d;
-    const int kend = d.nz - 2;
-    const int k0 = 1 + b * a.tr, kl = min(k0 + a.tr - 1, kend), ks = max(1, k0 - hz);
+    const GSBand band = gs_band(b, a.tr, hz, d.nz);
+    const int k0 = band.k0, kl = band.kl, ks = band.ks;
     GSSweepTile<T, MOM, NF> t;
     t.lane = threadIdx.x & 31;
     t.f0 = f0;
@@ -1745,7 +1746,7 @@ __device__ __forceinline__ void gs_sweep_tile(const GSSweepArgs<T>& a, GSSweepSh
     }
     __syncwarp();
     t.take(S, a, 0, ks - 1, D < n, t.Kp, t.below);
-    if (ks == 1 && t.own) {   // the ghost row under the grid
+    if (band.bottom && t.own) {   // the ghost row under the grid
 #pragma unroll
         for (int f = 0; f < NF; f++) {
             t.to[f] -= t.pitch;
@@ -1774,7 +1775,7 @@ __device__ __forceinline__ void gs_sweep_tile(const GSSweepArgs<T>& a, GSSweepSh
         q = (q + 1) & (D - 1);
         t.row(S.row[k - ks], Ku, vu, k >= k0);
     }
-    if (kl == kend && t.own) {   // the ghost row over the grid
+    if (band.top && t.own) {   // the ghost row over the grid
 #pragma unroll
         for (int f = 0; f < NF; f++) t.store4(f, t.v0[f]);
     }

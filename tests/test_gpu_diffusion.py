@@ -84,3 +84,34 @@ def test_repeated_passes_from_graphs(G, precision, dt):
         for n in ("zeta", "th", "qv", "qc", "qr", "u", "w"):
             assert np.array_equal(out.fields[n], ref.fields[n]), n
     b.close()
+
+
+def test_tails_over_a_whole_band_in_many_waves(G):
+    """Tails of 8 rows and more (dx = 100 m, dt = 8 s: B + C = 2 K dt / dx^2 =
+    0.016 at K's floor of 10 m^2/s, 9 rows) over bands of 8 rows, with more
+    tiles in one launch than the GPU holds at once: 64 cases of 128 x 64, about
+    2500 blocks. A band above the first starts at the ground then, and must
+    leave the rows of the bands under it alone whichever of them ran before.
+    Every case as alone, bit for bit (there all its tiles run at once)."""
+    from vvm_b200.initial_state import warm_bubble
+    kinds = [warm_bubble(128, 64, 100.0, 100.0, 8.0, amp=a, radius=800.0, zc=z) for a, z in ((0.2, 900.0), (0.4, 1200.0))]
+    ref = []
+    for st in kinds:
+        g = G.VVMGpu(st.grid, solver=G.VVM_SOLVER_SPECTRAL)
+        g.upload(st)
+        g.step(5)
+        ref.append(g.download())
+        g.close()
+        assert np.isfinite(ref[-1].fields["zeta"]).all()
+    sts = [kinds[j % 2] for j in range(64)]
+    b = G.VVMBatch([st.grid for st in sts], precision=0)
+    b.grouping(64)
+    b.upload(sts)
+    b.step(5)
+    b.synchronize()
+    assert b.grouping() == 1
+    for j, c in enumerate(b.cases):
+        out = c.download()
+        for n in ("zeta", "th", "qv", "qc", "qr", "u", "w", "RKM"):
+            assert np.array_equal(out.fields[n], ref[j % 2].fields[n]), (j, n)
+    b.close()
