@@ -442,18 +442,19 @@ inline void upload_now(void* dst, const void* src, size_t nb) {
 
 // Small allocations are carved from slabs: a context makes about a hundred,
 // and a cudaMalloc, a clear and a wait for each took most of its creation (128 x
-// 64: 2 ms). ptrs and bytes list the slabs.
+// 64: 2 ms). ptrs lists the slabs and the large allocations, used the bytes of
+// each that are handed out: what lies behind them belongs to nobody yet.
 struct Arena {
     static constexpr size_t kSlab = size_t(2) << 20, kAlign = 256;
     std::vector<void*> ptrs;
-    std::vector<size_t> bytes;
+    std::vector<size_t> used;
     char* slab = nullptr;
-    size_t left = 0;
+    size_t slab_at = 0, left = 0;   // the open slab, its index and its free bytes
     void* raw(size_t nb) {
         void* p = nullptr;
         CK(cudaMalloc(&p, nb));
         ptrs.push_back(p);
-        bytes.push_back(nb);
+        used.push_back(nb);
         CK(cudaMemset(p, 0, nb));
         // complete before returning: a context's stream may be non-blocking,
         // and work on it is not ordered after the legacy stream
@@ -466,11 +467,13 @@ struct Arena {
         if (nb > kSlab / 2) return static_cast<X*>(raw(nb));
         if (nb > left) {
             slab = static_cast<char*>(raw(kSlab));
+            slab_at = ptrs.size() - 1;
             left = kSlab;
         }
         X* p = reinterpret_cast<X*>(slab);
         slab += nb;
         left -= nb;
+        used[slab_at] = kSlab - left;
         return p;
     }
     ~Arena() {
@@ -3311,8 +3314,11 @@ int step_once(vvm_gpu_ctx* c) {
 
 // A device copy of every buffer of a context plus its host-side counters:
 // the autotuner runs real steps and puts the cases back exactly afterwards.
+// Buffers made later, which may lie behind the copied ones in a slab, are left
+// as they are.
 struct Snapshot {
     std::vector<void*> copies;
+    std::vector<size_t> bytes;   // of each: what was in use
     int step = 0, cur = 0, nsolves = 0, last_iters = 0;
     bool fut_is_now = false;
     double last_relres = 0;
@@ -3321,9 +3327,11 @@ struct Snapshot {
         CK(cudaStreamSynchronize(c->stream));
         for (size_t j = 0; j < c->ar.ptrs.size(); j++) {
             void* q = nullptr;
-            CK(cudaMalloc(&q, c->ar.bytes[j]));
-            CK(cudaMemcpyAsync(q, c->ar.ptrs[j], c->ar.bytes[j], cudaMemcpyDeviceToDevice, c->stream));
+            const size_t nb = c->ar.used[j];
+            CK(cudaMalloc(&q, nb));
             copies.push_back(q);
+            bytes.push_back(nb);
+            CK(cudaMemcpyAsync(q, c->ar.ptrs[j], nb, cudaMemcpyDeviceToDevice, c->stream));
         }
         CK(cudaStreamSynchronize(c->stream));
         step = c->step;
@@ -3337,7 +3345,7 @@ struct Snapshot {
     void restore(vvm_gpu_ctx* c) {
         CK(cudaStreamSynchronize(c->stream));
         for (size_t j = 0; j < copies.size(); j++)
-            CK(cudaMemcpyAsync(c->ar.ptrs[j], copies[j], c->ar.bytes[j], cudaMemcpyDeviceToDevice, c->stream));
+            CK(cudaMemcpyAsync(c->ar.ptrs[j], copies[j], bytes[j], cudaMemcpyDeviceToDevice, c->stream));
         CK(cudaStreamSynchronize(c->stream));
         c->step = step;
         c->cur = cur;
@@ -3818,8 +3826,13 @@ int batch_autotune(vvm_gpu_batch* b, int reps, int* ngroups) {
     CK(cudaStreamSynchronize(b->stream));
     std::vector<std::unique_ptr<Snapshot>> snaps(n);
     for (size_t i = 0; i < n; i++) {
+        // the solver first, so that its work arrays (the iterate a solve may
+        // start from) are put back too
+        vvm_gpu_ctx* c = b->cases[i];
+        ensure_poisson(c);
+        if (c->desc.solver == VVM_SOLVER_LEARNED) ensure_learned(c);
         snaps[i].reset(new Snapshot());
-        snaps[i]->take(b->cases[i]);
+        snaps[i]->take(c);
     }
     int rc = VVM_GPU_OK;
     // bring every case to a step that runs from a graph (restored below)

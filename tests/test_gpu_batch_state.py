@@ -1,0 +1,59 @@
+"""What a batch does to its cases' state, in the orders a program may call it.
+
+The autotuner straight after the upload, before any step: it builds the solver
+on the way, and must leave it whole. Every case then steps as it does alone
+with the tuned knobs, bit for bit, and a solve's residual, recomputed with the
+C restatement's copy of the matrix, is what the solve reports: 1e-10 asked,
+1e-9 allowed (the report is the same sum in another order, and a solve that
+reports 1e-10 with a broken weight is off by all of its right-hand side).
+"""
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+PROG = ("zeta", "th", "qv", "qc", "qr", "u", "w")
+
+
+@pytest.fixture(scope="module")
+def G():
+    from vvm_b200 import build, gpu
+    build.build()
+    return gpu
+
+
+def _same(a, b):
+    return all(np.array_equal(a.fields[f], b.fields[f]) for f in PROG)
+
+
+@pytest.mark.parametrize("precision,solver,shapes", [
+    (1, 2, [(64, 32), (64, 32), (128, 48)]),   # mixed, spectral, grouped and alone
+    (0, 2, [(256, 32)]),
+    (0, 0, [(64, 32), (96, 33)]),              # FP64, multigrid
+    (1, 0, [(64, 32)]),
+    (0, 1, [(64, 32)]),                        # the learned preconditioner, untrained
+])
+def test_autotune_before_the_first_step(G, port_lib, precision, solver, shapes):
+    from vvm_b200.initial_state import warm_bubble
+    sts = [warm_bubble(nx, nz, 200.0, 200.0, radius=max(400.0, nx * 25.0)) for nx, nz in shapes]
+    b = G.VVMBatch([s.grid for s in sts], precision=precision, solver=solver)
+    b.upload(sts)
+    b.autotune(reps=1)
+    b.step(4)
+    b.synchronize()
+    outs = [c.download() for c in b.cases]
+    for c, st, out in zip(b.cases, sts, outs):
+        g = G.VVMGpu(st.grid, precision=precision, solver=solver)
+        g.set_tuning(*c.tuning())
+        g.upload(st)
+        g.step(4)
+        assert _same(out, g.download())
+        g.close()
+        A = port_lib.PortModel(st.grid)
+        A.load(st)
+        rhs = np.random.default_rng(1).standard_normal(st.grid.NX * (st.grid.NZ - 1))
+        W, _, rel = c.poisson_solve(rhs, tol=1e-10)
+        assert rel <= 1e-10
+        assert np.linalg.norm(rhs - A.apply_A(W)) <= 1e-9 * np.linalg.norm(rhs)
+        A.close()
+    b.close()
