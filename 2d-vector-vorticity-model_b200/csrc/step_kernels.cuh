@@ -159,6 +159,7 @@ struct PZetaArgs {
     AB2 ab;
     PubarArgs<T> pubar;            // pubarTop_pt, by one block past the tiles
     int do_pubar;
+    unsigned* kmax;                // [2]: cleared by that block for this step's k_rkm_rkh
 };
 
 // Tile of k_pzeta: 31 x 8R zeta points a block of 32 x 8 threads, R rows a
@@ -228,7 +229,10 @@ __device__ __forceinline__ void k_pzeta_body(const FieldMaps<7>& maps, const PZe
     using Sh = PZetaShared<T, R>;
     constexpr int BZ = Sh::BZ, VZ = Sh::VZ, VX = kTileVX, AL = 16 / sizeof(T);
     if (a.do_pubar && blockIdx.y == 0) {   // the first row of blocks: it starts with the first wave
-        if (blockIdx.x == 0) k_pubartop_body<T>(a.pubar);
+        if (blockIdx.x == 0) {
+            if (threadIdx.x == 0 && threadIdx.y == 0) a.kmax[0] = a.kmax[1] = 0u;
+            k_pubartop_body<T>(a.pubar);
+        }
         return;
     }
     const int by = blockIdx.y - (a.do_pubar ? 1 : 0);
@@ -2283,7 +2287,6 @@ struct MeanArgs {
     double *thb, *qvb, *thvb;
     double* ubar;   // [0] ubarTop, [1] ubarTopp
     int rotate_ubar;
-    unsigned* kmax;   // [2]: cleared for the next step's k_rkm_rkh (may be null)
     const int* skip;  // nothing to do where *skip (may be null)
 };
 
@@ -2328,7 +2331,6 @@ __device__ __forceinline__ void k_update_mean_body(const MeanArgs<T>& a) {
         if (k == 1) { a.thb[0] = tb; a.qvb[0] = qb; a.thvb[0] = tv; }
         if (k == d.nz - 2) { a.thb[d.nz - 1] = tb; a.qvb[d.nz - 1] = qb; a.thvb[d.nz - 1] = tv; }
         if (k == 1 && a.rotate_ubar) a.ubar[0] = a.ubar[1];
-        if (k == 1 && a.kmax) a.kmax[0] = a.kmax[1] = 0u;
     }
 }
 template <typename T>

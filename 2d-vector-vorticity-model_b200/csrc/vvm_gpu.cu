@@ -1932,7 +1932,7 @@ void launch_pzeta_r(vvm_gpu_ctx* c) {
     PZetaArgs<T> a{c->d, c->c, c->profiles(), F.zeta[now], F.u, F.w, F.th[now], F.qv[now], F.qc[now], F.qr[now],
                    zeta_pre<T>(c), F.hist[H_ZETA][ab.sn], F.hist[H_ZETA][ab.so], F.hist[H_BUOY][ab.sn],
                    F.hist[H_BUOY][ab.so], c->d_err, ab, pubar_args<T>(c),
-                   c->in_step && !(c->desc.flags & VVM_FLAG_STREAMFUNCTION)};
+                   c->in_step && !(c->desc.flags & VVM_FLAG_STREAMFUNCTION), c->kmax};
     const T* staged[7] = {a.zeta, a.u, a.w, a.th, a.qv, a.qc, a.qr};
     FieldMaps<7> m;
     for (int f = 0; f < 7; f++)
@@ -2390,7 +2390,7 @@ void launch_turbulence(vvm_gpu_ctx* c, bool nudge, long long* recorded_in_loops 
     cudaStream_t st = c->stream;
     const GSSweepArgs<T> w = gs_sweep_args<T>(c, nudge);
     GSPasses<T> passes(c, w, recorded_in_loops != nullptr);
-    if (!recorded_in_loops) {   // a graph's steps leave both as they found them
+    if (!recorded_in_loops) {   // a graph's steps begin with both clear: k_pzeta clears kmax, the passes their state
         CK(cudaMemsetAsync(c->kmax, 0, 2 * sizeof(unsigned), st));
         CK(cudaMemsetAsync(c->gsctl, 0, sizeof(GSTileCtl), st));
     }
@@ -2438,7 +2438,7 @@ void launch_update_mean(vvm_gpu_ctx* c, bool rotate, const int* skip = nullptr) 
     Fields<T>& F = fields<T>(c);
     int fut = 1 - c->cur;
     MeanArgs<T> a{c->d, c->offset_th(), c->offset_qv(), F.th[fut], F.qv[fut], c->thb, c->qvb, c->thvb,
-                  c->ubar, rotate ? 1 : 0, c->in_step ? c->kmax : nullptr, skip};
+                  c->ubar, rotate ? 1 : 0, skip};
     klaunch<k_update_mean_body<T>, 256>(&c->stats, VVM_K_MEAN, c->stream, k_update_mean<T>, dim3(c->d.nz - 2),
                                         dim3(256), 0, a);
 }

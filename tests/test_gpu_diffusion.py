@@ -115,3 +115,37 @@ def test_tails_over_a_whole_band_in_many_waves(G):
         for n in ("zeta", "th", "qv", "qc", "qr", "u", "w", "RKM"):
             assert np.array_equal(out.fields[n], ref[j % 2].fields[n]), (j, n)
     b.close()
+
+
+@pytest.mark.parametrize("precision", [0, 1])
+def test_routine_turbulence_leaves_later_steps_alone(G, precision):
+    """The largest eddy coefficient of a routine call (K at its cap of 8000
+    m^2/s) does not reach the next captured step, which would ask for the
+    repeated passes: the same kernels run and give the same bits as without
+    the call."""
+    from vvm_b200.initial_state import random_state, warm_bubble
+    st = warm_bubble(128, 32, 200.0, 200.0, 4.0, radius=1000.0)
+    wild = random_state(128, 32, dt=4.0, seed=3)
+    for n in ("u", "w"):
+        wild.fields[n] *= 40.0
+    for n in ("zeta", "th", "qv", "qc", "qr"):
+        wild.fields[n + "p"] = wild.fields[n]
+    outs, counts = [], []
+    for disturb in (False, True):
+        g = G.VVMGpu(st.grid, precision=precision, solver=G.VVM_SOLVER_SPECTRAL, warm_start=False)
+        g.upload(st)
+        g.step(3)
+        if disturb:
+            g.upload(wild)
+            g.call("turbulence")
+            assert g.download().fields["RKM"].max() > 1000.0
+            g.call("next_step")
+        g.upload(st)
+        n0 = g.launch_count
+        g.step(2)
+        counts.append(g.launch_count - n0)
+        outs.append(g.download())
+        g.close()
+    assert counts[0] == counts[1]
+    for n in ("zeta", "th", "qv", "qc", "qr", "u", "w", "RKM"):
+        assert np.array_equal(outs[0].fields[n], outs[1].fields[n]), n
