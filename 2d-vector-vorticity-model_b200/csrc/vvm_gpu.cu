@@ -2445,14 +2445,17 @@ void launch_update_mean(vvm_gpu_ctx* c, bool rotate, const int* skip = nullptr) 
 
 // ---------------------------------------------------------------- Poisson
 
+// Threads of a row-FFT block: the knob's, within [32, half a row, 1024], or as
+// many as that allows (us both transforms of a step with 512 / 1024: 8192 x 256
+// 75 / 62, 2048 x 256 30 / 28).
+int fft_threads_used(int NX, int knob) {
+    const int most = std::min(std::max(32, NX / 2), 1024);
+    return knob > 0 ? std::max(32, std::min(knob, most)) : most;
+}
+
 // Applies the launch-shape knobs that live inside the solver objects.
 void apply_tuning(vvm_gpu_ctx* c) {
-    if (c->pcg64 && c->pcg64->spectral) {
-        const int half = std::max(32, (c->d.nx - 2) / 2);
-        // (us both transforms of a step with 512 / 1024: 8192 x 256 75 / 62, 2048 x 256 30 / 28)
-        const int def = std::min(half, 1024);
-        c->pcg64->sp.threads = c->tune_fft > 0 ? std::max(32, std::min(c->tune_fft, std::min(half, 1024))) : def;
-    }
+    if (c->pcg64 && c->pcg64->spectral) c->pcg64->sp.threads = fft_threads_used(c->d.nx - 2, c->tune_fft);
 }
 
 void ensure_poisson(vvm_gpu_ctx* c) {
@@ -5166,14 +5169,7 @@ int vvm_gpu_set_tuning(vvm_gpu_ctx* ctx, int gs_tile_rows, int fft_threads) {
 int vvm_gpu_get_tuning(vvm_gpu_ctx* ctx, int* gs_tile_rows_out, int* fft_threads) {
     if (!ctx) return VVM_GPU_EINVAL;
     if (gs_tile_rows_out) *gs_tile_rows_out = gs_tile_rows(ctx);   // kGSSchedCluster: the cluster schedule
-    if (fft_threads) {
-        *fft_threads = 0;
-        if (ctx->spectral) {
-            const int half = std::max(32, (ctx->d.nx - 2) / 2);
-            *fft_threads = ctx->tune_fft > 0 ? std::max(32, std::min(ctx->tune_fft, std::min(half, 1024)))
-                                             : std::min(half, 512);
-        }
-    }
+    if (fft_threads) *fft_threads = ctx->spectral ? fft_threads_used(ctx->d.nx - 2, ctx->tune_fft) : 0;
     return VVM_GPU_OK;
 }
 

@@ -57,3 +57,18 @@ def test_autotune_before_the_first_step(G, port_lib, precision, solver, shapes):
         assert np.linalg.norm(rhs - A.apply_A(W)) <= 1e-9 * np.linalg.norm(rhs)
         A.close()
     b.close()
+
+
+@pytest.mark.parametrize("NX", [4, 64, 1024, 2048, 8192])
+def test_tuning_reports_the_row_fft_block_in_use(G, NX):
+    """The automatic block is half a row, 32 to 1024 threads; setting what is
+    reported changes nothing."""
+    from vvm_b200.initial_state import warm_bubble
+    g = G.VVMGpu(warm_bubble(NX, 8, 200.0, 200.0).grid, solver=G.VVM_SOLVER_SPECTRAL)
+    auto = g.tuning()
+    assert auto[1] == min(max(32, NX // 2), 1024)
+    g.set_tuning(*auto)
+    assert g.tuning() == auto
+    g.set_tuning(0, 64)
+    assert g.tuning()[1] == min(64, auto[1])
+    g.close()
