@@ -170,7 +170,8 @@ def _prognostic_state(arrays):
     hs = HostState()
     words = np.frombuffer(hs, dtype=np.uint64)
     for (n, at), a in zip(_SLOT, arrays):
-        words[at] = a.__array_interface__["data"][0]
+        if a is not None:
+            words[at] = a.__array_interface__["data"][0]
     return hs
 
 
