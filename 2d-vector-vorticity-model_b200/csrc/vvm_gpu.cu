@@ -3819,10 +3819,11 @@ double batch_time(vvm_gpu_batch* b, const std::vector<int>& idx, int reps) {
 }
 
 // Autotuner: for each group of cases with the same grid, precision and
-// solver, coordinate descent over the launch-shape knobs that leave the
-// arithmetic unchanged (the Gauss-Seidel schedule: tile height or one cluster
-// a field; the row-FFT block; the cases a grouped launch takes), timing one
-// step of the group's cases as a graph per candidate. Every case is put back
+// solver, coordinate descent over the launch-shape knobs (the Gauss-Seidel
+// schedule: single pass or one cluster a field; the row-FFT block; the cases a
+// grouped launch takes), timing one step of the group's cases as a graph per
+// candidate. The tile heights are not candidates: they shape the repeated
+// passes alone, which the timed steps do not run. Every case is put back
 // exactly afterwards.
 int batch_autotune(vvm_gpu_batch* b, int reps, int* ngroups) {
     const size_t n = b->cases.size();
@@ -3872,17 +3873,20 @@ int batch_autotune(vvm_gpu_batch* b, int reps, int* ngroups) {
         vvm_gpu_ctx* c = b->cases[idx[0]];
         int best_cs = c->tune_gs_tr, best_fft = c->tune_fft;
         double best = batch_time(b, idx, reps);
-        for (int tr : {kGSSchedCluster, 4, 8, 16, 32}) {   // Gauss-Seidel schedule: cluster, tile rows
-            set_all(idx, tr, best_fft);
+        {   // the Gauss-Seidel schedule the cases do not have
+            const int other = best_cs == kGSSchedCluster ? 0 : kGSSchedCluster;
+            set_all(idx, other, best_fft);
             const double t = batch_time(b, idx, reps);
             if (t < best) {
                 best = t;
-                best_cs = tr;
+                best_cs = other;
             }
         }
         set_all(idx, best_cs, best_fft);
         if (c->spectral) {
-            for (int th : {128, 256, 512}) {
+            const int start_fft = fft_threads_used(c->d.nx - 2, best_fft);
+            for (int th : {128, 256, 512, 1024}) {   // blocks of their own, not the start's again
+                if (fft_threads_used(c->d.nx - 2, th) != th || th == start_fft) continue;
                 set_all(idx, best_cs, th);
                 const double t = batch_time(b, idx, reps);
                 if (t < best) {

@@ -72,3 +72,21 @@ def test_tuning_reports_the_row_fft_block_in_use(G, NX):
     g.set_tuning(0, 64)
     assert g.tuning()[1] == min(64, auto[1])
     g.close()
+
+
+def test_autotune_keeps_the_tile_height(G):
+    """The tile heights time alike (they shape passes a normal step does not
+    run), so the autotuner tries none: it leaves the single pass as it is set
+    or takes the cluster schedule. And it can come back from the cluster."""
+    from vvm_b200.initial_state import warm_bubble
+    sts = [warm_bubble(64, 32, 200.0, 200.0)] * 3
+    for rows in (0, 32, 1, 1, 1):
+        b = G.VVMBatch([s.grid for s in sts], precision=1, solver=G.VVM_SOLVER_SPECTRAL)
+        for c in b.cases:
+            c.set_tuning(rows, 0)
+        b.upload(sts)
+        b.step(3)
+        b.autotune(reps=1)
+        tr = {c.tuning()[0] for c in b.cases}
+        assert len(tr) == 1 and tr <= {1, 32 if rows == 32 else 8}
+        b.close()
