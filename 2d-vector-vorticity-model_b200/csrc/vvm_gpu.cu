@@ -1808,6 +1808,14 @@ struct vvm_gpu_ctx {
     Stats stats;
     std::string err;
 
+    // Counts the changes of what a batch's captured steps hold of the case: the
+    // numbers below, the solver's arrays, the knobs.
+    unsigned long long graph_gen = 0;
+    // What an uploaded state puts into kernel arguments by value (forced steps,
+    // which has_forcing_th concerns, are not captured).
+    std::array<double, 9> graph_args() const {
+        return {pf1, pf2, lv_rdz_up, lv_rdz_dn, lv_rdz_c, lv_hfac, gs_fz[0], gs_fz[1], double(has_q)};
+    }
     void drop_graphs() {
         for (auto& row : gexec)
             for (auto& g : row)
@@ -2461,6 +2469,7 @@ void apply_tuning(vvm_gpu_ctx* c) {
 void ensure_poisson(vvm_gpu_ctx* c) {
     if (c->poisson_ready) return;
     c->drop_graphs();
+    c->graph_gen++;
     int NX = c->d.nx - 2, NK = c->d.nz - 3;
     c->pcg64.reset(new PCG<double>());
     c->pcg64->stats = &c->stats;
@@ -3390,6 +3399,7 @@ struct vvm_gpu_batch {
     cudaEvent_t fork = nullptr, t0 = nullptr, t1 = nullptr;
     std::vector<cudaEvent_t> joins;
     cudaGraphExec_t gexec[2][2] = {};
+    unsigned long long graph_gen = 0;       // sum of the cases' graph_gen that gexec was captured at
     std::vector<long long> gstatic[2][2];   // kernels outside loops, per case
     std::vector<void*> gbufs[2][2];         // device arrays of the grouped launches of gexec
     int group_max = kGroupMaxDefault;       // cases a grouped launch takes at most (0: no grouping)
@@ -3752,10 +3762,12 @@ int batch_step(vvm_gpu_batch* b, int nsteps) {
     for (int s = 0; s < nsteps; s++) {
         vvm_gpu_ctx* c0 = b->cases[0];
         bool ready = true;
+        unsigned long long gen = 0;   // each case's only grows
         for (auto* c : b->cases) {
             if (c->step != c0->step || c->cur != c0->cur)
                 return batch_fail(b, VVM_GPU_ESTATE, "batch_step: the cases are not at the same step");
             ready = ready && graph_ready(c);
+            gen += c->graph_gen;
         }
         if (!ready) {   // the first steps, or timers on: each case on its own stream
             if (on_batch) {
@@ -3767,6 +3779,11 @@ int batch_step(vvm_gpu_batch* b, int nsteps) {
                 if (rc != VVM_GPU_OK) worst = rc;
             }
             continue;
+        }
+        if (gen != b->graph_gen) {   // a case has a new state, operator or knob
+            CK(cudaStreamSynchronize(b->stream));
+            b->drop_graphs();
+            b->graph_gen = gen;
         }
         const int bi = c0->cur, par = (c0->step + 1) & 1;
         if (!b->gexec[bi][par]) b->gexec[bi][par] = batch_capture(b, all, b->gstatic[bi][par], b->gbufs[bi][par]);
@@ -4646,7 +4663,9 @@ int vvm_gpu_upload_state(vvm_gpu_ctx* ctx, const vvm_gpu_host_state* st) {
     if (!st) return fail(ctx, VVM_GPU_EINVAL, "upload: NULL state");
     return guarded(ctx, [&] {
         ctx->drop_graphs();   // kernel arguments depend on the uploaded flags
+        const auto args = ctx->graph_args();
         int rc = upload_profiles(ctx, st);
+        if (ctx->graph_args() != args) ctx->graph_gen++;
         if (rc) return rc;
         if (ctx->poisson_ready) {   // a new state: no solver history
             CK(cudaMemsetAsync(ctx->W, 0, (size_t)ctx->pcg64->NK * ctx->pcg64->pitch * sizeof(double), ctx->stream));
@@ -5141,6 +5160,7 @@ int vvm_gpu_learned_config(vvm_gpu_ctx* ctx, int mode, int cap) {
         ctx->learned_mode = mode;
         ctx->learned_cap = cap;
         ctx->drop_graphs();   // mode and cap are recorded into the graphs
+        ctx->graph_gen++;
         return VVM_GPU_OK;
     });
 }
@@ -5166,6 +5186,7 @@ int vvm_gpu_set_tuning(vvm_gpu_ctx* ctx, int gs_tile_rows, int fft_threads) {
         ctx->tune_fft = fft_threads;
         apply_tuning(ctx);
         ctx->drop_graphs();
+        ctx->graph_gen++;
         return VVM_GPU_OK;
     });
 }

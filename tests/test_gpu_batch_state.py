@@ -90,3 +90,36 @@ def test_autotune_keeps_the_tile_height(G):
         tr = {c.tuning()[0] for c in b.cases}
         assert len(tr) == 1 and tr <= {1, 32 if rows == 32 else 8}
         b.close()
+
+
+@pytest.mark.parametrize("warm_start", [True, False])
+@pytest.mark.parametrize("limit", [32, 0])   # grouped launches, cases as branches
+def test_a_new_state_reaches_the_batch_graphs(G, warm_start, limit):
+    """A second state with other profiles (density, and with it the elliptic
+    operator and the diffusion's coefficients), uploaded after the batch has
+    captured its steps: every case as alone, bit for bit. Then new knobs."""
+    from vvm_b200.initial_state import warm_bubble
+    old = [warm_bubble(64, 32, 200.0, 200.0, radius=800.0) for _ in range(3)]
+    new = [warm_bubble(64, 32, 200.0, 200.0, radius=r, dthdz=6e-3, rh=0.5) for r in (600.0, 800.0, 1000.0)]
+    b = G.VVMBatch([s.grid for s in old], precision=0, solver=G.VVM_SOLVER_SPECTRAL, warm_start=warm_start)
+    b.grouping(limit)
+    b.upload(old)
+    b.step(6)
+    b.upload(new)
+    b.step(6)
+    b.synchronize()
+    outs = [c.download() for c in b.cases]
+    for c in b.cases:
+        c.set_tuning(1, 0)   # the cluster schedule: other last bits
+    b.step(2)
+    b.synchronize()
+    for c, st, out in zip(b.cases, new, outs):
+        g = G.VVMGpu(st.grid, precision=0, solver=G.VVM_SOLVER_SPECTRAL, warm_start=warm_start)
+        g.upload(st)
+        g.step(6)
+        assert _same(out, g.download())
+        g.set_tuning(1, 0)
+        g.step(2)
+        assert _same(c.download(), g.download())
+        g.close()
+    b.close()
