@@ -447,14 +447,49 @@ inline void upload_now(void* dst, const void* src, size_t nb) {
 struct Arena {
     static constexpr size_t kSlab = size_t(2) << 20, kAlign = 256;
     std::vector<void*> ptrs;
-    std::vector<size_t> used;
+    std::vector<size_t> bytes, used;
+    bool borrowed = false;          // ptrs[0] is another arena's
+    size_t next = 0;                // of ptrs: the next to hand out (below its size after a rewind)
     char* slab = nullptr;
     size_t slab_at = 0, left = 0;   // the open slab, its index and its free bytes
+    // The allocations that follow repeat the ones made so far, in the same
+    // order and sizes, and take their memory (cleared again).
+    void rewind() {
+        next = 0;
+        slab = nullptr;
+        left = 0;
+        if (borrowed) open(raw(bytes[0]));
+    }
+    // Starts with the free end of `from`'s open slab (a slab of its own costs a
+    // small grid's first step 0.4 ms); `from` must outlive this arena.
+    void borrow(Arena& from) {
+        if (!ptrs.empty() || !from.left) return;
+        ptrs.push_back(from.slab);
+        bytes.push_back(from.left);
+        used.push_back(0);
+        borrowed = true;
+        from.slab = nullptr;
+        from.left = 0;
+        next = 1;
+        open(ptrs[0]);
+    }
+    void open(void* p) {   // p: ptrs[next - 1]
+        slab = static_cast<char*>(p);
+        slab_at = next - 1;
+        left = bytes[slab_at];
+    }
     void* raw(size_t nb) {
         void* p = nullptr;
-        CK(cudaMalloc(&p, nb));
-        ptrs.push_back(p);
-        used.push_back(nb);
+        if (next < ptrs.size()) {
+            if (bytes[next] != nb) throw CudaError{"arena: an allocation differs from the one it repeats"};
+            p = ptrs[next];
+        } else {
+            CK(cudaMalloc(&p, nb));
+            ptrs.push_back(p);
+            bytes.push_back(nb);
+            used.push_back(0);
+        }
+        used[next++] = nb;
         CK(cudaMemset(p, 0, nb));
         // complete before returning: a context's stream may be non-blocking,
         // and work on it is not ordered after the legacy stream
@@ -465,19 +500,15 @@ struct Arena {
     X* alloc(size_t n) {
         const size_t nb = (std::max<size_t>(n, 1) * sizeof(X) + kAlign - 1) / kAlign * kAlign;
         if (nb > kSlab / 2) return static_cast<X*>(raw(nb));
-        if (nb > left) {
-            slab = static_cast<char*>(raw(kSlab));
-            slab_at = ptrs.size() - 1;
-            left = kSlab;
-        }
+        if (nb > left) open(raw(kSlab));
         X* p = reinterpret_cast<X*>(slab);
         slab += nb;
         left -= nb;
-        used[slab_at] = kSlab - left;
+        used[slab_at] = bytes[slab_at] - left;
         return p;
     }
     ~Arena() {
-        for (void* p : ptrs) cudaFree(p);
+        for (size_t j = borrowed ? 1 : 0; j < ptrs.size(); j++) cudaFree(ptrs[j]);
     }
 };
 
@@ -1585,9 +1616,8 @@ struct PCG {
         arrive = ar.alloc<unsigned>(1);
         CK(cudaMallocHost(&sc_host, sizeof(CGScalars)));
     }
-    void release() {
+    ~PCG() {
         if (sc_host) cudaFreeHost(sc_host);
-        sc_host = nullptr;
     }
     dim3 block() const { return dim3(64, 4); }
     dim3 grid() const { return dim3(cdiv(NX, 64), cdiv(NK, 4)); }
@@ -1732,7 +1762,7 @@ struct vvm_gpu_ctx {
     bool learned_collect = false;   // training-pair collection: solve with the plain solver
     int tune_fft = 0;        // threads of a row-FFT block (0: automatic)
     int tune_group = 0;      // in a batch: cases a grouped launch takes at most (0: the batch's limit)
-    Arena ar;
+    Arena ar, par;   // the fields and workspaces; what ensure_poisson builds anew for another density
     Fields<double> f64;
     Fields<float> f32;
     int cur = 0;       // buffer index of the "now" time level
@@ -1839,9 +1869,6 @@ struct vvm_gpu_ctx {
         for (auto& row : xev)
             for (auto e : row)
                 if (e) cudaEventDestroy(e);
-        if (pcg64) pcg64->release();
-        if (pcg32) pcg32->release();
-        if (pcg_psi) pcg_psi->release();
         if (sc_host) cudaFreeHost(sc_host);
         if (sc_host_i) cudaFreeHost(sc_host_i);
         if (err_host) cudaFreeHost(err_host);
@@ -2470,27 +2497,30 @@ void ensure_poisson(vvm_gpu_ctx* c) {
     if (c->poisson_ready) return;
     c->drop_graphs();
     c->graph_gen++;
+    // the grid fixes every size: a new operator takes the old one's place
+    if (c->par.ptrs.empty()) c->par.borrow(c->ar);
+    else c->par.rewind();
     int NX = c->d.nx - 2, NK = c->d.nz - 3;
     c->pcg64.reset(new PCG<double>());
     c->pcg64->stats = &c->stats;
     c->pcg64->spectral = c->spectral;
-    c->pcg64->build(c->ar, NX, NK, c->h_rhou, c->h_rhow, c->h_a, c->h_h);
+    c->pcg64->build(c->par, NX, NK, c->h_rhou, c->h_rhow, c->h_a, c->h_h);
     int pitch = c->pcg64->pitch;
-    c->Wf = c->ar.alloc<double>((size_t)NK * pitch);
-    c->W = c->ar.alloc<double>((size_t)NK * pitch);
-    c->r64 = c->ar.alloc<double>((size_t)NK * pitch);
-    c->Wprev = c->ar.alloc<double>((size_t)NK * pitch);
+    c->Wf = c->par.alloc<double>((size_t)NK * pitch);
+    c->W = c->par.alloc<double>((size_t)NK * pitch);
+    c->r64 = c->par.alloc<double>((size_t)NK * pitch);
+    c->Wprev = c->par.alloc<double>((size_t)NK * pitch);
     c->nsolves = 0;
     if (c->mixed && !c->spectral) {
         c->pcg32.reset(new PCG<float>());
         c->pcg32->stats = &c->stats;
-        c->pcg32->build(c->ar, NX, NK, c->h_rhou, c->h_rhow, c->h_a, c->h_h);
-        c->g32 = c->ar.alloc<float>((size_t)NK * pitch);
-        c->d32 = c->ar.alloc<float>((size_t)NK * pitch);
+        c->pcg32->build(c->par, NX, NK, c->h_rhou, c->h_rhow, c->h_a, c->h_h);
+        c->g32 = c->par.alloc<float>((size_t)NK * pitch);
+        c->d32 = c->par.alloc<float>((size_t)NK * pitch);
     }
     dim3 g(cdiv(NX, 64), cdiv(NK, 4));
     c->wnpart = g.x * g.y;
-    c->wpartial = c->ar.alloc<double>(c->wnpart);
+    c->wpartial = c->par.alloc<double>(c->wnpart);
     if (!c->sc_host) CK(cudaMallocHost(&c->sc_host, sizeof(double)));
     c->poisson_ready = true;
     apply_tuning(c);
@@ -3329,7 +3359,7 @@ int step_once(vvm_gpu_ctx* c) {
 // Buffers made later, which may lie behind the copied ones in a slab, are left
 // as they are.
 struct Snapshot {
-    std::vector<void*> copies;
+    std::vector<void*> copies, from;
     std::vector<size_t> bytes;   // of each: what was in use
     int step = 0, cur = 0, nsolves = 0, last_iters = 0;
     bool fut_is_now = false;
@@ -3337,14 +3367,16 @@ struct Snapshot {
     long long launches = 0;
     void take(vvm_gpu_ctx* c) {
         CK(cudaStreamSynchronize(c->stream));
-        for (size_t j = 0; j < c->ar.ptrs.size(); j++) {
-            void* q = nullptr;
-            const size_t nb = c->ar.used[j];
-            CK(cudaMalloc(&q, nb));
-            copies.push_back(q);
-            bytes.push_back(nb);
-            CK(cudaMemcpyAsync(q, c->ar.ptrs[j], nb, cudaMemcpyDeviceToDevice, c->stream));
-        }
+        for (const Arena* a : {&c->ar, &c->par})
+            for (size_t j = 0; j < a->ptrs.size(); j++) {
+                void* q = nullptr;
+                const size_t nb = a->used[j];
+                CK(cudaMalloc(&q, nb));
+                copies.push_back(q);
+                from.push_back(a->ptrs[j]);
+                bytes.push_back(nb);
+                CK(cudaMemcpyAsync(q, a->ptrs[j], nb, cudaMemcpyDeviceToDevice, c->stream));
+            }
         CK(cudaStreamSynchronize(c->stream));
         step = c->step;
         cur = c->cur;
@@ -3357,7 +3389,7 @@ struct Snapshot {
     void restore(vvm_gpu_ctx* c) {
         CK(cudaStreamSynchronize(c->stream));
         for (size_t j = 0; j < copies.size(); j++)
-            CK(cudaMemcpyAsync(c->ar.ptrs[j], copies[j], bytes[j], cudaMemcpyDeviceToDevice, c->stream));
+            CK(cudaMemcpyAsync(from[j], copies[j], bytes[j], cudaMemcpyDeviceToDevice, c->stream));
         CK(cudaStreamSynchronize(c->stream));
         c->step = step;
         c->cur = cur;
