@@ -90,9 +90,9 @@ __device__ __forceinline__ void cp_async_elem(T* smem, const T* gmem) {
 
 // ---------------------------------------------------------------------------
 // Domain-mean top wind tendency (PoissonSolver::pubarTop_pt,
-// PoissonSolver.cpp:655-676). One block of 256 threads; in a whole step an
-// extra block of k_pzeta, which reads the same time level (a launch of its own
-// stood 9 us at the head of the scalars' chain).
+// PoissonSolver.cpp:655-676). One block; in a whole step an extra block of
+// k_pzeta, which reads the same time level (a launch of its own stood 9 us at
+// the head of the scalars' chain).
 
 template <typename T>
 struct PubarArgs {
@@ -138,8 +138,9 @@ __device__ __forceinline__ void k_pubartop_body(const PubarArgs<T>& a) {
         a.ubar[1] = a.ubar[0] + 1.5 * a.c.dt * tend - 0.5 * a.c.dt * old;
     }
 }
+constexpr int kPubarThreads = 1024;   // of k_pubartop, at most
 template <typename T>
-__global__ void k_pubartop(PubarArgs<T> a) { k_pubartop_body<T>(a); }
+__global__ void __launch_bounds__(kPubarThreads) k_pubartop(PubarArgs<T> a) { k_pubartop_body<T>(a); }
 
 // ---------------------------------------------------------------------------
 // Vorticity advection + buoyancy + westdown halo of zetap

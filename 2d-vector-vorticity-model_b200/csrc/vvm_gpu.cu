@@ -2090,7 +2090,10 @@ void launch_halo_all(vvm_gpu_ctx* c) {
 
 template <typename T>
 void launch_pubartop(vvm_gpu_ctx* c) {
-    LAUNCH(&c->stats, VVM_K_PUBAR, c->stream, k_pubartop<T><<<1, 256, 0, c->stream>>>(pubar_args<T>(c)));
+    // long rows take as many threads as a block has (us a call with 256 / 1024,
+    // FP64: 128 columns 7.8 / 8.3, 2048 9 with either, 4096 11.1 / 10.3, 8192 14.7 / 12.4)
+    const int threads = c->d.nx - 2 > 2048 ? kPubarThreads : 256;
+    LAUNCH(&c->stats, VVM_K_PUBAR, c->stream, k_pubartop<T><<<1, threads, 0, c->stream>>>(pubar_args<T>(c)));
     CKL();
 }
 
