@@ -1825,15 +1825,18 @@ __device__ __forceinline__ void k_gs_inputs_body(const GSSweepArgs<T>& a) {
     const int i = blockIdx.x * blockDim.x + threadIdx.x, k = blockIdx.y * blockDim.y + threadIdx.y;
     if (i >= d.nx || k >= d.nz) return;
     const size_t id = d.at(i, k);
+    T v[5];   // all loads before the first store, which might change them for all the compiler knows
+#pragma unroll
+    for (int f = 0; f < 5; f++) v[f] = a.src[f][id];
 #pragma unroll
     for (int f = 0; f < 5; f++) {
-        T v = a.src[f][id];
         if (a.nvp && f >= 2) {
-            if (kPert<T> && f == 2) v = T(gs_finish(gs_factor(a.nvp, 2), a.p.ref[1][k] + (double)v) - a.p.ref[1][k]);
-            else v = gs_finish(T(gs_factor(a.nvp, f)), v);
+            if (kPert<T> && f == 2) v[f] = T(gs_finish(gs_factor(a.nvp, 2), a.p.ref[1][k] + (double)v[f]) - a.p.ref[1][k]);
+            else v[f] = gs_finish(T(gs_factor(a.nvp, f)), v[f]);
         }
-        a.dst[f][id] = v;
     }
+#pragma unroll
+    for (int f = 0; f < 5; f++) a.dst[f][id] = v[f];
 }
 template <typename T>
 __global__ void k_gs_inputs(GSSweepArgs<T> a) { k_gs_inputs_body<T>(a); }
