@@ -1,7 +1,7 @@
 // Grouped launches: many independent cases of one grid shape in one launch.
 //
 // A batch of cases steps as one CUDA graph. Launched case by case, a step of
-// a small case is ~25 short kernels, and a few hundred cases make thousands
+// a small case is a dozen short kernels, and a few hundred cases make thousands
 // of graph nodes: the GPU's launch rate, not its bandwidth, then sets the
 // step time. A grouped launch runs one kernel for every case of a group at
 // once: blockIdx.z is the case, and each case's arguments come from an array

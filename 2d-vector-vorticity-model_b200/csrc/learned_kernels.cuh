@@ -615,9 +615,11 @@ __global__ void k_net_up_add(const __nv_bfloat16* lo, const __nv_bfloat16* skip,
 // at the end. Pixels are the contraction: both operands lie with the channels
 // of a pixel together, so both are loaded transposed (ldmatrix), a tap's shift
 // being a shift of the rows it starts from. (A tap's product has 32 rows, below
-// the 64 that a tcgen05 operand needs at least, and taps cannot share one: each
-// meets dY at its own shift. At 16 MB of operands for 2.4 GFLOP the kernel is
-// bound by its loads and issue anyway.) Rows of X come by cp.async one row
+// the 64 that a tcgen05 operand needs at least; the nine taps meet the same dY,
+// so that stacked they would be one product of 288 rows, but their rows start
+// at nine shifts of the staged pixels, which no single operand descriptor
+// gives. At 16 MB of operands for 2.4 GFLOP the kernel is bound by its loads
+// and issue anyway.) Rows of X come by cp.async one row
 // ahead, each read once; a pixel's four 16-byte chunks are rotated by
 // (pixel / 2) mod 4 so that eight consecutive pixels meet all banks.
 // 128 x 1024 pixels: 21 us, from 295 with a multiply-add of two conversions

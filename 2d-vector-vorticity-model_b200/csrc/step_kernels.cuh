@@ -369,7 +369,7 @@ __device__ __forceinline__ void k_pzeta_body(const FieldMaps<7>& maps, const PZe
         store_westdown(a.zetap, d, i, k, zp);
     }
 }
-// Blocks a SM: what shared memory holds at the rows a thread of pzeta_rows.
+// Blocks a SM: what shared memory holds at launch_pzeta's rows a thread.
 template <typename T, int R>
 __global__ void __launch_bounds__(kTileLanes* kTileWarps, 4)
     k_pzeta(const __grid_constant__ FieldMaps<7> maps, PZetaArgs<T> a) {
@@ -1042,10 +1042,11 @@ __global__ void __launch_bounds__(256) k_rkm_rkh(RKArgs<T> a) { k_rkm_rkh_body<T
 // reproduce the sequential sweep over the tiles. The passes stop earlier, as
 // soon as no outflow that another tile reads changed bit for bit from one
 // pass to the next: the following pass would then read the same inflows and
-// repeat every value, so that is the fixed point the full count reaches. With
-// diffusion coefficients of a step (B, C ~ dt K / dx^2, 1e-3 for the minimum
-// K = 10 m^2/s at dx = 100 m) an inflow error shrinks about a thousandfold a
-// pass; three passes are typical.
+// repeat every value, so that is the fixed point the full count reaches. A
+// pass shrinks an inflow's error by about B + C. These passes are the schedule
+// for large coefficients alone: with those a step normally has (1e-3) the
+// single pass below (k_gs_sweep) gives the sweep to round-off, and none of
+// these runs unless it asks for them.
 //
 // Pass 1 reads the old values: it forms A0 from them and stores it, takes
 // its inflows from them (the guess), and writes no field, so every tile of it
@@ -1059,10 +1060,10 @@ __global__ void __launch_bounds__(256) k_rkm_rkh(RKArgs<T> a) { k_rkm_rkh_body<T
 // The last block of a pass (a thread-fence and counter, no waiting) decides
 // whether another pass follows, and sets the condition of the graph's WHILE
 // node when the passes run in a graph; the last pass of a sweep resets the
-// pass state for the next one (the host also clears it before each sweep). A
-// later pass launched after the sweep converged returns at once, so a graph
-// runs the typical count unconditionally and enters its WHILE node only when
-// more passes are needed.
+// pass state for the next one (the host's loop also clears it first). In a
+// graph they are the body of a conditional node that k_gs_sweep opens: the
+// inputs and pass 1 the first time round, a later pass each time; a pass that
+// finds the sweep converged returns at once.
 
 template <typename T>
 struct GSArgs {
@@ -1095,7 +1096,7 @@ inline bool gs_tile_rows_ok(int tr) { return tr == 4 || tr == 8 || tr == 16 || t
 template <typename T>
 constexpr int kGSTileMinBlocks = sizeof(T) == 8 ? 3 : 4;
 
-struct GSTileCtl {    // zeroed before a sweep
+struct GSTileCtl {    // zero before a sweep
     int pass;         // passes of the sweep completed
     int changed[2];   // by parity of the pass that wrote an outflow differing from its previous one
     int done;         // blocks of the current pass that finished
@@ -1474,8 +1475,8 @@ __global__ void __launch_bounds__(128, kGSTileMinBlocks<T>) k_gs_tiles(GSArgs<T>
 // field (shorter rows: least time where the grid has few tiles). Rows arrive
 // by cp.async kGWDepth ahead, each lane reading back only what it copied, so
 // no barrier is needed. Bound by the instruction issue of the few warps a
-// scheduler holds (about 350 instructions a row of a pair, 220 of a field, ~4
-// cycles each at one warp a scheduler). Measured at 2048 x 256 against the
+// scheduler holds (2048 x 256 FP64: 6.1 M warp instructions over 912 tiles of 22
+// rows, 306 a row, ~4 cycles each at one warp a scheduler). Measured at 2048 x 256 against the
 // three passes it replaces: 32 / 91 us FP64, 19 / 63 us FP32; 8192 x 256 FP64
 // 81 / 260, 128 x 64 12.6 / 81. A form that makes the rows' coefficients by
 // other warps first (shared memory, a barrier every 8 or 16 rows) took 34 us

@@ -137,24 +137,20 @@ def class_bytes(cls: str, launches: int, grid, elem: int, cg_iters: float) -> fl
         "gs": 12 * cells * elem,           # per STEP, not per launch: 5 fields read
                                            # and written + RKM, RKH (repeated passes
                                            # vary in number)
-        "cal_u": 3 * cells * elem / 2,     # w zetap in, u out (two launches)
+        "cal_u": 3 * cells * elem,         # w zetap in, u out
     }
     if cls in per_launch:
         return per_launch[cls] * launches
     if cls == "mg_sweep":
-        # one V-cycle: pre-sweeps read f, write x (2 arrays); post-sweeps read
-        # f, x, half a coarse array, write y (3.5 arrays); fine levels halve
-        nfine, total, n = 0, 0.0, grid.NX
-        while n > 32 and n % 2 == 0:
-            total += 5.5 * (grid.NZ - 1) * n * elem
-            nfine += 1
-            n //= 2
-        return total / max(2 * nfine, 1) * launches
+        # the direct solver's row transforms, FP64 inside: zetap in, the
+        # right-hand side and the spectra out; spectra in, W and w out (rows of
+        # up to 4096 columns have no multigrid sweeps)
+        return (2 * 8 + elem) * unk * launches
     if cls == "mg_coarse":
-        # the z solve of the modes (direct solver): spectra in and out, two factor
-        # arrays of half the size; with the row transforms of the multigrid's exact
-        # level, 2 arrays each, the mean of three launches is less
-        return 3 * unk * elem * launches
+        # the z solve of the modes: spectra in and out, two factor arrays of half
+        # the size; with the row transforms of the multigrid's exact level, 2
+        # arrays each, the mean of three launches is less
+        return 3 * 8 * unk * launches
     if cls == "cg":
         # per iteration: spmv 2, update 6, dot 2, direction 3 arrays of the unknowns
         return 13 * unk * elem * cg_iters

@@ -138,8 +138,10 @@ int vvm_gpu_last_error(vvm_gpu_ctx* ctx, char* buf, size_t len);
 int vvm_gpu_upload_state(vvm_gpu_ctx* ctx, const vvm_gpu_host_state* st);
 int vvm_gpu_download_state(vvm_gpu_ctx* ctx, vvm_gpu_host_state* st);
 /* Prognostic fields only (zeta, th, qv, qc, qr, u, w): the per-step traffic
- * of an output call. The copies run on the context's own copy stream, each
- * field's copy beside the previous field's layout kernel. The upload returns
+ * of an output call. Fields of more than 512 KB are copied on the context's own
+ * copy stream, each beside the previous field's layout kernel; smaller ones on
+ * the context's stream, seven copies and one layout kernel. A field whose
+ * pointer is null is skipped by the download. The upload returns
  * once the work is queued (work on the context's stream that follows sees the
  * fields; the host buffers must stay unchanged until then, as for any
  * asynchronous copy); the download returns with the host buffers filled. */
@@ -323,10 +325,12 @@ int vvm_gpu_get_tuning(vvm_gpu_ctx* ctx, int* gs_tile_rows, int* fft_threads);
  * upload, download, queries and the routine entries; every case must be at
  * the same step when vvm_gpu_batch_step runs (VVM_GPU_ESTATE otherwise).
  * vvm_gpu_batch_autotune times one step of each group of cases with the same
- * grid, precision and solver for each value of the launch-shape knobs above
- * and for the cases a grouped launch takes (`reps` graph launches per
- * candidate), keeps the fastest, and restores
- * every case's state exactly; *ngroups receives the number of groups.
+ * grid, precision and solver for the two Gauss-Seidel schedules (single pass as
+ * set, cluster), row-FFT blocks of 128 to 1024 threads and the cases a grouped
+ * launch takes (`reps` graph launches per candidate), keeps the fastest, and
+ * restores every case's state exactly; it needs an uploaded state, not a step.
+ * *ngroups receives the number of groups. A state, operator or knob that
+ * changes on a case reaches the batch's next step.
  * vvm_gpu_batch_synchronize waits for the batch and reports any case's
  * device error. Failures of batch calls: vvm_gpu_batch_last_error. */
 typedef struct vvm_gpu_batch vvm_gpu_batch;
