@@ -123,3 +123,32 @@ def test_a_new_state_reaches_the_batch_graphs(G, warm_start, limit):
         assert _same(c.download(), g.download())
         g.close()
     b.close()
+
+
+@pytest.mark.parametrize("precision", [0, 1])
+def test_a_member_that_holds_nan_is_stepped_like_any_other(G, precision):
+    """A member of an ensemble has blown up: the first steps, driven by the
+    host, take it as the captured ones do, and the others are as alone."""
+    from vvm_b200.initial_state import warm_bubble
+    sts = [warm_bubble(64, 32, 200.0, 200.0, amp=a, radius=800.0) for a in (1.0, 2.0, 3.0)]
+    sts[1].fields["zeta"][20, 10] = np.nan
+    b = G.VVMBatch([s.grid for s in sts], precision=precision, solver=G.VVM_SOLVER_SPECTRAL)
+    b.upload(sts)
+    for n in (1, 1, 1, 2):   # two steps by the host, three from graphs
+        b.step(n)
+    b.synchronize()
+    outs = [c.download() for c in b.cases]
+    assert np.isnan(outs[1].fields["w"]).any()
+    b.close()
+    for j in (0, 2):
+        g = G.VVMGpu(sts[j].grid, precision=precision, solver=G.VVM_SOLVER_SPECTRAL)
+        g.upload(sts[j])
+        g.step(5)
+        assert _same(outs[j], g.download())
+        g.close()
+    g = G.VVMGpu(sts[1].grid, precision=precision, solver=G.VVM_SOLVER_SPECTRAL)
+    g.upload(sts[1])
+    g.call("pzeta")
+    g.call("cal_w")      # the routine takes it too
+    assert np.isnan(g.download().fields["w"]).any()
+    g.close()
