@@ -952,8 +952,9 @@ __device__ __forceinline__ unsigned bits_up(float x) { return __float_as_uint(x)
 
 // R rows a thread: the rows between are loaded once, not three times, and all
 // of them at once, with a barrier and an atomic for R times as many cells.
-// Ri is compared as its numerator against its denominator (th > 0), so that
-// the cells of Ri >= 1/4, most of them, divide and take roots not at all.
+// Where the numerator of Ri is at least a quarter of a positive denominator, in
+// most cells, there is no mixing and neither a division nor a root is taken; Ri
+// itself decides everywhere else (whatever theta's sign, and where it is zero).
 template <typename T, int R>
 __device__ __forceinline__ void k_rkm_rkh_body(const RKArgs<T>& a) {
     const Dims& d = a.d;
@@ -987,14 +988,15 @@ __device__ __forceinline__ void k_rkm_rkh_body(const RKArgs<T>& a) {
                 dth += T(a.p.g0[0][k]);
             }
             const T def2 = Rzeta * Rzeta + T(2.) * (rot * rot);
-            const T num = T(a.c.gravity) * dth * T(a.p.r2dzcc[k]), den = th0 * def2;   // Ri = num / den
+            const T r2 = T(a.p.r2dzcc[k]), num = T(a.c.gravity) * dth * r2, den = th0 * def2;   // Ri = num / den
             T km = T(0.), kh = T(0.);
-            if (num < T(0.25) * den && num != T(0)) {
-                const T Ri = num / den, lam = T(a.p.lambda2[k]), ld = lam * sqrt(def2);
+            if (!(den > T(0) && num >= T(0.25) * den)) {
+                const T Ri = (T(a.c.gravity) / th0 * dth * r2) / def2;
+                const T lam = T(a.p.lambda2[k]), ld = lam * sqrt(def2);
                 if (Ri < T(0)) {
                     km = ld * sqrt(T(1.) - T(16.) * Ri);
                     kh = ld * T(1.4) * sqrt(T(1.) - T(40.) * Ri);
-                } else {
+                } else if (T(0) < Ri && Ri < T(0.25)) {
                     const T f = T(1.) - T(4.) * Ri, f4 = (f * f) * (f * f);
                     km = ld * f4;
                     kh = ld * T(1.4) * (T(1.) - T(1.2) * Ri) * f4;
