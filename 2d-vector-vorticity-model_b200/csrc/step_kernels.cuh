@@ -161,6 +161,7 @@ struct PZetaArgs {
     PubarArgs<T> pubar;            // pubarTop_pt, by one block past the tiles
     int do_pubar;
     unsigned* kmax;                // [2]: cleared by that block for this step's k_rkm_rkh
+    int* redo;                     // and this for its k_gs_sweep
 };
 
 // Tile of k_pzeta: 31 x 8R zeta points a block of 32 x 8 threads, R rows a
@@ -231,7 +232,10 @@ __device__ __forceinline__ void k_pzeta_body(const FieldMaps<7>& maps, const PZe
     constexpr int BZ = Sh::BZ, VZ = Sh::VZ, VX = kTileVX, AL = 16 / sizeof(T);
     if (a.do_pubar && blockIdx.y == 0) {   // the first row of blocks: it starts with the first wave
         if (blockIdx.x == 0) {
-            if (threadIdx.x == 0 && threadIdx.y == 0) a.kmax[0] = a.kmax[1] = 0u;
+            if (threadIdx.x == 0 && threadIdx.y == 0) {
+                a.kmax[0] = a.kmax[1] = 0u;
+                *a.redo = 0;
+            }
             k_pubartop_body<T>(a.pubar);
         }
         return;
@@ -1462,7 +1466,9 @@ __global__ void __launch_bounds__(128, kGSTileMinBlocks<T>) k_gs_tiles(GSArgs<T>
 // rows that puts this below 2^-56 (FP32: 2^-28), from the largest eddy
 // coefficient of the grid (k_rkm_rkh), usually 4 to 8; where more than
 // kGWHaloMax would be needed (B + C above about 0.1, FP32 0.3) the kernel
-// writes nothing and asks for the repeated passes above instead. Along a row
+// writes nothing and asks for the repeated passes above instead; so does a
+// tile that has met an infinity or NaN, which no tail outruns (whatever its
+// rows hold of these is still there in the last one). Along a row
 // the same bound cuts the scan short: y left of a lane's four cells is the
 // lanes' offsets of the 8 (B <= 2^-7, FP32 2^-3.5) or 16 cells before it.
 //
@@ -1502,12 +1508,20 @@ struct GSSweepArgs {
     int jobs;            // 3: zeta; th, qv; qc, qr. 5: every field on its own
     const unsigned* kmax;
     float fz[2];         // largest C / K over the rows: Mparam, Hparam
-    GSTileCtl* ctl;      // more: the repeated passes are needed
+    GSTileCtl* ctl;      // more: the repeated passes are needed (0 before)
     // a captured step that puts its rare loops at its end (run_step_direct):
-    // the solve's check has failed; set when the end has to run
+    // the solve's check has failed; set when the end has to run (0 before)
     const int* solve_more;
     int* redo;
 };
+
+// Asks for the repeated passes (ctl->more), and for the end of a captured step.
+template <typename T>
+__device__ __forceinline__ void gs_ask(const GSSweepArgs<T>& a, bool passes, cudaGraphConditionalHandle h) {
+    if (passes) a.ctl->more = 1;
+    if (a.redo) *a.redo = 1;
+    if (h) cudaGraphSetConditional(h, 1u);
+}
 
 template <typename T>
 struct GSSweepShared {
@@ -1692,8 +1706,9 @@ struct GSSweepTile {
     }
 };
 
+// False where the tile has met a value that is not finite.
 template <typename T, bool MOM, int NF>
-__device__ __forceinline__ void gs_sweep_tile(const GSSweepArgs<T>& a, GSSweepShared<T>& S, int f0, int b, int c, int hz,
+__device__ __forceinline__ bool gs_sweep_tile(const GSSweepArgs<T>& a, GSSweepShared<T>& S, int f0, int b, int c, int hz,
                                               bool wide) {
     constexpr int D = kGWDepth;
     const Dims& d = a.d;
@@ -1788,6 +1803,12 @@ __device__ __forceinline__ void gs_sweep_tile(const GSSweepArgs<T>& a, GSSweepSh
         for (int f = 0; f < NF; f++) t.store4(f, t.v0[f]);
     }
     cp_async_wait<0>();
+    bool finite = true;
+#pragma unroll
+    for (int f = 0; f < NF; f++)
+#pragma unroll
+        for (int e = 0; e < 4; e++) finite = finite && isfinite(t.below[f][e]);
+    return __all_sync(0xffffffffu, finite);
 }
 
 template <typename T>
@@ -1800,21 +1821,19 @@ __device__ __forceinline__ void k_gs_sweep_body(const GSSweepArgs<T>& a, cudaGra
     const float lx = -log2f(1.001f * cx * fmaxf(km, kh));
     const int hz = max(1, (int)ceilf(kGWBits<T> / l) - 1);
     const bool ok = km == km && kh == kh && l > 0.f && hz <= kGWHaloMax && 16.f * lx >= kGWBits<T>;
-    if (threadIdx.x == 0 && blockIdx.x == 0 && blockIdx.y == 0) {
-        a.ctl->more = ok ? 0 : 1;
-        const bool more = !ok || (a.solve_more && *a.solve_more);
-        if (a.redo) *a.redo = more;
-        if (h) cudaGraphSetConditional(h, more ? 1u : 0u);
-    }
+    if (threadIdx.x == 0 && blockIdx.x == 0 && blockIdx.y == 0)
+        if (!ok || (a.solve_more && *a.solve_more)) gs_ask(a, !ok, h);
     if (!ok) return;
     const int wid = threadIdx.x >> 5;
     const int tile = blockIdx.x * kGWWarps + wid;
     if (tile >= a.jobs * a.nb * a.nc) return;
     const int c = tile % a.nc, b = (tile / a.nc) % a.nb, job = tile / (a.nc * a.nb);
     const bool wide = 8.f * lx < kGWBits<T>;
-    if (job == 0) gs_sweep_tile<T, true, 1>(a, S[wid], 0, b, c, hz, wide);
-    else if (a.jobs == 3) gs_sweep_tile<T, false, 2>(a, S[wid], 2 * job - 1, b, c, hz, wide);
-    else gs_sweep_tile<T, false, 1>(a, S[wid], job, b, c, hz, wide);
+    bool finite;
+    if (job == 0) finite = gs_sweep_tile<T, true, 1>(a, S[wid], 0, b, c, hz, wide);
+    else if (a.jobs == 3) finite = gs_sweep_tile<T, false, 2>(a, S[wid], 2 * job - 1, b, c, hz, wide);
+    else finite = gs_sweep_tile<T, false, 1>(a, S[wid], job, b, c, hz, wide);
+    if (!finite && (threadIdx.x & 31) == 0) gs_ask(a, true, h);
 }
 template <typename T>
 __global__ void __launch_bounds__(32 * kGWWarps) k_gs_sweep(GSSweepArgs<T> a, cudaGraphConditionalHandle h) { k_gs_sweep_body<T>(a, h); }

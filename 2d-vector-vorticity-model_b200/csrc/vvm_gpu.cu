@@ -246,8 +246,12 @@ __global__ void k_spec_check(VecArgs<double> v, const double* f, const double* x
 }
 
 // The rare end of a captured step (run_step_direct): opens its CG loop if the
-// solve's check failed; counts the kernels it ran outside its loops.
-__global__ void k_redo_begin(const CGCtl* ctl, cudaGraphConditionalHandle solve) {
+// solve's check failed, and clears what the diffusion's second sweep asks with;
+// counts the kernels it ran outside its loops.
+__global__ void k_redo_begin(const CGCtl* ctl, GSTileCtl* gs, cudaGraphConditionalHandle solve,
+                             cudaGraphConditionalHandle passes) {
+    gs->more = 0;
+    cudaGraphSetConditional(passes, 0u);
     cudaGraphSetConditional(solve, ctl->more ? 1u : 0u);
 }
 __global__ void k_redo_end(long long* exec, int kernels) { *exec += kernels; }
@@ -1967,7 +1971,7 @@ void launch_pzeta_r(vvm_gpu_ctx* c) {
     PZetaArgs<T> a{c->d, c->c, c->profiles(), F.zeta[now], F.u, F.w, F.th[now], F.qv[now], F.qc[now], F.qr[now],
                    zeta_pre<T>(c), F.hist[H_ZETA][ab.sn], F.hist[H_ZETA][ab.so], F.hist[H_BUOY][ab.sn],
                    F.hist[H_BUOY][ab.so], c->d_err, ab, pubar_args<T>(c),
-                   c->in_step && !(c->desc.flags & VVM_FLAG_STREAMFUNCTION), c->kmax};
+                   c->in_step && !(c->desc.flags & VVM_FLAG_STREAMFUNCTION), c->kmax, c->redo};
     const T* staged[7] = {a.zeta, a.u, a.w, a.th, a.qv, a.qc, a.qr};
     FieldMaps<7> m;
     for (int f = 0; f < 7; f++)
@@ -2428,7 +2432,7 @@ void launch_turbulence(vvm_gpu_ctx* c, bool nudge, long long* recorded_in_loops 
     cudaStream_t st = c->stream;
     const GSSweepArgs<T> w = gs_sweep_args<T>(c, nudge);
     GSPasses<T> passes(c, w, recorded_in_loops != nullptr);
-    if (!recorded_in_loops) {   // a graph's steps begin with both clear: k_pzeta clears kmax, the passes their state
+    if (!recorded_in_loops) {   // a graph's steps find both clear: k_pzeta clears kmax, the passes leave their state so
         CK(cudaMemsetAsync(c->kmax, 0, 2 * sizeof(unsigned), st));
         CK(cudaMemsetAsync(c->gsctl, 0, sizeof(GSTileCtl), st));
     }
@@ -3156,7 +3160,7 @@ void run_step_direct(vvm_gpu_ctx* c, long long* in_loops) {
             OnStream os(c, bc.s);
             const long long n0 = c->stats.launches;
             const cudaGraphConditionalHandle hs = new_handle(&c->stats, bc.s), hp = new_handle(&c->stats, bc.s);
-            LAUNCH(&c->stats, VVM_K_CG, bc.s, k_redo_begin<<<1, 1, 0, bc.s>>>(c->pcg64->ctl, hs));
+            LAUNCH(&c->stats, VVM_K_CG, bc.s, k_redo_begin<<<1, 1, 0, bc.s>>>(c->pcg64->ctl, c->gsctl, hs, hp));
             CKL();
             PCG<double>& P = *c->pcg64;
             LAUNCH(&c->stats, VVM_K_CG, bc.s, k_cg_residual<double><<<P.grid(), P.block(), 0, bc.s>>>(P.vargs(), c->Wf, c->W, P.r, P.partial));

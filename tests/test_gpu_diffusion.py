@@ -149,3 +149,65 @@ def test_routine_turbulence_leaves_later_steps_alone(G, precision):
     assert counts[0] == counts[1]
     for n in ("zeta", "th", "qv", "qc", "qr", "u", "w", "RKM"):
         assert np.array_equal(outs[0].fields[n], outs[1].fields[n]), n
+
+
+@pytest.mark.parametrize("precision", [0, 1])
+@pytest.mark.parametrize("value", [np.nan, np.inf])
+@pytest.mark.parametrize("field,i,k", [("zeta", 5, 3), ("th", 107, 9), ("qc", 109, 24), ("qr", 200, 1)])
+def test_a_value_that_is_not_finite_spreads_as_in_the_sequential_sweep(G, field, i, k, value, precision):
+    """One such value reaches, through the recurrence, every cell above it and
+    to its right, far past the tails by which the tiles find their inflows."""
+    from oracle.models import PortModel
+    from vvm_b200.initial_state import random_state
+    st = random_state(215, 25, dt=1.0, seed=1)
+    for n in ("zeta", "th", "qv", "qc", "qr"):
+        st.fields[n + "p"] = st.fields[n].copy()
+    st.fields[field + "p"][i, k] = value
+    m = PortModel(st.grid)
+    m.load(st)
+    m.call("RKM_RKH")
+    ref = m.dump()
+    g = G.VVMGpu(st.grid, precision=precision)
+    g.upload(st)
+    g.call("turbulence")
+    out = g.download()
+    g.close()
+    for n, _ in PAIRS:
+        a, b = out.fields[n], ref.fields[n]
+        ok = np.isfinite(b)
+        assert np.array_equal(np.isfinite(a), ok), n
+        assert rel_l2(a[ok], b[ok]) <= (1e-13 if precision == 0 else 1e-5), n
+
+
+@pytest.mark.parametrize("precision", [0, 1])
+def test_steps_of_a_state_that_is_not_finite(G, precision):
+    """The same in whole steps: captured ones (alone, and in a group beside
+    sound cases) leave the bits of host-driven ones."""
+    from vvm_b200.initial_state import warm_bubble
+    st, bad = (warm_bubble(128, 40, 200.0, 200.0, radius=1000.0) for _ in range(2))
+    bad.fields["th"][40, 12] = np.nan
+    names = ("zeta", "th", "qv", "qc", "qr", "u", "w")
+    # warm_start off: the second step on runs from a graph
+    def alone(s, host):
+        g = G.VVMGpu(s.grid, precision=precision, solver=G.VVM_SOLVER_SPECTRAL, warm_start=False)
+        g.upload(s)
+        if host:
+            g.profile(True)
+        for _ in range(3):
+            g.step(1)
+        out = g.download()
+        g.close()
+        return out
+    ref = [alone(s, True) for s in (st, bad)]
+    assert np.isfinite(ref[0].fields["zeta"]).all() and not np.isfinite(ref[1].fields["zeta"]).all()
+    b = G.VVMBatch([s.grid for s in (st, bad, st)], precision=precision, warm_start=False)
+    b.upload([st, bad, st])
+    b.step(3)
+    b.synchronize()
+    assert b.grouping() == 1
+    outs = [c.download() for c in b.cases]
+    b.close()
+    for out, r in ((alone(st, False), ref[0]), (alone(bad, False), ref[1]), (outs[0], ref[0]), (outs[1], ref[1]),
+                   (outs[2], ref[0])):
+        for n in names:
+            assert np.array_equal(out.fields[n], r.fields[n], equal_nan=True), n
