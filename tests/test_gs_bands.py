@@ -54,5 +54,5 @@ def test_every_row_is_stored_once(lib, tr):
 def test_the_kernel_uses_the_rule():
     """No store of k_gs_sweep decides about a ghost row by anything else."""
     text = (CSRC / "step_kernels.cuh").read_text()
-    body = text[text.index("void gs_sweep_tile("):text.index("void k_gs_sweep_body(")]
+    body = text[text.index(" gs_sweep_tile("):text.index(" k_gs_sweep_body(")]
     assert "gs_band(" in body and "band.bottom" in body and "band.top" in body
